@@ -2749,12 +2749,28 @@ int step_batch_chunks(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_fields 
     fill_status(stats, M, EFDC_XM_CUDA_ERROR);
     return EFDC_XM_CUDA_ERROR;
   }
-  if ((rc = ensure_stages(c, std::max(nu, nd)))) {
+  // the upload j takes stage j and each download the stage of an upload of the
+  // same element size, or one of its own: a member's range in a stage starts at
+  // its element offset, so ranges of different element sizes overlap other
+  // members', whose chunks are still on their way
+  std::vector<size_t> dst(nd);
+  size_t nst = nu;
+  {
+    std::vector<char> taken(nu, 0);
+    for (size_t j = 0; j < nd; ++j) {
+      size_t i = 0;
+      while (i < nu && (taken[i] || esize(up[i].kind) != esize(dn[j].kind))) ++i;
+      if (i < nu) taken[i] = 1;
+      dst[j] = i < nu ? i : nst++;
+    }
+  }
+  if ((rc = ensure_stages(c, nst))) {
     fill_status(stats, M, rc);
     return rc;
   }
   for (size_t j = 0; j < nu; ++j) c->jobs_h[j] = CopyJob{c->stage[j], up[j].dev, up[j].kind};
-  for (size_t j = 0; j < nd; ++j) c->jobs_h[nu + j] = CopyJob{c->stage[j], dn[j].dev, dn[j].kind};
+  for (size_t j = 0; j < nd; ++j)
+    c->jobs_h[nu + j] = CopyJob{c->stage[dst[j]], dn[j].dev, dn[j].kind};
   CK(cudaMemcpyAsync(c->jobs_d, c->jobs_h, (nu + nd) * sizeof(CopyJob), cudaMemcpyHostToDevice,
                      c->stream));
   if ((rc = upload_small(c, f))) {  // waits for the solver stream: the job table is in place
@@ -2835,7 +2851,7 @@ int step_batch_chunks(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_fields 
     CK(cudaEventRecord(c->ev_g[k], c->dn_x));
     for (int s = 0; s < NPIPE; ++s) CK(cudaStreamWaitEvent(c->dn_stream[s], c->ev_g[k], 0));
     for (size_t j = 0; j < nd; ++j)
-      if ((rc = d2h_range(c, dn[j], reinterpret_cast<const char *>(c->stage[j]), mb[k],
+      if ((rc = d2h_range(c, dn[j], reinterpret_cast<const char *>(c->stage[dst[j]]), mb[k],
                           mb[k + 1], c->dn_stream, q, keep, NPIPE)))
         return fail(rc);
   }
