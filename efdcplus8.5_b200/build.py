@@ -22,6 +22,8 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler",
 SOURCES = {
     "xm_step.cu": ["-fmad=false"],
     "xm_mixed.cu": [],
+    "xm_resident.cu": ["-fmad=false"],
+    "xm_resident32.cu": [],
     "xm_capi.cu": [],
     "xm_noalloc.cu": ["-fmad=false"],
     "xm_adjoint.cu": [],

@@ -130,6 +130,18 @@ struct ChanSpec {
   double gw, gl;         // guest's WCHAN and cross length (DXP/DYP of LMDCHU or LMDCHV)
 };
 
+// The launches of a resident solve (xm_resident.cuh): its form and, for grid
+// groups that do not all fit the chip at once, one launch per run of members
+// that do.
+struct ResSet {
+  struct Wave {
+    int cta0, ncta;
+  };
+  xm::ResForm form{};
+  std::vector<Wave> waves;  // empty: some member does not fit
+  int4 *cta = nullptr;      // grid groups, device: (member, first quad, quads, 0)
+};
+
 struct efdc_xm_ctx {
   int device = 0;
   int M = 0;
@@ -171,6 +183,9 @@ struct efdc_xm_ctx {
        *sc_hd = nullptr;
   bool in_chunks = false;  // inside a chunked efdc_xm_step_batch (see to_device)
   double *part = nullptr;
+  ResSet res64, res32;          // resident solves, FP64 and MIXED
+  double2 *res_part = nullptr;   // their grid groups' partial sums
+  unsigned *res_count = nullptr; // and arrival counters
   int *lidx = nullptr;
   int *tile_member = nullptr;
   long long *moff = nullptr;
@@ -276,12 +291,11 @@ struct efdc_xm_ctx {
   int kvariant = 0, ctas_mv = 0, ctas_up = 0;
   int inner_margin_log10 = 0;   // MIXED inner target margin 10^-v
   int inner_tol_x10 = 60;       // MIXED inner relative tolerance 10^(-v/10) at least
-  bool small_solve = true;      // FP64: members small enough solve in one CTA each
+  bool resident = true;         // solves in one launch where the members fit the chip
   int fold_reduce = 1;          // member reductions folded into the CG kernels:
                                 // 0 never, 1 up to FOLD_MEMBERS members, 2 always
   int nchunk = 8;               // member chunks of a pipelined efdc_xm_step_batch
-  int small_slots = 0;          // the largest member window (its ghost tile and tiles)
-  int small_units = 0;          // the most 4-tile units of a member
+  int max_units = 0;            // the most 4-tile units of a member
   float poly_threshold = 10.f;  // MIXED: polynomial preconditioner above this Jacobi count
   xm::Launch L() const {
     xm::Launch l{grid,      grid_cg, grid_cg32, grid_up32,
@@ -649,23 +663,97 @@ int scaled_system(efdc_xm_ctx *c) {
   return EFDC_XM_OK;
 }
 
+constexpr int MAX_OUTER = 30;        // MIXED refinement passes per solve
+// inner: |r| down by at least 10^(-inner_tol_x10/10) (default 1e-6; FP32 reaches ~1e-7)
+double inner_rel_tol(const efdc_xm_ctx *c) { return std::pow(10.0, -0.1 * c->inner_tol_x10); }
+
 // FP64 CONGRAD of every active member on the scaled system in c->Y.  The
 // members iterate in lockstep launches; a member that has stopped is skipped
 // by the kernels.  On return c->ctl_h holds each member's outcome.
-// FP64 solves in one CTA per member (k_cg_small): every member's window fits
-// in a CTA's shared memory and no member has sub-grid channels (their terms
-// are separate kernels of the multi-kernel CG).
-bool small_solve(const efdc_xm_ctx *c) {
-  return c->small_solve && c->small_slots > 0 && xm::cg_small_fits(c->small_slots) &&
-         c->S.ch.n == 0;
+// How a solve runs: iteration kernels of every member in lockstep, or resident
+// groups of CTAs (contexts without sub-grid channels, whose terms are separate
+// kernels of the multi-kernel CG).
+bool resident_solve(const efdc_xm_ctx *c, bool mixed) {
+  return c->resident && c->S.ch.n == 0 && !(mixed ? c->res32 : c->res64).waves.empty();
+}
+
+// The form of a resident solve.  One cluster per member where the largest
+// member fits 16 CTAs, with as few quads per CTA as that takes (the members
+// are independent: a launch holds any number of clusters).  Else grid groups,
+// the first form that holds every member at once, or, up to max_waves, the
+// last in as few launches as that takes.  Several launches, one after another,
+// are still faster than the multi-kernel CG in FP64 (24 basins of 2.5 M cells:
+// 1.60 against 1.72 ms per step) and slower in MIXED (1.29 against 1.16 ms).
+bool build_resident(efdc_xm_ctx *c, int (*capacity)(const xm::ResForm &, bool, int),
+                    size_t max_waves, ResSet &out) {
+  const int M = c->M, mq = c->max_units;
+  auto cap_of = [&](const xm::ResForm &f) {
+    return std::min(capacity(f, false, c->nsm), capacity(f, true, c->nsm));
+  };
+  constexpr xm::ResForm forms[] = {{1, 1, 0}, {2, 1, 0}, {2, 2, 0}};
+  for (xm::ResForm f : forms) {
+    const int per = f.w * f.q, n = (mq + per - 1) / per;
+    if (n > 16) continue;
+    f.cluster = n;
+    if (cap_of(f) < 1) continue;
+    out.form = f;
+    out.waves = {{0, n * M}};
+    return true;
+  }
+  for (const xm::ResForm &f : forms) {
+    const int per = f.w * f.q, cap = cap_of(f);
+    const bool last = &f == std::end(forms) - 1;
+    // one CTA per SM exchanges faster than two: the narrow form only up to there
+    const int lim = f.w == 1 ? std::min(cap, c->nsm) : cap;
+    std::vector<int4> cta;
+    std::vector<ResSet::Wave> waves;
+    bool fits = cap > 0;
+    for (int m = 0; m < M && fits; ++m) {
+      const int q0 = c->qstart_h[m], q1 = c->qstart_h[m + 1], n = (q1 - q0 + per - 1) / per;
+      fits = n <= lim;
+      if (waves.empty() || waves.back().ncta + n > lim) waves.push_back({int(cta.size()), 0});
+      waves.back().ncta += n;
+      for (int q = q0; q < q1; q += per) cta.push_back(int4{m, q, std::min(per, q1 - q), 0});
+    }
+    if (!fits || (waves.size() > 1 && !last) || waves.size() > max_waves) continue;
+    out.cta = c->alloc<int4>(cta.size(), false);
+    if (!out.cta || cudaMemcpy(out.cta, cta.data(), cta.size() * sizeof(int4),
+                               cudaMemcpyHostToDevice) != cudaSuccess)
+      return false;
+    out.form = f;
+    out.waves = std::move(waves);
+    return true;
+  }
+  return true;
+}
+
+xm::ResPlan res_plan(const efdc_xm_ctx *c, const ResSet &r, const ResSet::Wave &w) {
+  return xm::ResPlan{r.cta ? r.cta + w.cta0 : nullptr, c->res_part, c->res_count};
+}
+
+void launch_resident64(efdc_xm_ctx *c, const xm::Launch &l, double *P) {
+  for (const ResSet::Wave &w : c->res64.waves)
+    xm::launch_cg_res(l, c->S, c->Y, P, c->ctl, c->glob, res_plan(c, c->res64, w),
+                      c->res64.form, w.ncta);
+}
+void launch_resident32(efdc_xm_ctx *c, const xm::Launch &l, double *P, double fac) {
+  for (const ResSet::Wave &w : c->res32.waves)
+    xm::launch_mx_res(l, c->S, c->mxview, c->Y, P, c->ctl, c->glob, res_plan(c, c->res32, w),
+                      c->res32.form, w.ncta, fac, inner_rel_tol(c), MAX_OUTER);
+}
+
+// No arrivals counted: at the start, and after a wait that ran out.
+int reset_resident(efdc_xm_ctx *c) {
+  CK(cudaMemsetAsync(c->res_count, 0, sizeof(unsigned) * xm::RES_COUNT_STRIDE * size_t(c->M),
+                     c->stream));
+  return EFDC_XM_OK;
 }
 
 int solve_fp64(efdc_xm_ctx *c, double *P) {
   const xm::Launch l = c->L();
   xm::launch_solve_reset(l, c->ctl, c->glob, c->act, c->M);
-  if (small_solve(c)) {  // the whole CG of each member in one CTA (k_cg_small)
-    xm::launch_cg_small(l, c->S, c->Y, P, c->ctl, c->glob, c->part, c->small_slots,
-                        c->small_units, c->M);
+  if (resident_solve(c, false)) {  // the whole CG of each member in one launch
+    launch_resident64(c, l, P);
     CK(cudaGetLastError());
     int rc = read_ctl(c);
     if (rc) return rc;
@@ -710,9 +798,6 @@ int solve_fp64(efdc_xm_ctx *c, double *P) {
   return EFDC_XM_OK;
 }
 
-constexpr int MAX_OUTER = 30;        // MIXED refinement passes per solve
-// inner: |r| down by at least 10^(-inner_tol_x10/10) (default 1e-6; FP32 reaches ~1e-7)
-double inner_rel_tol(const efdc_xm_ctx *c) { return std::pow(10.0, -0.1 * c->inner_tol_x10); }
 
 // MIXED: each member's inner preconditioner for the next solve, and the kinds
 // of inner solve the launches need; uploads the choice.  The Neumann
@@ -748,6 +833,21 @@ int solve_mixed(efdc_xm_ctx *c, double *P, double factor) {
   const xm::Launch lk = c->L();  // with the kinds in use
   xm::launch_chan_p0(lk, c->S, c->mxview, P, c->act);
   int rc = 0;
+  if (resident_solve(c, true)) {
+    launch_resident32(c, lk, P, fac);
+    CK(cudaGetLastError());
+    if ((rc = read_ctl(c))) return rc;
+    for (int m = 0; m < c->M; ++m) {
+      if (!c->act_h[m]) continue;
+      Ctl &k = c->ctl_h[m];
+      if (k.last_inner > 0) c->mem[m].last_inner = k.last_inner;
+      if (k.inner_first > 0)
+        c->mem[m].jac_est =
+            float(k.inner_first) * (c->mpoly_h[m] && !(k.asym & 1) ? 1.9f : 1.0f);
+      if (!k.done && k.status == 0) k.status = EFDC_XM_CG_MAXITER;
+    }
+    return EFDC_XM_OK;
+  }
   for (int o = 0; o < MAX_OUTER; ++o) {
     xm::launch_outer_reset(lk, c->glob);
     xm::launch_mx_resid(lk, c->S, c->mxview, c->Y, P, c->ctl, c->glob, c->part, fac,
@@ -1023,8 +1123,6 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
   c->ntile = ntile;
   c->nslot = ntile * TILE;
   c->stage_len = off;
-  for (const Member &mb : c->mem)  // the member windows of k_cg_small
-    c->small_slots = std::max(c->small_slots, (mb.tile1 - mb.tile0 + 1) * TILE);
   auto bail = [&](const char *what) -> efdc_xm_ctx * {
     if (g_last_error.empty()) set_error("efdc_xm_create: %s", what);
     efdc_xm_destroy(c);
@@ -1061,7 +1159,7 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
 
   // ---- host layout: tiles, quads (4-tile CG units, never across members), slots ----
   std::vector<int4> tnbr(ntile, int4{0, 0, 0, 0});
-  std::vector<int> tile_member(ntile, 0), tend(M), qstart(M + 1, 0);
+  std::vector<int> tile_member(ntile, 0), qstart(M + 1, 0);
   std::vector<int4> quads;
   std::vector<uint8_t> kind(c->nslot, xm::LAND);
   std::vector<int> lidx(c->nslot, 0);
@@ -1084,7 +1182,6 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
     }
     tnbr[mb.tile0 - 1] = int4{mb.tile0 - 1, mb.tile0 - 1, mb.tile0 - 1, mb.tile0 - 1};
     tile_member[mb.tile0 - 1] = m;
-    tend[m] = mb.tile1;
     qstart[m] = int(quads.size());
     for (int t = mb.tile0; t < mb.tile1; t += 4)
       quads.push_back(int4{m, t, std::min(4, mb.tile1 - t), 0});
@@ -1174,7 +1271,7 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
   int4 *tnbr_d = c->alloc<int4>(ntile);
   uint8_t *kind_d = c->alloc<uint8_t>(ns);
   int4 *quads_d = c->alloc<int4>(quads.size());
-  int *qstart_d = c->alloc<int>(M + 1), *tend_d = c->alloc<int>(M);
+  int *qstart_d = c->alloc<int>(M + 1);
   c->moff = c->alloc<long long>(M);
   c->mlc = c->alloc<int>(M);
   c->sc = c->alloc<xm::StepScalars>(M);
@@ -1183,8 +1280,11 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
   c->act = c->alloc<int>(M);
   c->mpoly = c->alloc<int>(M);
   c->part = c->alloc<double>(2 * size_t(c->nquad) + 64);
-  if (!c->lidx || !c->tile_member || !tnbr_d || !kind_d || !quads_d || !qstart_d || !tend_d ||
-      !c->moff || !c->mlc || !c->sc || !c->ctl || !c->glob || !c->act || !c->mpoly || !c->part)
+  c->res_part = c->alloc<double2>(2 * size_t(c->nquad), false);
+  c->res_count = c->alloc<unsigned>(xm::RES_COUNT_STRIDE * size_t(M), false);
+  if (!c->lidx || !c->tile_member || !tnbr_d || !kind_d || !quads_d || !qstart_d ||
+      !c->moff || !c->mlc || !c->sc || !c->ctl || !c->glob || !c->act || !c->mpoly || !c->part ||
+      !c->res_part || !c->res_count)
     return bail("cudaMalloc failed");
   {
     std::vector<long long> moff(M);
@@ -1205,11 +1305,13 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
   c->hp1_h.assign(M, 1.0);
   c->chan_start.assign(M + 1, 0);
   c->qstart_h = qstart;
-  for (int m = 0; m < M; ++m) c->small_units = std::max(c->small_units, qstart[m + 1] - qstart[m]);
+  for (int m = 0; m < M; ++m) c->max_units = std::max(c->max_units, qstart[m + 1] - qstart[m]);
   c->has_layers.assign(M, 0);
+  if (reset_resident(c) || !build_resident(c, xm::cg_res_capacity, SIZE_MAX, c->res64) ||
+      !build_resident(c, xm::mx_res_capacity, 1, c->res32))
+    return bail("cudaMalloc failed (resident solves)");
   cudaMemcpy(quads_d, quads.data(), quads.size() * sizeof(int4), cudaMemcpyHostToDevice);
   cudaMemcpy(qstart_d, qstart.data(), (M + 1) * sizeof(int), cudaMemcpyHostToDevice);
-  cudaMemcpy(tend_d, tend.data(), M * sizeof(int), cudaMemcpyHostToDevice);
   auto D = [&]() { return c->alloc<double>(ns); };
   auto I = [&]() { return c->alloc<int>(ns); };
   auto Fl = [&]() { return c->alloc<float>(ns); };
@@ -1220,7 +1322,6 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
   S.tile_member = c->tile_member;
   S.quads = quads_d;
   S.qstart = qstart_d;
-  S.tend = tend_d;
   S.sc = c->sc;
   S.nquad = c->nquad;
   S.nmember = M;
@@ -1838,7 +1939,7 @@ struct StepPlan {
   int mixed, istl, all, any_isdry, any_legacy, any99, any_waste, iters;
   int max_iterm, max_sweeps, grid, grid_cg, grid_cg32, grid_up32;
   int mx_jac, mx_poly, may_asym, chan, baro, obc_serial, any_may_asym, nmember;
-  int variant, ctas_mv, ctas_up, any_drag, small;
+  int variant, ctas_mv, ctas_up, any_drag, resident;
   double fac, inner_margin;
   const void *psol;
 };
@@ -1925,10 +2026,12 @@ cudaError_t capture_solve(efdc_xm_ctx *c, const StepPlan &pl, int d, StepGraph &
   l.stream = st;
   const int M = c->M, K = pl.iters;
   double *P = c->X.p;
-  if (!pl.mixed && pl.small) {  // one CTA per member, its loop inside (k_cg_small)
+  if (pl.resident) {  // the loops inside the kernel
     xm::launch_solve_reset(l, c->ctl, c->glob, c->act, M);
-    xm::launch_cg_small(l, c->S, c->Y, P, c->ctl, c->glob, c->part, c->small_slots,
-                        c->small_units, M);
+    if (pl.mixed)
+      launch_resident32(c, l, P, pl.fac);
+    else
+      launch_resident64(c, l, P);
     take_count(mark, mine);
     return cudaGetLastError();
   }
@@ -2110,10 +2213,11 @@ void drop_step_graphs(efdc_xm_ctx *c) {
 // A bounded wait in a kernel ran out (Glob::err): every member of the step
 // fails with EFDC_XM_DEVICE_TIMEOUT; the flag is cleared for the next call.
 int device_timeout(efdc_xm_ctx *c, efdc_xm_stats *stats, int m0, int m1) {
-  set_error("a bounded device-side wait ran out (bulk copies into shared memory did not "
-            "complete); the step's results are not valid");
+  set_error("a bounded device-side wait ran out (bulk copies into shared memory, or the sums of "
+            "another CTA of a resident solve, did not arrive); the results are not valid");
   for (int m = m0; m < m1; ++m) stats[m].status = EFDC_XM_DEVICE_TIMEOUT;
   CK(cudaMemsetAsync(&c->glob->err, 0, sizeof(int), c->stream));
+  if (const int rc = reset_resident(c)) return rc;
   return EFDC_XM_DEVICE_TIMEOUT;
 }
 
@@ -2335,7 +2439,7 @@ int tune_time(efdc_xm_ctx *c, bool mixed, double fac, int reps, double *ms) {
   const xm::Launch lk = c->L();
   StepPlan pl{};
   pl.mixed = mixed;
-  pl.small = !mixed && small_solve(c);
+  pl.resident = resident_solve(c, mixed);
   pl.iters = c->graph_iters;
   pl.max_iterm = 1;
   for (int m = 0; m < c->M; ++m) pl.max_iterm = std::max(pl.max_iterm, c->sc_h[m].iterm);
@@ -2369,7 +2473,7 @@ int tune_time(efdc_xm_ctx *c, bool mixed, double fac, int reps, double *ms) {
   if ((rc = read_glob(c))) return rc;
   if (c->glob_h->err) {  // a bounded wait ran out: this schedule is not usable here
     CK(cudaMemsetAsync(&c->glob->err, 0, sizeof(int), c->stream));
-    return EFDC_XM_OK;
+    return reset_resident(c);
   }
   std::sort(t.begin(), t.end());
   *ms = t[t.size() / 2];
@@ -2517,7 +2621,7 @@ int step_range(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_stats *stats, 
     StepPlan pl{};
     const xm::Launch lk = c->L();
     pl.mixed = mixed;
-    pl.small = !mixed && small_solve(c);
+    pl.resident = resident_solve(c, mixed);
     pl.istl = istl;
     pl.all = all;
     pl.any_isdry = any_isdry;
@@ -3847,6 +3951,7 @@ int32_t efdc_xm_congrad(efdc_xm_ctx *c, const double *ccc, const double *ccs, co
   rc = mixed ? solve_mixed(c, c->X.p, 0.0) : solve_fp64(c, c->X.p);
   if (rc) return rc;
   const Ctl k = c->ctl_h[0];
+  if (k.status == EFDC_XM_DEVICE_TIMEOUT) return device_timeout(c, nullptr, 0, 0);
   std::vector<Xfer> out = {{one(p), c->X.p, 0}};
   if ((rc = download_arrays(c, out))) return rc;
   if (iters) *iters = k.iter;
@@ -4005,8 +4110,8 @@ int32_t efdc_xm_set_option(efdc_xm_ctx *c, int32_t option, int32_t value) {
       return EFDC_XM_OK;
     case EFDC_XM_OPT_SMALL_SOLVE:
       if (value < 0 || value > 1) break;
-      if ((value != 0) != c->small_solve) {
-        c->small_solve = value != 0;
+      if ((value != 0) != c->resident) {
+        c->resident = value != 0;
         drop_graphs(c);
       }
       return EFDC_XM_OK;
@@ -4398,6 +4503,7 @@ int32_t efdc_xm_calib_adjoint_step(efdc_xm_ctx *c, const efdc_xm_params *prm, in
     if ((rc = solve_fp64(c, A.lam))) return rc;
     const Ctl &k = c->ctl_h[0];
     iters = k.iter;
+    if (k.status == EFDC_XM_DEVICE_TIMEOUT) return device_timeout(c, nullptr, 0, 0);
     if (k.status != EFDC_XM_OK) {
       set_error("adjoint CONGRAD: %s after %d iterations",
                 k.status == EFDC_XM_CG_MAXITER ? "maximum iterations exceeded"

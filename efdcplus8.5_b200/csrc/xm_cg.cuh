@@ -458,51 +458,58 @@ __device__ __forceinline__ void quad_sweep_v(const DevStatic &S, double *part, S
 // FP64 CONGRAD (congrad.f90): :88 RETURN on RPCG = 0; :124 ALPHA (also the
 // MIXED inner ALPHA); :143-169 BETA, RSQ and the stop test.  With no_stop the
 // iteration continues past RSQM and ITERM (kernel timing).
-__device__ __forceinline__ void cg_init_epi(Ctl &k, Glob *glob, double rpcg) {
+// The *_step forms work on a Ctl alone and return true when the member has
+// finished (the resident solves keep theirs in registers); the *_epi forms
+// also record it in the member's Ctl and in glob.
+__device__ __forceinline__ bool cg_init_step(Ctl &k, double rpcg) {
   k.rpcg = rpcg;
   k.beta = 0.0;
   k.parity = 0;
   k.iter = 0;
   k.rsq = 0.0;
   k.status = 0;
-  if (rpcg == 0.0 || !isfinite(rpcg)) {  // :88 RETURN
-    if (!isfinite(rpcg)) k.status = EFDC_XM_NONFINITE;
-    k.done = 1;
-    atomicAdd(&glob->ndone, 1);
-  }
+  if (!isfinite(rpcg)) k.status = EFDC_XM_NONFINITE;
+  return rpcg == 0.0 || !isfinite(rpcg);  // :88 RETURN
+}
+__device__ __forceinline__ void member_done(Ctl &k, Glob *glob) {
+  k.done = 1;
+  atomicAdd(&glob->ndone, 1);
+}
+__device__ __forceinline__ void cg_init_epi(Ctl &k, Glob *glob, double rpcg) {
+  if (cg_init_step(k, rpcg)) member_done(k, glob);
 }
 __device__ __forceinline__ void cg_matvec_epi(Ctl &k, double pap) {
   k.papcg = pap;
   k.alpha = k.rpcg / pap;  // :124
 }
-__device__ __forceinline__ void cg_update_epi(Ctl &k, Glob *glob, const StepScalars &c,
-                                              double rpcgn, double rsq, int no_stop) {
+__device__ __forceinline__ bool cg_update_step(Ctl &k, double rsqm, int iterm, double rpcgn,
+                                               double rsq, int no_stop) {
   k.beta = rpcgn / k.rpcg;
   k.rpcg = rpcgn;
   k.rsq = rsq;
   const int it = k.iter + 1;
   k.iter = it;
-  int fin = 0;
   if (!isfinite(rsq) || !isfinite(k.alpha)) {
     k.status = EFDC_XM_NONFINITE;
-    fin = 1;
-  } else if (!no_stop && rsq <= c.rsqm) {
-    fin = 1;
-  } else if (!no_stop && it >= c.iterm) {
+    return true;
+  }
+  if (!no_stop && rsq <= rsqm) return true;
+  if (!no_stop && it >= iterm) {
     k.status = EFDC_XM_CG_MAXITER;
-    fin = 1;
-  } else {
-    k.parity ^= 1;
+    return true;
   }
-  if (fin) {
-    k.done = 1;
-    atomicAdd(&glob->ndone, 1);
-  }
+  k.parity ^= 1;
+  return false;
+}
+__device__ __forceinline__ void cg_update_epi(Ctl &k, Glob *glob, const StepScalars &c,
+                                              double rpcgn, double rsq, int no_stop) {
+  if (cg_update_step(k, c.rsqm, c.iterm, rpcgn, rsq, no_stop)) member_done(k, glob);
 }
 
 // MIXED inner iteration: BETA = r.z / r.z_old and the inner stop test on r.r
 // (its target, ITERM, or cap_fac*ITERM + 50 inner iterations over all passes).
-__device__ __forceinline__ void mx_update_epi(Ctl &k, Glob *glob, int iterm, double rz, double rr,
+// Returns 1 when the inner solve has finished, 2 when the member has failed.
+__device__ __forceinline__ int mx_update_step(Ctl &k, int iterm, double rz, double rr,
                                               double cap_fac, int no_stop) {
   k.beta = rz / k.rpcg;
   k.rpcg = rz;
@@ -512,15 +519,57 @@ __device__ __forceinline__ void mx_update_epi(Ctl &k, Glob *glob, int iterm, dou
   k.iter += 1;
   if (!isfinite(rr) || !isfinite(rz) || !isfinite(k.alpha)) {
     k.status = EFDC_XM_NONFINITE;
-    k.done = 1;
-    atomicAdd(&glob->ndone, 1);
-  } else if (!no_stop && (rr <= k.rsq_target || it >= iterm ||
-                          k.iter >= int(cap_fac * iterm) + 50)) {
+    return 2;
+  }
+  if (!no_stop &&
+      (rr <= k.rsq_target || it >= iterm || k.iter >= int(cap_fac * iterm) + 50))
+    return 1;
+  k.parity ^= 1;
+  return 0;
+}
+__device__ __forceinline__ void mx_update_epi(Ctl &k, Glob *glob, int iterm, double rz, double rr,
+                                              double cap_fac, int no_stop) {
+  const int fin = mx_update_step(k, iterm, rz, rr, cap_fac, no_stop);
+  if (fin == 2) {
+    member_done(k, glob);
+  } else if (fin == 1) {
     k.idone = 1;
     atomicAdd(&glob->nidone, 1);
-  } else {
-    k.parity ^= 1;
   }
+}
+
+// MIXED: the member's epilogue of the refinement residual: RSQ (of the scaled
+// system, as CONGRAD measures it), the stop test on the FP64 RSQ, and the
+// inner solve's target.  True when the member has finished.
+__device__ __forceinline__ bool mx_resid_step(Ctl &k, double c_rsqm, int iterm, const RedArgs &ra,
+                                              double rsq, double rz) {
+  if (ra.unscaled) {
+    const double ccmnm = fmin(k.ccmnm_int, k.ccmnm_bc);
+    rsq = rsq / (ccmnm * ccmnm);
+  }
+  const double rsqm = c_rsqm * ra.rsqm_fac;
+  k.rsq64 = rsq;
+  k.rsq = rsq;
+  k.rpcg = rz;
+  k.beta = 0.0;
+  k.parity = 0;
+  k.inner_iter = 0;
+  k.idone = 0;
+  k.outer += 1;
+  // inner stop on the scaled residual: reduce it by the factor the FP64
+  // residual needs to reach 0.1*RSQM, and by at least rel_tol (in norm)
+  const double need = (rsq > 0.0) ? ra.margin * 0.1 * rsqm / rsq : 1.0;
+  k.rsq_target = rz * fmax(fmin(need, 1.0), ra.rel_tol * ra.rel_tol);
+  if (!isfinite(rsq)) {
+    k.status = EFDC_XM_NONFINITE;
+    return true;
+  }
+  if (!ra.no_stop && (rsq <= rsqm || rz == 0.0)) return true;
+  if (!ra.no_stop && k.iter >= 2 * iterm + 50) {
+    k.status = EFDC_XM_CG_MAXITER;  // inner iterations of all passes exhausted
+    return true;
+  }
+  return false;
 }
 
 // The member-reduce kernels: member m (one CTA per member, grid-stride) sums
@@ -556,57 +605,13 @@ __device__ __forceinline__ void quad_apply(const DevStatic &S, Skip skip, Body b
 // PCG = CCCI*RCG + BETA*PCG (congrad.f90:133-159) on the cell's row vector and
 // its N/S rows and E/W neighbours, then APCG = CCC*P + CCS*PS + CCN*PN + CCW*PW
 // + CCE*PE (congrad.f90:114).  Stores p_new and Ap; returns the cell part of
-// p.Ap.  With asym == false, CCN(L) = CCS(LN) and CCE(L) = CCW(LE).
-template <class T>
-__device__ __forceinline__ double matvec_row(const RowGeo &g, bool valid, const T *__restrict__ r,
-                                             const T *__restrict__ ccc,
-                                             const T *__restrict__ pold, T *__restrict__ pnew,
-                                             const T *__restrict__ ccs, const T *__restrict__ ccw,
-                                             const T *__restrict__ cce, const T *__restrict__ ccn,
-                                             T *__restrict__ ap, T beta, bool asym) {
-  const V4<T> r0 = ld4(r + g.d0), c0 = ld4(ccc + g.d0), o0 = ld4(pold + g.d0);
-  const V4<T> rn = ld4(r + g.dn), cn_ = ld4(ccc + g.dn), on = ld4(pold + g.dn);
-  const V4<T> rs = ld4(r + g.ds), cs_ = ld4(ccc + g.ds), os = ld4(pold + g.ds);
-  auto pc = [&](T rr, T cc, T po) { return rcpT(cc) * rr + beta * po; };
-  const V4<T> p = {pc(r0.x, c0.x, o0.x), pc(r0.y, c0.y, o0.y), pc(r0.z, c0.z, o0.z),
-                   pc(r0.w, c0.w, o0.w)};
-  const V4<T> pn = {pc(rn.x, cn_.x, on.x), pc(rn.y, cn_.y, on.y), pc(rn.z, cn_.z, on.z),
-                    pc(rn.w, cn_.w, on.w)};
-  const V4<T> ps = {pc(rs.x, cs_.x, os.x), pc(rs.y, cs_.y, os.y), pc(rs.z, cs_.z, os.z),
-                    pc(rs.w, cs_.w, os.w)};
-  T pw = from_west(p), pe = from_east(p);
-  if (g.cx == 0) pw = pc(r[g.dwe], ccc[g.dwe], pold[g.dwe]);
-  if (g.cx == ROWT - 1) pe = pc(r[g.dee], ccc[g.dee], pold[g.dee]);
-  const V4<T> ks = ld4(ccs + g.d0), kw = ld4(ccw + g.d0);
-  V4<T> kn, ke;
-  if (asym) {
-    kn = ld4(ccn + g.d0);
-    ke = ld4(cce + g.d0);
-  } else {
-    kn = ld4(ccs + g.dn);
-    T kwe = from_east(kw);
-    if (g.cx == ROWT - 1) kwe = ccw[g.dee];
-    ke = {kw.y, kw.z, kw.w, kwe};
-  }
-  V4<T> a;
-  a.x = c0.x * p.x + ks.x * ps.x + kn.x * pn.x + kw.x * pw + ke.x * p.y;
-  a.y = c0.y * p.y + ks.y * ps.y + kn.y * pn.y + kw.y * p.x + ke.y * p.z;
-  a.z = c0.z * p.z + ks.z * ps.z + kn.z * pn.z + kw.z * p.y + ke.z * p.w;
-  a.w = c0.w * p.w + ks.w * ps.w + kn.w * pn.w + kw.w * p.z + ke.w * pe;
-  if (!valid) return 0.0;
-  st4(pnew + g.d0, p);
-  st4(ap + g.d0, a);
-  return double(a.x) * double(p.x) + double(a.y) * double(p.y) + double(a.z) * double(p.z) +
-         double(a.w) * double(p.w);
-}
-
-
-// FP64: as matvec_row, with z = CCCI*r stored by the kernels that write r, so
-// that the halo rows need z and p_old only: p = z + beta*p_old has the same
-// roundings as CCCI*r + beta*p_old formed in place.  With x and dox, also the
-// previous iteration's x += alpha*p_old, the statement the update pass would
-// have run (same operands, same rounding): that pass then reads neither x nor
-// p, and the last iteration's term is applied after the loop (k_cg_finish).
+// p.Ap.  With asym == false, CCN(L) = CCS(LN) and CCE(L) = CCW(LE).  z = CCCI*r
+// is stored by the kernels that write r, so that the halo rows need z and p_old
+// only: p = z + beta*p_old has the same roundings as CCCI*r + beta*p_old formed
+// in place.  With x and dox, also the previous iteration's x += alpha*p_old, the
+// statement the update pass would have run (same operands, same rounding): that
+// pass then reads neither x nor p, and the last iteration's term is applied
+// after the loop (k_cg_finish).
 __device__ __forceinline__ double matvec_row_z(const RowGeo &g, bool valid,
                                                const double *__restrict__ z,
                                                const double *__restrict__ ccc,
@@ -653,6 +658,40 @@ __device__ __forceinline__ double matvec_row_z(const RowGeo &g, bool valid,
   st4(pnew + g.d0, p);
   st4(ap + g.d0, a);
   return a.x * p.x + a.y * p.y + a.z * p.z + a.w * p.w;
+}
+
+// The FP32 rows of the inner iteration, with the fused multiply-adds written
+// out: every kernel that forms one -- the variants below, the staged and the
+// resident ones -- rounds alike, whatever the compiler would contract there.
+// Ap = p + AS*pS + AN*pN + AW*pW + AE*pE on a row vector
+__device__ __forceinline__ V4<float> scaled_ap(const V4<float> &p, const V4<float> &ps,
+                                               const V4<float> &pn, float pw, float pe,
+                                               const V4<float> &ks, const V4<float> &kn,
+                                               const V4<float> &kw, const V4<float> &ke) {
+  return {fmaf(ke.x, p.y, fmaf(kw.x, pw, fmaf(kn.x, pn.x, fmaf(ks.x, ps.x, p.x)))),
+          fmaf(ke.y, p.z, fmaf(kw.y, p.x, fmaf(kn.y, pn.y, fmaf(ks.y, ps.y, p.y)))),
+          fmaf(ke.z, p.w, fmaf(kw.z, p.y, fmaf(kn.z, pn.z, fmaf(ks.z, ps.z, p.z)))),
+          fmaf(ke.w, pe, fmaf(kw.w, p.z, fmaf(kn.w, pn.w, fmaf(ks.w, ps.w, p.w))))};
+}
+// z = (2I - Ahat) r = r - (AS*rS + AN*rN + AW*rW + AE*rE)
+__device__ __forceinline__ float neumann(float r, float ks, float rs, float kn, float rn,
+                                         float kw, float rw, float ke, float re) {
+  return r - fmaf(ke, re, fmaf(kw, rw, fmaf(ks, rs, __fmul_rn(kn, rn))));
+}
+__device__ __forceinline__ V4<float> neumann_row(const V4<float> &r, const V4<float> &rs,
+                                                 const V4<float> &rn, float rw, float re,
+                                                 const V4<float> &ks, const V4<float> &kn,
+                                                 const V4<float> &kw, const V4<float> &ke) {
+  return {neumann(r.x, ks.x, rs.x, kn.x, rn.x, kw.x, rw, ke.x, r.y),
+          neumann(r.y, ks.y, rs.y, kn.y, rn.y, kw.y, r.x, ke.y, r.z),
+          neumann(r.z, ks.z, rs.z, kn.z, rn.z, kw.z, r.y, ke.z, r.w),
+          neumann(r.w, ks.w, rs.w, kn.w, rn.w, kw.w, r.z, ke.w, re)};
+}
+// the FP64 dot product of two FP32 row vectors (the products are exact)
+__device__ __forceinline__ double dot4(const V4<float> &a, const V4<float> &b) {
+  double s = __fma_rn(double(a.y), double(b.y), __dmul_rn(double(a.x), double(b.x)));
+  s = __fma_rn(double(a.z), double(b.z), s);
+  return __fma_rn(double(a.w), double(b.w), s);
 }
 
 // MIXED inner iteration: x += alpha*p of the previous iteration, which the
@@ -705,17 +744,12 @@ __device__ __forceinline__ double matvec_row_scaled(const RowGeo &g, bool valid,
     if (g.cx == ROWT - 1) kwe = aw[g.dee];
     ke = {kw.y, kw.z, kw.w, kwe};
   }
-  V4<float> a;
-  a.x = p.x + ks.x * ps.x + kn.x * pn.x + kw.x * pw + ke.x * p.y;
-  a.y = p.y + ks.y * ps.y + kn.y * pn.y + kw.y * p.x + ke.y * p.z;
-  a.z = p.z + ks.z * ps.z + kn.z * pn.z + kw.z * p.y + ke.z * p.w;
-  a.w = p.w + ks.w * ps.w + kn.w * pn.w + kw.w * p.z + ke.w * pe;
+  const V4<float> a = scaled_ap(p, ps, pn, pw, pe, ks, kn, kw, ke);
   if (!valid) return 0.0;
   if (dox) st4(x + g.d0, x_plus_alpha_p(x0, alpha_prev, o0));
   st4(pnew + g.d0, p);
   st4(ap + g.d0, a);
-  return double(a.x) * double(p.x) + double(a.y) * double(p.y) + double(a.z) * double(p.z) +
-         double(a.w) * double(p.w);
+  return dot4(a, p);
 }
 
 // MIXED, polynomial-preconditioned: r -= alpha*Ap at the cell
@@ -753,18 +787,13 @@ __device__ __forceinline__ void update_row_poly(const RowGeo &g, bool valid,
     float kwe = from_east(kw);
     if (g.cx == ROWT - 1) kwe = aw[g.dee];
     const V4<float> ke = {kw.y, kw.z, kw.w, kwe};
-    zv.x = rn0.x - (ks.x * nS.x + kn.x * nN.x + kw.x * nw + ke.x * rn0.y);
-    zv.y = rn0.y - (ks.y * nS.y + kn.y * nN.y + kw.y * rn0.x + ke.y * rn0.z);
-    zv.z = rn0.z - (ks.z * nS.z + kn.z * nN.z + kw.z * rn0.y + ke.z * rn0.w);
-    zv.w = rn0.w - (ks.w * nS.w + kn.w * nN.w + kw.w * rn0.z + ke.w * ne);
+    zv = neumann_row(rn0, nS, nN, nw, ne, ks, kn, kw, ke);
   }
   if (!valid) return;
   st4(rnew + g.d0, rn0);
   st4(z + g.d0, zv);
-  rz += double(rn0.x) * double(zv.x) + double(rn0.y) * double(zv.y) +
-        double(rn0.z) * double(zv.z) + double(rn0.w) * double(zv.w);
-  rr += double(rn0.x) * double(rn0.x) + double(rn0.y) * double(rn0.y) +
-        double(rn0.z) * double(rn0.z) + double(rn0.w) * double(rn0.w);
+  rz += dot4(rn0, zv);
+  rr += dot4(rn0, rn0);
 }
 
 // MIXED: z0 = (2I - Ahat) r (or r) for the first inner iteration, p_old = 0,
@@ -785,16 +814,12 @@ __device__ __forceinline__ double zinit_row(const RowGeo &g, bool valid,
     float kwe = from_east(kw);
     if (g.cx == ROWT - 1) kwe = aw[g.dee];
     const V4<float> ke = {kw.y, kw.z, kw.w, kwe};
-    zv.x = r0.x - (ks.x * rS.x + kn.x * rN.x + kw.x * rw + ke.x * r0.y);
-    zv.y = r0.y - (ks.y * rS.y + kn.y * rN.y + kw.y * r0.x + ke.y * r0.z);
-    zv.z = r0.z - (ks.z * rS.z + kn.z * rN.z + kw.z * r0.y + ke.z * r0.w);
-    zv.w = r0.w - (ks.w * rS.w + kn.w * rN.w + kw.w * r0.z + ke.w * re);
+    zv = neumann_row(r0, rS, rN, rw, re, ks, kn, kw, ke);
   }
   if (!valid) return 0.0;
   st4(z + g.d0, zv);
   st4(pold + g.d0, V4<float>{0.f, 0.f, 0.f, 0.f});
-  return double(r0.x) * double(zv.x) + double(r0.y) * double(zv.y) + double(r0.z) * double(zv.z) +
-         double(r0.w) * double(zv.w);
+  return dot4(r0, zv);
 }
 
 // Variant 3 of the MIXED inner iteration: matvec_row_scaled and
@@ -841,17 +866,12 @@ __device__ __forceinline__ double matvec_row_scaled_eager(const RowGeo &g, bool 
     if (east) kwe = kwe_edge;
     ke = {kw.y, kw.z, kw.w, kwe};
   }
-  V4<float> a;
-  a.x = p.x + ks.x * ps.x + kn.x * pn.x + kw.x * pw + ke.x * p.y;
-  a.y = p.y + ks.y * ps.y + kn.y * pn.y + kw.y * p.x + ke.y * p.z;
-  a.z = p.z + ks.z * ps.z + kn.z * pn.z + kw.z * p.y + ke.z * p.w;
-  a.w = p.w + ks.w * ps.w + kn.w * pn.w + kw.w * p.z + ke.w * pe;
+  const V4<float> a = scaled_ap(p, ps, pn, pw, pe, ks, kn, kw, ke);
   if (!valid) return 0.0;
   if (dox) st4(x + g.d0, x_plus_alpha_p(x0, alpha_prev, o0));
   st4(pnew + g.d0, p);
   st4(ap + g.d0, a);
-  return double(a.x) * double(p.x) + double(a.y) * double(p.y) + double(a.z) * double(p.z) +
-         double(a.w) * double(p.w);
+  return dot4(a, p);
 }
 
 __device__ __forceinline__ void update_row_poly_eager(const RowGeo &g, bool valid,
@@ -899,18 +919,13 @@ __device__ __forceinline__ void update_row_poly_eager(const RowGeo &g, bool vali
     float kwe = from_east(kw);
     if (east) kwe = kwe_edge;
     const V4<float> ke = {kw.y, kw.z, kw.w, kwe};
-    zv.x = rn0.x - (ks.x * nS.x + kn.x * nN.x + kw.x * nw + ke.x * rn0.y);
-    zv.y = rn0.y - (ks.y * nS.y + kn.y * nN.y + kw.y * rn0.x + ke.y * rn0.z);
-    zv.z = rn0.z - (ks.z * nS.z + kn.z * nN.z + kw.z * rn0.y + ke.z * rn0.w);
-    zv.w = rn0.w - (ks.w * nS.w + kn.w * nN.w + kw.w * rn0.z + ke.w * ne);
+    zv = neumann_row(rn0, nS, nN, nw, ne, ks, kn, kw, ke);
   }
   if (!valid) return;
   st4(rnew + g.d0, rn0);
   st4(z + g.d0, zv);
-  rz += double(rn0.x) * double(zv.x) + double(rn0.y) * double(zv.y) +
-        double(rn0.z) * double(zv.z) + double(rn0.w) * double(zv.w);
-  rr += double(rn0.x) * double(rn0.x) + double(rn0.y) * double(rn0.y) +
-        double(rn0.z) * double(rn0.z) + double(rn0.w) * double(rn0.w);
+  rz += dot4(rn0, zv);
+  rr += dot4(rn0, rn0);
 }
 
 // MIXED, Jacobi: r -= alpha*Ap (into the other residual buffer) and the part
@@ -929,8 +944,7 @@ __device__ __forceinline__ void update_row_jac(const RowGeo &g, bool valid,
   rv.z = fmaf(-alpha, av.z, rv.z);
   rv.w = fmaf(-alpha, av.w, rv.w);
   st4(rnew + g.d0, rv);
-  rr += double(rv.x) * double(rv.x) + double(rv.y) * double(rv.y) + double(rv.z) * double(rv.z) +
-        double(rv.w) * double(rv.w);
+  rr += dot4(rv, rv);
 }
 
 // X = X + ALPHA*PCG, RCG = RCG - ALPHA*APCG, TMPCG = CCCI*RCG (congrad.f90:
@@ -1072,16 +1086,12 @@ __device__ __forceinline__ double zinit_row_eager(const RowGeo &g, bool valid,
     float kwe = from_east(kw);
     if (east) kwe = kwe_edge;
     const V4<float> ke = {kw.y, kw.z, kw.w, kwe};
-    zv.x = r0.x - (ks.x * rS.x + kn.x * rN.x + kw.x * rw + ke.x * r0.y);
-    zv.y = r0.y - (ks.y * rS.y + kn.y * rN.y + kw.y * r0.x + ke.y * r0.z);
-    zv.z = r0.z - (ks.z * rS.z + kn.z * rN.z + kw.z * r0.y + ke.z * r0.w);
-    zv.w = r0.w - (ks.w * rS.w + kn.w * rN.w + kw.w * r0.z + ke.w * re);
+    zv = neumann_row(r0, rS, rN, rw, re, ks, kn, kw, ke);
   }
   if (!valid) return 0.0;
   st4(z + g.d0, zv);
   st4(pold + g.d0, V4<float>{0.f, 0.f, 0.f, 0.f});
-  return double(r0.x) * double(zv.x) + double(r0.y) * double(zv.y) + double(r0.z) * double(zv.z) +
-         double(r0.w) * double(zv.w);
+  return dot4(r0, zv);
 }
 
 // The Jacobi scaling of the MIXED inner system, 1/sqrt(c) for a diagonal c

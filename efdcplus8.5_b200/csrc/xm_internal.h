@@ -138,7 +138,6 @@ struct DevStatic {
   const int4 *quads;      // [nquad] (member, first tile, tiles of the member in it (1..4), 0):
                           // the 4-tile units of the CG kernels
   const int *qstart;      // [M+1] first quad of each member
-  const int *tend;        // [M] one past the member's last tile
   const StepScalars *sc;  // [M] per-member scalars of the current step
   int nquad;
   int nmember;

@@ -59,14 +59,29 @@ void launch_explicit(const Launch &l, const DevStatic &S, const MomDev &M, const
 void launch_implicit_drag(const Launch &l, const DevStatic &S, const DevState &X,
                           const int *act);
 void launch_put(cudaStream_t st, const int *idx, const double *val, int n, double *dst);
-// CONGRAD of small members, one CTA each with its vectors in shared memory
-// (k_cg_small): the windows of every member fit when cg_small_fits(the
-// largest window's slots); the same iterates as the multi-kernel CG.
-constexpr int SMALL_SMEM_MAX = 200 * 1024;
-bool cg_small_fits(int slots);
-void launch_cg_small(const Launch &l, const DevStatic &S, const DevSystem &Y, double *P,
-                     Ctl *ctl, Glob *glob, double *part, int max_slots, int max_units,
-                     int nmember);
+// Solves that stay on the chip (xm_resident.cuh): a form is the quads side by
+// side in a CTA (w), its rows of quads (q), and the CTAs of a member as a
+// cluster (cluster > 0; else groups of any size that wait on a counter).
+struct ResForm {
+  int w, q, cluster;
+};
+struct ResPlan {
+  const int4 *cta;  // grid groups: [ncta] (member, first quad, quads, 0)
+  double2 *part;    // grid groups: [2][nquad] the quads' partial sums, by turns
+  unsigned *count;  // grid groups: [M*RES_COUNT_STRIDE] the member's arrivals, and next to it
+                    // the arrivals at the end of its last launch
+};
+constexpr int RES_COUNT_STRIDE = 32;  // a 128-byte line per member
+// FP64 CONGRAD: the CTAs (clusters) of a form that can be resident at once, and
+// a launch of ncta CTAs
+int cg_res_capacity(const ResForm &f, bool may_asym, int nsm);
+void launch_cg_res(const Launch &l, const DevStatic &S, const DevSystem &Y, double *P, Ctl *ctl,
+                   Glob *glob, const ResPlan &R, const ResForm &f, int ncta);
+// The MIXED solve (all its refinement passes, at most max_outer)
+int mx_res_capacity(const ResForm &f, bool may_asym, int nsm);
+void launch_mx_res(const Launch &l, const DevStatic &S, const SysView &V, const DevSystem &Y,
+                   double *P, Ctl *ctl, Glob *glob, const ResPlan &R, const ResForm &f, int ncta,
+                   double rsqm_fac, double rel_tol, int max_outer);
 void launch_put_int(cudaStream_t st, const int *idx, const int *val, int n, int *dst);
 // sub-grid channels (xm_chan.cu); each does nothing unless l.chan
 void launch_chan_entry(const Launch &l, const DevStatic &S, const DevState &X, const int *act);

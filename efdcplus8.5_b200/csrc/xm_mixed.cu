@@ -273,17 +273,12 @@ __global__ void __launch_bounds__(NT, 3) k_mx_matvec_st(DevStatic S, DevSystem Y
           if (g.cx == ROWT - 1) kwe = e.e2;
           ke = {kw.y, kw.z, kw.w, kwe};
         }
-        V4<float> ap;
-        ap.x = p.x + ks.x * ps.x + kn.x * pn.x + kw.x * pw + ke.x * p.y;
-        ap.y = p.y + ks.y * ps.y + kn.y * pn.y + kw.y * p.x + ke.y * p.z;
-        ap.z = p.z + ks.z * ps.z + kn.z * pn.z + kw.z * p.y + ke.z * p.w;
-        ap.w = p.w + ks.w * ps.w + kn.w * pn.w + kw.w * p.z + ke.w * pe;
+        const V4<float> ap = scaled_ap(p, ps, pn, pw, pe, ks, kn, kw, ke);
         if (!valid) return;
         if (a.dox) st4(Y.x32 + g.d0, x_plus_alpha_p(ld4(Y.x32 + g.d0), a.alpha, o0));
         st4(a.pnew + g.d0, p);
         st4(Y.ap32 + g.d0, ap);
-        v[0] = double(ap.x) * double(p.x) + double(ap.y) * double(p.y) +
-               double(ap.z) * double(p.z) + double(ap.w) * double(p.w);
+        v[0] = dot4(ap, p);
       },
       fold_if<FOLD>(ctl, [&](int m, const double *sum) {
         if (threadIdx.x == 0) cg_matvec_epi(ctl[m], sum[0]);
@@ -349,18 +344,12 @@ __global__ void __launch_bounds__(NT, 3) k_mx_update_poly_st(DevStatic S, DevSys
         float kwe = from_east(kw);
         if (g.cx == ROWT - 1) kwe = e.e2;
         const V4<float> ke = {kw.y, kw.z, kw.w, kwe};
-        V4<float> zv;
-        zv.x = rn0.x - (ks.x * nS.x + kn.x * nN.x + kw.x * nw + ke.x * rn0.y);
-        zv.y = rn0.y - (ks.y * nS.y + kn.y * nN.y + kw.y * rn0.x + ke.y * rn0.z);
-        zv.z = rn0.z - (ks.z * nS.z + kn.z * nN.z + kw.z * rn0.y + ke.z * rn0.w);
-        zv.w = rn0.w - (ks.w * nS.w + kn.w * nN.w + kw.w * rn0.z + ke.w * ne);
+        const V4<float> zv = neumann_row(rn0, nS, nN, nw, ne, ks, kn, kw, ke);
         if (!valid) return;
         st4(a.rnew + g.d0, rn0);
         st4(Y.z32 + g.d0, zv);
-        v[0] = double(rn0.x) * double(zv.x) + double(rn0.y) * double(zv.y) +
-               double(rn0.z) * double(zv.z) + double(rn0.w) * double(zv.w);
-        v[1] = double(rn0.x) * double(rn0.x) + double(rn0.y) * double(rn0.y) +
-               double(rn0.z) * double(rn0.z) + double(rn0.w) * double(rn0.w);
+        v[0] = dot4(rn0, zv);
+        v[1] = dot4(rn0, rn0);
       },
       fold_if<FOLD>(ctl, [&](int m, const double *sum) {
         if (threadIdx.x == 0)
@@ -398,8 +387,7 @@ __global__ void __launch_bounds__(NT, 4) k_mx_update_jac_st(DevStatic S, DevSyst
         rv.z = fmaf(-alpha, av.z, rv.z);
         rv.w = fmaf(-alpha, av.w, rv.w);
         st4(a.rnew + g.d0, rv);
-        const double rr = double(rv.x) * double(rv.x) + double(rv.y) * double(rv.y) +
-                          double(rv.z) * double(rv.z) + double(rv.w) * double(rv.w);
+        const double rr = dot4(rv, rv);
         v[0] = rr;
         v[1] = rr;
       },

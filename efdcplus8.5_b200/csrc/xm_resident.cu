@@ -1,0 +1,234 @@
+// xm_resident.cu -- the FP64 CONGRAD of a member in one launch, its vectors in
+// registers (see xm_resident.cuh).  Compiled without FMA contraction, like the
+// multi-kernel CG (xm_step.cu): each statement rounds as in congrad.f90.
+
+#include "xm_resident.cuh"
+
+namespace xm {
+
+constexpr int RES_NC = 5;  // CCC, CCS, CCW, CCN and CCCI (symmetric) or CCE (MA)
+template <int W, int Q>
+using Coef64 = ResCoef<double, W, Q, RES_NC, Q == 1>;
+template <int W, int Q>
+constexpr size_t res_smem64() {
+  return size_t(W) * Q * TILES_PER_CTA * TILE * sizeof(double) + Coef64<W, Q>::bytes;
+}
+
+// congrad.f90:54-187 for one member per group of CTAs.  What bounds it is the
+// exchange (see xm_resident.cuh) and the latency of the row work around it.
+// Measured against the multi-kernel CG with folded reductions (one CTA per
+// member before, for members of up to 4,000 slots), ms per step, device-resident:
+// 60x60 cells 0.35 -> 0.13, 260x250 0.36 -> 0.17, 500x500 0.45 -> 0.24, 700x700
+// 0.57 -> 0.34, 256 lakes of 1,100 cells in one batch 0.50 -> 0.38.
+// 128 registers a thread: one row of quads keeps the coefficients in registers
+// too, two keep them in shared memory.
+template <bool MA, int W, int Q, bool CLUSTER>
+__global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1) k_cg_res(DevStatic S, DevSystem Y, double *P,
+                                                        Ctl *ctl, Glob *glob, ResPlan R) {
+  extern __shared__ __align__(16) double dyn[];
+  __shared__ ResShared<W, Q, CLUSTER> sh;
+  const ResCta me = res_cta<W, Q, CLUSTER>(R, S);
+  const int m = me.m;
+  if (ctl[m].done) return;  // the same for the member's CTAs: it is set after their exchanges
+  if constexpr (CLUSTER) cluster_barrier();  // every CTA has started: its shared memory is there
+  const double rsqm = S.sc[m].rsqm;
+  const int iterm = S.sc[m].iterm;
+  const bool asym = unsym<MA>(ctl[m]);
+  ResBarrier bar{CLUSTER ? 0u : R.count[size_t(m) * RES_COUNT_STRIDE + 1], 0};
+  double *stage = dyn;
+  Coef64<W, Q> C;
+  C.sm = dyn + W * Q * TILES_PER_CTA * TILE;
+  const bool north = res_north(), south = res_south(), west = res_west(), east = res_east();
+  const int w0 = W > 1 ? int(threadIdx.x) / NT : 0;  // quad q0 + i*W + w0 is the thread's row i
+  auto none = [] {};
+
+  ResRow row[Q];
+  V4<double> x[Q], r[Q], p[Q], ap[Q];
+  double kwe[Q];  // symmetric: CCW of the cell east of the row vector
+  Ctl k;  // of it: rpcg, papcg, alpha, beta, rsq, iter, status, parity
+  k.alpha = 0.0;
+  bool fin;
+  double v0[Q][1];
+  {  // :54-88
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+      const int j = i * W + w0;
+      const RowGeo g = res_geo(S, me.q0 + j, j < me.nq, row[i]);
+      r[i] = residual_row(g, S.kind, P, Y, asym);
+      x[i] = ld4(P + g.d0);
+      const V4<double> c = ld4(Y.ccc + g.d0), kw = ld4(Y.ccw + g.d0);
+      const V4<double> ci = {rcpT(c.x), rcpT(c.y), rcpT(c.z), rcpT(c.w)};
+      p[i] = {r[i].x * ci.x, r[i].y * ci.y, r[i].z * ci.z, r[i].w * ci.w};
+      C.put(i, 0, c);
+      C.put(i, 1, ld4(Y.ccs + g.d0));
+      C.put(i, 2, kw);
+      C.put(i, 3, asym ? ld4(Y.ccn + g.d0) : ld4(Y.ccs + g.dn));
+      kwe[i] = from_east(kw);
+      if (east) kwe[i] = Y.ccw[g.dee];
+      if constexpr (MA)
+        C.put(i, 4, asym ? ld4(Y.cce + g.d0) : V4<double>{kw.y, kw.z, kw.w, kwe[i]});
+      else
+        C.put(i, 4, ci);
+      st_border(Y.z, row[i], p[i]);
+      st_border(Y.pa, row[i], p[i]);
+      v0[i][0] = row[i].valid ? r[i].x * p[i].x + r[i].y * p[i].y + r[i].z * p[i].z +
+                                    r[i].w * p[i].w
+                              : 0.0;
+    }
+  }
+  auto cci = [&](int i) {  // CCCI
+    if constexpr (MA) {
+      const V4<double> c = C.get(i, 0);
+      return V4<double>{rcpT(c.x), rcpT(c.y), rcpT(c.z), rcpT(c.w)};
+    } else {
+      return C.get(i, 4);
+    }
+  };
+  // what the neighbour tiles hold of z and p_old, for the next A*p
+  V4<double> hz[Q], ho[Q];
+  double ez[Q], eo[Q];
+  auto halo = [&](const double *pold) {
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+      if (north || south) {
+        hz[i] = ldx4(Y.z + row[i].hv);
+        ho[i] = ldx4(pold + row[i].hv);
+      }
+      if (west || east) {
+        ez[i] = __ldcg(Y.z + row[i].hx);
+        eo[i] = __ldcg(pold + row[i].hx);
+      }
+    }
+  };
+  {
+    double sum[1];
+    if (!res_exchange(R, S, me, sh, bar, v0, sum, [&] { halo(Y.pa); }))
+      return res_fail(ctl[m], Y.err);
+    fin = cg_init_step(k, sum[0]);
+  }
+  while (!fin) {  // ITERM bounds the loop
+    {  // :93-125, and :133 of the previous iteration
+      const double beta = k.beta, alpha = k.alpha;
+      double *pnew = k.parity ? Y.pa : Y.pb;
+      const bool dox = k.iter > 0;
+      double v[Q][1], sum[1];
+#pragma unroll
+      for (int i = 0; i < Q; ++i) {
+        const V4<double> ci = cci(i);
+        if (dox)
+          x[i] = {x[i].x + alpha * p[i].x, x[i].y + alpha * p[i].y, x[i].z + alpha * p[i].z,
+                  x[i].w + alpha * p[i].w};
+        p[i] = {ci.x * r[i].x + beta * p[i].x, ci.y * r[i].y + beta * p[i].y,
+                ci.z * r[i].z + beta * p[i].z, ci.w * r[i].w + beta * p[i].w};
+        st4(res_stage<W>(stage, i), p[i]);
+        st_border(pnew, row[i], p[i]);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < Q; ++i) {
+        V4<double> h{};
+        double e = 0.0;
+        if (north || south)
+          h = {hz[i].x + beta * ho[i].x, hz[i].y + beta * ho[i].y, hz[i].z + beta * ho[i].z,
+               hz[i].w + beta * ho[i].w};
+        if (west || east) e = ez[i] + beta * eo[i];
+        const double *st = res_stage<W>(stage, i);
+        const V4<double> pn = north ? h : ld4(st + TX), ps = south ? h : ld4(st - TX);
+        double pw = from_west(p[i]), pe = from_east(p[i]);
+        if (west) pw = e;
+        if (east) pe = e;
+        const V4<double> c0 = C.get(i, 0), ks = C.get(i, 1), kw = C.get(i, 2), kn = C.get(i, 3);
+        V4<double> ke;
+        if constexpr (MA)
+          ke = C.get(i, 4);
+        else
+          ke = {kw.y, kw.z, kw.w, kwe[i]};
+        const V4<double> q = p[i];
+        V4<double> a;
+        a.x = c0.x * q.x + ks.x * ps.x + kn.x * pn.x + kw.x * pw + ke.x * q.y;
+        a.y = c0.y * q.y + ks.y * ps.y + kn.y * pn.y + kw.y * q.x + ke.y * q.z;
+        a.z = c0.z * q.z + ks.z * ps.z + kn.z * pn.z + kw.z * q.y + ke.z * q.w;
+        a.w = c0.w * q.w + ks.w * ps.w + kn.w * pn.w + kw.w * q.z + ke.w * pe;
+        ap[i] = a;
+        v[i][0] = row[i].valid ? a.x * q.x + a.y * q.y + a.z * q.z + a.w * q.w : 0.0;
+      }
+      if (!res_exchange(R, S, me, sh, bar, v, sum, none)) return res_fail(ctl[m], Y.err);
+      cg_matvec_epi(k, sum[0]);
+    }
+    {  // :134-169
+      const double alpha = k.alpha;
+      double v[Q][2], sum[2];
+#pragma unroll
+      for (int i = 0; i < Q; ++i) {
+        const V4<double> ci = cci(i);
+        V4<double> rv = r[i];
+        rv.x = rv.x - alpha * ap[i].x;
+        rv.y = rv.y - alpha * ap[i].y;
+        rv.z = rv.z - alpha * ap[i].z;
+        rv.w = rv.w - alpha * ap[i].w;
+        r[i] = rv;
+        const V4<double> z = {ci.x * rv.x, ci.y * rv.y, ci.z * rv.z, ci.w * rv.w};
+        st_border(Y.z, row[i], z);
+        v[i][0] = row[i].valid ? rv.x * z.x + rv.y * z.y + rv.z * z.z + rv.w * z.w : 0.0;
+        v[i][1] = row[i].valid ? rv.x * rv.x + rv.y * rv.y + rv.z * rv.z + rv.w * rv.w : 0.0;
+      }
+      const double *pold = k.parity ? Y.pa : Y.pb;  // the next A*p's: the p just stored
+      if (!res_exchange(R, S, me, sh, bar, v, sum, [&] { halo(pold); }))
+        return res_fail(ctl[m], Y.err);
+      fin = cg_update_step(k, rsqm, iterm, sum[0], sum[1], 0);
+    }
+  }
+  if (k.iter > 0) {  // :133 of the last iteration
+    const double alpha = k.alpha;
+#pragma unroll
+    for (int i = 0; i < Q; ++i)
+      if (row[i].valid)
+        st4(P + row[i].d0,
+            V4<double>{x[i].x + alpha * p[i].x, x[i].y + alpha * p[i].y,
+                       x[i].z + alpha * p[i].z, x[i].w + alpha * p[i].w});
+  }
+  if (me.q0 == me.qm0 && me.nq > 0 && threadIdx.x == 0) {  // every CTA of the member has read its entry values
+    Ctl &o = ctl[m];
+    o.rpcg = k.rpcg;
+    o.beta = k.beta;
+    o.rsq = k.rsq;
+    if (k.iter > 0) {
+      o.papcg = k.papcg;
+      o.alpha = k.alpha;
+    }
+    o.iter = k.iter;
+    o.status = k.status;
+    o.parity = k.parity;
+    member_done(o, glob);
+    if (!CLUSTER) R.count[size_t(m) * RES_COUNT_STRIDE + 1] = bar.count;
+  }
+}
+
+int cg_res_capacity(const ResForm &f, bool may_asym, int nsm) {
+  int cap = 0;
+  res_form(f, [&](auto w, auto q, auto cl) {
+    constexpr int W = decltype(w)::value, Q = decltype(q)::value;
+    constexpr bool CL = decltype(cl)::value;
+    cap = may_asym
+              ? res_cap(k_cg_res<true, W, Q, CL>, NT * W, res_smem64<W, Q>(), nsm, f.cluster)
+              : res_cap(k_cg_res<false, W, Q, CL>, NT * W, res_smem64<W, Q>(), nsm, f.cluster);
+  });
+  return cap;
+}
+
+void launch_cg_res(const Launch &l, const DevStatic &S, const DevSystem &Y, double *P, Ctl *ctl,
+                   Glob *glob, const ResPlan &R, const ResForm &f, int ncta) {
+  res_form(f, [&](auto w, auto q, auto cl) {
+    constexpr int W = decltype(w)::value, Q = decltype(q)::value;
+    constexpr bool CL = decltype(cl)::value;
+    if (l.may_asym)
+      launch_resident(k_cg_res<true, W, Q, CL>, ncta, NT * W, res_smem64<W, Q>(), f.cluster,
+                      l.stream, S, Y, P, ctl, glob, R);
+    else
+      launch_resident(k_cg_res<false, W, Q, CL>, ncta, NT * W, res_smem64<W, Q>(), f.cluster,
+                      l.stream, S, Y, P, ctl, glob, R);
+  });
+  count_launches(1);
+}
+
+}  // namespace xm

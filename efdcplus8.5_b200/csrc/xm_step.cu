@@ -724,240 +724,14 @@ __global__ void __launch_bounds__(NT) k_cg_finish(DevStatic S, DevSystem Y, doub
 }
 
 // ---------------------------------------------------------------------------
-// CONGRAD of small members, the whole solve in one CTA per member: the
-// member's CG vectors (P, r, z, p double-buffered, Ap) stay in shared memory
-// from the first residual to the stop test, its units run SMALL_UNITS at a
-// time, and the coefficient arrays are read from global memory.  The rows
-// (the same row functions), the per-unit partial sums (warp sums added in
-// warp order), the member sums (reduce_partials of a 256-thread CTA) and the
-// epilogues are those of k_cg_init, k_cg_matvec, k_cg_update and their member
-// reductions, so the iterates equal theirs bit for bit; one launch replaces
-// 2 + 4 per iteration.  The rows of a unit past the member's last tile work
-// on the member's ghost tile with stores off, so that every access stays in
-// the member's window of slots, [its ghost tile, its last tile].
-constexpr int SMALL_UNITS = 2;
-constexpr int SMALL_NT = SMALL_UNITS * NT;
-constexpr int SMALL_CACHED = 2;  // passes whose geometry a thread keeps in registers
-
-// reduce_partials of a 256-thread CTA, by a CTA of SMALL_NT threads (the
-// threads past the first 256 add nothing, as block_sum's last stage reads 8
-// warps), from the partials in shared memory
-constexpr int SMALL_MAX_UNITS = 64;
-__device__ __forceinline__ double reduce_partials_256(const double *part, int nblk, double *sh) {
-  double s = 0.0;
-  for (int base = 0; base < nblk; base += 8 * NT) {
-    double v[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int i = base + j * NT + int(threadIdx.x);
-      v[j] = (threadIdx.x < NT && i < nblk) ? part[i] : 0.0;
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) s += v[j];
-  }
-  return block_sum(s, sh);
-}
-
-template <bool MA, int NP>
-__global__ void __launch_bounds__(SMALL_NT) k_cg_small(DevStatic S, DevSystem Y, double *P,
-                                                      Ctl *ctl, Glob *glob, double *part) {
-  extern __shared__ double smv[];
-  __shared__ double sh[32];
-  __shared__ double wp[2][SMALL_NT / 32];
-  __shared__ double qp[2][SMALL_MAX_UNITS];  // the member's per-unit partials
-  __shared__ double s_beta, s_alpha;          // the member's control values, as thread 0
-  __shared__ int s_done, s_parity;            // leaves them in ctl[m]
-  const int m = blockIdx.x;
-  if (ctl[m].done) return;  // not in this sweep
-  // thread 0 runs the epilogues on ctl[m] and shares what the loop reads
-  auto share = [&] {
-    if (threadIdx.x == 0) {
-      const Ctl &k = ctl[m];
-      s_done = k.done;
-      s_parity = k.parity;
-      s_beta = k.beta;
-      s_alpha = k.alpha;
-    }
-    __syncthreads();
-  };
-  const int q0 = S.qstart[m], q1 = S.qstart[m + 1], nq = q1 - q0;
-  const int ghost = S.quads[q0].y - 1;  // the member's ghost tile, before its tiles
-  const int base = ghost * TILE, nsl = (S.tend[m] - ghost) * TILE;
-  double *gv[6] = {P, Y.r, Y.z, Y.pa, Y.pb, Y.ap};
-  for (int i = threadIdx.x; i < nsl; i += SMALL_NT)
-#pragma unroll
-    for (int k = 0; k < 6; ++k) smv[k * nsl + i] = gv[k][base + i];
-  __syncthreads();
-  // pointers that take the slot d of the window to shared memory
-  double *const Ps = smv - base;
-  DevSystem Ys = Y;
-  Ys.r = smv + nsl - base;
-  Ys.z = smv + 2 * nsl - base;
-  Ys.pa = smv + 3 * nsl - base;
-  Ys.pb = smv + 4 * nsl - base;
-  Ys.ap = smv + 5 * nsl - base;
-  const int qi = threadIdx.x / NT, tq = threadIdx.x % NT;
-  const int sub = tq / TPT, q = tq % TPT;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool asym = unsym<MA>(ctl[m]);
-
-  // where a thread's rows are in pass p (units u0 + qi, u0 = q0 + p*SMALL_UNITS)
-  struct Pass {
-    RowGeo g;
-    bool have, valid;
-  };
-  auto pass_of = [&](int u0) {
-    const int qd = u0 + qi;
-    const bool have = qd < q1;
-    const int4 cur = have ? S.quads[qd] : int4{m, ghost, 0, 0};
-    const bool valid = have && sub < cur.z;
-    const int ti = valid ? cur.y + sub : ghost;
-    return Pass{row_geo_nb(__ldg(&S.tnbr[ti]), ti, q), have, valid};
-  };
-  // NP > 0: the member has at most NP passes, whose geometry is formed once
-  // here and kept in registers (the loop then has no dependent loads of the
-  // unit table and the tile neighbours)
-  Pass pc[NP > 0 ? NP : 1];
-  if constexpr (NP > 0) {
-#pragma unroll
-    for (int p = 0; p < NP; ++p) pc[p] = pass_of(q0 + p * SMALL_UNITS);
-  }
-
-  // one sweep of a row body over the member's units, as quad_sweep makes it
-  auto sweep = [&](auto body, auto ns_tag) {
-    constexpr int NS = decltype(ns_tag)::value;
-    auto unit = [&](int u0, const Pass &ps) {
-      const int qd = u0 + qi;
-      double v[NS];
-#pragma unroll
-      for (int s = 0; s < NS; ++s) v[s] = 0.0;
-      body(ps.g, ps.valid, v);
-#pragma unroll
-      for (int s = 0; s < NS; ++s) {
-        const double x = warp_sum(v[s]);
-        if (lane == 0) wp[s][warp] = x;
-      }
-      __syncthreads();
-      if (tq == 0 && ps.have) {
-#pragma unroll
-        for (int s = 0; s < NS; ++s) {
-          double a = 0.0;
-#pragma unroll
-          for (int w = 0; w < NWARP; ++w) a += wp[s][qi * NWARP + w];
-          qp[s][qd - q0] = a;
-        }
-      }
-      __syncthreads();
-    };
-    if constexpr (NP > 0) {
-#pragma unroll
-      for (int p = 0; p < NP; ++p)
-        if (q0 + p * SMALL_UNITS < q1) unit(q0 + p * SMALL_UNITS, pc[p]);  // CTA-uniform
-    } else {
-      for (int u0 = q0; u0 < q1; u0 += SMALL_UNITS) unit(u0, pass_of(u0));
-    }
-  };
-  using One = std::integral_constant<int, 1>;
-  using Two = std::integral_constant<int, 2>;
-
-  // :54-88
-  sweep(
-      [&](const RowGeo &g, bool valid, double *v) {
-        const V4<double> r = residual_row(g, S.kind, Ps, Ys, asym);
-        const V4<double> c = ld4(Y.ccc + g.d0);
-        const V4<double> z = {r.x * rcpT(c.x), r.y * rcpT(c.y), r.z * rcpT(c.z),
-                              r.w * rcpT(c.w)};
-        if (valid) {
-          st4(Ys.r + g.d0, r);
-          st4(Ys.pa + g.d0, z);
-          st4(Ys.z + g.d0, z);
-          v[0] = r.x * z.x + r.y * z.y + r.z * z.z + r.w * z.w;
-        }
-      },
-      One{});
-  {
-    const double rpcg = reduce_partials_256(qp[0], nq, sh);
-    if (threadIdx.x == 0) cg_init_epi(ctl[m], glob, rpcg);
-    share();
-  }
-  // :91-169, ITERM bounds the loop (cg_update_epi sets done)
-  while (!s_done) {
-    {
-      const bool par = s_parity;
-      const double beta = s_beta;
-      const double *pold = par ? Ys.pb : Ys.pa;
-      double *pnew = par ? Ys.pa : Ys.pb;
-      sweep(
-          [&](const RowGeo &g, bool valid, double *v) {
-            v[0] = matvec_row_z(g, valid, Ys.z, Y.ccc, pold, pnew, Y.ccs, Y.ccw, Y.cce, Y.ccn,
-                                Ys.ap, beta, asym);
-          },
-          One{});
-      const double pap = reduce_partials_256(qp[0], nq, sh);
-      if (threadIdx.x == 0) cg_matvec_epi(ctl[m], pap);
-      share();
-    }
-    {
-      const double alpha = s_alpha;
-      const double *pnew = s_parity ? Ys.pa : Ys.pb;
-      sweep(
-          [&](const RowGeo &g, bool valid, double *v) {
-            update_row<double>(g, valid, Ps, pnew, Ys.r, Ys.ap, Y.ccc, alpha, v[0], v[1], Ys.z);
-          },
-          Two{});
-      const double rz = reduce_partials_256(qp[0], nq, sh);
-      const double rr = reduce_partials_256(qp[1], nq, sh);
-      if (threadIdx.x == 0) cg_update_epi(ctl[m], glob, S.sc[m], rz, rr, 0);
-      share();
-    }
-  }
-  for (int i = threadIdx.x; i < nsl; i += SMALL_NT)
-#pragma unroll
-    for (int k = 0; k < 6; ++k) gv[k][base + i] = smv[k * nsl + i];
-}
-
-// ---------------------------------------------------------------------------
 // MIXED outer step: r = b - A*P in FP64 (the FP64 refinement residual), RSQ
 // in FP64, and the FP32 scaled inner system's rhs rhat = D^-1/2 r with
 // x = 0 and p0 = rhat (k_mx_zinit then forms z0 = M^-1 rhat and p_old = 0 for
 // the polynomial members).  rsqm_fac scales the member's RSQM (the MIXED stop,
 // below RSQM).  EAGER: the row's loads issued first (kernel variant 3).
-// The member's epilogue of the refinement residual: RSQ (of the scaled system,
-// as CONGRAD measures it), the stop test on the FP64 RSQ, and the inner
-// solve's target.
-__device__ __forceinline__ void mx_resid_epi(Ctl &k, const StepScalars &c, const RedArgs &ra,
-                                             double rsq, double rz) {
-  if (ra.unscaled) {
-    const double ccmnm = fmin(k.ccmnm_int, k.ccmnm_bc);
-    rsq = rsq / (ccmnm * ccmnm);
-  }
-  const double rsqm = c.rsqm * ra.rsqm_fac;
-  k.rsq64 = rsq;
-  k.rsq = rsq;
-  k.rpcg = rz;
-  k.beta = 0.0;
-  k.parity = 0;
-  k.inner_iter = 0;
-  k.idone = 0;
-  k.outer += 1;
-  // inner stop on the scaled residual: reduce it by the factor the FP64
-  // residual needs to reach 0.1*RSQM, and by at least rel_tol (in norm)
-  const double need = (rsq > 0.0) ? ra.margin * 0.1 * rsqm / rsq : 1.0;
-  k.rsq_target = rz * fmax(fmin(need, 1.0), ra.rel_tol * ra.rel_tol);
-  int fin = 0;
-  if (!isfinite(rsq)) {
-    k.status = EFDC_XM_NONFINITE;
-    fin = 1;
-  } else if (!ra.no_stop && (rsq <= rsqm || rz == 0.0)) {
-    fin = 1;
-  } else if (!ra.no_stop && k.iter >= 2 * c.iterm + 50) {
-    k.status = EFDC_XM_CG_MAXITER;  // inner iterations of all passes exhausted
-    fin = 1;
-  }
-  if (fin) {
-    k.done = 1;
-    atomicAdd(&ra.glob->ndone, 1);
-  }
+__device__ __forceinline__ void mx_resid_epi(Ctl &k, Glob *glob, const StepScalars &c,
+                                             const RedArgs &ra, double rsq, double rz) {
+  if (mx_resid_step(k, c.rsqm, c.iterm, ra, rsq, rz)) member_done(k, glob);
 }
 
 template <bool MA, bool EAGER, bool FOLD>
@@ -988,7 +762,7 @@ __global__ void __launch_bounds__(NT) k_mx_resid(DevStatic S, SysView V, DevSyst
         }
       },
       fold_if<FOLD>(ctl, [&](int m, const double *sum) {
-        if (threadIdx.x == 0) mx_resid_epi(ctl[m], S.sc[m], ra, sum[0], sum[1]);
+        if (threadIdx.x == 0) mx_resid_epi(ctl[m], ra.glob, S.sc[m], ra, sum[0], sum[1]);
       }));
 }
 __global__ void __launch_bounds__(NT) k_red_mx_resid(DevStatic S, Ctl *ctl, const double *part,
@@ -996,7 +770,7 @@ __global__ void __launch_bounds__(NT) k_red_mx_resid(DevStatic S, Ctl *ctl, cons
   member_reduce<2>(
       S, part, [&](int m) { return ctl[m].done != 0; },
       [&](int m, const double *sum) {
-        if (threadIdx.x == 0) mx_resid_epi(ctl[m], S.sc[m], ra, sum[0], sum[1]);
+        if (threadIdx.x == 0) mx_resid_epi(ctl[m], ra.glob, S.sc[m], ra, sum[0], sum[1]);
       });
 }
 
@@ -1591,43 +1365,6 @@ void launch_cg_init(const Launch &l, const DevStatic &S, const DevSystem &Y, dou
   cg_init_kernel<false>(l, S, Y, P, ctl, part, ra);
   launch_chan_res64(l, S, Y, P, ctl, part);
   k_red_cg_init<<<reduce_grid(S), NT, 0, l.stream>>>(S, ctl, glob, part);
-  count_launches(1);
-}
-// Shared memory of k_cg_small for windows of up to `slots` slots (its six
-// vectors); false when that is more than a CTA can have.
-bool cg_small_fits(int slots) {
-  return size_t(slots) * 6 * sizeof(double) <= size_t(SMALL_SMEM_MAX) &&
-         slots / (TILES_PER_CTA * TILE) <= SMALL_MAX_UNITS;
-}
-void launch_cg_small(const Launch &l, const DevStatic &S, const DevSystem &Y, double *P,
-                     Ctl *ctl, Glob *glob, double *part, int max_slots, int max_units,
-                     int nmember) {
-  const size_t smem = size_t(max_slots) * 6 * sizeof(double);
-  static std::mutex mu;
-  static bool set = false;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (!set) {
-      for (const void *k : {reinterpret_cast<const void *>(k_cg_small<true, 0>),
-                            reinterpret_cast<const void *>(k_cg_small<false, 0>),
-                            reinterpret_cast<const void *>(k_cg_small<true, SMALL_CACHED>),
-                            reinterpret_cast<const void *>(k_cg_small<false, SMALL_CACHED>)})
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMALL_SMEM_MAX);
-      set = true;
-    }
-  }
-  // members of at most SMALL_CACHED passes keep their geometry in registers
-  const bool cached = max_units <= SMALL_CACHED * SMALL_UNITS;
-  if (l.may_asym && cached)
-    k_cg_small<true, SMALL_CACHED><<<nmember, SMALL_NT, smem, l.stream>>>(S, Y, P, ctl, glob,
-                                                                         part);
-  else if (l.may_asym)
-    k_cg_small<true, 0><<<nmember, SMALL_NT, smem, l.stream>>>(S, Y, P, ctl, glob, part);
-  else if (cached)
-    k_cg_small<false, SMALL_CACHED><<<nmember, SMALL_NT, smem, l.stream>>>(S, Y, P, ctl, glob,
-                                                                          part);
-  else
-    k_cg_small<false, 0><<<nmember, SMALL_NT, smem, l.stream>>>(S, Y, P, ctl, glob, part);
   count_launches(1);
 }
 template <bool F>

@@ -558,12 +558,12 @@ int64_t efdc_xm_host_waits(void);
  *   EFDC_XM_OPT_INNER_TOL (default 60, 40..75): a MIXED inner solve reduces
  *     its residual by at least 10^(-value/10) in norm before the next FP64
  *     refinement pass, where the FP64 stop needs more than that.
- *   EFDC_XM_OPT_SMALL_SOLVE (default 1): 1 runs the FP64 CG of contexts
- *     whose members are all small (up to about 4,000 slots of 32x8 tiles,
- *     e.g. basins of a few thousand cells) and have no sub-grid channels as
- *     one launch with one CTA per member, its vectors in shared memory; 0
- *     runs it as the kernels of every other context.  Both give the same
- *     results bit for bit.
+ *   EFDC_XM_OPT_SMALL_SOLVE (default 1): 1 runs the solves of contexts whose
+ *     members fit the chip (FP64: up to about 600,000 cells each; MIXED: all
+ *     members together up to about that) and have no sub-grid channels as one
+ *     launch per solve, or per run of members that fit, with the vectors in
+ *     registers; 0 runs them as the kernels of every other context.  Both give
+ *     the same results bit for bit.
  *   EFDC_XM_OPT_FOLD_REDUCE (default 1, 0..2): 2 finishes each member's CG
  *     sums (its dot products, ALPHA, BETA and stop tests) inside the kernel
  *     that forms them, in the CTA that stores the member's last partial sum;
