@@ -216,7 +216,8 @@ struct efdc_xm_ctx {
   cudaStream_t cap_stream[4] = {};  // capture streams of the nested loop bodies
   bool mx_jac = true, mx_poly = false;  // kinds of MIXED inner solve in use
   xm::SysView mxview{};  // the system the MIXED solve refines (the step's assembly, or CONGRAD's)
-  bool last_mixed = false;  // the last step ran MIXED: the scaled FP64 system is formed on request
+  bool last_mixed = false;  // the last step ran MIXED
+  bool scaled_ready = true;  // Y holds the last step's scaled FP64 system (else formed on request)
   bool sys_external = false;  // the system being solved is a caller's (efdc_xm_congrad)
   // calibration (efdc_xm_calib_*): adjoint state, step-start snapshots,
   // the CG solution of the last step, gauge gathers
@@ -651,15 +652,17 @@ int run_iters(efdc_xm_ctx *c, bool mixed, double *P, int n) {
   return EFDC_XM_OK;
 }
 
-// The scaled FP64 system of the last step (calpuv2c.f90:371-399), which a
-// MIXED step does not form itself; for downloads and FP64 kernel timing.
+// The scaled FP64 system of the last step (calpuv2c.f90:371-399), which MIXED
+// and resident solves do not form; for downloads, FP64 kernel timing and the
+// adjoint solve.
 int scaled_system(efdc_xm_ctx *c) {
   for (int m = 0; m < c->M; ++m) c->act_h[m] = 1;
   int rc = write_act(c);
   if (rc) return rc;
-  xm::launch_scale(c->L(), c->S, c->X, c->Y, c->ctl, c->act, 0, 1);
+  xm::launch_scale(c->L(), c->S, c->X, c->Y, c->ctl, c->act, 0, c->any_may_asym ? 1 : 2);
   CK(cudaGetLastError());
   c->last_mixed = false;
+  c->scaled_ready = true;
   return EFDC_XM_OK;
 }
 
@@ -731,15 +734,17 @@ xm::ResPlan res_plan(const efdc_xm_ctx *c, const ResSet &r, const ResSet::Wave &
   return xm::ResPlan{r.cta ? r.cta + w.cta0 : nullptr, c->res_part, c->res_count};
 }
 
-void launch_resident64(efdc_xm_ctx *c, const xm::Launch &l, double *P) {
+void launch_resident64(efdc_xm_ctx *c, const xm::Launch &l, const xm::SysView &V, double *P,
+                       const xm::ResEnds &ends) {
   for (const ResSet::Wave &w : c->res64.waves)
-    xm::launch_cg_res(l, c->S, c->Y, P, c->ctl, c->glob, res_plan(c, c->res64, w),
-                      c->res64.form, w.ncta);
+    xm::launch_cg_res(l, c->S, V, c->Y, P, c->ctl, c->glob, res_plan(c, c->res64, w),
+                      c->res64.form, w.ncta, ends);
 }
-void launch_resident32(efdc_xm_ctx *c, const xm::Launch &l, double *P, double fac) {
+void launch_resident32(efdc_xm_ctx *c, const xm::Launch &l, double *P, double fac,
+                       const xm::ResEnds &ends) {
   for (const ResSet::Wave &w : c->res32.waves)
     xm::launch_mx_res(l, c->S, c->mxview, c->Y, P, c->ctl, c->glob, res_plan(c, c->res32, w),
-                      c->res32.form, w.ncta, fac, inner_rel_tol(c), MAX_OUTER);
+                      c->res32.form, w.ncta, fac, inner_rel_tol(c), MAX_OUTER, ends);
 }
 
 // No arrivals counted: at the start, and after a wait that ran out.
@@ -749,11 +754,13 @@ int reset_resident(efdc_xm_ctx *c) {
   return EFDC_XM_OK;
 }
 
-int solve_fp64(efdc_xm_ctx *c, double *P) {
+// Of the system V: a resident solve's, the step's unscaled assembly or Y's
+// scaled system; the multi-kernel CG takes Y's whatever V is.
+int solve_fp64(efdc_xm_ctx *c, const xm::SysView &V, double *P) {
   const xm::Launch l = c->L();
   xm::launch_solve_reset(l, c->ctl, c->glob, c->act, c->M);
   if (resident_solve(c, false)) {  // the whole CG of each member in one launch
-    launch_resident64(c, l, P);
+    launch_resident64(c, l, V, P, xm::ResEnds{});
     CK(cudaGetLastError());
     int rc = read_ctl(c);
     if (rc) return rc;
@@ -806,7 +813,7 @@ int solve_fp64(efdc_xm_ctx *c, double *P) {
 // turns out unsymmetric (its flag is set on the device) runs Jacobi whatever
 // the choice, so the Jacobi kernels are launched too wherever that can
 // happen: a radiation boundary, or a caller's standalone system.
-int choose_inner(efdc_xm_ctx *c) {
+void choose_inner(efdc_xm_ctx *c) {
   const xm::Launch l = c->L();
   c->mx_jac = c->mx_poly = false;
   for (int m = 0; m < c->M; ++m) {
@@ -821,6 +828,8 @@ int choose_inner(efdc_xm_ctx *c) {
       if (c->mem[m].may_asym || c->sys_external) c->mx_jac = true;
     }
   }
+}
+int send_inner(efdc_xm_ctx *c) {
   return to_device(c, c->mpoly, c->mpoly_h, c->mpoly_hd, sizeof(int) * c->M);
 }
 
@@ -829,12 +838,13 @@ int choose_inner(efdc_xm_ctx *c) {
 int solve_mixed(efdc_xm_ctx *c, double *P, double factor) {
   const double fac = factor > 0 ? factor : 0.1;  // stop at fac*RSQM in FP64
   xm::launch_solve_reset(c->L(), c->ctl, c->glob, c->act, c->M);
-  if (int rc0 = choose_inner(c)) return rc0;
+  choose_inner(c);
+  if (int rc0 = send_inner(c)) return rc0;
   const xm::Launch lk = c->L();  // with the kinds in use
   xm::launch_chan_p0(lk, c->S, c->mxview, P, c->act);
   int rc = 0;
   if (resident_solve(c, true)) {
-    launch_resident32(c, lk, P, fac);
+    launch_resident32(c, lk, P, fac, xm::ResEnds{});
     CK(cudaGetLastError());
     if ((rc = read_ctl(c))) return rc;
     for (int m = 0; m < c->M; ++m) {
@@ -1904,8 +1914,8 @@ int download_batch(efdc_xm_ctx *c, efdc_xm_fields *f, bool skip_unchanged, int l
   uint32_t got = 0;
   int rc = plan_download(c, f, skip_unchanged, levels, xs, ls, &got);
   if (rc) return rc;
-  if (c->last_mixed && wants_system(f)) {
-    // a MIXED step solves from the unscaled assembly: the scaled system
+  if (!c->scaled_ready && wants_system(f)) {
+    // the solve read the unscaled assembly: the scaled system
     // (calpuv2c.f90:371-399) is formed when it is asked for
     if ((rc = scaled_system(c))) return rc;
   }
@@ -2019,24 +2029,26 @@ void take_count(long long *mark, long long *n) {
   } while (0)
 
 // The solve of one sweep, captured on level d (stream c->cap_stream[d]).
+// step: within a step's graph, whose first kernel (or the end of the sweep
+// before) has reset the members.
 cudaError_t capture_solve(efdc_xm_ctx *c, const StepPlan &pl, int d, StepGraph &sg,
-                          long long *mark, long long *mine) {
+                          long long *mark, long long *mine, bool step) {
   cudaStream_t st = c->cap_stream[d];
   xm::Launch l = c->L();
   l.stream = st;
   const int M = c->M, K = pl.iters;
   double *P = c->X.p;
+  if (!step) xm::launch_solve_reset(l, c->ctl, c->glob, c->act, M);
   if (pl.resident) {  // the loops inside the kernel
-    xm::launch_solve_reset(l, c->ctl, c->glob, c->act, M);
+    const xm::ResEnds ends{step ? c->act : nullptr, step && !c->any_may_asym ? 1 : 0};
     if (pl.mixed)
-      launch_resident32(c, l, P, pl.fac);
+      launch_resident32(c, l, P, pl.fac, ends);
     else
-      launch_resident64(c, l, P);
+      launch_resident64(c, l, c->mxview, P, ends);
     take_count(mark, mine);
     return cudaGetLastError();
   }
   if (!pl.mixed) {
-    xm::launch_solve_reset(l, c->ctl, c->glob, c->act, M);
     xm::launch_cg_init(l, c->S, c->Y, P, c->ctl, c->glob, c->part);
     cudaGraphConditionalHandle h;
     CKG(cond_handle(st, &h));
@@ -2054,7 +2066,6 @@ cudaError_t capture_solve(efdc_xm_ctx *c, const StepPlan &pl, int d, StepGraph &
     take_count(mark, mine);
     return cudaGetLastError();
   }
-  xm::launch_solve_reset(l, c->ctl, c->glob, c->act, M);
   xm::launch_chan_p0(l, c->S, c->mxview, P, c->act);
   cudaGraphConditionalHandle ho, hi;
   CKG(cond_handle(st, &ho));
@@ -2085,6 +2096,22 @@ cudaError_t capture_solve(efdc_xm_ctx *c, const StepPlan &pl, int d, StepGraph &
   return end_body(lo.stream);
 }
 
+// What a step's graph reads from the host at its start, and where it leaves the
+// control blocks at its end: the mapped mirrors, in place of small copies around
+// the graph.
+bool mirrors_mapped(const efdc_xm_ctx *c) {
+  return c->ctl_hd && c->glob_hd && c->act_hd && c->mpoly_hd && c->sc_hd;
+}
+xm::StepIn step_in(const efdc_xm_ctx *c) {
+  if (!mirrors_mapped(c)) return {c->sc, c->act, c->mpoly};
+  return {static_cast<const xm::StepScalars *>(c->sc_hd), static_cast<const int *>(c->act_hd),
+          static_cast<const int *>(c->mpoly_hd)};
+}
+xm::StepOut step_out(const efdc_xm_ctx *c) {
+  if (!mirrors_mapped(c)) return {nullptr, nullptr};
+  return {static_cast<Ctl *>(c->ctl_hd), static_cast<Glob *>(c->glob_hd)};
+}
+
 // Captures the whole step into sg (the host has set the views, the swaps,
 // the scalars and the members' activity; see step_range).
 // x_pre: the state views before the time-level rotation of CALPUV9C(3), on
@@ -2102,7 +2129,7 @@ cudaError_t capture_step(efdc_xm_ctx *c, const StepPlan &pl, const xm::DevState 
   CKG(cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
   cudaError_t err = cudaSuccess;
   [&] {
-    xm::launch_step_enter(s0, c->ctl, c->act, c->glob, M);
+    xm::launch_step_enter(s0, step_in(c), c->sc, c->act, c->mpoly, c->ctl, c->glob, M);
     if (pl.istl == 0) {
       xm::launch_chan_entry(l, c->S, c->X, c->act);
       xm::launch_begin(l, c->S, c->X, c->act, !pl.all);
@@ -2114,38 +2141,44 @@ cudaError_t capture_step(efdc_xm_ctx *c, const StepPlan &pl, const xm::DevState 
       if (pl.istl == 3) xm::launch_advance3(l, c->S, c->X);
     }
     if (pl.any_isdry) xm::launch_obc_reset(l, c->S, c->B, c->X, c->act);
-    cudaGraphConditionalHandle hs;
-    if ((err = cond_handle(s0, &hs)) != cudaSuccess) return;
-    xm::launch_loop_enter(s0, c->glob, xm::LOOP_SWEEP, hs, 0, M);
-    take_count(&mark, &sg.n_top);
-    if ((err = begin_while(s0, hs, s1)) != cudaSuccess) return;
-    // the sweep body (1000 CONTINUE of calpuv2c.f90)
+    // the sweep (1000 CONTINUE of calpuv2c.f90), repeated while a member's faces
+    // change: a loop where some member has wetting and drying
+    const bool loop = pl.any_isdry;
+    cudaGraphConditionalHandle hs{};
     xm::Launch lw = l;
-    lw.stream = s1;
-    xm::launch_sweep_reset(lw, c->ctl, c->act, M);
+    if (loop) {
+      if ((err = cond_handle(s0, &hs)) != cudaSuccess) return;
+      xm::launch_loop_enter(s0, c->glob, xm::LOOP_SWEEP, hs, 0, M);
+      take_count(&mark, &sg.n_top);
+      if ((err = begin_while(s0, hs, s1)) != cudaSuccess) return;
+      lw.stream = s1;
+    }
+    long long *const n = loop ? &sg.n_body[xm::LOOP_SWEEP] : &sg.n_top;
     xm::launch_assemble(lw, c->S, c->X, c->ctl, c->act);
-    xm::launch_obc(lw, c->S, c->X, c->B, c->ctl, c->act, c->obc_serial, c->any_may_asym ? 1 : 0);
-    xm::launch_chan_sub(lw, c->S, c->X, c->ctl, c->act, -1);
-    xm::launch_scale(lw, c->S, c->X, c->Y, c->ctl, c->act, pl.mixed, c->any_may_asym ? 1 : 0);
-    if ((err = capture_solve(c, pl, 1, sg, &mark, &sg.n_body[xm::LOOP_SWEEP])) != cudaSuccess)
-      return;
+    const int cross = c->any_may_asym ? 1 : 0;
+    xm::launch_obc(lw, c->S, c->X, c->B, c->ctl, c->act, c->obc_serial, cross,
+                   cross || !pl.resident);
+    xm::launch_chan_sub(lw, c->S, c->X, c->ctl, c->act, loop ? -1 : 1);
+    if (!pl.resident) xm::launch_scale(lw, c->S, c->X, c->Y, c->ctl, c->act, pl.mixed, cross);
+    if ((err = capture_solve(c, pl, loop ? 1 : 0, sg, &mark, n, true)) != cudaSuccess) return;
     if (c->psol) {  // calibration: the adjoint needs P' before P is refreshed from HP
       if ((err = cudaMemcpyAsync(c->psol, c->X.p, size_t(c->nslot) * sizeof(double),
-                                 cudaMemcpyDeviceToDevice, s1)) != cudaSuccess)
+                                 cudaMemcpyDeviceToDevice, lw.stream)) != cudaSuccess)
         return;
     }
-    xm::launch_after_solve(s1, c->ctl, c->act, M, pl.mixed);
+    if (!pl.resident) xm::launch_after_solve(lw.stream, c->ctl, c->act, M, pl.mixed);
     xm::launch_chan_flow(lw, c->S, c->X, c->act);
     xm::launch_backsub(lw, c->S, c->X, c->act);
-    xm::launch_obc_hp(lw, c->S, c->X, c->B, c->act);
+    if (loop) xm::launch_obc_hp(lw, c->S, c->X, c->B, c->act);
     xm::launch_chan_exch(lw, c->S, c->X, c->act);
-    if (pl.any_isdry) xm::launch_wetdry(lw, c->S, c->X, c->ctl, c->act, pl.any_legacy, pl.any99);
-    xm::launch_sweep_next(s1, c->S, c->ctl, c->act, c->glob, hs, pl.max_sweeps + 1, M);
-    take_count(&mark, &sg.n_body[xm::LOOP_SWEEP]);
-    if ((err = end_body(s1)) != cudaSuccess) return;
+    if (loop) {
+      xm::launch_wetdry(lw, c->S, c->X, c->ctl, c->act, pl.any_legacy, pl.any99);
+      xm::launch_sweep_next(s1, c->S, c->ctl, c->act, c->glob, hs, pl.max_sweeps + 1, M);
+      take_count(&mark, n);
+      if ((err = end_body(s1)) != cudaSuccess) return;
+    }
     // finalisation of the members whose sweeps ended normally
-    xm::launch_fin_prepare(s0, c->ctl, c->act, M);
-    xm::launch_final(l, c->S, c->X, c->ctl, c->act, pl.any_waste);
+    xm::launch_final(l, c->S, c->X, c->ctl, nullptr, pl.any_waste, c->glob, step_out(c));
     take_count(&mark, &sg.n_top);
   }();
   cudaGraph_t g = nullptr;
@@ -2229,10 +2262,7 @@ int run_step_graph(efdc_xm_ctx *c, const StepPlan &pl, const xm::DevState &x_pre
   StepGraph *sg = step_graph(c, pl, x_pre);
   if (!sg) return -1;
   CK(cudaGraphLaunch(sg->exec, c->stream));
-  if (c->in_chunks && c->ctl_hd && c->glob_hd) {
-    xm::launch_words(c->stream, c->ctl_hd, c->ctl, sizeof(Ctl) * c->M);
-    xm::launch_words(c->stream, c->glob_hd, c->glob, sizeof(Glob));
-  } else {
+  if (!mirrors_mapped(c)) {
     CK(cudaMemcpyAsync(c->ctl_h, c->ctl, sizeof(Ctl) * c->M, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaMemcpyAsync(c->glob_h, c->glob, sizeof(Glob), cudaMemcpyDeviceToHost, c->stream));
   }
@@ -2405,7 +2435,7 @@ cudaError_t capture_solve_graph(efdc_xm_ctx *c, const StepPlan &pl, cudaGraphExe
   long long mine = 0;
   cudaError_t err = cudaStreamBeginCapture(c->cap_stream[0], cudaStreamCaptureModeThreadLocal);
   if (err != cudaSuccess) return err;
-  err = capture_solve(c, pl, 0, sg, &mark, &mine);
+  err = capture_solve(c, pl, 0, sg, &mark, &mine, false);
   cudaGraph_t g = nullptr;
   const cudaError_t e_end = cudaStreamEndCapture(c->cap_stream[0], &g);
   g_launches.fetch_sub(g_launches.load() - start);
@@ -2435,11 +2465,15 @@ int tune_time(efdc_xm_ctx *c, bool mixed, double fac, int reps, double *ms) {
   for (int m = 0; m < c->M; ++m) c->act_h[m] = 1;
   int rc = write_act(c);
   if (rc) return rc;
-  if (mixed && (rc = choose_inner(c))) return rc;
+  if (mixed) {
+    choose_inner(c);
+    if ((rc = send_inner(c))) return rc;
+  }
   const xm::Launch lk = c->L();
   StepPlan pl{};
   pl.mixed = mixed;
   pl.resident = resident_solve(c, mixed);
+  if (!mixed && !pl.resident && !c->scaled_ready && (rc = scaled_system(c))) return rc;
   pl.iters = c->graph_iters;
   pl.max_iterm = 1;
   for (int m = 0; m < c->M; ++m) pl.max_iterm = std::max(pl.max_iterm, c->sc_h[m].iterm);
@@ -2551,6 +2585,8 @@ int step_range(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_stats *stats, 
   const bool mixed = prm[0].precision == EFDC_XM_PREC_MIXED;
   c->mxview = xm::SysView{c->X.fp, c->X.cc, c->X.cs, c->X.cw, c->X.ce, c->X.cn, 1};
   c->last_mixed = mixed;
+  const bool resident = resident_solve(c, mixed);
+  c->scaled_ready = !mixed && !resident;
   c->sys_external = false;
   c->step_baro = false;
   for (int m = m0; m < m1; ++m) c->step_baro |= prm[m].bsc > 1.E-6;
@@ -2576,14 +2612,23 @@ int step_range(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_stats *stats, 
   }
   // what the step writes no longer matches the caller's arrays
   c->synced &= ~(any_isdry ? STEP_WRITES : STEP_WRITES_DRYFREE);
-  int rc = to_device(c, c->sc, c->sc_h, c->sc_hd, sizeof(xm::StepScalars) * M);
-  if (rc) return rc;
-  if (c->in_chunks)  // counters of this step (no copy engine: see to_device)
-    xm::launch_words(c->stream, c->ctl, nullptr, sizeof(Ctl) * M);
-  else
-    CK(cudaMemsetAsync(c->ctl, 0, sizeof(Ctl) * M, c->stream));
-  rc = write_act(c);
-  if (rc) return rc;
+  // the step's control blocks on the device: a graph's first kernel brings them
+  // there from the mapped mirrors
+  auto controls = [&]() -> int {
+    int r = to_device(c, c->sc, c->sc_h, c->sc_hd, sizeof(xm::StepScalars) * M);
+    if (r) return r;
+    if (c->in_chunks)  // counters of this step (no copy engine: see to_device)
+      xm::launch_words(c->stream, c->ctl, nullptr, sizeof(Ctl) * M);
+    else
+      CK(cudaMemsetAsync(c->ctl, 0, sizeof(Ctl) * M, c->stream));
+    return write_act(c);
+  };
+  int rc = 0;
+  bool sent = false;
+  if (!c->device_loops || !mirrors_mapped(c)) {
+    if ((rc = controls())) return rc;
+    sent = true;
+  }
   // the two-level advance UHDY1E=UHDYE, VHDX1E=VHDXE, H1P=HP
   // (calpuv2c.f90:256-264): a buffer swap when every member steps (then the
   // others are rewritten for every water cell before they are read), per-cell
@@ -2617,11 +2662,14 @@ int step_range(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_stats *stats, 
   }
   if (c->device_loops) {
     // the whole step as one graph, its loops on the device
-    if (mixed && (rc = choose_inner(c))) return rc;
+    if (mixed) {
+      choose_inner(c);
+      if (!mirrors_mapped(c) && (rc = send_inner(c))) return rc;
+    }
     StepPlan pl{};
     const xm::Launch lk = c->L();
     pl.mixed = mixed;
-    pl.resident = resident_solve(c, mixed);
+    pl.resident = resident;
     pl.istl = istl;
     pl.all = all;
     pl.any_isdry = any_isdry;
@@ -2661,6 +2709,7 @@ int step_range(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_stats *stats, 
       return rc;
     }
     // no graph with conditional nodes here: the host-driven step below
+    if (!sent && (rc = controls())) return rc;
   }
   if (istl == 0) {
     xm::launch_chan_entry(l, c->S, c->X, c->act);
@@ -2677,11 +2726,15 @@ int step_range(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_stats *stats, 
   for (int sweep = 0;; ++sweep) {  // 1000 CONTINUE, for the members still sweeping
     xm::launch_sweep_reset(l, c->ctl, c->act, M);
     xm::launch_assemble(l, c->S, c->X, c->ctl, c->act);
-    xm::launch_obc(l, c->S, c->X, c->B, c->ctl, c->act, c->obc_serial, c->any_may_asym ? 1 : 0);
+    xm::launch_obc(l, c->S, c->X, c->B, c->ctl, c->act, c->obc_serial, c->any_may_asym ? 1 : 0,
+                   true);
     xm::launch_chan_sub(l, c->S, c->X, c->ctl, c->act, sweep == 0 ? 1 : 0);
-    xm::launch_scale(l, c->S, c->X, c->Y, c->ctl, c->act, mixed ? 1 : 0, c->any_may_asym ? 1 : 0);
+    if (!resident)
+      xm::launch_scale(l, c->S, c->X, c->Y, c->ctl, c->act, mixed ? 1 : 0,
+                       c->any_may_asym ? 1 : 0);
     CK(cudaGetLastError());
-    rc = mixed ? solve_mixed(c, c->X.p, prm[0].mixed_rsq_factor) : solve_fp64(c, c->X.p);
+    rc = mixed ? solve_mixed(c, c->X.p, prm[0].mixed_rsq_factor)
+               : solve_fp64(c, c->mxview, c->X.p);
     if (rc) return rc;
     if ((rc = read_glob(c))) return rc;
     if (c->glob_h->err) return device_timeout(c, stats, m0, m1);
@@ -2758,7 +2811,7 @@ int step_range(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_stats *stats, 
   }
   if (any_fin) {
     if ((rc = write_act(c))) return rc;
-    xm::launch_final(l, c->S, c->X, c->ctl, c->act, any_waste);
+    xm::launch_final(l, c->S, c->X, c->ctl, c->act, any_waste, c->glob, xm::StepOut{});
     CK(cudaGetLastError());
   }
   if ((rc = read_ctl(c))) return rc;
@@ -3945,10 +3998,11 @@ int32_t efdc_xm_congrad(efdc_xm_ctx *c, const double *ccc, const double *ccs, co
   const bool mixed = precision == EFDC_XM_PREC_MIXED;
   c->mxview = xm::SysView{c->Y.fptmp, c->Y.ccc, c->Y.ccs, c->Y.ccw, c->Y.cce, c->Y.ccn, 0};
   c->last_mixed = false;
+  c->scaled_ready = true;
   c->sys_external = true;
   xm::launch_sys_prepare(c->L(), c->S, c->Y, c->ctl, mixed ? 1 : 0);
   CK(cudaGetLastError());
-  rc = mixed ? solve_mixed(c, c->X.p, 0.0) : solve_fp64(c, c->X.p);
+  rc = mixed ? solve_mixed(c, c->X.p, 0.0) : solve_fp64(c, c->mxview, c->X.p);
   if (rc) return rc;
   const Ctl k = c->ctl_h[0];
   if (k.status == EFDC_XM_DEVICE_TIMEOUT) return device_timeout(c, nullptr, 0, 0);
@@ -4165,7 +4219,7 @@ int32_t efdc_xm_time_kernels(efdc_xm_ctx *c, int32_t precision, int32_t reps, ef
   CK(cudaSetDevice(c->device));
   const xm::Launch l = c->L();
   const bool mixed = precision == EFDC_XM_PREC_MIXED;
-  if (!mixed && c->last_mixed) {
+  if (!mixed && !c->scaled_ready) {
     const int rc0 = scaled_system(c);
     if (rc0) return rc0;
   }
@@ -4486,6 +4540,7 @@ int32_t efdc_xm_calib_adjoint_step(efdc_xm_ctx *c, const efdc_xm_params *prm, in
   A.u0 = c->snap[slot][4];
   A.v0 = c->snap[slot][5];
   A.psol = c->psol;
+  if (!c->scaled_ready && (rc = scaled_system(c))) return rc;
   xm::launch_adj_pre(l, c->S, c->X, c->B, A);
   CK(cudaMemsetAsync(c->bsq, 0, sizeof(double), c->stream));
   xm::launch_adj_rhs(l, c->S, c->Y, c->ctl, A, c->bsq);
@@ -4500,7 +4555,8 @@ int32_t efdc_xm_calib_adjoint_step(efdc_xm_ctx *c, const efdc_xm_params *prm, in
                        c->stream));
     c->act_h[0] = 1;
     if ((rc = write_act(c))) return rc;
-    if ((rc = solve_fp64(c, A.lam))) return rc;
+    const xm::SysView V{c->Y.fptmp, c->Y.ccc, c->Y.ccs, c->Y.ccw, c->Y.cce, c->Y.ccn, 0};
+    if ((rc = solve_fp64(c, V, A.lam))) return rc;
     const Ctl &k = c->ctl_h[0];
     iters = k.iter;
     if (k.status == EFDC_XM_DEVICE_TIMEOUT) return device_timeout(c, nullptr, 0, 0);

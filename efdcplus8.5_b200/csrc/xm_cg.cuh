@@ -506,6 +506,59 @@ __device__ __forceinline__ void cg_update_epi(Ctl &k, Glob *glob, const StepScal
   if (cg_update_step(k, c.rsqm, c.iterm, rpcgn, rsq, no_stop)) member_done(k, glob);
 }
 
+// Whether a face of cell d with a water neighbour has two different
+// coefficients (see k_obc_asym).
+__device__ __forceinline__ bool unsymmetric_faces(const DevStatic &S, const SysView &V, int d) {
+  const Nb q = neighbours_of_slot(S.tnbr, d);
+  bool a = false;
+  if (S.kind[q.e] != LAND) a |= V.ce[d] != V.cw[q.e];
+  if (S.kind[q.w] != LAND) a |= V.cw[d] != V.ce[q.w];
+  if (S.kind[q.n] != LAND) a |= V.cn[d] != V.cs[q.n];
+  if (S.kind[q.s] != LAND) a |= V.cs[d] != V.cn[q.s];
+  return a;
+}
+
+// Start of a sweep of a member (1000 CONTINUE): its minimum diagonals and
+// flags, and its solve; a member out of the sweep is finished from the start.
+__device__ __forceinline__ void member_sweep_reset(Ctl &k, bool active) {
+  if (active) {
+    k.ccmnm_int = 1.e+18;
+    k.ccmnm_bc = 1.e+18;
+    k.asym = 0;
+    k.icordry = 0;
+  }
+  k.done = active ? 0 : 1;
+  k.idone = 0;
+  k.iter = 0;
+  k.inner_iter = 0;
+  k.outer = 0;
+  k.status = 0;
+  k.parity = 0;
+  k.beta = 0.0;
+  k.counter = 0u;
+}
+// After a solve: the member's statistics, and a member whose solve failed
+// leaves the step before its back-substitution (its status is kept).  asym:
+// the member's symmetry flags, which the solve may just have set.
+__device__ __forceinline__ void member_after_solve(Ctl &k, int &act, int asym, bool mixed) {
+  k.iters_last = k.iter;
+  k.iters_total += k.iter;
+  k.solves += 1;
+  k.rsq_last = mixed ? k.rsq64 : k.rsq;
+  k.outer_total += k.outer;
+  k.ccmnm_last = fmin(k.ccmnm_int, k.ccmnm_bc);
+  if (!k.done && k.status == 0) k.status = EFDC_XM_CG_MAXITER;
+  int st = EFDC_XM_OK;
+  if (asym & 2)
+    st = EFDC_XM_UNSUPPORTED;
+  else if (k.status != EFDC_XM_OK)
+    st = k.status;
+  if (st != EFDC_XM_OK) {
+    k.mstatus = st;
+    act = 0;
+  }
+}
+
 // MIXED inner iteration: BETA = r.z / r.z_old and the inner stop test on r.r
 // (its target, ITERM, or cap_fac*ITERM + 50 inner iterations over all passes).
 // Returns 1 when the inner solve has finished, 2 when the member has failed.

@@ -93,8 +93,23 @@ struct Glob {
   int nidone;    // members whose inner (FP32) solve finished
   int nicordry;  // members that need another wet/dry sweep
   int err;       // nonzero: a bounded device-side wait ran out (a timeout status)
+  unsigned arrive;  // arrivals of the step's last kernel (k_fin), zero at its start
   int loop[NLOOP];  // body executions of the loop now running (each loop's cap)
   int tot[NLOOP];   // body executions in the step (the launch count)
+};
+
+// What the host gives a step that runs as one graph, in its page-locked mirrors
+// (mapped: the graph's first kernel reads them), or, where those are not
+// mapped, the device arrays themselves (already copied).
+struct StepIn {
+  const StepScalars *sc;
+  const int *act, *mpoly;
+};
+// Where a step's last kernel leaves the control blocks for the host (mapped;
+// null: the host copies them).
+struct StepOut {
+  Ctl *ctl;
+  Glob *glob;
 };
 
 // Static per-slot model data (FP64).  Land slots hold element LC.

@@ -72,16 +72,23 @@ struct ResPlan {
                     // the arrivals at the end of its last launch
 };
 constexpr int RES_COUNT_STRIDE = 32;  // a 128-byte line per member
-// FP64 CONGRAD: the CTAs (clusters) of a form that can be resident at once, and
-// a launch of ncta CTAs
+// What a resident solve does at its ends besides solving.
+struct ResEnds {
+  int *act;      // not null: member_after_solve of each member, at its end
+  int check;     // open-boundary cells report an unsymmetric operator (symmetric contexts)
+};
+// FP64 CONGRAD of the system V (scaled by the member's minimum diagonal as it
+// is read where V is unscaled): the CTAs (clusters) of a form that can be
+// resident at once, and a launch of ncta CTAs
 int cg_res_capacity(const ResForm &f, bool may_asym, int nsm);
-void launch_cg_res(const Launch &l, const DevStatic &S, const DevSystem &Y, double *P, Ctl *ctl,
-                   Glob *glob, const ResPlan &R, const ResForm &f, int ncta);
-// The MIXED solve (all its refinement passes, at most max_outer)
+void launch_cg_res(const Launch &l, const DevStatic &S, const SysView &V, const DevSystem &Y,
+                   double *P, Ctl *ctl, Glob *glob, const ResPlan &R, const ResForm &f, int ncta,
+                   const ResEnds &ends);
+// The MIXED solve of V (all its refinement passes, at most max_outer)
 int mx_res_capacity(const ResForm &f, bool may_asym, int nsm);
 void launch_mx_res(const Launch &l, const DevStatic &S, const SysView &V, const DevSystem &Y,
                    double *P, Ctl *ctl, Glob *glob, const ResPlan &R, const ResForm &f, int ncta,
-                   double rsqm_fac, double rel_tol, int max_outer);
+                   double rsqm_fac, double rel_tol, int max_outer, const ResEnds &ends);
 void launch_put_int(cudaStream_t st, const int *idx, const int *val, int n, int *dst);
 // sub-grid channels (xm_chan.cu); each does nothing unless l.chan
 void launch_chan_entry(const Launch &l, const DevStatic &S, const DevState &X, const int *act);
@@ -103,7 +110,7 @@ void launch_sweep_reset(const Launch &l, Ctl *ctl, const int *act, int nmember);
 void launch_assemble(const Launch &l, const DevStatic &S, const DevState &X, Ctl *ctl,
                      const int *act);
 void launch_obc(const Launch &l, const DevStatic &S, const DevState &X, const DevObc &B, Ctl *ctl,
-                const int *act, bool serial, int write_cross);
+                const int *act, bool serial, int write_cross, bool check);
 void launch_obc_reset(const Launch &l, const DevStatic &S, const DevObc &B, const DevState &X,
                       const int *act);
 void launch_scale(const Launch &l, const DevStatic &S, const DevState &X, const DevSystem &Y,
@@ -140,8 +147,9 @@ void launch_obc_hp(const Launch &l, const DevStatic &S, const DevState &X, const
                    const int *act);
 void launch_wetdry(const Launch &l, const DevStatic &S, const DevState &X, Ctl *ctl,
                    const int *act, bool any_legacy, bool any99);
+// act null: the members the graph's sweeps left in order; out: see StepOut
 void launch_final(const Launch &l, const DevStatic &S, const DevState &X, Ctl *ctl,
-                  const int *act, bool any_waste);
+                  const int *act, bool any_waste, Glob *glob, const StepOut &out);
 void launch_reciprocals(const Launch &l, const DevStatic &S, const DevState &X, int t0, int t1);
 // the autotuner's initial guess of a timed solve: P at the last step's entry
 void launch_tune_guess(const Launch &l, const DevStatic &S, const DevState &X, double *out);
@@ -181,12 +189,12 @@ void launch_loop_enter(cudaStream_t st, Glob *g, int which, cudaGraphConditional
                        int pending, int nmember);
 void launch_loop_next(cudaStream_t st, Glob *g, int which, cudaGraphConditionalHandle h, int cap,
                       int inner, int nmember);
-void launch_step_enter(cudaStream_t st, Ctl *ctl, const int *act, Glob *g, int nmember);
+void launch_step_enter(cudaStream_t st, const StepIn &in, StepScalars *sc, int *act, int *mpoly,
+                       Ctl *ctl, Glob *g, int nmember);
 void launch_inner_done(cudaStream_t st, Ctl *ctl, const int *act, int nmember);
 void launch_after_solve(cudaStream_t st, Ctl *ctl, int *act, int nmember, int mixed);
 void launch_sweep_next(cudaStream_t st, const DevStatic &S, Ctl *ctl, int *act, Glob *g,
                        cudaGraphConditionalHandle h, int cap, int nmember);
-void launch_fin_prepare(cudaStream_t st, const Ctl *ctl, int *act, int nmember);
 
 // sets the message returned by efdc_xm_last_error() for this thread
 void set_last_error_str(const char *msg);

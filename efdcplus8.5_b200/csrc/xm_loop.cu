@@ -13,6 +13,9 @@
 // step, the sweep count and its cap) is done here too, so a step needs no
 // host synchronisation until it has finished.
 
+#include <algorithm>
+
+#include "xm_cg.cuh"
 #include "xm_kernels.h"
 
 namespace xm {
@@ -35,10 +38,40 @@ __global__ void k_loop_next(Glob *g, int which, cudaGraphConditionalHandle h, in
   cudaGraphSetConditional(h, (more && c < cap) ? 1u : 0u);
 }
 
-// Start of a step: the members taking part, the step counters of Glob.
-__global__ void k_step_enter(Ctl *ctl, const int *act, Glob *g, int nmember) {
-  for (int m = threadIdx.x; m < nmember; m += blockDim.x) ctl[m].stepping = act[m] ? 1 : 0;
-  if (threadIdx.x < NLOOP) g->tot[threadIdx.x] = 0;
+// Start of a step, and of its first sweep: the members' scalars, activity and
+// inner preconditioner from the host's mirrors, their control blocks, the
+// step's counters.  One kernel of the graph in place of four small copies
+// before it.
+__global__ void k_step_enter(StepIn in, StepScalars *sc, int *act, int *mpoly, Ctl *ctl, Glob *g,
+                             int nmember) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  const unsigned *src = reinterpret_cast<const unsigned *>(in.sc);
+  unsigned *dst = reinterpret_cast<unsigned *>(sc);
+  if (in.sc != sc)
+    for (int i = t; i < nmember * int(sizeof(StepScalars) / 4); i += nt) dst[i] = src[i];
+  for (int m = t; m < nmember; m += nt) {
+    const int a = in.act[m];
+    act[m] = a;
+    mpoly[m] = in.mpoly[m];
+    Ctl k{};
+    k.stepping = a ? 1 : 0;
+    member_sweep_reset(k, a != 0);
+    ctl[m] = k;
+  }
+  if (blockIdx.x == 0) {
+    __shared__ int out;
+    if (threadIdx.x == 0) out = 0;
+    __syncthreads();
+    for (int m = threadIdx.x; m < nmember; m += blockDim.x)
+      if (!in.act[m]) atomicAdd(&out, 1);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      g->ndone = out;
+      g->nidone = 0;
+      g->arrive = 0u;
+    }
+    if (threadIdx.x < NLOOP) g->tot[threadIdx.x] = 0;
+  }
 }
 
 // MIXED, after an inner loop: the inner iterations of the pass (those of the
@@ -52,65 +85,45 @@ __global__ void k_inner_done(Ctl *ctl, const int *act, int nmember) {
   }
 }
 
-// After a solve: the member's statistics, and a member whose solve failed
-// leaves the step before its back-substitution (its status is kept).
 __global__ void k_after_solve(Ctl *ctl, int *act, int nmember, int mixed) {
-  for (int m = threadIdx.x; m < nmember; m += blockDim.x) {
-    if (!act[m]) continue;
-    Ctl &k = ctl[m];
-    k.iters_last = k.iter;
-    k.iters_total += k.iter;
-    k.solves += 1;
-    k.rsq_last = mixed ? k.rsq64 : k.rsq;
-    k.outer_total += k.outer;
-    k.ccmnm_last = fmin(k.ccmnm_int, k.ccmnm_bc);
-    if (!k.done && k.status == 0) k.status = EFDC_XM_CG_MAXITER;
-    int st = EFDC_XM_OK;
-    if (k.asym & 2)
-      st = EFDC_XM_UNSUPPORTED;
-    else if (k.status != EFDC_XM_OK)
-      st = k.status;
-    if (st != EFDC_XM_OK) {
-      k.mstatus = st;
-      act[m] = 0;
-    }
-  }
+  for (int m = threadIdx.x; m < nmember; m += blockDim.x)
+    if (act[m]) member_after_solve(ctl[m], act[m], ctl[m].asym, mixed != 0);
 }
 
 // End of a sweep (calpuv2c.f90:597-601, 726-749): a member whose faces
 // changed sweeps again unless it has reached its cap (then its status is
-// WETDRY_MAXSWEEP); the sweep loop runs again while some member does.
+// WETDRY_MAXSWEEP); the sweep loop runs again while some member does, and
+// the members are reset for it.
 __global__ void k_sweep_next(DevStatic S, Ctl *ctl, int *act, Glob *g,
                              cudaGraphConditionalHandle h, int cap, int nmember) {
   __shared__ int any;
   if (threadIdx.x == 0) any = 0;
   __syncthreads();
   for (int m = threadIdx.x; m < nmember; m += blockDim.x) {
-    if (!act[m]) continue;
     Ctl &k = ctl[m];
-    const StepScalars &c = S.sc[m];
     int next = 0;
-    if (c.isdry > 0 && c.isdry != 98 && k.icordry) {
-      if (++k.sweep < c.max_sweeps)
-        next = 1;
-      else
-        k.mstatus = EFDC_XM_WETDRY_MAXSWEEP;
+    if (act[m]) {
+      const StepScalars &c = S.sc[m];
+      if (c.isdry > 0 && c.isdry != 98 && k.icordry) {
+        if (++k.sweep < c.max_sweeps)
+          next = 1;
+        else
+          k.mstatus = EFDC_XM_WETDRY_MAXSWEEP;
+      }
+      act[m] = next;
+      if (next) atomicAdd(&any, 1);
     }
-    act[m] = next;
-    if (next) any = 1;
   }
   __syncthreads();
+  if (any)
+    for (int m = threadIdx.x; m < nmember; m += blockDim.x) member_sweep_reset(ctl[m], act[m] != 0);
   if (threadIdx.x == 0) {
+    g->ndone = nmember - any;
+    g->nidone = 0;
     g->tot[LOOP_SWEEP] += 1;
     const int c = ++g->loop[LOOP_SWEEP];
     cudaGraphSetConditional(h, (any && c < cap) ? 1u : 0u);
   }
-}
-
-// Before the finalisation: the members whose sweeps ended normally.
-__global__ void k_fin_prepare(const Ctl *ctl, int *act, int nmember) {
-  for (int m = threadIdx.x; m < nmember; m += blockDim.x)
-    act[m] = (ctl[m].stepping && ctl[m].mstatus == EFDC_XM_OK) ? 1 : 0;
 }
 
 void launch_loop_enter(cudaStream_t st, Glob *g, int which, cudaGraphConditionalHandle h,
@@ -123,8 +136,11 @@ void launch_loop_next(cudaStream_t st, Glob *g, int which, cudaGraphConditionalH
   k_loop_next<<<1, 1, 0, st>>>(g, which, h, cap, inner, nmember);
   count_launches(1);
 }
-void launch_step_enter(cudaStream_t st, Ctl *ctl, const int *act, Glob *g, int nmember) {
-  k_step_enter<<<1, 256, 0, st>>>(ctl, act, g, nmember);
+void launch_step_enter(cudaStream_t st, const StepIn &in, StepScalars *sc, int *act, int *mpoly,
+                       Ctl *ctl, Glob *g, int nmember) {
+  const int words = nmember * int(sizeof(StepScalars) / 4);
+  k_step_enter<<<std::min(64, (words + 255) / 256), 256, 0, st>>>(in, sc, act, mpoly, ctl, g,
+                                                                 nmember);
   count_launches(1);
 }
 void launch_inner_done(cudaStream_t st, Ctl *ctl, const int *act, int nmember) {
@@ -140,9 +156,4 @@ void launch_sweep_next(cudaStream_t st, const DevStatic &S, Ctl *ctl, int *act, 
   k_sweep_next<<<1, 256, 0, st>>>(S, ctl, act, g, h, cap, nmember);
   count_launches(1);
 }
-void launch_fin_prepare(cudaStream_t st, const Ctl *ctl, int *act, int nmember) {
-  k_fin_prepare<<<1, 256, 0, st>>>(ctl, act, nmember);
-  count_launches(1);
-}
-
 }  // namespace xm

@@ -23,8 +23,9 @@ constexpr size_t res_smem64() {
 // 128 registers a thread: one row of quads keeps the coefficients in registers
 // too, two keep them in shared memory.
 template <bool MA, int W, int Q, bool CLUSTER>
-__global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1) k_cg_res(DevStatic S, DevSystem Y, double *P,
-                                                        Ctl *ctl, Glob *glob, ResPlan R) {
+__global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
+    k_cg_res(DevStatic S, SysView V, DevSystem Y, double *P, Ctl *ctl, Glob *glob, ResPlan R,
+             ResEnds ends) {
   extern __shared__ __align__(16) double dyn[];
   __shared__ ResShared<W, Q, CLUSTER> sh;
   const ResCta me = res_cta<W, Q, CLUSTER>(R, S);
@@ -50,25 +51,53 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1) k_cg_res(Dev
   bool fin;
   double v0[Q][1];
   {  // :54-88
+    // the scaling of calpuv2c.f90:371-399, as the system is read (k_scale's products)
+    const double sc = V.unscaled ? 1. / fmin(ctl[m].ccmnm_int, ctl[m].ccmnm_bc) : 1.0;
+    auto ld = [&](const double *a, int d) {
+      const V4<double> v = ld4(a + d);
+      return V4<double>{v.x * sc, v.y * sc, v.z * sc, v.w * sc};
+    };
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
       const int j = i * W + w0;
       const RowGeo g = res_geo(S, me.q0 + j, j < me.nq, row[i]);
-      r[i] = residual_row(g, S.kind, P, Y, asym);
-      x[i] = ld4(P + g.d0);
-      const V4<double> c = ld4(Y.ccc + g.d0), kw = ld4(Y.ccw + g.d0);
-      const V4<double> ci = {rcpT(c.x), rcpT(c.y), rcpT(c.z), rcpT(c.w)};
-      p[i] = {r[i].x * ci.x, r[i].y * ci.y, r[i].z * ci.z, r[i].w * ci.w};
-      C.put(i, 0, c);
-      C.put(i, 1, ld4(Y.ccs + g.d0));
-      C.put(i, 2, kw);
-      C.put(i, 3, asym ? ld4(Y.ccn + g.d0) : ld4(Y.ccs + g.dn));
+      const V4<double> X0 = ld4(P + g.d0), xn = ld4(P + g.dn), xs = ld4(P + g.ds);
+      const V4<double> b = ld(V.fp, g.d0), ks = ld(V.cs, g.d0), kw = ld(V.cw, g.d0);
+      const V4<double> kn = asym ? ld(V.cn, g.d0) : ld(V.cs, g.dn);
+      V4<double> c = ld(V.cc, g.d0);
+      const uchar4 kd = *reinterpret_cast<const uchar4 *>(S.kind + g.d0);
+      double xw = from_west(X0), xe = from_east(X0);
       kwe[i] = from_east(kw);
-      if (east) kwe[i] = Y.ccw[g.dee];
-      if constexpr (MA)
-        C.put(i, 4, asym ? ld4(Y.cce + g.d0) : V4<double>{kw.y, kw.z, kw.w, kwe[i]});
-      else
-        C.put(i, 4, ci);
+      if (west) xw = P[g.dwe];
+      if (east) {
+        xe = P[g.dee];
+        kwe[i] = V.cw[g.dee] * sc;
+      }
+      const V4<double> ke = asym ? ld(V.ce, g.d0) : V4<double>{kw.y, kw.z, kw.w, kwe[i]};
+      // land slots are inert: CCC = 1, r = 0
+      if (kd.x == LAND) c.x = 1.;
+      if (kd.y == LAND) c.y = 1.;
+      if (kd.z == LAND) c.z = 1.;
+      if (kd.w == LAND) c.w = 1.;
+      V4<double> d;
+      d.x = b.x - c.x * X0.x - kn.x * xn.x - ks.x * xs.x - kw.x * xw - ke.x * X0.y;
+      d.y = b.y - c.y * X0.y - kn.y * xn.y - ks.y * xs.y - kw.y * X0.x - ke.y * X0.z;
+      d.z = b.z - c.z * X0.z - kn.z * xn.z - ks.z * xs.z - kw.z * X0.y - ke.z * X0.w;
+      d.w = b.w - c.w * X0.w - kn.w * xn.w - ks.w * xs.w - kw.w * X0.z - ke.w * xe;
+      if (kd.x == LAND) d.x = 0.;
+      if (kd.y == LAND) d.y = 0.;
+      if (kd.z == LAND) d.z = 0.;
+      if (kd.w == LAND) d.w = 0.;
+      res_check_faces(S, V, ctl[m], row[i], kd, ends);
+      r[i] = d;
+      x[i] = X0;
+      const V4<double> ci = {rcpT(c.x), rcpT(c.y), rcpT(c.z), rcpT(c.w)};
+      p[i] = {d.x * ci.x, d.y * ci.y, d.z * ci.z, d.w * ci.w};
+      C.put(i, 0, c);
+      C.put(i, 1, ks);
+      C.put(i, 2, kw);
+      C.put(i, 3, kn);
+      C.put(i, 4, MA ? ke : ci);
       st_border(Y.z, row[i], p[i]);
       st_border(Y.pa, row[i], p[i]);
       v0[i][0] = row[i].valid ? r[i].x * p[i].x + r[i].y * p[i].y + r[i].z * p[i].z +
@@ -200,6 +229,7 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1) k_cg_res(Dev
     o.status = k.status;
     o.parity = k.parity;
     member_done(o, glob);
+    if (ends.act) member_after_solve(o, ends.act[m], atomicOr(&o.asym, 0), false);
     if (!CLUSTER) R.count[size_t(m) * RES_COUNT_STRIDE + 1] = bar.count;
   }
 }
@@ -216,17 +246,18 @@ int cg_res_capacity(const ResForm &f, bool may_asym, int nsm) {
   return cap;
 }
 
-void launch_cg_res(const Launch &l, const DevStatic &S, const DevSystem &Y, double *P, Ctl *ctl,
-                   Glob *glob, const ResPlan &R, const ResForm &f, int ncta) {
+void launch_cg_res(const Launch &l, const DevStatic &S, const SysView &V, const DevSystem &Y,
+                   double *P, Ctl *ctl, Glob *glob, const ResPlan &R, const ResForm &f, int ncta,
+                   const ResEnds &ends) {
   res_form(f, [&](auto w, auto q, auto cl) {
     constexpr int W = decltype(w)::value, Q = decltype(q)::value;
     constexpr bool CL = decltype(cl)::value;
     if (l.may_asym)
       launch_resident(k_cg_res<true, W, Q, CL>, ncta, NT * W, res_smem64<W, Q>(), f.cluster,
-                      l.stream, S, Y, P, ctl, glob, R);
+                      l.stream, S, V, Y, P, ctl, glob, R, ends);
     else
       launch_resident(k_cg_res<false, W, Q, CL>, ncta, NT * W, res_smem64<W, Q>(), f.cluster,
-                      l.stream, S, Y, P, ctl, glob, R);
+                      l.stream, S, V, Y, P, ctl, glob, R, ends);
   });
   count_launches(1);
 }

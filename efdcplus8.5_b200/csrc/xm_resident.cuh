@@ -208,12 +208,17 @@ __device__ __forceinline__ bool res_exchange(const ResPlan &R, const DevStatic &
       }
     }
     if (__syncthreads_or(dead)) return false;
+    // reduce_partials: thread i adds partials i, i + 256, ... (the first before the
+    // halo's loads, which may queue behind it)
+    const bool red = t < NT;
+    double2 first = make_double2(0.0, 0.0);
+    if (red && t < c.nqm) first = __ldcg(part + c.qm0 + t);
     halo();
-    if (t < NT) {  // reduce_partials: thread i adds partials i, i + 256, ...
+    if (red) {
       double z[NS];
-#pragma unroll
-      for (int s = 0; s < NS; ++s) z[s] = 0.0;
-      for (int i = t; i < c.nqm; i += NT) {
+      z[0] = 0.0 + first.x;
+      if constexpr (NS > 1) z[1] = 0.0 + first.y;
+      for (int i = t + NT; i < c.nqm; i += NT) {
         const double2 a = __ldcg(part + c.qm0 + i);
         z[0] += a.x;
         if constexpr (NS > 1) z[1] += a.y;
@@ -235,6 +240,18 @@ __device__ __forceinline__ bool res_exchange(const ResPlan &R, const DevStatic &
     }
   }
   return true;
+}
+
+// The open-boundary cells of a row vector report an unsymmetric operator
+// (k_obc_asym's test, for contexts whose kernels assume a symmetric one).
+__device__ __forceinline__ void res_check_faces(const DevStatic &S, const SysView &V, Ctl &k,
+                                                const ResRow &r, const uchar4 &kd,
+                                                const ResEnds &ends) {
+  if (!ends.check || !r.valid) return;
+  const uint8_t kinds[CPT] = {kd.x, kd.y, kd.z, kd.w};
+#pragma unroll
+  for (int c = 0; c < CPT; ++c)
+    if (kinds[c] == OPENBC && unsymmetric_faces(S, V, r.d0 + c)) atomicOr(&k.asym, 2);
 }
 
 // A wait ran out: the step fails with a timeout status.

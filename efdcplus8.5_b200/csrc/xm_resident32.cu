@@ -38,9 +38,9 @@ constexpr size_t res_smem32() {
 // multi-kernel form, ms per MIXED step: 60x60 cells 0.33 -> 0.13, 260x250 0.35 ->
 // 0.17, 500x500 0.38 -> 0.21, 700x700 0.45 -> 0.29.
 template <bool MA, int W, int Q, bool CLUSTER>
-__global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1) k_mx_res(DevStatic S, SysView V, DevSystem Y,
-                                                        double *P, Ctl *ctl, Glob *glob,
-                                                        ResPlan R, RedArgs ra, int max_outer) {
+__global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
+    k_mx_res(DevStatic S, SysView V, DevSystem Y, double *P, Ctl *ctl, Glob *glob, ResPlan R,
+             RedArgs ra, int max_outer, ResEnds ends) {
   extern __shared__ __align__(16) float dyn32[];
   __shared__ ResShared<W, Q, CLUSTER> sh;
   const ResCta me = res_cta<W, Q, CLUSTER>(R, S);
@@ -73,13 +73,57 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1) k_mx_res(Dev
   for (int i = 0; i < Q; ++i) {
     const int j = i * W + w0;
     const RowGeo g = res_geo(S, me.q0 + j, j < me.nq, row[i]);
-    const V4<float> kw = ld4(Y.aw32 + g.d0);
-    C.put(i, 0, ld4(Y.as32 + g.d0));
-    C.put(i, 1, kw);
-    C.put(i, 2, asym ? ld4(Y.an32 + g.d0) : ld4(Y.as32 + g.dn));
-    float kwe = from_east(kw);
-    if (east) kwe = Y.aw32[g.dee];
-    C.put(i, 3, asym ? ld4(Y.ae32 + g.d0) : V4<float>{kw.y, kw.z, kw.w, kwe});
+    // the Jacobi-scaled operator, as the system is read (k_scale32's products):
+    // a coupling towards or from land is 0
+    const V4<double> cc = ld4(V.cc + g.d0), cs = ld4(V.cs + g.d0), cw = ld4(V.cw + g.d0);
+    const V4<double> cn = ld4(V.cc + g.dn), cS = ld4(V.cc + g.ds), csn = ld4(V.cs + g.dn);
+    const uchar4 kd = *reinterpret_cast<const uchar4 *>(S.kind + g.d0);
+    const uchar4 kN = *reinterpret_cast<const uchar4 *>(S.kind + g.dn);
+    const uchar4 kS = *reinterpret_cast<const uchar4 *>(S.kind + g.ds);
+    auto inv4 = [](const V4<double> &c) {
+      return V4<double>{inv_sqrt_diag(c.x), inv_sqrt_diag(c.y), inv_sqrt_diag(c.z),
+                        inv_sqrt_diag(c.w)};
+    };
+    auto off = [](double c, double d, double dn, bool wet, bool wetn) {  // C(L)*D(L)*D(LN)
+      return wet && wetn ? float(mul(mul(c, d), dn)) : 0.f;
+    };
+    const V4<double> D = inv4(cc), DN = inv4(cn), DS = inv4(cS);
+    const bool wx = kd.x != LAND, wy = kd.y != LAND, wz = kd.z != LAND, ww = kd.w != LAND;
+    double dw = from_west(D), de = from_east(D), cwe = 0.;
+    // the wet flags of the cells west of the first and east of the last
+    bool wetw = __shfl_up_sync(0xffffffffu, int(ww), 1, ROWT) != 0;
+    bool wete = __shfl_down_sync(0xffffffffu, int(wx), 1, ROWT) != 0;
+    cwe = from_east(cw);
+    if (west) {
+      dw = inv_sqrt_diag(V.cc[g.dwe]);
+      wetw = S.kind[g.dwe] != LAND;
+    }
+    if (east) {
+      de = inv_sqrt_diag(V.cc[g.dee]);
+      wete = S.kind[g.dee] != LAND;
+      cwe = V.cw[g.dee];
+    }
+    const V4<float> as = {off(cs.x, D.x, DS.x, wx, kS.x != LAND), off(cs.y, D.y, DS.y, wy, kS.y != LAND),
+                          off(cs.z, D.z, DS.z, wz, kS.z != LAND), off(cs.w, D.w, DS.w, ww, kS.w != LAND)};
+    const V4<float> aw = {off(cw.x, D.x, dw, wx, wetw), off(cw.y, D.y, D.x, wy, wx),
+                          off(cw.z, D.z, D.y, wz, wy), off(cw.w, D.w, D.z, ww, wz)};
+    V4<float> an, ae;
+    if (asym) {
+      const V4<double> c1 = ld4(V.cn + g.d0), c2 = ld4(V.ce + g.d0);
+      an = {off(c1.x, D.x, DN.x, wx, kN.x != LAND), off(c1.y, D.y, DN.y, wy, kN.y != LAND),
+            off(c1.z, D.z, DN.z, wz, kN.z != LAND), off(c1.w, D.w, DN.w, ww, kN.w != LAND)};
+      ae = {off(c2.x, D.x, D.y, wx, wy), off(c2.y, D.y, D.z, wy, wz),
+            off(c2.z, D.z, D.w, wz, ww), off(c2.w, D.w, de, ww, wete)};
+    } else {  // AN(L) = AS(LN), AE(L) = AW(LE)
+      an = {off(csn.x, DN.x, D.x, kN.x != LAND, wx), off(csn.y, DN.y, D.y, kN.y != LAND, wy),
+            off(csn.z, DN.z, D.z, kN.z != LAND, wz), off(csn.w, DN.w, D.w, kN.w != LAND, ww)};
+      ae = {aw.y, aw.z, aw.w, off(cwe, de, D.w, wete, ww)};
+    }
+    C.put(i, 0, as);
+    C.put(i, 1, aw);
+    C.put(i, 2, an);
+    C.put(i, 3, ae);
+    res_check_faces(S, V, ctl[m], row[i], kd, ends);
   }
   auto fail = [&] { res_fail(ctl[m], Y.err); };
   // what the neighbour tiles hold of one or two vectors, for the next row work
@@ -329,6 +373,7 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1) k_mx_res(Dev
     t.last_inner = last_inner;
     t.inner_first = inner_first;
     if (done) member_done(t, glob);
+    if (ends.act) member_after_solve(t, ends.act[m], atomicOr(&t.asym, 0), true);
     if (!CLUSTER) R.count[size_t(m) * RES_COUNT_STRIDE + 1] = bar.count;
   }
 }
@@ -347,7 +392,7 @@ int mx_res_capacity(const ResForm &f, bool may_asym, int nsm) {
 
 void launch_mx_res(const Launch &l, const DevStatic &S, const SysView &V, const DevSystem &Y,
                    double *P, Ctl *ctl, Glob *glob, const ResPlan &R, const ResForm &f, int ncta,
-                   double rsqm_fac, double rel_tol, int max_outer) {
+                   double rsqm_fac, double rel_tol, int max_outer, const ResEnds &ends) {
   RedArgs ra{};
   ra.rsqm_fac = rsqm_fac;
   ra.rel_tol = rel_tol;
@@ -358,10 +403,10 @@ void launch_mx_res(const Launch &l, const DevStatic &S, const SysView &V, const 
     constexpr bool CL = decltype(cl)::value;
     if (l.may_asym)
       launch_resident(k_mx_res<true, W, Q, CL>, ncta, NT * W, res_smem32<W, Q>(), f.cluster,
-                      l.stream, S, V, Y, P, ctl, glob, R, ra, max_outer);
+                      l.stream, S, V, Y, P, ctl, glob, R, ra, max_outer, ends);
     else
       launch_resident(k_mx_res<false, W, Q, CL>, ncta, NT * W, res_smem32<W, Q>(), f.cluster,
-                      l.stream, S, V, Y, P, ctl, glob, R, ra, max_outer);
+                      l.stream, S, V, Y, P, ctl, glob, R, ra, max_outer, ends);
   });
   count_launches(1);
 }

@@ -128,7 +128,7 @@ __device__ __forceinline__ double fp1_cell(const DevStatic &S, const StepScalars
 __device__ __forceinline__ double assemble_cell(const DevStatic &S, const DevState &X,
                                                 const StepScalars &c, const Nb &q, double fp1,
                                                 double fuh, double fuhe, double fvh,
-                                                double fvhn) {
+                                                double fvhn, bool cross) {
   const int d = q.d;
   // the loads first (the stores below could alias them for the compiler)
   const double sub = X.sub[d], svb = X.svb[d], sube = X.sub[q.e], svbn = X.svb[q.n];
@@ -147,8 +147,10 @@ __device__ __forceinline__ double assemble_cell(const DevStatic &S, const DevSta
   const double cc = c.delti * dxyp - cs - cw - ce - cn;
   X.cs[d] = cs;
   X.cw[d] = cw;
-  X.ce[d] = ce;
-  X.cn[d] = cn;
+  // a symmetric member's CE, CN are read next to its open-boundary cells only
+  // (unsymmetric_faces)
+  if (cross || S.kind[q.e] == OPENBC) X.ce[d] = ce;
+  if (cross || S.kind[q.n] == OPENBC) X.cn[d] = cn;
   X.cc[d] = cc;
   return cc;
 }
@@ -348,8 +350,8 @@ __global__ void k_sweep_reset(Ctl *ctl, const int *act, int nmember) {
 // calpuv2c.f90:306-344 (FP, CS, CW, CE, CN, CC) and the member's minimum of
 // CC over its non-open-boundary cells (:360-368; the open-boundary cells' CC
 // is replaced by SETOPENBC and enters through k_obc_*).  CC > 0 here.
-__global__ void __launch_bounds__(NT) k_assemble(DevStatic S, DevState X, int ntile, Ctl *ctl,
-                                                const int *act) {
+__global__ void __launch_bounds__(NT, 4) k_assemble(DevStatic S, DevState X, int ntile, Ctl *ctl,
+                                                const int *act, bool cross) {
   __shared__ double sh[32];
   TILE_LOOP(ntile) {
     TILE_MEMBER(S);
@@ -360,7 +362,7 @@ __global__ void __launch_bounds__(NT) k_assemble(DevStatic S, DevState X, int nt
     double mn = 1.e+18;
     if (kd != LAND) {
       const double cc = assemble_cell(S, X, c, q, X.fp1[d], X.fuhdye[d], X.fuhdye[q.e],
-                                      X.fvhdxe[d], X.fvhdxe[q.n]);
+                                      X.fvhdxe[d], X.fvhdxe[q.n], cross);
       if (kd == WATER) mn = cc;
     }
     mn = block_min(mn, sh);
@@ -371,69 +373,56 @@ __global__ void __launch_bounds__(NT) k_assemble(DevStatic S, DevState X, int nt
 // ---------------------------------------------------------------------------
 // SETOPENBC (setopenbc.f90:22-206) + SETOPENBC2 (setopenbc2.f90:17-46) for one
 // boundary cell k.  Returns CC of the cell.
+// Its loads first, one round trip for all of them: a store before a load would
+// hold the load back (the arrays could alias).  10.4 -> 8.5 us per launch (ncu).
 __device__ __forceinline__ double obc_cell(const DevStatic &S, const DevState &X,
                                            const DevObc &B, const StepScalars &c, int k, int mt) {
   const int d = B.slot[k], nb = B.nbr[k], side = B.side[k], ispb = B.ispb[k];
+  double fp = B.pser ? B.pser[k] : 0.0;
   const double D = c.deltd2, G = c.g, HDRY2 = 0.2 * c.hdry;
-  X.cc[d] = c.delti * S.dxyp[d];
-  X.cs[d] = 0.;
-  X.cw[d] = 0.;
-  X.ce[d] = 0.;
-  X.cn[d] = 0.;
-  if (!X.lopenbcdry[d]) {
-    double fp = B.pser ? B.pser[k] : 0.0;
-    for (int t = 0; t < mt; ++t) {
-      const double TC = c.cosv[t], TS = c.sinv[t];
-      fp = fp + B.pcb[k * B.mtmax + t] * TC + B.psb[k * B.mtmax + t] * TS;
-    }
+  // the boundary's face: at LEC(L) for W, LNC(L) for S, the cell's own for E, N
+  const bool u = side < 2, far = side == 0 || side == 2;
+  const int f = far ? nb : d;
+  const int dry = X.lopenbcdry[d];
+  const double h = u ? X.huc[f] : X.hvc[f], hr = u ? S.hruo[f] : S.hrvo[f];
+  const double rc = u ? rc_x(X, c, f) : rc_y(X, c, f);
+  const double fu = u ? X.fuhdye[f] : X.fvhdxe[f];
+  const double di = u ? S.dxiu[f] : S.dyiv[f], dj = u ? S.dyiu[f] : S.dxiv[f];
+  const double bd = S.belv[d], bn = S.belv[nb], dxyp = S.dxyp[d], fpn = X.fp[nb];
+  for (int t = 0; t < mt; ++t) {
+    const double TC = c.cosv[t], TS = c.sinv[t];
+    fp = fp + B.pcb[k * B.mtmax + t] * TC + B.psb[k * B.mtmax + t] * TS;
+  }
+  double cc = c.delti * dxyp, cf = 0.;  // cf: the face's coefficient of a radiation cell
+  if (!dry) {
     if (ispb == 1 || ispb == 2) {  // radiation
-      if (side == 0) {  // W, face at LEC(L)
-        const double CET = 0.5 * D * G * S.hruo[nb] * rc_x(X, c, nb) * X.huc[nb];
-        const double TMP = D * sqrt(G * X.huc[nb]) * S.dxiu[nb];
-        X.cc[d] = CET * (1. + TMP) / TMP;
-        X.ce[d] = -CET;
-        fp = CET * (2. * fp - sqrt(G * X.huc[nb]) * X.fuhdye[nb] * S.dyiu[nb] / X.huc[nb]) / TMP;
-      } else if (side == 1) {  // E, own west face
-        const double CWT = 0.5 * D * G * S.hruo[d] * rc_x(X, c, d) * X.huc[d];
-        const double TMP = D * sqrt(G * X.huc[d]) * S.dxiu[d];
-        X.cc[d] = CWT * (1. + TMP) / TMP;
-        X.cw[d] = -CWT;
-        fp = CWT * (2. * fp + sqrt(G * X.huc[d]) * X.fuhdye[d] * S.dyiu[d] / X.huc[d]) / TMP;
-      } else if (side == 2) {  // S, face at LNC(L)
-        const double CNT = 0.5 * D * G * S.hrvo[nb] * rc_y(X, c, nb) * X.hvc[nb];
-        const double TMP = D * sqrt(G * X.hvc[nb]) * S.dyiv[nb];
-        X.cc[d] = CNT * (1. + TMP) / TMP;
-        X.cn[d] = -CNT;
-        fp = CNT * (2. * fp - sqrt(G * X.hvc[nb]) * X.fvhdxe[nb] * S.dxiv[nb] / X.hvc[nb]) / TMP;
-      } else {  // N, own south face
-        const double CST = 0.5 * D * G * S.hrvo[d] * rc_y(X, c, d) * X.hvc[d];
-        const double TMP = D * sqrt(G * X.hvc[d]) * S.dyiv[d];
-        X.cc[d] = CST * (1. + TMP) / TMP;
-        X.cs[d] = -CST;
-        fp = CST * (2. * fp + sqrt(G * X.hvc[d]) * X.fvhdxe[d] * S.dxiv[d] / X.hvc[d]) / TMP;
-      }
+      const double CT = 0.5 * D * G * hr * rc * h;
+      const double TMP = D * sqrt(G * h) * di;
+      cc = CT * (1. + TMP) / TMP;
+      cf = -CT;
+      fp = far ? CT * (2. * fp - sqrt(G * h) * fu * dj / h) / TMP
+               : CT * (2. * fp + sqrt(G * h) * fu * dj / h) / TMP;
     } else {  // clamped elevation
       const double FP1G = fp / G - HDRY2;
       double CT;
-      if (FP1G < S.belv[d] || FP1G < S.belv[nb]) {
-        fp = (S.belv[d] + HDRY2) * G;
+      if (FP1G < bd || FP1G < bn) {
+        fp = (bd + HDRY2) * G;
         CT = 0.;
         X.lopenbcdry[d] = 1;
-      } else if (side == 0) {
-        CT = 0.5 * D * G * S.hruo[nb] * rc_x(X, c, nb) * X.huc[nb];
-      } else if (side == 1) {
-        CT = 0.5 * D * G * S.hruo[d] * rc_x(X, c, d) * X.huc[d];
-      } else if (side == 2) {
-        CT = 0.5 * D * G * S.hrvo[nb] * rc_y(X, c, nb) * X.hvc[nb];
       } else {
-        CT = 0.5 * D * G * S.hrvo[d] * rc_y(X, c, d) * X.hvc[d];
+        CT = 0.5 * D * G * hr * rc * h;
       }
-      X.fp[nb] = X.fp[nb] + CT * fp;
-      fp = c.delti * S.dxyp[d] * fp;
+      X.fp[nb] = fpn + CT * fp;
+      fp = c.delti * dxyp * fp;
     }
     X.fp[d] = fp;
   }
-  return X.cc[d];
+  X.cc[d] = cc;
+  X.ce[d] = side == 0 ? cf : 0.;
+  X.cw[d] = side == 1 ? cf : 0.;
+  X.cn[d] = side == 2 ? cf : 0.;
+  X.cs[d] = side == 3 ? cf : 0.;
+  return cc;
 }
 
 __device__ __forceinline__ void obc2_cell(const DevState &X, const DevObc &B, int k) {
@@ -485,7 +474,8 @@ __global__ void k_obc_reset(DevStatic S, DevObc B, DevState X, const int *act) {
 // ---------------------------------------------------------------------------
 // calpuv2c.f90:371-399: scale by the member's minimum diagonal.  CE and CN
 // are scaled only when the batch holds a possibly unsymmetric member
-// (write_cross); otherwise the CG reads CCE(L) = CCW(LE), CCN(L) = CCS(LN).
+// (write_cross = 1); otherwise the CG reads CCE(L) = CCW(LE), CCN(L) = CCS(LN),
+// and so does a download that asks for them (write_cross = 2).
 __global__ void __launch_bounds__(NT) k_scale(DevStatic S, DevState X, DevSystem Y, int ntile,
                                              Ctl *ctl, const int *act, int write_cross) {
   TILE_LOOP(ntile) {
@@ -499,9 +489,13 @@ __global__ void __launch_bounds__(NT) k_scale(DevStatic S, DevState X, DevSystem
     Y.ccw[d] = X.cw[d] * CCMNMI;
     Y.ccc[d] = X.cc[d] * CCMNMI;
     Y.fptmp[d] = X.fp[d] * CCMNMI;
-    if (write_cross) {
+    if (write_cross == 1) {
       Y.cce[d] = X.ce[d] * CCMNMI;
       Y.ccn[d] = X.cn[d] * CCMNMI;
+    } else if (write_cross == 2) {
+      const Nb q = neighbours(S.tnbr, tile, threadIdx.x);
+      Y.cce[d] = X.cw[q.e] * CCMNMI;
+      Y.ccn[d] = X.cs[q.n] * CCMNMI;
     }
   }
 }
@@ -557,14 +551,8 @@ __global__ void k_obc_asym(DevStatic S, DevState X, DevObc B, Ctl *ctl, const in
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < B.n; k += gridDim.x * blockDim.x) {
     const int m = B.member[k];
     if (!act[m]) continue;
-    const int d = B.slot[k];
-    const Nb q = neighbours_of_slot(S.tnbr, d);
-    bool a = false;
-    if (S.kind[q.e] != LAND) a |= X.ce[d] != X.cw[q.e];
-    if (S.kind[q.w] != LAND) a |= X.cw[d] != X.ce[q.w];
-    if (S.kind[q.n] != LAND) a |= X.cn[d] != X.cs[q.n];
-    if (S.kind[q.s] != LAND) a |= X.cs[d] != X.cn[q.s];
-    if (a) atomicOr(&ctl[m].asym, write_cross ? 1 : 2);
+    if (unsymmetric_faces(S, SysView{X.fp, X.cc, X.cs, X.cw, X.ce, X.cn, 1}, B.slot[k]))
+      atomicOr(&ctl[m].asym, write_cross ? 1 : 2);
   }
 }
 
@@ -822,48 +810,76 @@ __global__ void __launch_bounds__(NT) k_sys_prepare(DevStatic S, DevSystem Y, in
 
 // ---------------------------------------------------------------------------
 // calpuv2c.f90:416-437 face discharges and unit-width discharges.
-__global__ void __launch_bounds__(NT) k_backsub(DevStatic S, DevState X, int ntile,
+//
+// Back-substitution and continuity in one kernel: the continuity takes the new
+// discharges of the cell's east and north faces from the next lane (a warp is a
+// tile row) and, through shared memory, from the warp of the next row; only the
+// tile's last column and row form the neighbour tile's again from its inputs.
+// Two kernels read the discharges back from memory: 184 instead of 168 B per
+// cell and one more launch (2.5 M cells: 4 CTAs per SM 1.12 ms per MIXED step, 3 or
+// fewer 1.15; two kernels 1.16).  Open-boundary cells of members without wetting and
+// drying get their depth here (:489-490); the others' is k_obc_hp's.
+__device__ __forceinline__ double face_flow(const StepScalars &c, double sw, double f, double hr,
+                                            double rc, double h, double P, double PB) {
+  return sw * (f - c.deltd2 * hr * rc * h * (P - PB));
+}
+// UHDYE (VHDXE) of slot x, whose west (south) neighbour has elevation PB: formed
+// as its own thread does, or the ghost value a land slot holds
+__device__ __forceinline__ double flow_u(const DevStatic &S, const DevState &X,
+                                         const StepScalars &c, int x, double PB) {
+  if (S.kind[x] == LAND) return X.uhdye[x];
+  return face_flow(c, X.sub[x], X.fuhdye[x], S.hruo[x], rc_x(X, c, x), X.huc[x], X.p[x], PB);
+}
+__device__ __forceinline__ double flow_v(const DevStatic &S, const DevState &X,
+                                         const StepScalars &c, int x, double PB) {
+  if (S.kind[x] == LAND) return X.vhdxe[x];
+  return face_flow(c, X.svb[x], X.fvhdxe[x], S.hrvo[x], rc_y(X, c, x), X.hvc[x], X.p[x], PB);
+}
+__global__ void __launch_bounds__(NT, 4) k_backsub(DevStatic S, DevState X, int ntile,
                                                const int *act) {
+  __shared__ double sv[2][TILE];
+  int turn = 0;
   TILE_LOOP(ntile) {
     TILE_MEMBER(S);
     if (!act[m]) continue;
     const Nb q = neighbours(S.tnbr, tile, threadIdx.x);
     const int d = q.d;
-    if (S.kind[d] == LAND) continue;
+    const uint8_t kd = S.kind[d];
     // the loads first (the stores below could alias them for the compiler)
     const double P = X.p[d], PW = X.p[q.w], PS = X.p[q.s];
     const double sub = X.sub[d], svb = X.svb[d], fuh = X.fuhdye[d], fvh = X.fvhdxe[d];
     const double hruo = S.hruo[d], hrvo = S.hrvo[d], huc = X.huc[d], hvc = X.hvc[d];
     const double rx = rc_x(X, c, d), ry = rc_y(X, c, d), dyiu = S.dyiu[d], dxiv = S.dxiv[d];
-    const double u = sub * (fuh - c.deltd2 * hruo * rx * huc * (P - PW));
-    const double v = svb * (fvh - c.deltd2 * hrvo * ry * hvc * (P - PS));
+    const double *U = X.ub, *V = X.vb;
+    const double u1 = U[d], u1e = U[q.e], v1 = V[d], v1n = V[q.n];
+    const double hb = X.hb[d], dxyip = S.dxyip[d], qsume = X.qsume[d];
+    const bool east = (threadIdx.x & (TX - 1)) == TX - 1, north = threadIdx.x / TX == TY - 1;
+    double ue = 0., vn = 0.;
+    if (east) ue = flow_u(S, X, c, q.e, P);
+    if (north) vn = flow_v(S, X, c, q.n, P);
+    const double u = kd == LAND ? X.uhdye[d] : face_flow(c, sub, fuh, hruo, rx, huc, P, PW);
+    const double v = kd == LAND ? X.vhdxe[d] : face_flow(c, svb, fvh, hrvo, ry, hvc, P, PS);
+    sv[turn][threadIdx.x] = v;
+    const double ul = __shfl_down_sync(0xffffffffu, u, 1);
+    __syncthreads();
+    if (!east) ue = ul;
+    if (!north) vn = sv[turn][threadIdx.x + TX];
+    turn ^= 1;
+    if (kd == LAND) continue;
+    // :466-486 from H1P, UHDY1E, VHDX1E; CALPUV9C's (calpuv9c.f90:500-525) is
+    // written DELT*(Q - S/2), from H2P, UHDY2E, VHDX2E for ISTL_ = 3 (the views
+    // hb, ub, vb)
+    double hp;
+    if (c.istl == 0)
+      hp = hb + c.deltd2 * dxyip * (2. * qsume - (ue + u1e - u - u1 + vn + v1n - v - v1));
+    else
+      hp = hb + c.delt * dxyip * (qsume - 0.5 * (ue + u1e - u - u1 + vn + v1n - v - v1));
+    if (kd == OPENBC && c.isdry == 0) hp = c.gi * P - S.belv[d];
     X.uhdye[d] = u;
     X.vhdxe[d] = v;
     X.uhe[d] = u * dyiu;
     X.vhe[d] = v * dxiv;
-  }
-}
-
-// calpuv2c.f90:466-486 continuity from H1P, UHDY1E, VHDX1E; CALPUV9C's
-// (calpuv9c.f90:500-525) is written DELT*(Q - S/2), from H2P, UHDY2E, VHDX2E
-// for ISTL_ = 3 (the views hb, ub, vb).
-__global__ void __launch_bounds__(NT) k_continuity(DevStatic S, DevState X, int ntile,
-                                                  const int *act) {
-  TILE_LOOP(ntile) {
-    TILE_MEMBER(S);
-    if (!act[m]) continue;
-    const Nb q = neighbours(S.tnbr, tile, threadIdx.x);
-    const int d = q.d;
-    if (S.kind[d] == LAND) continue;
-    const double *U = X.ub, *V = X.vb;
-    if (c.istl == 0)
-      X.hp[d] = X.hb[d] + c.deltd2 * S.dxyip[d] *
-                              (2. * X.qsume[d] - (X.uhdye[q.e] + U[q.e] - X.uhdye[d] - U[d] +
-                                                  X.vhdxe[q.n] + V[q.n] - X.vhdxe[d] - V[d]));
-    else
-      X.hp[d] = X.hb[d] + c.delt * S.dxyip[d] *
-                              (X.qsume[d] - 0.5 * (X.uhdye[q.e] + U[q.e] - X.uhdye[d] - U[d] +
-                                                   X.vhdxe[q.n] + V[q.n] - X.vhdxe[d] - V[d]));
+    X.hp[d] = hp;
   }
 }
 
@@ -874,9 +890,10 @@ __global__ void k_obc_hp(DevStatic S, DevState X, DevObc B, const int *act) {
     const int m = B.member[k];
     if (!act[m]) continue;
     const StepScalars &c = S.sc[m];
+    if (c.isdry == 0) continue;  // k_backsub's
     const int d = B.slot[k];
     double hp = c.gi * X.p[d] - S.belv[d];
-    if (c.isdry > 0) {
+    {
       const double h1p = X.h1p[d];
       const int obd = X.lopenbcdry[d];
       if ((obd || (h1p < 0.9 * c.hdry && hp < h1p) || hp < 0.) && X.iscdry[d] == 0) {
@@ -1079,11 +1096,15 @@ __global__ void __launch_bounds__(NT) k_wd99_commit(DevStatic S, DevState X, int
 // ---------------------------------------------------------------------------
 // :838-889 volume wasting of isolated wet cells (ISDRY>0, NDRYSTP<0) and the
 // later H1P/QDWASTE fix-up of the wasted cells (:1003-1025).
+// act null: the members whose sweeps ended normally (a step as one graph).
+__device__ __forceinline__ bool finishes(const int *act, const Ctl *ctl, int m) {
+  return act ? act[m] != 0 : ctl[m].stepping && ctl[m].mstatus == EFDC_XM_OK;
+}
 __global__ void __launch_bounds__(NT) k_fin_waste(DevStatic S, DevState X, int ntile, Ctl *ctl,
                                                  const int *act) {
   TILE_LOOP(ntile) {
     TILE_MEMBER(S);
-    if (!act[m] || c.isdry <= 0 || c.ndrystp >= 0) continue;
+    if (!finishes(act, ctl, m) || c.isdry <= 0 || c.ndrystp >= 0) continue;
     const int NTMP = abs(c.ndrystp);
     const Nb q = neighbours(S.tnbr, tile, threadIdx.x);
     const int d = q.d;
@@ -1127,12 +1148,13 @@ __global__ void __launch_bounds__(NT) k_fin_waste(DevStatic S, DevState X, int n
 }
 
 // :893-931 final P (ISDRY=0), HU, HV, LMASKDRY; NEGDEP count (the reciprocals
-// HPI, HUI, HVI are formed when downloaded: k_reciprocals).
+// HPI, HUI, HVI are formed when downloaded: k_reciprocals).  out: the CTA that
+// arrives last leaves the control blocks in the host's mapped mirrors.
 __global__ void __launch_bounds__(NT) k_fin(DevStatic S, DevState X, int ntile, Ctl *ctl,
-                                           const int *act) {
+                                           const int *act, Glob *glob, StepOut out) {
   TILE_LOOP(ntile) {
     TILE_MEMBER(S);
-    if (!act[m]) continue;
+    if (!finishes(act, ctl, m)) continue;
     const Nb q = neighbours(S.tnbr, tile, threadIdx.x);
     const int d = q.d;
     int neg = 0, bad = 0;
@@ -1167,6 +1189,14 @@ __global__ void __launch_bounds__(NT) k_fin(DevStatic S, DevState X, int ntile, 
       if (neg) atomicAdd(&ctl[m].nneg, neg);
       if (bad) atomicAdd(&ctl[m].nnonfinite, bad);
     }
+  }
+  if (out.ctl && arrive_last(&glob->arrive)) {
+    auto words = [](void *dst, const void *src, int n) {
+      for (int i = threadIdx.x; i < n; i += NT)
+        static_cast<unsigned *>(dst)[i] = __ldcg(static_cast<const unsigned *>(src) + i);
+    };
+    words(out.ctl, ctl, S.nmember * int(sizeof(Ctl) / 4));
+    words(out.glob, glob, int(sizeof(Glob) / 4));
   }
 }
 
@@ -1281,18 +1311,20 @@ void launch_sweep_reset(const Launch &l, Ctl *ctl, const int *act, int nmember) 
 }
 void launch_assemble(const Launch &l, const DevStatic &S, const DevState &X, Ctl *ctl,
                      const int *act) {
-  k_assemble<<<cell_grid(l, k_assemble), NT, 0, l.stream>>>(S, X, l.ntile, ctl, act);
+  k_assemble<<<cell_grid(l, k_assemble), NT, 0, l.stream>>>(S, X, l.ntile, ctl, act, l.may_asym);
   count_launches(1);
 }
 void launch_obc(const Launch &l, const DevStatic &S, const DevState &X, const DevObc &B, Ctl *ctl,
-                const int *act, bool serial, int write_cross) {
+                const int *act, bool serial, int write_cross, bool check) {
   if (B.n == 0) return;
   if (serial)
     k_obc_serial<<<1, 1, 0, l.stream>>>(S, X, B, ctl, act);
   else
     k_obc_parallel<<<(B.n + NT - 1) / NT, NT, 0, l.stream>>>(S, X, B, ctl, act);
+  count_launches(1);
+  if (!check) return;
   k_obc_asym<<<(B.n + NT - 1) / NT, NT, 0, l.stream>>>(S, X, B, ctl, act, write_cross);
-  count_launches(2);
+  count_launches(1);
 }
 void launch_obc_reset(const Launch &l, const DevStatic &S, const DevObc &B, const DevState &X,
                       const int *act) {
@@ -1463,8 +1495,6 @@ void launch_mx_apply(const Launch &l, const DevStatic &S, const SysView &V, cons
 void launch_backsub(const Launch &l, const DevStatic &S, const DevState &X, const int *act) {
   k_backsub<<<cell_grid(l, k_backsub), NT, 0, l.stream>>>(S, X, l.ntile, act);
   count_launches(1);
-  k_continuity<<<l.grid, NT, 0, l.stream>>>(S, X, l.ntile, act);
-  count_launches(1);
 }
 void launch_obc_hp(const Launch &l, const DevStatic &S, const DevState &X, const DevObc &B,
                    const int *act) {
@@ -1488,12 +1518,12 @@ void launch_wetdry(const Launch &l, const DevStatic &S, const DevState &X, Ctl *
   }
 }
 void launch_final(const Launch &l, const DevStatic &S, const DevState &X, Ctl *ctl,
-                  const int *act, bool any_waste) {
+                  const int *act, bool any_waste, Glob *glob, const StepOut &out) {
   if (any_waste) {
     k_fin_waste<<<l.grid, NT, 0, l.stream>>>(S, X, l.ntile, ctl, act);
     count_launches(1);
   }
-  k_fin<<<l.grid, NT, 0, l.stream>>>(S, X, l.ntile, ctl, act);
+  k_fin<<<l.grid, NT, 0, l.stream>>>(S, X, l.ntile, ctl, act, glob, out);
   count_launches(1);
 }
 // The autotuner's initial guess for timing a solve: P at the entry of the
