@@ -14,26 +14,29 @@
 //
 // The algorithm is CONGRAD's Jacobi-preconditioned CG (congrad.f90:54-187) in
 // FP64 on the reference's own layout: cells L=2..LA in CELLMAP order with the
-// LNC/LSC/LEC/LWC neighbour maps (so periodic links work too), one thread per
-// cell, three kernels per iteration like the reference's three loops.
+// LNC/LSC/LEC/LWC neighbour maps (so periodic links work too).  One cooperative
+// launch runs the whole solve: a thread keeps its cells' P, RCG, PCG and APCG
+// in registers, the others read z = CCCI*RCG and PCG from the scratch, and the
+// two reductions of an iteration are also its barriers.
 
 #include <cstdarg>
 #include <cstdio>
 #include <mutex>
 
 #include "../../include/efdc_xm.h"
-#include "xm_common.cuh"
 #include "xm_kernels.h"
+#include "xm_resident.cuh"
 
 namespace {
 
 constexpr int NA_MAX_CELLS = EFDC_XM_NOALLOC_MAX_CELLS;  // water cells, LA-1
 constexpr int NA_LEN = ((NA_MAX_CELLS + 2 + 31) / 32) * 32;  // elements 1..LC, padded
-constexpr int NA_GRID = 296;                          // CTAs (2 per SM of a B200)
+constexpr int NA_GRID = 296;                          // partial sums: blocks of 256 threads
+constexpr int NA_HALVES = 2;                          // such blocks per CTA
 constexpr int NA_CTL = 16;                            // doubles of the control block
-constexpr size_t NA_DOUBLES = size_t(3) * NA_LEN + 2 * NA_GRID + NA_CTL;
+constexpr size_t NA_DOUBLES = size_t(3) * NA_LEN + 4 * NA_GRID + NA_CTL;
 
-// The scratch: r | p | Ap | partial sums | control block.  In host code this
+// The scratch: z | p | p (by turns) | partial sums (by turns) | control block.  In host code this
 // name is only a stand-in for the symbol; its device address comes from
 // cudaGetSymbolAddress (see scratch_ptr).
 static __device__ __align__(256) double g_na_scratch[NA_DOUBLES];
@@ -50,125 +53,188 @@ struct NaArgs {
   const int *lnc, *lsc, *lec, *lwc;
   const double *ccc, *ccs, *ccn, *ccw, *cce, *fptmp;
   double *P;
-  double *r, *p, *ap, *part;
+  double *z, *pa, *pb, *part;
   NaCtl *ctl;
 };
 
-using xm::arrive_last;
-using xm::block_sum;
 using xm::NT;
-using xm::reduce_partials;
+using xm::NWARP;
 
-// :54-88 RCG = FPTMP - A*P; PCG = RCG*CCCI; RPCG.  Also zeroes the ghost
-// elements 1 and LC of PCG (congrad.f90:42: PCG(1)=PCG(LC)=0).
-__global__ void __launch_bounds__(NT) k_na_init(NaArgs a) {
-  __shared__ double sh[32];
-  double acc = 0.0;
+constexpr int NA_NT = NA_HALVES * NT;
+
+// The sums of NS values over all blocks, in every thread, and the barrier of the
+// grid: each block of 256 threads (half a CTA) sums its values and stores them,
+// the CTA adds its arrival with release semantics and waits for the others'
+// (bounded), then sums the blocks' values as one block of 256 threads does.
+// False (in every thread) when the wait ran out.
+template <int NS>
+__device__ __forceinline__ bool na_sum(const NaArgs &a, unsigned &count, int &turn,
+                                       const double (&v)[NS], double (&out)[NS]) {
+  __shared__ double sh[NS][NA_HALVES][NWARP];
+  __shared__ double red[NS][NWARP];
+  const int t = threadIdx.x, lane = t & 31, half = t / NT, warp = (t % NT) >> 5;
+  const int nblk = gridDim.x * NA_HALVES;
+  double2 *part = reinterpret_cast<double2 *>(a.part) + turn * NA_GRID;
+  turn ^= 1;
+  auto tree = [](const double *w) {  // block_sum's last stage (its further lanes add zeros)
+    return ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
+  };
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const double x = xm::warp_sum(v[s]);
+    if (lane == 0) sh[s][half][warp] = x + 0.0;
+  }
+  __syncthreads();  // also: every thread's z or p is before the release below
+  count += gridDim.x;
+  int dead = 0;
+  if (t < 32) {
+    if (t < NA_HALVES)
+      part[blockIdx.x * NA_HALVES + t] =
+          make_double2(tree(sh[0][t]), NS > 1 ? tree(sh[NS - 1][t]) : 0.0);
+    __syncwarp();
+    if (t == 0) {
+      xm::red_release(&a.ctl->counter, 1u);
+      for (int k = 0; int(xm::ld_acquire(&a.ctl->counter) - count) < 0; ++k)
+        if (k >= xm::RES_TRIES) {
+          dead = 1;
+          break;
+        }
+    }
+  }
+  if (__syncthreads_or(dead)) return false;
+  if (t < NT) {  // reduce_partials
+    double z[NS];
+#pragma unroll
+    for (int s = 0; s < NS; ++s) z[s] = 0.0;
+    for (int i = t; i < nblk; i += NT) {
+      const double2 x = __ldcg(part + i);
+      z[0] += x.x;
+      if constexpr (NS > 1) z[1] += x.y;
+    }
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      const double x = xm::warp_sum(z[s]);
+      if (lane == 0) red[s][warp] = x + 0.0;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < NS; ++s) out[s] = tree(red[s]);
+  return true;
+}
+
+// congrad.f90:54-187 with NC cells per thread.  What bounds it is the exchange,
+// as for the resident solves (xm_resident.cuh): three kernels per iteration and a
+// copy to the host every 8 took 410 us for 16 iterations on 112,000 cells; one
+// launch takes 181 us (a call of efdc_xm_congrad_noalloc, its copy of P included).
+template <int NC>
+__global__ void __launch_bounds__(NA_NT) k_na_solve(NaArgs a, double rsqm, int iterm) {
+  const int first = 2 + int(blockIdx.x) * NA_NT + int(threadIdx.x), stride = gridDim.x * NA_NT;
+  unsigned count = 0u;
+  int turn = 0;
+  double x[NC], r[NC], p[NC], ap[NC], ci[NC];
+  if (blockIdx.x == 0 && threadIdx.x == 0)  // congrad.f90:42: PCG(1)=PCG(LC)=0
+    for (double *q : {a.z, a.pa, a.pb}) {
+      q[0] = 0.0;
+      q[a.lc - 1] = 0.0;
+    }
+  auto fail = [&] {
+    if (threadIdx.x == 0) {
+      a.ctl->status = EFDC_XM_DEVICE_TIMEOUT;
+      a.ctl->done = 1;
+    }
+  };
+  double rpcg, alpha = 0.0, beta = 0.0, rsq = 0.0;
+  int iter = 0, status = 0;
+  bool done;
+  {  // :54-88
+    double v[1] = {0.0}, sum[1];
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+      const int L = first + k * stride;
+      if (L > a.la) continue;
+      const int i = L - 1;
+      x[k] = a.P[i];
+      const double c = a.ccc[i];
+      r[k] = a.fptmp[i] - c * x[k] - a.ccn[i] * a.P[a.lnc[i] - 1] -
+             a.ccs[i] * a.P[a.lsc[i] - 1] - a.ccw[i] * a.P[a.lwc[i] - 1] -
+             a.cce[i] * a.P[a.lec[i] - 1];
+      ci[k] = 1. / c;
+      p[k] = r[k] * ci[k];
+      a.z[i] = p[k];
+      a.pa[i] = p[k];
+      v[0] += r[k] * p[k];
+    }
+    if (!na_sum(a, count, turn, v, sum)) return fail();
+    rpcg = sum[0];
+    if (!isfinite(rpcg)) status = EFDC_XM_NONFINITE;
+    done = rpcg == 0.0 || !isfinite(rpcg);
+  }
+  while (!done) {  // ITERM bounds the loop
+    const double *pold = iter & 1 ? a.pb : a.pa;
+    double *pnew = iter & 1 ? a.pa : a.pb;
+    {  // :151-162 of the iteration before, :107-125
+      double v[1] = {0.0}, sum[1];
+#pragma unroll
+      for (int k = 0; k < NC; ++k) {
+        const int L = first + k * stride;
+        if (L > a.la) continue;
+        const int i = L - 1;
+        auto at = [&](int n) { return __ldcg(a.z + n) + beta * __ldcg(pold + n); };
+        const double ps = at(__ldg(a.lsc + i) - 1), pn = at(__ldg(a.lnc + i) - 1),
+                     pw = at(__ldg(a.lwc + i) - 1), pe = at(__ldg(a.lec + i) - 1);
+        p[k] = ci[k] * r[k] + beta * p[k];
+        pnew[i] = p[k];
+        ap[k] = __ldg(a.ccc + i) * p[k] + __ldg(a.ccs + i) * ps + __ldg(a.ccn + i) * pn +
+                __ldg(a.ccw + i) * pw + __ldg(a.cce + i) * pe;
+        v[0] += ap[k] * p[k];
+      }
+      if (!na_sum(a, count, turn, v, sum)) return fail();
+      alpha = rpcg / sum[0];
+    }
+    {  // :127-149
+      double v[2] = {0.0, 0.0}, sum[2];
+#pragma unroll
+      for (int k = 0; k < NC; ++k) {
+        const int L = first + k * stride;
+        if (L > a.la) continue;
+        x[k] = x[k] + alpha * p[k];
+        r[k] = r[k] - alpha * ap[k];
+        const double z = ci[k] * r[k];
+        a.z[L - 1] = z;
+        v[0] += r[k] * z;
+        v[1] += r[k] * r[k];
+      }
+      if (!na_sum(a, count, turn, v, sum)) return fail();
+      beta = sum[0] / rpcg;
+      rpcg = sum[0];
+      rsq = sum[1];
+    }
+    ++iter;
+    if (!isfinite(rsq) || !isfinite(alpha)) {
+      status = EFDC_XM_NONFINITE;
+      done = true;
+    } else if (rsq <= rsqm) {
+      done = true;
+    } else if (iter >= iterm) {
+      status = EFDC_XM_CG_MAXITER;
+      done = true;
+    }
+  }
+  if (iter > 0)
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+      const int L = first + k * stride;
+      if (L <= a.la) a.P[L - 1] = x[k];
+    }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    a.p[0] = 0.0;
-    a.p[a.lc - 1] = 0.0;
-  }
-  for (int L = 2 + blockIdx.x * NT + threadIdx.x; L <= a.la; L += gridDim.x * NT) {
-    const int i = L - 1;
-    const double r = a.fptmp[i] - a.ccc[i] * a.P[i] - a.ccn[i] * a.P[a.lnc[i] - 1] -
-                     a.ccs[i] * a.P[a.lsc[i] - 1] - a.ccw[i] * a.P[a.lwc[i] - 1] -
-                     a.cce[i] * a.P[a.lec[i] - 1];
-    const double z = r * (1. / a.ccc[i]);
-    a.r[i] = r;
-    a.p[i] = z;
-    acc += r * z;
-  }
-  acc = block_sum(acc, sh);
-  if (threadIdx.x == 0) a.part[blockIdx.x] = acc;
-  if (arrive_last(&a.ctl->counter)) {
-    const double rpcg = reduce_partials<>(a.part, gridDim.x, sh);
-    if (threadIdx.x == 0) {
-      a.ctl->rpcg = rpcg;
-      a.ctl->iter = 0;
-      a.ctl->status = 0;
-      a.ctl->done = (rpcg == 0.0) ? 1 : 0;
-      if (!isfinite(rpcg)) {
-        a.ctl->done = 1;
-        a.ctl->status = EFDC_XM_NONFINITE;
-      }
-      a.ctl->counter = 0;
-    }
-  }
-}
-
-// :107-125 APCG and ALPHA
-__global__ void __launch_bounds__(NT) k_na_matvec(NaArgs a) {
-  __shared__ double sh[32];
-  if (a.ctl->done) return;
-  double acc = 0.0;
-  for (int L = 2 + blockIdx.x * NT + threadIdx.x; L <= a.la; L += gridDim.x * NT) {
-    const int i = L - 1;
-    const double p = a.p[i];
-    const double ap = a.ccc[i] * p + a.ccs[i] * a.p[a.lsc[i] - 1] + a.ccn[i] * a.p[a.lnc[i] - 1] +
-                      a.ccw[i] * a.p[a.lwc[i] - 1] + a.cce[i] * a.p[a.lec[i] - 1];
-    a.ap[i] = ap;
-    acc += ap * p;
-  }
-  acc = block_sum(acc, sh);
-  if (threadIdx.x == 0) a.part[blockIdx.x] = acc;
-  if (arrive_last(&a.ctl->counter)) {
-    const double papcg = reduce_partials<>(a.part, gridDim.x, sh);
-    if (threadIdx.x == 0) {
-      a.ctl->alpha = a.ctl->rpcg / papcg;
-      a.ctl->counter = 0;
-    }
-  }
-}
-
-// :127-149 P, RCG, RPCGN, RSQ, BETA and the stop test
-__global__ void __launch_bounds__(NT) k_na_update(NaArgs a, double rsqm, int iterm) {
-  __shared__ double sh[32];
-  if (a.ctl->done) return;
-  const double alpha = a.ctl->alpha;
-  double a1 = 0.0, a2 = 0.0;
-  for (int L = 2 + blockIdx.x * NT + threadIdx.x; L <= a.la; L += gridDim.x * NT) {
-    const int i = L - 1;
-    a.P[i] = a.P[i] + alpha * a.p[i];
-    const double r = a.r[i] - alpha * a.ap[i];
-    a.r[i] = r;
-    const double z = (1. / a.ccc[i]) * r;
-    a1 += r * z;
-    a2 += r * r;
-  }
-  a1 = block_sum(a1, sh);
-  if (threadIdx.x == 0) a.part[blockIdx.x] = a1;
-  a2 = block_sum(a2, sh);
-  if (threadIdx.x == 0) a.part[gridDim.x + blockIdx.x] = a2;
-  if (arrive_last(&a.ctl->counter)) {
-    const double rpcgn = reduce_partials<>(a.part, gridDim.x, sh);
-    const double rsq = reduce_partials<>(a.part + gridDim.x, gridDim.x, sh);
-    if (threadIdx.x == 0) {
-      a.ctl->beta = rpcgn / a.ctl->rpcg;
-      a.ctl->rpcg = rpcgn;
-      a.ctl->rsq = rsq;
-      const int it = a.ctl->iter + 1;
-      a.ctl->iter = it;
-      if (!isfinite(rsq) || !isfinite(a.ctl->alpha)) {
-        a.ctl->done = 1;
-        a.ctl->status = EFDC_XM_NONFINITE;
-      } else if (rsq <= rsqm) {
-        a.ctl->done = 1;
-      } else if (it >= iterm) {
-        a.ctl->done = 1;
-        a.ctl->status = EFDC_XM_CG_MAXITER;
-      }
-      a.ctl->counter = 0;
-    }
-  }
-}
-
-// :151-162 PCG = TMPCG + BETA*PCG
-__global__ void __launch_bounds__(NT) k_na_pupdate(NaArgs a) {
-  if (a.ctl->done) return;
-  const double beta = a.ctl->beta;
-  for (int L = 2 + blockIdx.x * NT + threadIdx.x; L <= a.la; L += gridDim.x * NT) {
-    const int i = L - 1;
-    a.p[i] = (1. / a.ccc[i]) * a.r[i] + beta * a.p[i];
+    a.ctl->rpcg = rpcg;
+    a.ctl->alpha = alpha;
+    a.ctl->beta = beta;
+    a.ctl->rsq = rsq;
+    a.ctl->iter = iter;
+    a.ctl->status = status;
+    a.ctl->done = 1;
   }
 }
 
@@ -252,39 +318,38 @@ int32_t efdc_xm_congrad_noalloc(int32_t la, const int32_t *lnc, const int32_t *l
   a.cce = cce;
   a.fptmp = fptmp;
   a.P = p;
-  a.r = base;
-  a.p = base + NA_LEN;
-  a.ap = base + 2 * size_t(NA_LEN);
+  a.z = base;
+  a.pa = base + NA_LEN;
+  a.pb = base + 2 * size_t(NA_LEN);
   a.part = base + 3 * size_t(NA_LEN);
-  a.ctl = reinterpret_cast<NaCtl *>(base + 3 * size_t(NA_LEN) + 2 * NA_GRID);
-  const int grid = std::max(1, std::min(NA_GRID, (la - 1 + NT - 1) / NT));
+  a.ctl = reinterpret_cast<NaCtl *>(base + 3 * size_t(NA_LEN) + 4 * NA_GRID);
+  // one CTA per SM of a B200 at most: the exchange is the cheaper the fewer there are
+  const int grid = std::max(1, std::min(NA_GRID / NA_HALVES, (la - 1 + NA_NT - 1) / NA_NT));
   // the control block keeps the previous call's contents: start from zero
   auto fail = [&](cudaError_t err, const char *what) {
     na_error("efdc_xm_congrad_noalloc: %s: %s", what, cudaGetErrorString(err));
     return EFDC_XM_CUDA_ERROR;
   };
   if ((e = cudaMemsetAsync(a.ctl, 0, sizeof(NaCtl), st)) != cudaSuccess) return fail(e, "memset");
-  k_na_init<<<grid, NT, 0, st>>>(a);
-  if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "launch");
+  const int nc = (la - 1 + grid * NA_NT - 1) / (grid * NA_NT);
+  static_assert((NA_MAX_CELLS + NA_GRID * NT - 1) / (NA_GRID * NT) <= 8, "cells per thread");
+  const void *kernel = nc <= 1   ? reinterpret_cast<const void *>(k_na_solve<1>)
+                       : nc <= 2 ? reinterpret_cast<const void *>(k_na_solve<2>)
+                       : nc <= 4 ? reinterpret_cast<const void *>(k_na_solve<4>)
+                                 : reinterpret_cast<const void *>(k_na_solve<8>);
+  void *args[] = {&a, &rsqm, &iterm};
+  if ((e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(NA_NT), args, 0, st)) !=
+      cudaSuccess)
+    return fail(e, "launch");
   NaCtl h{};
-  int launched = 0;
-  while (launched < iterm) {
-    const int chunk = std::min(8, iterm - launched);
-    for (int k = 0; k < chunk; ++k) {
-      k_na_matvec<<<grid, NT, 0, st>>>(a);
-      k_na_update<<<grid, NT, 0, st>>>(a, rsqm, iterm);
-      k_na_pupdate<<<grid, NT, 0, st>>>(a);
-    }
-    launched += chunk;
-    if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "launch");
-    if ((e = cudaMemcpyAsync(&h, a.ctl, sizeof(NaCtl), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
-      return fail(e, "copy of the control block");
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return fail(e, "synchronize");
-    if (h.done) break;
-  }
+  if ((e = cudaMemcpyAsync(&h, a.ctl, sizeof(NaCtl), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
+    return fail(e, "copy of the control block");
+  if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return fail(e, "synchronize");
   if (iters) *iters = h.iter;
   if (rsq) *rsq = h.rsq;
-  if (!h.done) return EFDC_XM_CG_MAXITER;
+  if (h.status == EFDC_XM_DEVICE_TIMEOUT)
+    na_error("efdc_xm_congrad_noalloc: a bounded device-side wait ran out; the result is not "
+             "valid");
   if (h.status == EFDC_XM_CG_MAXITER)
     na_error("efdc_xm_congrad_noalloc: maximum iterations exceeded (RSQ=%g)", h.rsq);
   if (h.status == EFDC_XM_NONFINITE)

@@ -638,10 +638,11 @@ int32_t efdc_xm_time_kernels(efdc_xm_ctx *ctx, int32_t precision, int32_t reps,
  *   - all calls share the array: calls that overlap on the GPU (other
  *     streams, other host threads) race; the call returns after its work on
  *     `stream` (a cudaStream_t, NULL = legacy default stream) finished;
- *   - every call reads its stop test back to the host: it copies the control
- *     block to host memory and synchronizes `stream` after every 8
- *     iterations, so it must not be called while a stream capture is active
- *     (on `stream` or, in global capture mode, anywhere in the process). */
+ *   - a call is one cooperative launch of up to 148 CTAs that wait on one
+ *     another (bounded: EFDC_XM_DEVICE_TIMEOUT); it copies its control block to
+ *     host memory and synchronizes `stream`, so it must not be called while a
+ *     stream capture is active (on `stream` or, in global capture mode, anywhere
+ *     in the process). */
 #define EFDC_XM_NOALLOC_MAX_CELLS 524288
 int32_t efdc_xm_congrad_noalloc(int32_t la, const int32_t *lnc, const int32_t *lsc,
                                 const int32_t *lec, const int32_t *lwc, const double *ccc,
