@@ -686,14 +686,17 @@ bool resident_solve(const efdc_xm_ctx *c, bool mixed) {
 // the first form that holds every member at once, or, up to max_waves, the
 // last in as few launches as that takes.  Several launches, one after another,
 // are still faster than the multi-kernel CG in FP64 (24 basins of 2.5 M cells:
-// 1.60 against 1.72 ms per step) and slower in MIXED (1.29 against 1.16 ms).
+// 1.46 against 1.72 ms per step) and slower in MIXED (1.29 against 1.16 ms).  Four
+// rows of quads exist in FP64 only: of the same form in MIXED, a basin of 770,000
+// cells took 0.50 ms against the multi-kernel CG's 0.49, one of a million 0.53
+// against 0.56.
 bool build_resident(efdc_xm_ctx *c, int (*capacity)(const xm::ResForm &, bool, int),
                     size_t max_waves, ResSet &out) {
   const int M = c->M, mq = c->max_units;
   auto cap_of = [&](const xm::ResForm &f) {
     return std::min(capacity(f, false, c->nsm), capacity(f, true, c->nsm));
   };
-  constexpr xm::ResForm forms[] = {{1, 1, 0}, {2, 1, 0}, {2, 2, 0}};
+  constexpr xm::ResForm forms[] = {{1, 1, 0}, {2, 1, 0}, {2, 2, 0}, {2, 4, 0}};
   for (xm::ResForm f : forms) {
     const int per = f.w * f.q, n = (mq + per - 1) / per;
     if (n > 16) continue;

@@ -6,9 +6,15 @@
 
 namespace xm {
 
+// What a form keeps where.  One row of quads: the coefficients in registers.  Two:
+// in shared memory.  Four (the lean form): P and PCG live in shared memory too --
+// PCG where the rows above and below read it anyway --, CCCI as well, and the
+// other coefficients are read and scaled anew (24 of the 112 B per cell-iteration
+// of the multi-kernel CG, from L2).
+__host__ __device__ constexpr bool res_lean(int Q) { return Q == 4; }
 constexpr int RES_NC = 5;  // CCC, CCS, CCW, CCN and CCCI (symmetric) or CCE (MA)
 template <int W, int Q>
-using Coef64 = ResCoef<double, W, Q, RES_NC, Q == 1>;
+using Coef64 = ResCoef<double, W, Q, res_lean(Q) ? 2 : RES_NC, Q == 1>;  // lean: CCCI, P
 template <int W, int Q>
 constexpr size_t res_smem64() {
   return size_t(W) * Q * TILES_PER_CTA * TILE * sizeof(double) + Coef64<W, Q>::bytes;
@@ -19,9 +25,11 @@ constexpr size_t res_smem64() {
 // Measured against the multi-kernel CG with folded reductions (one CTA per
 // member before, for members of up to 4,000 slots), ms per step, device-resident:
 // 60x60 cells 0.35 -> 0.13, 260x250 0.36 -> 0.17, 500x500 0.45 -> 0.24, 700x700
-// 0.57 -> 0.34, 256 lakes of 1,100 cells in one batch 0.50 -> 0.38.
+// 0.57 -> 0.33, 256 lakes of 1,100 cells in one batch 0.50 -> 0.38; lean: 900x860
+// 0.65 -> 0.49, 1,000x1,000 0.80 -> 0.56 (an iteration 31 -> 20 us, of which the row
+// work is 13, the exchanges' waits for the slowest CTA 3 and the exchanges 4).
 // 128 registers a thread: one row of quads keeps the coefficients in registers
-// too, two keep them in shared memory.
+// too, two keep them in shared memory, four read them (see res_lean).
 template <bool MA, int W, int Q, bool CLUSTER>
 __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
     k_cg_res(DevStatic S, SysView V, DevSystem Y, double *P, Ctl *ctl, Glob *glob, ResPlan R,
@@ -43,20 +51,45 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
   const int w0 = W > 1 ? int(threadIdx.x) / NT : 0;  // quad q0 + i*W + w0 is the thread's row i
   auto none = [] {};
 
+  constexpr bool LEAN = res_lean(Q);
   ResRow row[Q];
-  V4<double> x[Q], r[Q], p[Q], ap[Q];
-  double kwe[Q];  // symmetric: CCW of the cell east of the row vector
+  V4<double> xr[LEAN ? 1 : Q] = {}, pr[LEAN ? 1 : Q] = {};  // (the registers of the other forms)
+  V4<double> r[Q], ap[Q];
+  double kwe[LEAN ? 1 : Q];  // symmetric: CCW of the cell east of the row vector
+  auto get_x = [&](int i) {
+    if constexpr (LEAN)
+      return C.get(i, 1);
+    else
+      return xr[i];
+  };
+  auto put_x = [&](int i, const V4<double> &v) {
+    if constexpr (LEAN)
+      C.put(i, 1, v);
+    else
+      xr[i] = v;
+  };
+  auto get_p = [&](int i) {
+    if constexpr (LEAN)
+      return ld_stage(res_stage<W>(stage, i));
+    else
+      return pr[i];
+  };
+  auto put_p = [&](int i, const V4<double> &v) {
+    st_stage(res_stage<W>(stage, i), v);
+    if constexpr (!LEAN) pr[i] = v;
+  };
   Ctl k;  // of it: rpcg, papcg, alpha, beta, rsq, iter, status, parity
   k.alpha = 0.0;
   bool fin;
   double v0[Q][1];
+  // the scaling of calpuv2c.f90:371-399, as the system is read (k_scale's products)
+  const double sc = V.unscaled ? 1. / fmin(ctl[m].ccmnm_int, ctl[m].ccmnm_bc) : 1.0;
+  auto ld = [&](const double *a, int d) {
+    const V4<double> v = ld4(a + d);
+    return V4<double>{v.x * sc, v.y * sc, v.z * sc, v.w * sc};
+  };
+  unsigned land = 0;  // lean: a bit per cell of the rows
   {  // :54-88
-    // the scaling of calpuv2c.f90:371-399, as the system is read (k_scale's products)
-    const double sc = V.unscaled ? 1. / fmin(ctl[m].ccmnm_int, ctl[m].ccmnm_bc) : 1.0;
-    auto ld = [&](const double *a, int d) {
-      const V4<double> v = ld4(a + d);
-      return V4<double>{v.x * sc, v.y * sc, v.z * sc, v.w * sc};
-    };
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
       const int j = i * W + w0;
@@ -67,13 +100,13 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
       V4<double> c = ld(V.cc, g.d0);
       const uchar4 kd = *reinterpret_cast<const uchar4 *>(S.kind + g.d0);
       double xw = from_west(X0), xe = from_east(X0);
-      kwe[i] = from_east(kw);
+      double kwee = from_east(kw);
       if (west) xw = P[g.dwe];
       if (east) {
         xe = P[g.dee];
-        kwe[i] = V.cw[g.dee] * sc;
+        kwee = V.cw[g.dee] * sc;
       }
-      const V4<double> ke = asym ? ld(V.ce, g.d0) : V4<double>{kw.y, kw.z, kw.w, kwe[i]};
+      const V4<double> ke = asym ? ld(V.ce, g.d0) : V4<double>{kw.y, kw.z, kw.w, kwee};
       // land slots are inert: CCC = 1, r = 0
       if (kd.x == LAND) c.x = 1.;
       if (kd.y == LAND) c.y = 1.;
@@ -90,44 +123,57 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
       if (kd.w == LAND) d.w = 0.;
       res_check_faces(S, V, ctl[m], row[i], kd, ends);
       r[i] = d;
-      x[i] = X0;
       const V4<double> ci = {rcpT(c.x), rcpT(c.y), rcpT(c.z), rcpT(c.w)};
-      p[i] = {d.x * ci.x, d.y * ci.y, d.z * ci.z, d.w * ci.w};
-      C.put(i, 0, c);
-      C.put(i, 1, ks);
-      C.put(i, 2, kw);
-      C.put(i, 3, kn);
-      C.put(i, 4, MA ? ke : ci);
-      st_border(Y.z, row[i], p[i]);
-      st_border(Y.pa, row[i], p[i]);
-      v0[i][0] = row[i].valid ? r[i].x * p[i].x + r[i].y * p[i].y + r[i].z * p[i].z +
-                                    r[i].w * p[i].w
-                              : 0.0;
+      const V4<double> z = {d.x * ci.x, d.y * ci.y, d.z * ci.z, d.w * ci.w};
+      if constexpr (LEAN) {
+        land |= unsigned((kd.x == LAND) | (kd.y == LAND) << 1 | (kd.z == LAND) << 2 |
+                         (kd.w == LAND) << 3)
+                << 4 * i;
+        C.put(i, 0, ci);
+      } else {
+        kwe[i] = kwee;
+        C.put(i, 0, c);
+        C.put(i, 1, ks);
+        C.put(i, 2, kw);
+        C.put(i, 3, kn);
+        C.put(i, 4, MA ? ke : ci);
+      }
+      put_x(i, X0);
+      put_p(i, z);
+      st_border(Y.z, row[i], z);
+      st_border(Y.pa, row[i], z);
+      v0[i][0] = row[i].valid ? d.x * z.x + d.y * z.y + d.z * z.z + d.w * z.w : 0.0;
     }
   }
   auto cci = [&](int i) {  // CCCI
-    if constexpr (MA) {
+    if constexpr (LEAN) {
+      return C.get(i, 0);
+    } else if constexpr (MA) {
       const V4<double> c = C.get(i, 0);
       return V4<double>{rcpT(c.x), rcpT(c.y), rcpT(c.z), rcpT(c.w)};
     } else {
       return C.get(i, 4);
     }
   };
-  // what the neighbour tiles hold of z and p_old, for the next A*p
-  V4<double> hz[Q], ho[Q];
-  double ez[Q], eo[Q];
+  // what the neighbour tiles hold of z and p_old, for the next A*p: of every row,
+  // loaded under the exchange, or (lean) of the first, each next row's under the
+  // one before
+  constexpr int NH = LEAN ? 1 : Q;
+  V4<double> hz[NH], ho[NH];
+  double ez[NH], eo[NH];
+  auto halo_row = [&](const double *pold, int i, int h) {
+    if (north || south) {
+      hz[h] = ldx4(Y.z + row[i].hv);
+      ho[h] = ldx4(pold + row[i].hv);
+    }
+    if (west || east) {
+      ez[h] = __ldcg(Y.z + row[i].hx);
+      eo[h] = __ldcg(pold + row[i].hx);
+    }
+  };
   auto halo = [&](const double *pold) {
 #pragma unroll
-    for (int i = 0; i < Q; ++i) {
-      if (north || south) {
-        hz[i] = ldx4(Y.z + row[i].hv);
-        ho[i] = ldx4(pold + row[i].hv);
-      }
-      if (west || east) {
-        ez[i] = __ldcg(Y.z + row[i].hx);
-        eo[i] = __ldcg(pold + row[i].hx);
-      }
-    }
+    for (int i = 0; i < NH; ++i) halo_row(pold, i, i);
   };
   {
     double sum[1];
@@ -138,41 +184,64 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
   while (!fin) {  // ITERM bounds the loop
     {  // :93-125, and :133 of the previous iteration
       const double beta = k.beta, alpha = k.alpha;
+      const double *pold = k.parity ? Y.pb : Y.pa;
       double *pnew = k.parity ? Y.pa : Y.pb;
       const bool dox = k.iter > 0;
       double v[Q][1], sum[1];
 #pragma unroll
       for (int i = 0; i < Q; ++i) {
-        const V4<double> ci = cci(i);
-        if (dox)
-          x[i] = {x[i].x + alpha * p[i].x, x[i].y + alpha * p[i].y, x[i].z + alpha * p[i].z,
-                  x[i].w + alpha * p[i].w};
-        p[i] = {ci.x * r[i].x + beta * p[i].x, ci.y * r[i].y + beta * p[i].y,
-                ci.z * r[i].z + beta * p[i].z, ci.w * r[i].w + beta * p[i].w};
-        st4(res_stage<W>(stage, i), p[i]);
-        st_border(pnew, row[i], p[i]);
+        const V4<double> ci = cci(i), po = get_p(i);
+        if (dox) {
+          const V4<double> x0 = get_x(i);
+          put_x(i, {x0.x + alpha * po.x, x0.y + alpha * po.y, x0.z + alpha * po.z,
+                    x0.w + alpha * po.w});
+        }
+        const V4<double> q = {ci.x * r[i].x + beta * po.x, ci.y * r[i].y + beta * po.y,
+                              ci.z * r[i].z + beta * po.z, ci.w * r[i].w + beta * po.w};
+        put_p(i, q);
+        st_border(pnew, row[i], q);
       }
       __syncthreads();
 #pragma unroll
       for (int i = 0; i < Q; ++i) {
+        const int hi = LEAN ? 0 : i;
         V4<double> h{};
         double e = 0.0;
         if (north || south)
-          h = {hz[i].x + beta * ho[i].x, hz[i].y + beta * ho[i].y, hz[i].z + beta * ho[i].z,
-               hz[i].w + beta * ho[i].w};
-        if (west || east) e = ez[i] + beta * eo[i];
+          h = {hz[hi].x + beta * ho[hi].x, hz[hi].y + beta * ho[hi].y,
+               hz[hi].z + beta * ho[hi].z, hz[hi].w + beta * ho[hi].w};
+        if (west || east) e = ez[hi] + beta * eo[hi];
+        V4<double> c0, ks, kw, kn, ke;
+        if constexpr (LEAN) {
+          const int d0 = row[i].d0;
+          c0 = ld(V.cc, d0);
+          if (land >> 4 * i & 1) c0.x = 1.;
+          if (land >> 4 * i & 2) c0.y = 1.;
+          if (land >> 4 * i & 4) c0.z = 1.;
+          if (land >> 4 * i & 8) c0.w = 1.;
+          ks = ld(V.cs, d0);
+          kw = ld(V.cw, d0);
+          kn = asym ? ld(V.cn, d0) : ld(V.cs, north ? row[i].hv : d0 + TX);  // CCN(L) = CCS(LN)
+          double kwee = from_east(kw);
+          if (east) kwee = V.cw[row[i].hx] * sc;
+          ke = asym ? ld(V.ce, d0) : V4<double>{kw.y, kw.z, kw.w, kwee};
+          if (i + 1 < Q) halo_row(pold, i + 1, 0);
+        } else {
+          c0 = C.get(i, 0);
+          ks = C.get(i, 1);
+          kw = C.get(i, 2);
+          kn = C.get(i, 3);
+          if constexpr (MA)
+            ke = C.get(i, 4);
+          else
+            ke = {kw.y, kw.z, kw.w, kwe[i]};
+        }
         const double *st = res_stage<W>(stage, i);
-        const V4<double> pn = north ? h : ld4(st + TX), ps = south ? h : ld4(st - TX);
-        double pw = from_west(p[i]), pe = from_east(p[i]);
+        const V4<double> pn = north ? h : ld_stage(st + TX), ps = south ? h : ld_stage(st - TX);
+        const V4<double> q = get_p(i);
+        double pw = from_west(q), pe = from_east(q);
         if (west) pw = e;
         if (east) pe = e;
-        const V4<double> c0 = C.get(i, 0), ks = C.get(i, 1), kw = C.get(i, 2), kn = C.get(i, 3);
-        V4<double> ke;
-        if constexpr (MA)
-          ke = C.get(i, 4);
-        else
-          ke = {kw.y, kw.z, kw.w, kwe[i]};
-        const V4<double> q = p[i];
         V4<double> a;
         a.x = c0.x * q.x + ks.x * ps.x + kn.x * pn.x + kw.x * pw + ke.x * q.y;
         a.y = c0.y * q.y + ks.y * ps.y + kn.y * pn.y + kw.y * q.x + ke.y * q.z;
@@ -210,11 +279,12 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
   if (k.iter > 0) {  // :133 of the last iteration
     const double alpha = k.alpha;
 #pragma unroll
-    for (int i = 0; i < Q; ++i)
+    for (int i = 0; i < Q; ++i) {
+      const V4<double> x0 = get_x(i), po = get_p(i);
       if (row[i].valid)
-        st4(P + row[i].d0,
-            V4<double>{x[i].x + alpha * p[i].x, x[i].y + alpha * p[i].y,
-                       x[i].z + alpha * p[i].z, x[i].w + alpha * p[i].w});
+        st4(P + row[i].d0, V4<double>{x0.x + alpha * po.x, x0.y + alpha * po.y,
+                                      x0.z + alpha * po.z, x0.w + alpha * po.w});
+    }
   }
   if (me.q0 == me.qm0 && me.nq > 0 && threadIdx.x == 0) {  // every CTA of the member has read its entry values
     Ctl &o = ctl[m];
@@ -236,7 +306,7 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
 
 int cg_res_capacity(const ResForm &f, bool may_asym, int nsm) {
   int cap = 0;
-  res_form(f, [&](auto w, auto q, auto cl) {
+  res_form<true>(f, [&](auto w, auto q, auto cl) {
     constexpr int W = decltype(w)::value, Q = decltype(q)::value;
     constexpr bool CL = decltype(cl)::value;
     cap = may_asym
@@ -249,7 +319,7 @@ int cg_res_capacity(const ResForm &f, bool may_asym, int nsm) {
 void launch_cg_res(const Launch &l, const DevStatic &S, const SysView &V, const DevSystem &Y,
                    double *P, Ctl *ctl, Glob *glob, const ResPlan &R, const ResForm &f, int ncta,
                    const ResEnds &ends) {
-  res_form(f, [&](auto w, auto q, auto cl) {
+  res_form<true>(f, [&](auto w, auto q, auto cl) {
     constexpr int W = decltype(w)::value, Q = decltype(q)::value;
     constexpr bool CL = decltype(cl)::value;
     if (l.may_asym)

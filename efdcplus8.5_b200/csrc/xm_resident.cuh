@@ -112,11 +112,29 @@ struct ResCta {
   int m, q0, nq, qm0, nqm;
 };
 
-// A thread's row vectors of the CTA's quads in shared memory, as the tiles
-// hold them ([row][quad][tile][row][column]), for the rows above and below.
-template <int W, class T>
-__device__ __forceinline__ T *res_stage(T *stage, int i) {
+// A thread's row vectors of the CTA's quads in shared memory ([row][quad][tile]
+// [row][column]), for the rows above and below: TX elements from them.  Of a row
+// of 64-bit columns the first halves of its threads' vectors come first, then the
+// second: eight threads read 128 bytes in one go.
+template <int W>
+__device__ __forceinline__ float *res_stage(float *stage, int i) {
   return stage + i * (W * TILES_PER_CTA * TILE) + int(threadIdx.x) * CPT;
+}
+template <int W>
+__device__ __forceinline__ double *res_stage(double *stage, int i) {
+  return stage + i * (W * TILES_PER_CTA * TILE) + int(threadIdx.x) / ROWT * TX +
+         int(threadIdx.x) % ROWT * 2;
+}
+__device__ __forceinline__ V4<float> ld_stage(const float *p) { return ld4(p); }
+__device__ __forceinline__ V4<double> ld_stage(const double *p) {
+  const double2 a = *reinterpret_cast<const double2 *>(p);
+  const double2 b = *reinterpret_cast<const double2 *>(p + TX / 2);
+  return {a.x, a.y, b.x, b.y};
+}
+__device__ __forceinline__ void st_stage(float *p, const V4<float> &v) { st4(p, v); }
+__device__ __forceinline__ void st_stage(double *p, const V4<double> &v) {
+  *reinterpret_cast<double2 *>(p) = make_double2(v.x, v.y);
+  *reinterpret_cast<double2 *>(p + TX / 2) = make_double2(v.z, v.w);
 }
 
 constexpr int RES_CLUSTER_QUADS = 128;  // of a member in a cluster, at most
@@ -380,9 +398,9 @@ void launch_resident(void (*kernel)(P...), int ncta, int threads, size_t smem, i
   cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
-// Calls f with a form as compile-time constants; false for one that is not
-// compiled.
-template <class F>
+// Calls go with a form as compile-time constants; false for one that is not
+// compiled (LEAN: four rows of quads are, for grid groups).
+template <bool LEAN, class F>
 bool res_form(const ResForm &f, F &&go) {
   auto call = [&](auto w, auto q) {
     if (f.cluster > 0)
@@ -396,6 +414,9 @@ bool res_form(const ResForm &f, F &&go) {
   if (f.w == 1 && f.q == 1) return call(I1{}, I1{});
   if (f.w == 2 && f.q == 1) return call(I2{}, I1{});
   if (f.w == 2 && f.q == 2) return call(I2{}, I2{});
+  if constexpr (LEAN)
+    if (f.w == 2 && f.q == 4 && f.cluster == 0)
+      return go(I2{}, std::integral_constant<int, 4>{}, std::false_type{}), true;
   return false;
 }
 

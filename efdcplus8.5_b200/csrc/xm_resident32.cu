@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
 
 int mx_res_capacity(const ResForm &f, bool may_asym, int nsm) {
   int cap = 0;
-  res_form(f, [&](auto w, auto q, auto cl) {
+  res_form<false>(f, [&](auto w, auto q, auto cl) {
     constexpr int W = decltype(w)::value, Q = decltype(q)::value;
     constexpr bool CL = decltype(cl)::value;
     cap = may_asym
@@ -398,7 +398,7 @@ void launch_mx_res(const Launch &l, const DevStatic &S, const SysView &V, const 
   ra.rel_tol = rel_tol;
   ra.margin = l.inner_margin;
   ra.unscaled = V.unscaled;
-  res_form(f, [&](auto w, auto q, auto cl) {
+  res_form<false>(f, [&](auto w, auto q, auto cl) {
     constexpr int W = decltype(w)::value, Q = decltype(q)::value;
     constexpr bool CL = decltype(cl)::value;
     if (l.may_asym)

@@ -3,7 +3,7 @@ launch, its vectors on the chip, against the multi-kernel CG of the same
 context, bit for bit -- states, CG iterations, refinement passes.
 
 Sizes at which the launch changes its form: a member of one 4-tile unit (no
-exchange between CTAs), ragged last units, one, two and four units per CTA, and
+exchange between CTAs), ragged last units, one, two, four and eight units per CTA, and
 batches that take several launches; with radiation boundaries (the four-array
 operator), wetting and drying, three time levels, the standalone CONGRAD and
 the adjoint's solve.
@@ -80,6 +80,17 @@ def test_forms(precision, device_loops):
     for m in mem:
         same([m], precision, 6, device_loops=device_loops)
     same(mem, precision, 6, device_loops=device_loops)
+
+
+@pytest.mark.parametrize("names", [("radiation_all_sides", "legacy_dry_1"),
+                                   ("radiation_closed_face", "tidal_flat_99")])
+def test_four_rows_of_quads(names):
+    """The FP64 form of members of more than 592 units, which reads the operator in
+    each iteration: small members with both operators beside a basin that takes it,
+    and (two launches) beside two."""
+    small = [cases.build(n)[0] for n in names]
+    same([basin(830, 801)] + small, X.PREC_FP64)
+    same(small + [basin(1010, 640, seed=k) for k in (3, 4)], X.PREC_FP64, 2)
 
 
 @pytest.mark.parametrize("precision", [X.PREC_FP64, X.PREC_MIXED])
