@@ -443,11 +443,11 @@ __device__ __forceinline__ void quad_sweep_staged(const DevStatic &S, double *pa
 }
 
 // The quad sweep of a kernel variant: 0 prefetches one quad ahead in
-// registers, 1 and 3 load the descriptors in batches (quad_sweep_batched).
+// registers, 1 loads the descriptors in batches (quad_sweep_batched).
 template <int NS, int VAR, class Setup, class Body, class Epi>
 __device__ __forceinline__ void quad_sweep_v(const DevStatic &S, double *part, Setup setup,
                                              Body body, const Fold<Epi> &f) {
-  if constexpr (VAR == 1 || VAR == 3)
+  if constexpr (VAR == 1)
     quad_sweep_batched<NS>(S, part, setup, body, f);
   else
     quad_sweep<NS>(S, part, setup, body, f);
@@ -762,126 +762,10 @@ __device__ __forceinline__ V4<float> x_plus_alpha_p(const V4<float> &x, float al
 // at the row vector and its halo, Ap = p + AS*pS + AN*pN + AW*pW + AE*pE, and
 // the part of p.Ap.  Symmetric: AN(L) = AS(LN), AE(L) = AW(LE).  With dox,
 // also the previous iteration's x += alpha*p (x_plus_alpha_p).
+// Here and in the other MIXED rows every global load is issued before the first
+// shuffle or dependent operation, so that one round trip to memory serves the row:
+// more values live, fewer CTAs per SM (see mx_ctas).
 __device__ __forceinline__ double matvec_row_scaled(const RowGeo &g, bool valid,
-                                                    const float *__restrict__ r,
-                                                    const float *__restrict__ pold,
-                                                    float *__restrict__ pnew,
-                                                    const float *__restrict__ as,
-                                                    const float *__restrict__ aw,
-                                                    const float *__restrict__ ae,
-                                                    const float *__restrict__ an,
-                                                    float *__restrict__ ap, float beta, bool asym,
-                                                    float *__restrict__ x, float alpha_prev,
-                                                    bool dox) {
-  const V4<float> r0 = ld4(r + g.d0), o0 = ld4(pold + g.d0);
-  const V4<float> x0 = dox ? ld4(x + g.d0) : V4<float>{0.f, 0.f, 0.f, 0.f};
-  const V4<float> rn = ld4(r + g.dn), on = ld4(pold + g.dn);
-  const V4<float> rs = ld4(r + g.ds), os = ld4(pold + g.ds);
-  const V4<float> p = {fmaf(beta, o0.x, r0.x), fmaf(beta, o0.y, r0.y), fmaf(beta, o0.z, r0.z),
-                       fmaf(beta, o0.w, r0.w)};
-  const V4<float> pn = {fmaf(beta, on.x, rn.x), fmaf(beta, on.y, rn.y), fmaf(beta, on.z, rn.z),
-                        fmaf(beta, on.w, rn.w)};
-  const V4<float> ps = {fmaf(beta, os.x, rs.x), fmaf(beta, os.y, rs.y), fmaf(beta, os.z, rs.z),
-                        fmaf(beta, os.w, rs.w)};
-  float pw = from_west(p), pe = from_east(p);
-  if (g.cx == 0) pw = fmaf(beta, pold[g.dwe], r[g.dwe]);
-  if (g.cx == ROWT - 1) pe = fmaf(beta, pold[g.dee], r[g.dee]);
-  const V4<float> ks = ld4(as + g.d0), kw = ld4(aw + g.d0);
-  V4<float> kn, ke;
-  if (asym) {
-    kn = ld4(an + g.d0);
-    ke = ld4(ae + g.d0);
-  } else {
-    kn = ld4(as + g.dn);
-    float kwe = from_east(kw);
-    if (g.cx == ROWT - 1) kwe = aw[g.dee];
-    ke = {kw.y, kw.z, kw.w, kwe};
-  }
-  const V4<float> a = scaled_ap(p, ps, pn, pw, pe, ks, kn, kw, ke);
-  if (!valid) return 0.0;
-  if (dox) st4(x + g.d0, x_plus_alpha_p(x0, alpha_prev, o0));
-  st4(pnew + g.d0, p);
-  st4(ap + g.d0, a);
-  return dot4(a, p);
-}
-
-// MIXED, polynomial-preconditioned: r -= alpha*Ap at the cell
-// and (recomputed from r and Ap) at its four neighbours, then
-// z = (2I - Ahat) r = r - N r (N: the couplings AS, AW, AN = AS(LN),
-// AE = AW(LE)) -- the two-term Neumann series of Ahat^-1, symmetric positive
-// definite for a symmetric unit-diagonal Ahat with eigenvalues in (0, 2).
-// With poly == false z = r (Jacobi; unsymmetric operators).  Stores the new
-// r (into the other residual buffer: neighbours still read the old r for
-// their own halo) and z; adds r.z and r.r.  (x += alpha*p: the next
-// matrix-vector pass, x_plus_alpha_p.)
-__device__ __forceinline__ void update_row_poly(const RowGeo &g, bool valid,
-                                                const float *__restrict__ r,
-                                                float *__restrict__ rnew,
-                                                const float *__restrict__ ap,
-                                                const float *__restrict__ as,
-                                                const float *__restrict__ aw,
-                                                float *__restrict__ z, float alpha, bool poly,
-                                                double &rz, double &rr) {
-  const V4<float> r0 = ld4(r + g.d0), a0 = ld4(ap + g.d0);
-  const V4<float> rn0 = {fmaf(-alpha, a0.x, r0.x), fmaf(-alpha, a0.y, r0.y),
-                         fmaf(-alpha, a0.z, r0.z), fmaf(-alpha, a0.w, r0.w)};
-  V4<float> zv = rn0;
-  if (poly) {
-    const V4<float> rN = ld4(r + g.dn), aN = ld4(ap + g.dn);
-    const V4<float> rS = ld4(r + g.ds), aS = ld4(ap + g.ds);
-    const V4<float> nN = {fmaf(-alpha, aN.x, rN.x), fmaf(-alpha, aN.y, rN.y),
-                          fmaf(-alpha, aN.z, rN.z), fmaf(-alpha, aN.w, rN.w)};
-    const V4<float> nS = {fmaf(-alpha, aS.x, rS.x), fmaf(-alpha, aS.y, rS.y),
-                          fmaf(-alpha, aS.z, rS.z), fmaf(-alpha, aS.w, rS.w)};
-    float nw = from_west(rn0), ne = from_east(rn0);
-    if (g.cx == 0) nw = fmaf(-alpha, ap[g.dwe], r[g.dwe]);
-    if (g.cx == ROWT - 1) ne = fmaf(-alpha, ap[g.dee], r[g.dee]);
-    const V4<float> ks = ld4(as + g.d0), kw = ld4(aw + g.d0), kn = ld4(as + g.dn);
-    float kwe = from_east(kw);
-    if (g.cx == ROWT - 1) kwe = aw[g.dee];
-    const V4<float> ke = {kw.y, kw.z, kw.w, kwe};
-    zv = neumann_row(rn0, nS, nN, nw, ne, ks, kn, kw, ke);
-  }
-  if (!valid) return;
-  st4(rnew + g.d0, rn0);
-  st4(z + g.d0, zv);
-  rz += dot4(rn0, zv);
-  rr += dot4(rn0, rn0);
-}
-
-// MIXED: z0 = (2I - Ahat) r (or r) for the first inner iteration, p_old = 0,
-// and the part of r.z.
-__device__ __forceinline__ double zinit_row(const RowGeo &g, bool valid,
-                                           const float *__restrict__ r,
-                                           const float *__restrict__ as,
-                                           const float *__restrict__ aw, float *__restrict__ z,
-                                           float *__restrict__ pold, bool poly) {
-  const V4<float> r0 = ld4(r + g.d0);
-  V4<float> zv = r0;
-  if (poly) {
-    const V4<float> rN = ld4(r + g.dn), rS = ld4(r + g.ds);
-    float rw = from_west(r0), re = from_east(r0);
-    if (g.cx == 0) rw = r[g.dwe];
-    if (g.cx == ROWT - 1) re = r[g.dee];
-    const V4<float> ks = ld4(as + g.d0), kw = ld4(aw + g.d0), kn = ld4(as + g.dn);
-    float kwe = from_east(kw);
-    if (g.cx == ROWT - 1) kwe = aw[g.dee];
-    const V4<float> ke = {kw.y, kw.z, kw.w, kwe};
-    zv = neumann_row(r0, rS, rN, rw, re, ks, kn, kw, ke);
-  }
-  if (!valid) return 0.0;
-  st4(z + g.d0, zv);
-  st4(pold + g.d0, V4<float>{0.f, 0.f, 0.f, 0.f});
-  return dot4(r0, zv);
-}
-
-// Variant 3 of the MIXED inner iteration: matvec_row_scaled and
-// update_row_poly with every global load of the row issued before the first
-// shuffle or dependent operation (above, the coefficient rows and x, p_new
-// wait for the first loads' values), so that one round trip to memory serves
-// the row; the same operations on the same values, hence the same results.
-// It holds more values live: its kernels run at fewer CTAs per SM.
-__device__ __forceinline__ double matvec_row_scaled_eager(const RowGeo &g, bool valid,
                                                     const float *__restrict__ r,
                                                     const float *__restrict__ pold,
                                                     float *__restrict__ pnew,
@@ -927,7 +811,16 @@ __device__ __forceinline__ double matvec_row_scaled_eager(const RowGeo &g, bool 
   return dot4(a, p);
 }
 
-__device__ __forceinline__ void update_row_poly_eager(const RowGeo &g, bool valid,
+// MIXED, polynomial-preconditioned: r -= alpha*Ap at the cell
+// and (recomputed from r and Ap) at its four neighbours, then
+// z = (2I - Ahat) r = r - N r (N: the couplings AS, AW, AN = AS(LN),
+// AE = AW(LE)) -- the two-term Neumann series of Ahat^-1, symmetric positive
+// definite for a symmetric unit-diagonal Ahat with eigenvalues in (0, 2).
+// With poly == false z = r (Jacobi; unsymmetric operators).  Stores the new
+// r (into the other residual buffer: neighbours still read the old r for
+// their own halo) and z; adds r.z and r.r.  (x += alpha*p: the next
+// matrix-vector pass, x_plus_alpha_p.)
+__device__ __forceinline__ void update_row_poly(const RowGeo &g, bool valid,
                                                 const float *__restrict__ r,
                                                 float *__restrict__ rnew,
                                                 const float *__restrict__ ap,
@@ -979,6 +872,46 @@ __device__ __forceinline__ void update_row_poly_eager(const RowGeo &g, bool vali
   st4(z + g.d0, zv);
   rz += dot4(rn0, zv);
   rr += dot4(rn0, rn0);
+}
+
+// MIXED: z0 = (2I - Ahat) r (or r) for the first inner iteration, p_old = 0,
+// and the part of r.z.
+__device__ __forceinline__ double zinit_row(const RowGeo &g, bool valid,
+                                           const float *__restrict__ r,
+                                           const float *__restrict__ as,
+                                           const float *__restrict__ aw, float *__restrict__ z,
+                                           float *__restrict__ pold, bool poly) {
+  // every load first, so that one round trip serves the row
+  const V4<float> r0 = ld4(r + g.d0);
+  V4<float> rN{}, rS{}, ks{}, kw{}, kn{};
+  float rw_edge = 0.f, re_edge = 0.f, kwe_edge = 0.f;
+  const bool west = g.cx == 0, east = g.cx == ROWT - 1;
+  if (poly) {
+    rN = ld4(r + g.dn);
+    rS = ld4(r + g.ds);
+    ks = ld4(as + g.d0);
+    kw = ld4(aw + g.d0);
+    kn = ld4(as + g.dn);
+    if (west) rw_edge = r[g.dwe];
+    if (east) {
+      re_edge = r[g.dee];
+      kwe_edge = aw[g.dee];
+    }
+  }
+  V4<float> zv = r0;
+  if (poly) {
+    float rw = from_west(r0), re = from_east(r0);
+    if (west) rw = rw_edge;
+    if (east) re = re_edge;
+    float kwe = from_east(kw);
+    if (east) kwe = kwe_edge;
+    const V4<float> ke = {kw.y, kw.z, kw.w, kwe};
+    zv = neumann_row(r0, rS, rN, rw, re, ks, kn, kw, ke);
+  }
+  if (!valid) return 0.0;
+  st4(z + g.d0, zv);
+  st4(pold + g.d0, V4<float>{0.f, 0.f, 0.f, 0.f});
+  return dot4(r0, zv);
 }
 
 // MIXED, Jacobi: r -= alpha*Ap (into the other residual buffer) and the part
@@ -1039,46 +972,6 @@ __device__ __forceinline__ void update_row(const RowGeo &g, bool valid, T *__res
 __device__ __forceinline__ V4<double> residual_row(const RowGeo &g, const uint8_t *kind,
                                                    const double *__restrict__ P,
                                                    const SysView &V, bool asym) {
-  const V4<double> x = ld4(P + g.d0), xn = ld4(P + g.dn), xs = ld4(P + g.ds);
-  double xw = from_west(x), xe = from_east(x);
-  if (g.cx == 0) xw = P[g.dwe];
-  if (g.cx == ROWT - 1) xe = P[g.dee];
-  const V4<double> b = ld4(V.fp + g.d0), c = ld4(V.cc + g.d0), ks = ld4(V.cs + g.d0),
-                   kw = ld4(V.cw + g.d0);
-  V4<double> kn, ke;
-  if (asym) {
-    kn = ld4(V.cn + g.d0);
-    ke = ld4(V.ce + g.d0);
-  } else {  // CCN(L) = CCS(LN), CCE(L) = CCW(LE)
-    kn = ld4(V.cs + g.dn);
-    double kwe = from_east(kw);
-    if (g.cx == ROWT - 1) kwe = V.cw[g.dee];
-    ke = {kw.y, kw.z, kw.w, kwe};
-  }
-  const uchar4 kd = *reinterpret_cast<const uchar4 *>(kind + g.d0);
-  V4<double> r;
-  r.x = b.x - c.x * x.x - kn.x * xn.x - ks.x * xs.x - kw.x * xw - ke.x * x.y;
-  r.y = b.y - c.y * x.y - kn.y * xn.y - ks.y * xs.y - kw.y * x.x - ke.y * x.z;
-  r.z = b.z - c.z * x.z - kn.z * xn.z - ks.z * xs.z - kw.z * x.y - ke.z * x.w;
-  r.w = b.w - c.w * x.w - kn.w * xn.w - ks.w * xs.w - kw.w * x.z - ke.w * xe;
-  if (kd.x == LAND) r.x = 0.;
-  if (kd.y == LAND) r.y = 0.;
-  if (kd.z == LAND) r.z = 0.;
-  if (kd.w == LAND) r.w = 0.;
-  return r;
-}
-
-__device__ __forceinline__ V4<double> residual_row(const RowGeo &g, const uint8_t *kind,
-                                                   const double *__restrict__ P,
-                                                   const DevSystem &Y, bool asym) {
-  return residual_row(g, kind, P, SysView{Y.fptmp, Y.ccc, Y.ccs, Y.ccw, Y.cce, Y.ccn, 0}, asym);
-}
-
-// residual_row and zinit_row with every load of the row issued first (the
-// refinement kernels of variant 3, see matvec_row_scaled_eager).
-__device__ __forceinline__ V4<double> residual_row_eager(const RowGeo &g, const uint8_t *kind,
-                                                   const double *__restrict__ P,
-                                                   const SysView &V, bool asym) {
   // every load first, so that one round trip serves the row
   const V4<double> x = ld4(P + g.d0), xn = ld4(P + g.dn), xs = ld4(P + g.ds);
   const V4<double> b = ld4(V.fp + g.d0), c = ld4(V.cc + g.d0), ks = ld4(V.cs + g.d0),
@@ -1109,42 +1002,10 @@ __device__ __forceinline__ V4<double> residual_row_eager(const RowGeo &g, const 
   return r;
 }
 
-__device__ __forceinline__ double zinit_row_eager(const RowGeo &g, bool valid,
-                                           const float *__restrict__ r,
-                                           const float *__restrict__ as,
-                                           const float *__restrict__ aw, float *__restrict__ z,
-                                           float *__restrict__ pold, bool poly) {
-  // every load first, so that one round trip serves the row
-  const V4<float> r0 = ld4(r + g.d0);
-  V4<float> rN{}, rS{}, ks{}, kw{}, kn{};
-  float rw_edge = 0.f, re_edge = 0.f, kwe_edge = 0.f;
-  const bool west = g.cx == 0, east = g.cx == ROWT - 1;
-  if (poly) {
-    rN = ld4(r + g.dn);
-    rS = ld4(r + g.ds);
-    ks = ld4(as + g.d0);
-    kw = ld4(aw + g.d0);
-    kn = ld4(as + g.dn);
-    if (west) rw_edge = r[g.dwe];
-    if (east) {
-      re_edge = r[g.dee];
-      kwe_edge = aw[g.dee];
-    }
-  }
-  V4<float> zv = r0;
-  if (poly) {
-    float rw = from_west(r0), re = from_east(r0);
-    if (west) rw = rw_edge;
-    if (east) re = re_edge;
-    float kwe = from_east(kw);
-    if (east) kwe = kwe_edge;
-    const V4<float> ke = {kw.y, kw.z, kw.w, kwe};
-    zv = neumann_row(r0, rS, rN, rw, re, ks, kn, kw, ke);
-  }
-  if (!valid) return 0.0;
-  st4(z + g.d0, zv);
-  st4(pold + g.d0, V4<float>{0.f, 0.f, 0.f, 0.f});
-  return dot4(r0, zv);
+__device__ __forceinline__ V4<double> residual_row(const RowGeo &g, const uint8_t *kind,
+                                                   const double *__restrict__ P,
+                                                   const DevSystem &Y, bool asym) {
+  return residual_row(g, kind, P, SysView{Y.fptmp, Y.ccc, Y.ccs, Y.ccw, Y.cce, Y.ccn, 0}, asym);
 }
 
 // The Jacobi scaling of the MIXED inner system, 1/sqrt(c) for a diagonal c

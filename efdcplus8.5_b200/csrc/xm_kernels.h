@@ -23,8 +23,8 @@ struct Launch {
   bool chan = false;     // sub-grid channel terms (a step of a context with channels)
   bool baro = false;     // some member of the step has the baroclinic terms (CALEBI)
   // schedule (efdc_xm_set_schedule): the FP32 CG kernels' variant (0: quad
-  // descriptors prefetched one quad ahead, 1: in shared-memory batches) and,
-  // for variant 1, caps on their resident CTAs per SM (0: occupancy)
+  // descriptors prefetched one quad ahead, 1 and 3: in shared-memory batches, 2: those
+  // and staged rows) and, for 1 to 3, caps on their resident CTAs per SM (0: occupancy)
   int variant = 0;
   int ctas_mv = 0, ctas_up = 0;
   // MIXED: the inner solve's target is the reduction the FP64 residual needs

@@ -25,17 +25,14 @@ namespace xm {
 
 // p = z + beta*p_old at the cell and its halo (z = r for Jacobi members),
 // Ahat*p, p.Ap (per member).
-// CTAs per SM the launch bounds ask for, by variant (3 holds more values live)
-constexpr int mx_ctas(int var) { return var == 1 ? 5 : var == 3 ? 4 : 6; }
-// variant 3's matrix-vector and update kernels (measured on the 256-member
-// ensemble: 3 for the first, no spills at 72 registers, is even; 5 for the
-// second spills and is 3 % slower)
-constexpr int MV3_CTAS = 4, UP3_CTAS = 4;
-constexpr int mv_ctas(int var) { return var == 3 ? MV3_CTAS : mx_ctas(var); }
-constexpr int up_ctas(int var) { return var == 3 ? UP3_CTAS : mx_ctas(var); }
+// CTAs per SM the launch bounds ask for.  Measured, ms per step, rows that wait for
+// their first loads at 6 CTAs -> every load first at 4: 2,048x2,048 cells 1.72 -> 1.58,
+// 1,500x1,400 0.857 -> 0.807, 24 basins of 2.5 M cells 1.12 -> 1.06, 256 of 8.7 M 2.77
+// -> 2.59 (3 CTAs are even, 5 spill and are 3 % slower).
+constexpr int MX_CTAS = 4;
 
 template <bool MA, int VAR, bool FOLD>
-__global__ void __launch_bounds__(NT, mv_ctas(VAR)) k_mx_matvec(DevStatic S, DevSystem Y, Ctl *ctl,
+__global__ void __launch_bounds__(NT, MX_CTAS) k_mx_matvec(DevStatic S, DevSystem Y, Ctl *ctl,
                                                     double *part) {
   struct A {
     bool skip, asym, dox;
@@ -58,12 +55,8 @@ __global__ void __launch_bounds__(NT, mv_ctas(VAR)) k_mx_matvec(DevStatic S, Dev
                  poly ? Y.z32 : (par ? Y.r32b : Y.r32)};
       },
       [&](const A &a, const RowGeo &g, bool valid, double *v) {
-        if constexpr (VAR == 3)
-          v[0] = matvec_row_scaled_eager(g, valid, a.z, a.pold, a.pnew, Y.as32, Y.aw32, Y.ae32,
-                                         Y.an32, Y.ap32, a.beta, a.asym, Y.x32, a.alpha, a.dox);
-        else
-          v[0] = matvec_row_scaled(g, valid, a.z, a.pold, a.pnew, Y.as32, Y.aw32, Y.ae32,
-                                   Y.an32, Y.ap32, a.beta, a.asym, Y.x32, a.alpha, a.dox);
+        v[0] = matvec_row_scaled(g, valid, a.z, a.pold, a.pnew, Y.as32, Y.aw32, Y.ae32,
+                                 Y.an32, Y.ap32, a.beta, a.asym, Y.x32, a.alpha, a.dox);
       },
       fold_if<FOLD>(ctl, [&](int m, const double *sum) {
         if (threadIdx.x == 0) cg_matvec_epi(ctl[m], sum[0]);
@@ -82,7 +75,7 @@ __global__ void __launch_bounds__(NT) k_red_mx_matvec(DevStatic S, Ctl *ctl, con
 // and r.r (FP64 sums): the members that use it.  x += alpha*p is the next
 // matrix-vector kernel's (or, after the last iteration, k_mx_apply's).
 template <int VAR, bool FOLD>
-__global__ void __launch_bounds__(NT, up_ctas(VAR)) k_mx_update_poly(DevStatic S, DevSystem Y,
+__global__ void __launch_bounds__(NT, MX_CTAS) k_mx_update_poly(DevStatic S, DevSystem Y,
                                                          Ctl *ctl, double *part, RedArgs ra) {
   struct A {
     bool skip;
@@ -100,12 +93,8 @@ __global__ void __launch_bounds__(NT, up_ctas(VAR)) k_mx_update_poly(DevStatic S
                  par ? Y.r32 : Y.r32b};
       },
       [&](const A &a, const RowGeo &g, bool valid, double *v) {
-        if constexpr (VAR == 3)
-          update_row_poly_eager(g, valid, a.r, a.rnew, Y.ap32, Y.as32, Y.aw32, Y.z32, a.alpha,
-                                true, v[0], v[1]);
-        else
-          update_row_poly(g, valid, a.r, a.rnew, Y.ap32, Y.as32, Y.aw32, Y.z32, a.alpha, true,
-                          v[0], v[1]);
+        update_row_poly(g, valid, a.r, a.rnew, Y.ap32, Y.as32, Y.aw32, Y.z32, a.alpha, true,
+                        v[0], v[1]);
       },
       fold_if<FOLD>(ctl, [&](int m, const double *sum) {
         if (threadIdx.x == 0)
@@ -157,7 +146,7 @@ __global__ void __launch_bounds__(NT) k_red_mx_update(DevStatic S, Ctl *ctl, Glo
 
 // First inner iteration of the polynomial members: z0 = (2I - Ahat) r0,
 // p_old = 0, RPCG = r0.z0 (Jacobi members start from k_mx_resid's p0 = r0).
-template <bool EAGER, bool FOLD>
+template <bool FOLD>
 __global__ void __launch_bounds__(NT) k_mx_zinit(DevStatic S, DevSystem Y, Ctl *ctl,
                                                 double *part) {
   struct A {
@@ -167,10 +156,7 @@ __global__ void __launch_bounds__(NT) k_mx_zinit(DevStatic S, DevSystem Y, Ctl *
       S, part,
       [&](int m) { return A{ctl[m].done != 0 || !Y.mpoly[m] || unsym<true>(ctl[m]), false}; },
       [&](const A &, const RowGeo &g, bool valid, double *v) {
-        if constexpr (EAGER)
-          v[0] = zinit_row_eager(g, valid, Y.r32, Y.as32, Y.aw32, Y.z32, Y.pa32, true);
-        else
-          v[0] = zinit_row(g, valid, Y.r32, Y.as32, Y.aw32, Y.z32, Y.pa32, true);
+        v[0] = zinit_row(g, valid, Y.r32, Y.as32, Y.aw32, Y.z32, Y.pa32, true);
       },
       fold_if<FOLD>(ctl, [&](int m, const double *sum) {
         if (threadIdx.x == 0) ctl[m].rpcg = sum[0];
@@ -470,19 +456,12 @@ static void mx_matvec_kernel(const Launch &l, const DevStatic &S, const DevSyste
       k_mx_matvec_st<false, F><<<staged_grid(l, S, k_mx_matvec_st<false, F>, sm, l.ctas_mv), NT,
                                  sm, l.stream>>>(S, Y, ctl, part);
     }
-  } else if (l.variant == 1) {
+  } else if (l.variant != 0) {
     if (l.may_asym)
       k_mx_matvec<true, 1, F><<<grid_of(l, S, k_mx_matvec<true, 1, F>, l.ctas_mv), NT, 0,
                                 l.stream>>>(S, Y, ctl, part);
     else
       k_mx_matvec<false, 1, F><<<grid_of(l, S, k_mx_matvec<false, 1, F>, l.ctas_mv), NT, 0,
-                                 l.stream>>>(S, Y, ctl, part);
-  } else if (l.variant == 3) {
-    if (l.may_asym)
-      k_mx_matvec<true, 3, F><<<grid_of(l, S, k_mx_matvec<true, 3, F>, l.ctas_mv), NT, 0,
-                                l.stream>>>(S, Y, ctl, part);
-    else
-      k_mx_matvec<false, 3, F><<<grid_of(l, S, k_mx_matvec<false, 3, F>, l.ctas_mv), NT, 0,
                                  l.stream>>>(S, Y, ctl, part);
   } else if (l.may_asym) {
     k_mx_matvec<true, 0, F><<<l.grid_cg32, NT, 0, l.stream>>>(S, Y, ctl, part);
@@ -511,7 +490,7 @@ static void mx_update_kernels(const Launch &l, const DevStatic &S, const DevSyst
                             l.stream>>>(S, Y, ctl, part, ra);
     count_launches(1);
   } else if (l.mx_jac) {
-    if (l.variant == 1 || l.variant == 3)  // the Jacobi row already loads first
+    if (l.variant != 0)
       k_mx_update_jac<1, F><<<grid_of(l, S, k_mx_update_jac<1, F>, l.ctas_up), NT, 0,
                               l.stream>>>(S, Y, ctl, part, ra);
     else
@@ -524,11 +503,8 @@ static void mx_update_kernels(const Launch &l, const DevStatic &S, const DevSyst
                              l.stream>>>(S, Y, ctl, part, ra);
     count_launches(1);
   } else if (l.mx_poly) {
-    if (l.variant == 1)
+    if (l.variant != 0)
       k_mx_update_poly<1, F><<<grid_of(l, S, k_mx_update_poly<1, F>, l.ctas_up), NT, 0,
-                               l.stream>>>(S, Y, ctl, part, ra);
-    else if (l.variant == 3)
-      k_mx_update_poly<3, F><<<grid_of(l, S, k_mx_update_poly<3, F>, l.ctas_up), NT, 0,
                                l.stream>>>(S, Y, ctl, part, ra);
     else
       k_mx_update_poly<0, F><<<l.grid_up32, NT, 0, l.stream>>>(S, Y, ctl, part, ra);
@@ -552,19 +528,11 @@ void launch_mx_zinit(const Launch &l, const DevStatic &S, const DevSystem &Y, Ct
                      double *part) {
   if (!l.mx_poly) return;
   if (l.fold) {
-    if (l.variant == 3)
-      k_mx_zinit<true, true><<<grid_of(l, S, k_mx_zinit<true, true>, 0), NT, 0, l.stream>>>(
-          S, Y, ctl, part);
-    else
-      k_mx_zinit<false, true><<<l.grid_up32, NT, 0, l.stream>>>(S, Y, ctl, part);
+    k_mx_zinit<true><<<grid_of(l, S, k_mx_zinit<true>, 0), NT, 0, l.stream>>>(S, Y, ctl, part);
     count_launches(1);
     return;
   }
-  if (l.variant == 3)
-    k_mx_zinit<true, false><<<grid_of(l, S, k_mx_zinit<true, false>, 0), NT, 0, l.stream>>>(
-        S, Y, ctl, part);
-  else
-    k_mx_zinit<false, false><<<l.grid_up32, NT, 0, l.stream>>>(S, Y, ctl, part);
+  k_mx_zinit<false><<<grid_of(l, S, k_mx_zinit<false>, 0), NT, 0, l.stream>>>(S, Y, ctl, part);
   k_red_mx_zinit<<<reduce_grid(S), NT, 0, l.stream>>>(S, Y, ctl, part);
   count_launches(2);
 }

@@ -716,13 +716,13 @@ __global__ void __launch_bounds__(NT) k_cg_finish(DevStatic S, DevSystem Y, doub
 // in FP64, and the FP32 scaled inner system's rhs rhat = D^-1/2 r with
 // x = 0 and p0 = rhat (k_mx_zinit then forms z0 = M^-1 rhat and p_old = 0 for
 // the polynomial members).  rsqm_fac scales the member's RSQM (the MIXED stop,
-// below RSQM).  EAGER: the row's loads issued first (kernel variant 3).
+// below RSQM).
 __device__ __forceinline__ void mx_resid_epi(Ctl &k, Glob *glob, const StepScalars &c,
                                              const RedArgs &ra, double rsq, double rz) {
   if (mx_resid_step(k, c.rsqm, c.iterm, ra, rsq, rz)) member_done(k, glob);
 }
 
-template <bool MA, bool EAGER, bool FOLD>
+template <bool MA, bool FOLD>
 __global__ void __launch_bounds__(NT) k_mx_resid(DevStatic S, SysView V, DevSystem Y,
                                                 const double *P, Ctl *ctl, double *part,
                                                 RedArgs ra) {
@@ -732,11 +732,7 @@ __global__ void __launch_bounds__(NT) k_mx_resid(DevStatic S, SysView V, DevSyst
   quad_sweep<2>(
       S, part, [&](int m) { return A{ctl[m].done != 0, unsym<MA>(ctl[m])}; },
       [&](const A &a, const RowGeo &g, bool valid, double *v) {
-        V4<double> r;
-        if constexpr (EAGER)
-          r = residual_row_eager(g, S.kind, P, V, a.asym);
-        else
-          r = residual_row(g, S.kind, P, V, a.asym);
+        const V4<double> r = residual_row(g, S.kind, P, V, a.asym);
         const V4<double> c = ld4(V.cc + g.d0);
         const V4<float> r32 = {float(r.x * inv_sqrt_diag(c.x)), float(r.y * inv_sqrt_diag(c.y)),
                                float(r.z * inv_sqrt_diag(c.z)), float(r.w * inv_sqrt_diag(c.w))};
@@ -1451,20 +1447,12 @@ template <bool F>
 static void mx_resid_kernel(const Launch &l, const DevStatic &S, const SysView &V,
                             const DevSystem &Y, const double *P, Ctl *ctl, double *part,
                             const RedArgs &ra) {
-  if (l.variant == 3) {
-    if (l.may_asym)
-      k_mx_resid<true, true, F><<<quad_grid(l, S, k_mx_resid<true, true, F>), NT, 0,
-                                  l.stream>>>(S, V, Y, P, ctl, part, ra);
-    else
-      k_mx_resid<false, true, F><<<quad_grid(l, S, k_mx_resid<false, true, F>), NT, 0,
-                                   l.stream>>>(S, V, Y, P, ctl, part, ra);
-  } else if (l.may_asym) {
-    k_mx_resid<true, false, F><<<quad_grid(l, S, k_mx_resid<true, false, F>), NT, 0,
-                                 l.stream>>>(S, V, Y, P, ctl, part, ra);
-  } else {
-    k_mx_resid<false, false, F><<<quad_grid(l, S, k_mx_resid<false, false, F>), NT, 0,
-                                  l.stream>>>(S, V, Y, P, ctl, part, ra);
-  }
+  if (l.may_asym)
+    k_mx_resid<true, F><<<quad_grid(l, S, k_mx_resid<true, F>), NT, 0, l.stream>>>(
+        S, V, Y, P, ctl, part, ra);
+  else
+    k_mx_resid<false, F><<<quad_grid(l, S, k_mx_resid<false, F>), NT, 0, l.stream>>>(
+        S, V, Y, P, ctl, part, ra);
   count_launches(1);
 }
 void launch_mx_resid(const Launch &l, const DevStatic &S, const SysView &V, const DevSystem &Y,
@@ -1720,7 +1708,7 @@ int occupancy_blocks_per_sm_cg() {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_mx_apply, NT, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cg_update<false>, NT, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_cg_init<true, false>, NT, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, k_mx_resid<true, false, false>, NT, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, k_mx_resid<true, false>, NT, 0);
   const int m = std::min(std::min(a, b), std::min(c, d));
   return m > 0 ? m : 1;
 }
