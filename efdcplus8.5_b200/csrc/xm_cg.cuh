@@ -760,8 +760,10 @@ __device__ __forceinline__ V4<float> x_plus_alpha_p(const V4<float> &x, float al
 
 // MIXED inner CG on the Jacobi-scaled system (unit diagonal): p = r + beta*p
 // at the row vector and its halo, Ap = p + AS*pS + AN*pN + AW*pW + AE*pE, and
-// the part of p.Ap.  Symmetric: AN(L) = AS(LN), AE(L) = AW(LE).  With dox,
-// also the previous iteration's x += alpha*p (x_plus_alpha_p).
+// the part of p.Ap.  Symmetric: AN(L) = AS(LN), AE(L) = AW(LE).  After
+// the pass's first iteration (iter > 0) also the previous one's x += alpha*p
+// (x_plus_alpha_p).  A pass starts from p_old = x = 0, which are not read (nor
+// stored: 20 of a pass's 56 n + 113 B per cell).
 // Here and in the other MIXED rows every global load is issued before the first
 // shuffle or dependent operation, so that one round trip to memory serves the row:
 // more values live, fewer CTAs per SM (see mx_ctas).
@@ -775,19 +777,21 @@ __device__ __forceinline__ double matvec_row_scaled(const RowGeo &g, bool valid,
                                                     const float *__restrict__ an,
                                                     float *__restrict__ ap, float beta, bool asym,
                                                     float *__restrict__ x, float alpha_prev,
-                                                    bool dox) {
+                                                    int iter) {
   // every load first, so that one round trip serves the row (x is read at
   // the ghost tile's inert slots too when the row is not valid)
-  const V4<float> r0 = ld4(r + g.d0), o0 = ld4(pold + g.d0);
-  const V4<float> x0 = dox ? ld4(x + g.d0) : V4<float>{0.f, 0.f, 0.f, 0.f};
-  const V4<float> rn = ld4(r + g.dn), on = ld4(pold + g.dn);
-  const V4<float> rs = ld4(r + g.ds), os = ld4(pold + g.ds);
+  constexpr V4<float> Z = {0.f, 0.f, 0.f, 0.f};
+  const bool po = iter > 0;
+  const V4<float> r0 = ld4(r + g.d0), o0 = po ? ld4(pold + g.d0) : Z;
+  const V4<float> x0 = iter > 1 ? ld4(x + g.d0) : Z;
+  const V4<float> rn = ld4(r + g.dn), on = po ? ld4(pold + g.dn) : Z;
+  const V4<float> rs = ld4(r + g.ds), os = po ? ld4(pold + g.ds) : Z;
   const V4<float> ks = ld4(as + g.d0), kw = ld4(aw + g.d0);
   const V4<float> kn = asym ? ld4(an + g.d0) : ld4(as + g.dn);
   V4<float> ke = asym ? ld4(ae + g.d0) : V4<float>{0.f, 0.f, 0.f, 0.f};
   const bool west = g.cx == 0, east = g.cx == ROWT - 1;
-  const float rw = west ? r[g.dwe] : 0.f, ow = west ? pold[g.dwe] : 0.f;
-  const float re = east ? r[g.dee] : 0.f, oe = east ? pold[g.dee] : 0.f;
+  const float rw = west ? r[g.dwe] : 0.f, ow = west && po ? pold[g.dwe] : 0.f;
+  const float re = east ? r[g.dee] : 0.f, oe = east && po ? pold[g.dee] : 0.f;
   const float kwe_edge = (east && !asym) ? aw[g.dee] : 0.f;
   const V4<float> p = {fmaf(beta, o0.x, r0.x), fmaf(beta, o0.y, r0.y), fmaf(beta, o0.z, r0.z),
                        fmaf(beta, o0.w, r0.w)};
@@ -805,7 +809,7 @@ __device__ __forceinline__ double matvec_row_scaled(const RowGeo &g, bool valid,
   }
   const V4<float> a = scaled_ap(p, ps, pn, pw, pe, ks, kn, kw, ke);
   if (!valid) return 0.0;
-  if (dox) st4(x + g.d0, x_plus_alpha_p(x0, alpha_prev, o0));
+  if (po) st4(x + g.d0, x_plus_alpha_p(x0, alpha_prev, o0));
   st4(pnew + g.d0, p);
   st4(ap + g.d0, a);
   return dot4(a, p);
@@ -874,13 +878,13 @@ __device__ __forceinline__ void update_row_poly(const RowGeo &g, bool valid,
   rr += dot4(rn0, rn0);
 }
 
-// MIXED: z0 = (2I - Ahat) r (or r) for the first inner iteration, p_old = 0,
-// and the part of r.z.
+// MIXED: z0 = (2I - Ahat) r (or r) for the first inner iteration, and the part
+// of r.z.
 __device__ __forceinline__ double zinit_row(const RowGeo &g, bool valid,
                                            const float *__restrict__ r,
                                            const float *__restrict__ as,
                                            const float *__restrict__ aw, float *__restrict__ z,
-                                           float *__restrict__ pold, bool poly) {
+                                           bool poly) {
   // every load first, so that one round trip serves the row
   const V4<float> r0 = ld4(r + g.d0);
   V4<float> rN{}, rS{}, ks{}, kw{}, kn{};
@@ -910,7 +914,6 @@ __device__ __forceinline__ double zinit_row(const RowGeo &g, bool valid,
   }
   if (!valid) return 0.0;
   st4(z + g.d0, zv);
-  st4(pold + g.d0, V4<float>{0.f, 0.f, 0.f, 0.f});
   return dot4(r0, zv);
 }
 

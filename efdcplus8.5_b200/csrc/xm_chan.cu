@@ -313,7 +313,6 @@ __global__ void k_chan_resmx(DevStatic S, SysView V, DevSystem Y, const double *
       const float r32o = Y.r32[d];
       const float r32n = float(r * inv_sqrt_diag(V.cc[d]));
       Y.r32[d] = r32n;
-      Y.pa32[d] = r32n;
       part[q] += r * r - r5 * r5;
       part[size_t(S.nquad) + q] +=
           double(r32n) * double(r32n) - double(r32o) * double(r32o);

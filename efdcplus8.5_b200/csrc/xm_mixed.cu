@@ -35,7 +35,8 @@ template <bool MA, int VAR, bool FOLD>
 __global__ void __launch_bounds__(NT, MX_CTAS) k_mx_matvec(DevStatic S, DevSystem Y, Ctl *ctl,
                                                     double *part) {
   struct A {
-    bool skip, asym, dox;
+    bool skip, asym;
+    int iter;
     float beta, alpha;
     const float *pold;
     float *pnew;
@@ -48,15 +49,14 @@ __global__ void __launch_bounds__(NT, MX_CTAS) k_mx_matvec(DevStatic S, DevSyste
         const bool par = k.parity;
         const bool asym = unsym<MA>(k);
         const bool poly = Y.mpoly[m] && !asym;
-        // after the pass's first iteration: the previous x += alpha*p, with
-        // p_old that p and alpha still the previous ALPHA
-        return A{(k.done | k.idone) != 0, asym, k.inner_iter > 0, float(k.beta),
+        // (alpha: still the previous ALPHA)
+        return A{(k.done | k.idone) != 0, asym, k.inner_iter, float(k.beta),
                  float(k.alpha), par ? Y.pb32 : Y.pa32, par ? Y.pa32 : Y.pb32,
                  poly ? Y.z32 : (par ? Y.r32b : Y.r32)};
       },
       [&](const A &a, const RowGeo &g, bool valid, double *v) {
         v[0] = matvec_row_scaled(g, valid, a.z, a.pold, a.pnew, Y.as32, Y.aw32, Y.ae32,
-                                 Y.an32, Y.ap32, a.beta, a.asym, Y.x32, a.alpha, a.dox);
+                                 Y.an32, Y.ap32, a.beta, a.asym, Y.x32, a.alpha, a.iter);
       },
       fold_if<FOLD>(ctl, [&](int m, const double *sum) {
         if (threadIdx.x == 0) cg_matvec_epi(ctl[m], sum[0]);
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(NT) k_red_mx_update(DevStatic S, Ctl *ctl, Glo
 }
 
 // First inner iteration of the polynomial members: z0 = (2I - Ahat) r0,
-// p_old = 0, RPCG = r0.z0 (Jacobi members start from k_mx_resid's p0 = r0).
+// RPCG = r0.z0 (Jacobi members: z0 = r0, k_mx_resid's sum).
 template <bool FOLD>
 __global__ void __launch_bounds__(NT) k_mx_zinit(DevStatic S, DevSystem Y, Ctl *ctl,
                                                 double *part) {
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(NT) k_mx_zinit(DevStatic S, DevSystem Y, Ctl *
       S, part,
       [&](int m) { return A{ctl[m].done != 0 || !Y.mpoly[m] || unsym<true>(ctl[m]), false}; },
       [&](const A &, const RowGeo &g, bool valid, double *v) {
-        v[0] = zinit_row(g, valid, Y.r32, Y.as32, Y.aw32, Y.z32, Y.pa32, true);
+        v[0] = zinit_row(g, valid, Y.r32, Y.as32, Y.aw32, Y.z32, true);
       },
       fold_if<FOLD>(ctl, [&](int m, const double *sum) {
         if (threadIdx.x == 0) ctl[m].rpcg = sum[0];
@@ -196,7 +196,8 @@ template <bool MA, bool FOLD>
 __global__ void __launch_bounds__(NT, 3) k_mx_matvec_st(DevStatic S, DevSystem Y, Ctl *ctl,
                                                        double *part) {
   struct A {
-    bool skip, asym, dox;
+    bool skip, asym;
+    int iter;
     float beta, alpha;
     float *pnew;
     const float *b[4];
@@ -209,7 +210,7 @@ __global__ void __launch_bounds__(NT, 3) k_mx_matvec_st(DevStatic S, DevSystem Y
         const bool asym = unsym<MA>(k);
         const bool poly = Y.mpoly[m] && !asym;
         const float *z = poly ? Y.z32 : (par ? Y.r32b : Y.r32);
-        return A{(k.done | k.idone) != 0, asym, k.inner_iter > 0, float(k.beta), float(k.alpha),
+        return A{(k.done | k.idone) != 0, asym, k.inner_iter, float(k.beta), float(k.alpha),
                  par ? Y.pa32 : Y.pb32, {z, par ? Y.pb32 : Y.pa32, Y.as32, Y.aw32}};
       },
       [&](const A &a, const RowGeo &g, const StageRow &row) {
@@ -236,9 +237,13 @@ __global__ void __launch_bounds__(NT, 3) k_mx_matvec_st(DevStatic S, DevSystem Y
       [&](const A &a, const MvStage &st, const StageRow &row, const RowGeo &g, bool valid,
           const Halo &e, double *v) {
         const float beta = a.beta;
-        const V4<float> r0 = st_body(st, 0, row), o0 = st_body(st, 1, row);
-        const V4<float> rn = st_north(st, 0, row, e.h0), on = st_north(st, 1, row, e.h1);
-        const V4<float> rs = st_south(st, 0, row, e.h0), os = st_south(st, 1, row, e.h1);
+        constexpr V4<float> Z = {0.f, 0.f, 0.f, 0.f};
+        const bool po = a.iter > 0;  // (the first p_old and x: zeros, not stored)
+        const V4<float> r0 = st_body(st, 0, row), o0 = po ? st_body(st, 1, row) : Z;
+        const V4<float> rn = st_north(st, 0, row, e.h0),
+                        on = po ? st_north(st, 1, row, e.h1) : Z;
+        const V4<float> rs = st_south(st, 0, row, e.h0),
+                        os = po ? st_south(st, 1, row, e.h1) : Z;
         const V4<float> p = {fmaf(beta, o0.x, r0.x), fmaf(beta, o0.y, r0.y),
                              fmaf(beta, o0.z, r0.z), fmaf(beta, o0.w, r0.w)};
         const V4<float> pn = {fmaf(beta, on.x, rn.x), fmaf(beta, on.y, rn.y),
@@ -246,8 +251,8 @@ __global__ void __launch_bounds__(NT, 3) k_mx_matvec_st(DevStatic S, DevSystem Y
         const V4<float> ps = {fmaf(beta, os.x, rs.x), fmaf(beta, os.y, rs.y),
                               fmaf(beta, os.z, rs.z), fmaf(beta, os.w, rs.w)};
         float pw = from_west(p), pe = from_east(p);
-        if (g.cx == 0) pw = fmaf(beta, e.w1, e.w0);
-        if (g.cx == ROWT - 1) pe = fmaf(beta, e.e1, e.e0);
+        if (g.cx == 0) pw = fmaf(beta, po ? e.w1 : 0.f, e.w0);
+        if (g.cx == ROWT - 1) pe = fmaf(beta, po ? e.e1 : 0.f, e.e0);
         const V4<float> ks = st_body(st, 2, row), kw = st_body(st, 3, row);
         V4<float> kn, ke;
         if (a.asym) {
@@ -261,7 +266,8 @@ __global__ void __launch_bounds__(NT, 3) k_mx_matvec_st(DevStatic S, DevSystem Y
         }
         const V4<float> ap = scaled_ap(p, ps, pn, pw, pe, ks, kn, kw, ke);
         if (!valid) return;
-        if (a.dox) st4(Y.x32 + g.d0, x_plus_alpha_p(ld4(Y.x32 + g.d0), a.alpha, o0));
+        if (po)
+          st4(Y.x32 + g.d0, x_plus_alpha_p(a.iter > 1 ? ld4(Y.x32 + g.d0) : Z, a.alpha, o0));
         st4(a.pnew + g.d0, p);
         st4(Y.ap32 + g.d0, ap);
         v[0] = dot4(ap, p);

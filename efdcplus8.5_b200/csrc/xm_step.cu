@@ -713,9 +713,8 @@ __global__ void __launch_bounds__(NT) k_cg_finish(DevStatic S, DevSystem Y, doub
 
 // ---------------------------------------------------------------------------
 // MIXED outer step: r = b - A*P in FP64 (the FP64 refinement residual), RSQ
-// in FP64, and the FP32 scaled inner system's rhs rhat = D^-1/2 r with
-// x = 0 and p0 = rhat (k_mx_zinit then forms z0 = M^-1 rhat and p_old = 0 for
-// the polynomial members).  rsqm_fac scales the member's RSQM (the MIXED stop,
+// in FP64, and the FP32 scaled inner system's rhs rhat = D^-1/2 r (k_mx_zinit
+// then forms z0 = M^-1 rhat for the polynomial members).  rsqm_fac scales the member's RSQM (the MIXED stop,
 // below RSQM).
 __device__ __forceinline__ void mx_resid_epi(Ctl &k, Glob *glob, const StepScalars &c,
                                              const RedArgs &ra, double rsq, double rz) {
@@ -738,8 +737,6 @@ __global__ void __launch_bounds__(NT) k_mx_resid(DevStatic S, SysView V, DevSyst
                                float(r.z * inv_sqrt_diag(c.z)), float(r.w * inv_sqrt_diag(c.w))};
         if (valid) {
           st4(Y.r32 + g.d0, r32);
-          st4(Y.pa32 + g.d0, r32);
-          st4(Y.x32 + g.d0, V4<float>{0.f, 0.f, 0.f, 0.f});
           v[0] = r.x * r.x + r.y * r.y + r.z * r.z + r.w * r.w;
           v[1] = double(r32.x) * double(r32.x) + double(r32.y) * double(r32.y) +
                  double(r32.z) * double(r32.z) + double(r32.w) * double(r32.w);
@@ -770,7 +767,8 @@ __global__ void __launch_bounds__(NT) k_mx_apply(DevStatic S, SysView V, DevSyst
         const V4<double> c = ld4(V.cc + g.d0);
         // the inner solution with its last iteration's alpha*p (which the
         // matrix-vector pass of a next iteration would have added)
-        V4<float> d = ld4(Y.x32 + g.d0);
+        V4<float> d = {0.f, 0.f, 0.f, 0.f};  // of one iteration: x was not stored
+        if (k.inner_iter > 1) d = ld4(Y.x32 + g.d0);
         if (k.inner_iter > 0)
           d = x_plus_alpha_p(d, float(k.alpha), ld4((k.parity ? Y.pa32 : Y.pb32) + g.d0));
         x.x = x.x + double(d.x) * inv_sqrt_diag(c.x);
