@@ -42,6 +42,11 @@ struct CopyJob {
   void *dev;               // tile-order device array
   int is_int;              // 0 double, 1 LOGICAL (0/1), 2 raw int, 3 double water-only
 };
+// The jobs of a small transfer, as a kernel argument.
+struct JobTable {
+  static constexpr int CAP = 64;
+  CopyJob j[CAP];
+};
 
 // copy: the two-level advance as per-cell copies (a subset of the members
 // steps), else the host has swapped the buffers
@@ -169,6 +174,11 @@ void launch_scatter(cudaStream_t st, const CopyJob *jobs, int njob, const int *l
                     int d1);
 void launch_gather(cudaStream_t st, const CopyJob *jobs, int njob, const int *lidx,
                    const int *tile_member, const long long *moff, int d0, int d1);
+void launch_scatter_table(cudaStream_t st, const JobTable &jobs, int njob, const int *lidx,
+                          const int *tile_member, const long long *moff, const int *mlc, int d0,
+                          int d1);
+void launch_gather_table(cudaStream_t st, const JobTable &jobs, int njob, const int *lidx,
+                         const int *tile_member, const long long *moff, int d0, int d1);
 void launch_sys_prepare(const Launch &l, const DevStatic &S, const DevSystem &Y, Ctl *ctl,
                         int mixed);
 

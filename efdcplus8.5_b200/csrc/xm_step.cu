@@ -1199,11 +1199,9 @@ __global__ void __launch_bounds__(NT) k_fin(DevStatic S, DevState X, int ntile, 
 // back to back (member m at element offset moff[m], LC = mlc[m] elements).  A
 // land slot receives element LC of its member's array (the ghost value);
 // gathers write water slots only.  Both cover the slots [d0, d1).
-__global__ void k_scatter(const CopyJob *jobs, int njob, const int *lidx, const int *tile_member,
-                          const long long *moff, const int *mlc, int d0, int d1) {
-  const int j = blockIdx.y;
-  if (j >= njob) return;
-  const CopyJob J = jobs[j];
+__device__ __forceinline__ void scatter_job(const CopyJob &J, const int *lidx,
+                                            const int *tile_member, const long long *moff,
+                                            const int *mlc, int d0, int d1) {
   for (int d = d0 + blockIdx.x * blockDim.x + threadIdx.x; d < d1; d += gridDim.x * blockDim.x) {
     const int L = lidx[d];
     if (L < 2 && J.is_int == 3) continue;  // water-only: leave land slots as they are
@@ -1218,11 +1216,9 @@ __global__ void k_scatter(const CopyJob *jobs, int njob, const int *lidx, const 
   }
 }
 
-__global__ void k_gather(const CopyJob *jobs, int njob, const int *lidx, const int *tile_member,
-                         const long long *moff, int d0, int d1) {
-  const int j = blockIdx.y;
-  if (j >= njob) return;
-  const CopyJob J = jobs[j];
+__device__ __forceinline__ void gather_job(const CopyJob &J, const int *lidx,
+                                           const int *tile_member, const long long *moff, int d0,
+                                           int d1) {
   for (int d = d0 + blockIdx.x * blockDim.x + threadIdx.x; d < d1; d += gridDim.x * blockDim.x) {
     const int L = lidx[d];
     if (L < 2) continue;
@@ -1233,6 +1229,24 @@ __global__ void k_gather(const CopyJob *jobs, int njob, const int *lidx, const i
       static_cast<double *>(const_cast<void *>(J.host_order))[dst] =
           static_cast<const double *>(J.dev)[d];
   }
+}
+// The jobs from memory, or (small transfers) from the kernel's arguments.
+__global__ void k_scatter(const CopyJob *jobs, const int *lidx, const int *tile_member,
+                          const long long *moff, const int *mlc, int d0, int d1) {
+  scatter_job(jobs[blockIdx.y], lidx, tile_member, moff, mlc, d0, d1);
+}
+__global__ void k_scatter_table(const __grid_constant__ JobTable jobs, const int *lidx,
+                                const int *tile_member, const long long *moff, const int *mlc,
+                                int d0, int d1) {
+  scatter_job(jobs.j[blockIdx.y], lidx, tile_member, moff, mlc, d0, d1);
+}
+__global__ void k_gather(const CopyJob *jobs, const int *lidx, const int *tile_member,
+                         const long long *moff, int d0, int d1) {
+  gather_job(jobs[blockIdx.y], lidx, tile_member, moff, d0, d1);
+}
+__global__ void k_gather_table(const __grid_constant__ JobTable jobs, const int *lidx,
+                               const int *tile_member, const long long *moff, int d0, int d1) {
+  gather_job(jobs.j[blockIdx.y], lidx, tile_member, moff, d0, d1);
 }
 
 // ---------------------------------------------------------------------------
@@ -1672,14 +1686,29 @@ void launch_scatter(cudaStream_t st, const CopyJob *jobs, int njob, const int *l
                     int d1) {
   if (njob == 0 || d1 <= d0) return;
   dim3 g(std::min((d1 - d0 + 255) / 256, 2048), njob);
-  k_scatter<<<g, 256, 0, st>>>(jobs, njob, lidx, tile_member, moff, mlc, d0, d1);
+  k_scatter<<<g, 256, 0, st>>>(jobs, lidx, tile_member, moff, mlc, d0, d1);
   count_launches(1);
 }
 void launch_gather(cudaStream_t st, const CopyJob *jobs, int njob, const int *lidx,
                    const int *tile_member, const long long *moff, int d0, int d1) {
   if (njob == 0 || d1 <= d0) return;
   dim3 g(std::min((d1 - d0 + 255) / 256, 2048), njob);
-  k_gather<<<g, 256, 0, st>>>(jobs, njob, lidx, tile_member, moff, d0, d1);
+  k_gather<<<g, 256, 0, st>>>(jobs, lidx, tile_member, moff, d0, d1);
+  count_launches(1);
+}
+void launch_scatter_table(cudaStream_t st, const JobTable &jobs, int njob, const int *lidx,
+                          const int *tile_member, const long long *moff, const int *mlc, int d0,
+                          int d1) {
+  if (njob == 0 || d1 <= d0) return;
+  dim3 g(std::min((d1 - d0 + 255) / 256, 2048), njob);
+  k_scatter_table<<<g, 256, 0, st>>>(jobs, lidx, tile_member, moff, mlc, d0, d1);
+  count_launches(1);
+}
+void launch_gather_table(cudaStream_t st, const JobTable &jobs, int njob, const int *lidx,
+                         const int *tile_member, const long long *moff, int d0, int d1) {
+  if (njob == 0 || d1 <= d0) return;
+  dim3 g(std::min((d1 - d0 + 255) / 256, 2048), njob);
+  k_gather_table<<<g, 256, 0, st>>>(jobs, lidx, tile_member, moff, d0, d1);
   count_launches(1);
 }
 void launch_sys_prepare(const Launch &l, const DevStatic &S, const DevSystem &Y, Ctl *ctl,

@@ -387,20 +387,26 @@ def same_bits(names) -> int:
     return b
 
 
+_FIELD_WORDS = [(k, getattr(Fields, k).offset // 8, np.dtype(d))
+                for names, d in ((FIELD_DOUBLE_INOUT + FIELD_IN + FIELD_OUT + FIELD_CHAN +
+                                  FIELD_TL3 + FIELD_DRAG, np.float64), (FIELD_INT_INOUT, np.int32))
+                for k in names]
+
+
 def make_fields(st: dict, *, diag: bool = False, lists: bool = False, unchanged: int = 0):
     """Build a Fields struct over the numpy arrays of a state dict (in place).
     unchanged: efdc_xm_fields.unchanged (see same_bits)."""
     s = Fields()
     s.unchanged = unchanged
     keep = []
-    for k in FIELD_DOUBLE_INOUT + FIELD_IN + FIELD_OUT + FIELD_CHAN + FIELD_TL3 + FIELD_DRAG:
+    # the addresses as words of the struct: a third of the time of 31 pointer objects
+    words = np.frombuffer(s, np.uint64)
+    for k, word, dtype in _FIELD_WORDS:
         a = st.get(k)
         if a is not None:
-            setattr(s, k, _dp(a))
-    for k in FIELD_INT_INOUT:
-        a = st.get(k)
-        if a is not None:
-            setattr(s, k, _ip(a))
+            assert a.dtype == dtype and a.flags.c_contiguous
+            words[word] = a.ctypes.data
+            keep.append(a)
     for k, side in enumerate(SIDES):
         a = st["pser"].get(side) if "pser" in st else None
         if a is not None and a.size:
