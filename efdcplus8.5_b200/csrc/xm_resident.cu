@@ -15,9 +15,10 @@ __host__ __device__ constexpr bool res_lean(int Q) { return Q == 4; }
 constexpr int RES_NC = 5;  // CCC, CCS, CCW, CCN and CCCI (symmetric) or CCE (MA)
 template <int W, int Q>
 using Coef64 = ResCoef<double, W, Q, res_lean(Q) ? 2 : RES_NC, Q == 1>;  // lean: CCCI, P
-template <int W, int Q>
+template <int W, int Q, bool CLUSTER>
 constexpr size_t res_smem64() {
-  return size_t(W) * Q * TILES_PER_CTA * TILE * sizeof(double) + Coef64<W, Q>::bytes;
+  return size_t(W) * Q * TILES_PER_CTA * TILE * sizeof(double) + Coef64<W, Q>::bytes +
+         (CLUSTER ? 2 * res_edges<W, Q>() * sizeof(double) : 0);
 }
 
 // congrad.f90:54-187 for one member per group of CTAs.  What bounds it is the
@@ -49,6 +50,12 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
   C.sm = dyn + W * Q * TILES_PER_CTA * TILE;
   const bool north = res_north(), south = res_south(), west = res_west(), east = res_east();
   const int w0 = W > 1 ? int(threadIdx.x) / NT : 0;  // quad q0 + i*W + w0 is the thread's row i
+  // cluster: the edges of z and of p_old
+  constexpr int NE = res_edges<W, Q>();
+  double *edge = C.sm + Coef64<W, Q>::bytes / sizeof(double);
+  if constexpr (CLUSTER)
+    for (int t = threadIdx.x; t < 2 * RES_EDGE; t += W * NT)  // the zeros of the ghost tile
+      edge[(t < RES_EDGE ? 1 : 2) * NE - RES_EDGE + t % RES_EDGE] = 0.0;
   auto none = [] {};
 
   constexpr bool LEAN = res_lean(Q);
@@ -140,8 +147,14 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
       }
       put_x(i, X0);
       put_p(i, z);
-      st_border(Y.z, row[i], z);
-      st_border(Y.pa, row[i], z);
+      if constexpr (CLUSTER) {
+        res_peers<W, Q>(edge, me, S.quads[me.qm0].y, row[i]);
+        st_edge(edge, j, z);
+        st_edge(edge + NE, j, z);
+      } else {
+        st_border(Y.z, row[i], z);
+        st_border(Y.pa, row[i], z);
+      }
       v0[i][0] = row[i].valid ? d.x * z.x + d.y * z.y + d.z * z.z + d.w * z.w : 0.0;
     }
   }
@@ -162,13 +175,25 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
   V4<double> hz[NH], ho[NH];
   double ez[NH], eo[NH];
   auto halo_row = [&](const double *pold, int i, int h) {
-    if (north || south) {
-      hz[h] = ldx4(Y.z + row[i].hv);
-      ho[h] = ldx4(pold + row[i].hv);
-    }
-    if (west || east) {
-      ez[h] = __ldcg(Y.z + row[i].hx);
-      eo[h] = __ldcg(pold + row[i].hx);
+    if constexpr (CLUSTER) {
+      constexpr unsigned P_OLD = NE * sizeof(double);
+      if (north || south) {
+        hz[h] = ld_peer4(row[i].hv);
+        ho[h] = ld_peer4(row[i].hv + P_OLD);
+      }
+      if (west || east) {
+        ez[h] = ld_peer1(row[i].hx);
+        eo[h] = ld_peer1(row[i].hx + P_OLD);
+      }
+    } else {
+      if (north || south) {
+        hz[h] = ldx4(Y.z + row[i].hv);
+        ho[h] = ldx4(pold + row[i].hv);
+      }
+      if (west || east) {
+        ez[h] = __ldcg(Y.z + row[i].hx);
+        eo[h] = __ldcg(pold + row[i].hx);
+      }
     }
   };
   auto halo = [&](const double *pold) {
@@ -199,7 +224,7 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
         const V4<double> q = {ci.x * r[i].x + beta * po.x, ci.y * r[i].y + beta * po.y,
                               ci.z * r[i].z + beta * po.z, ci.w * r[i].w + beta * po.w};
         put_p(i, q);
-        st_border(pnew, row[i], q);
+        if constexpr (!CLUSTER) st_border(pnew, row[i], q);
       }
       __syncthreads();
 #pragma unroll
@@ -266,7 +291,12 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
         rv.w = rv.w - alpha * ap[i].w;
         r[i] = rv;
         const V4<double> z = {ci.x * rv.x, ci.y * rv.y, ci.z * rv.z, ci.w * rv.w};
-        st_border(Y.z, row[i], z);
+        if constexpr (CLUSTER) {  // p_old too: the last row work's readers are past the exchange
+          st_edge(edge, i * W + w0, z);
+          st_edge(edge + NE, i * W + w0, get_p(i));
+        } else {
+          st_border(Y.z, row[i], z);
+        }
         v[i][0] = row[i].valid ? rv.x * z.x + rv.y * z.y + rv.z * z.z + rv.w * z.w : 0.0;
         v[i][1] = row[i].valid ? rv.x * rv.x + rv.y * rv.y + rv.z * rv.z + rv.w * rv.w : 0.0;
       }
@@ -276,6 +306,7 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
       fin = cg_update_step(k, rsqm, iterm, sum[0], sum[1], 0);
     }
   }
+  if constexpr (CLUSTER) cluster_barrier();  // the edges have been read
   if (k.iter > 0) {  // :133 of the last iteration
     const double alpha = k.alpha;
 #pragma unroll
@@ -310,8 +341,8 @@ int cg_res_capacity(const ResForm &f, bool may_asym, int nsm) {
     constexpr int W = decltype(w)::value, Q = decltype(q)::value;
     constexpr bool CL = decltype(cl)::value;
     cap = may_asym
-              ? res_cap(k_cg_res<true, W, Q, CL>, NT * W, res_smem64<W, Q>(), nsm, f.cluster)
-              : res_cap(k_cg_res<false, W, Q, CL>, NT * W, res_smem64<W, Q>(), nsm, f.cluster);
+              ? res_cap(k_cg_res<true, W, Q, CL>, NT * W, res_smem64<W, Q, CL>(), nsm, f.cluster)
+              : res_cap(k_cg_res<false, W, Q, CL>, NT * W, res_smem64<W, Q, CL>(), nsm, f.cluster);
   });
   return cap;
 }
@@ -323,10 +354,10 @@ void launch_cg_res(const Launch &l, const DevStatic &S, const SysView &V, const 
     constexpr int W = decltype(w)::value, Q = decltype(q)::value;
     constexpr bool CL = decltype(cl)::value;
     if (l.may_asym)
-      launch_resident(k_cg_res<true, W, Q, CL>, ncta, NT * W, res_smem64<W, Q>(), f.cluster,
+      launch_resident(k_cg_res<true, W, Q, CL>, ncta, NT * W, res_smem64<W, Q, CL>(), f.cluster,
                       l.stream, S, V, Y, P, ctl, glob, R, ends);
     else
-      launch_resident(k_cg_res<false, W, Q, CL>, ncta, NT * W, res_smem64<W, Q>(), f.cluster,
+      launch_resident(k_cg_res<false, W, Q, CL>, ncta, NT * W, res_smem64<W, Q, CL>(), f.cluster,
                       l.stream, S, V, Y, P, ctl, glob, R, ends);
   });
   count_launches(1);

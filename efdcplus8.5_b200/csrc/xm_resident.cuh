@@ -5,8 +5,8 @@
 // with W quads side by side (256*W threads) and Q such rows of quads one after
 // another, a thread holding its row vectors of each quad in registers from the
 // first residual to the stop test.  What leaves a CTA is the border of its
-// tiles (the rows and columns a neighbour tile reads), through L2, and one
-// partial sum per quad.  The multi-kernel CG pays two kernel boundaries per
+// tiles (the rows and columns a neighbour tile reads) and one partial sum per
+// quad, through L2 (FP64 clusters: through shared memory).  The multi-kernel CG pays two kernel boundaries per
 // iteration (launch, ramp, tail and a folded reduction: 7 us each on a
 // 60,000-cell basin whose row work is below 1 us); here a boundary is one
 // exchange between the CTAs of the member, which is also their barrier:
@@ -135,6 +135,64 @@ __device__ __forceinline__ void st_stage(float *p, const V4<float> &v) { st4(p, 
 __device__ __forceinline__ void st_stage(double *p, const V4<double> &v) {
   *reinterpret_cast<double2 *>(p) = make_double2(v.x, v.y);
   *reinterpret_cast<double2 *>(p + TX / 2) = make_double2(v.z, v.w);
+}
+
+// Cluster groups hold what their CTAs read of one another's tiles in shared memory:
+// the borders of the CTA's tiles in two vectors (z and p_old), a tile as [S row][N row]
+// [W column][E column], and past the last tile one of zeros for the ghost tile (where
+// every vector is zero).  In global memory they cost the cluster barrier the stores'
+// round trip to L2 and the row work behind it another: FP64 steps of 44x28 cells 0.088
+// -> 0.079 ms, 60x60 0.091 -> 0.083, 180x150 0.115 -> 0.105, 260x250 (four quads a CTA,
+// bound by its row work) 0.131 -> 0.130.
+constexpr int RES_EDGE = 2 * TX + 2 * TY;
+template <int W, int Q>
+__host__ __device__ constexpr int res_edges() {  // elements of one vector
+  return (W * Q * TILES_PER_CTA + 1) * RES_EDGE;
+}
+__device__ __forceinline__ void ld_peer(unsigned a, double &x, double &y) {
+  asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(x), "=d"(y) : "r"(a) : "memory");
+}
+__device__ __forceinline__ V4<double> ld_peer4(unsigned a) {  // a row: see res_stage
+  V4<double> v;
+  ld_peer(a, v.x, v.y);
+  ld_peer(a + TX / 2 * sizeof(double), v.z, v.w);
+  return v;
+}
+__device__ __forceinline__ double ld_peer1(unsigned a) {
+  double x;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(x) : "r"(a) : "memory");
+  return x;
+}
+// The row's hv and hx: no slots, the addresses of those cells in the CTAs' edges.
+template <int W, int Q>
+__device__ __forceinline__ void res_peers(const double *edge, const ResCta &c, int t0,
+                                          ResRow &r) {
+  const int q = res_q(), cx = q % ROWT, ty = q / ROWT;
+  auto at = [&](int slot, int e) {
+    const int lt = slot / TILE - t0;  // before the member's tiles: a ghost tile
+    const int j = lt < 0 ? W * Q : lt / TILES_PER_CTA % (W * Q);
+    const int rank = lt < 0 ? (c.q0 - c.qm0) / (W * Q) : lt / TILES_PER_CTA / (W * Q);
+    const double *p = edge + (j * TILES_PER_CTA + (lt < 0 ? 0 : lt % TILES_PER_CTA)) * RES_EDGE + e;
+    unsigned a = unsigned(__cvta_generic_to_shared(p)), peer;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(a), "r"(rank));
+    return int(peer);
+  };
+  r.hv = at(r.hv, (res_north() ? 0 : TX) + 2 * cx);
+  r.hx = at(r.hx, 2 * TX + (res_west() ? TY : 0) + ty);
+}
+// The thread's part of its tile's edge (j: the quad of the CTA).
+__device__ __forceinline__ void st_edge(double *edge, int j, const V4<double> &v) {
+  const int q = res_q(), cx = q % ROWT, ty = q / ROWT;
+  double *e = edge + (j * TILES_PER_CTA + threadIdx.x % NT / TPT) * RES_EDGE;
+  if (res_north() || res_south()) {
+    double2 *p = reinterpret_cast<double2 *>(e + (res_north() ? TX : 0) + 2 * cx);
+    p[0] = make_double2(v.x, v.y);
+    p[TX / 4] = make_double2(v.z, v.w);
+  }
+  if (res_west())
+    e[2 * TX + ty] = v.x;
+  else if (res_east())
+    e[2 * TX + TY + ty] = v.w;
 }
 
 constexpr int RES_CLUSTER_QUADS = 128;  // of a member in a cluster, at most
