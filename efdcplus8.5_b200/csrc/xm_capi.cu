@@ -644,7 +644,9 @@ size_t group_size(efdc_xm_ctx *c, size_t n) {
   return g;
 }
 
-int upload_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs, bool wait = true) {
+// ring = false: without the ring of pageable arrays.
+int upload_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs, bool wait = true,
+                  bool ring = true) {
   if (xs.empty()) return EFDC_XM_OK;
   if (xs.size() > size_t(MAX_JOBS)) {
     set_error("internal: too many arrays in one transfer");
@@ -652,7 +654,6 @@ int upload_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs, bool wait = true)
   }
   if (packed(c, xs.size())) return upload_packed(c, xs, wait);
   const size_t G = group_size(c, xs.size());
-  const bool pieces = pieces_ready(c);
   for (size_t j = 0; j < xs.size(); ++j)
     c->jobs_h[j] = CopyJob{c->stage[j % G], xs[j].dev, xs[j].kind};
   CK(cudaMemcpyAsync(c->jobs_d, c->jobs_h, xs.size() * sizeof(CopyJob), cudaMemcpyHostToDevice,
@@ -665,7 +666,7 @@ int upload_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs, bool wait = true)
     std::vector<Piece> v;
     for (size_t j = g0; j < g1; ++j) {
       char *stage = reinterpret_cast<char *>(c->stage[j % G]);
-      if (pieces && pageable(c, xs[j])) {
+      if (ring && pageable(c, xs[j]) && pieces_ready(c)) {
         const size_t es = esize(xs[j].kind);
         for (int m = 0; m < c->M; ++m)
           add_pieces(v, static_cast<char *>(const_cast<void *>(xs[j].host[m])),
@@ -692,7 +693,6 @@ int download_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs) {
   }
   if (packed(c, xs.size())) return download_packed(c, xs);
   const size_t G = group_size(c, xs.size());
-  const bool pieces = pieces_ready(c);
   for (size_t j = 0; j < xs.size(); ++j)
     c->jobs_h[j] = CopyJob{c->stage[j % G], xs[j].dev, xs[j].kind};
   CK(cudaMemcpyAsync(c->jobs_d, c->jobs_h, xs.size() * sizeof(CopyJob), cudaMemcpyHostToDevice,
@@ -709,7 +709,7 @@ int download_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs) {
     std::vector<Piece> v;
     for (size_t j = g0; j < g1; ++j) {
       char *stage = reinterpret_cast<char *>(c->stage[j % G]);
-      if (pieces && pageable(c, xs[j])) {
+      if (pageable(c, xs[j]) && pieces_ready(c)) {
         const size_t es = esize(xs[j].kind);
         for (int m = 0; m < c->M; ++m)  // the water elements L = 2..LA
           add_pieces(v, static_cast<char *>(const_cast<void *>(xs[j].host[m])) + es,
@@ -1642,7 +1642,8 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
       {&efdc_xm_grid::sbxo, st[12]},  {&efdc_xm_grid::sbyo, st[13]}, {&efdc_xm_grid::belv, st[14]}};
   std::vector<Xfer> xs;
   for (const auto &mt : metrics) xs.push_back(Xfer{per(mt.first), mt.second, 0});
-  if (upload_arrays(c, xs) != EFDC_XM_OK) return bail("upload of the static arrays failed");
+  if (upload_arrays(c, xs, true, false) != EFDC_XM_OK)
+    return bail("upload of the static arrays failed");
   if (cudaDeviceSynchronize() != cudaSuccess) return bail("device error during set-up");
   for (int m = 0; m < M; ++m) c->mem[m].slot_of = std::move(slot_of[m]);
   return c;
@@ -1929,7 +1930,9 @@ int upload_batch(efdc_xm_ctx *c, const efdc_xm_fields *f, bool skip_wetdry, bool
   std::vector<Xfer> xs;
   uint32_t sent = 0;
   int rc = plan_upload(c, f, skip_wetdry, skip_sbxy, levels, xs, &sent);
-  if (!rc) rc = upload_arrays(c, xs, false);  // upload_small waits
+  // (upload_small waits); an upload by itself may be the only one: it sets up no ring,
+  // whose page-locking takes several milliseconds
+  if (!rc) rc = upload_arrays(c, xs, false, !wait || c->ring_h);
   if (!rc && !levels) rc = copy_levels(c, f, 0, size_t(c->nslot), c->stream);
   if (!rc) rc = upload_small(c, f, wait);
   if (rc) {

@@ -28,6 +28,9 @@
 // the multi-kernel CG: the iterates are equal bit for bit.
 #pragma once
 
+#include <map>
+#include <mutex>
+#include <tuple>
 #include <utility>
 
 #include "xm_cg.cuh"
@@ -419,7 +422,17 @@ int res_cap(K kernel, int threads, size_t smem, int nsm, int cluster) {
     cfg.dynamicSmemBytes = smem;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
+    // (a millisecond; the answer is the device's: asked once per kernel and size)
+    static std::mutex mu;
+    static std::map<std::tuple<int, const void *, int>, int> known;
+    int dev = 0;
+    ok = ok && cudaGetDevice(&dev) == cudaSuccess;
+    std::lock_guard<std::mutex> lock(mu);
+    const auto key = std::make_tuple(dev, reinterpret_cast<const void *>(kernel), cluster);
+    const auto it = known.find(key);
+    if (it != known.end()) return ok ? it->second : 0;
     ok = ok && cudaOccupancyMaxActiveClusters(&b, kernel, &cfg) == cudaSuccess;
+    if (ok) known[key] = b;
   } else {
     ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, threads, smem) ==
                    cudaSuccess;
