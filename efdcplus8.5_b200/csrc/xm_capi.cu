@@ -857,14 +857,17 @@ bool resident_solve(const efdc_xm_ctx *c, bool mixed) {
 // 1.46 against 1.72 ms per step) and slower in MIXED (1.29 against 1.16 ms).  Four
 // rows of quads exist in FP64 only: of the same form in MIXED, a basin of 770,000
 // cells took 0.50 ms against the multi-kernel CG's 0.49, one of a million 0.53
-// against 0.56.
+// against 0.56.  Two quads a CTA: one after another in FP64, each thread with the
+// registers of two (500x500 cells 0.186 -> 0.177 ms per step, 160x150 0.102 -> 0.099),
+// side by side in MIXED (0.159 against 0.173 and 0.110 against 0.119).
+const std::vector<xm::ResForm> FORMS64 = {{1, 1, 0}, {1, 2, 0}, {2, 2, 0}, {2, 4, 0}};
+const std::vector<xm::ResForm> FORMS32 = {{1, 1, 0}, {2, 1, 0}, {2, 2, 0}};
 bool build_resident(efdc_xm_ctx *c, int (*capacity)(const xm::ResForm &, bool, int),
-                    size_t max_waves, ResSet &out) {
+                    const std::vector<xm::ResForm> &forms, size_t max_waves, ResSet &out) {
   const int M = c->M, mq = c->max_units;
   auto cap_of = [&](const xm::ResForm &f) {
     return std::min(capacity(f, false, c->nsm), capacity(f, true, c->nsm));
   };
-  constexpr xm::ResForm forms[] = {{1, 1, 0}, {2, 1, 0}, {2, 2, 0}, {2, 4, 0}};
   for (xm::ResForm f : forms) {
     const int per = f.w * f.q, n = (mq + per - 1) / per;
     if (n > 16) continue;
@@ -876,7 +879,7 @@ bool build_resident(efdc_xm_ctx *c, int (*capacity)(const xm::ResForm &, bool, i
   }
   for (const xm::ResForm &f : forms) {
     const int per = f.w * f.q, cap = cap_of(f);
-    const bool last = &f == std::end(forms) - 1;
+    const bool last = &f == &forms.back();
     // one CTA per SM exchanges faster than two: the narrow form only up to there
     const int lim = f.w == 1 ? std::min(cap, c->nsm) : cap;
     std::vector<int4> cta;
@@ -1491,8 +1494,8 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
   c->qstart_h = qstart;
   for (int m = 0; m < M; ++m) c->max_units = std::max(c->max_units, qstart[m + 1] - qstart[m]);
   c->has_layers.assign(M, 0);
-  if (reset_resident(c) || !build_resident(c, xm::cg_res_capacity, SIZE_MAX, c->res64) ||
-      !build_resident(c, xm::mx_res_capacity, 1, c->res32))
+  if (reset_resident(c) || !build_resident(c, xm::cg_res_capacity, FORMS64, SIZE_MAX, c->res64) ||
+      !build_resident(c, xm::mx_res_capacity, FORMS32, 1, c->res32))
     return bail("cudaMalloc failed (resident solves)");
   cudaMemcpy(quads_d, quads.data(), quads.size() * sizeof(int4), cudaMemcpyHostToDevice);
   cudaMemcpy(qstart_d, qstart.data(), (M + 1) * sizeof(int), cudaMemcpyHostToDevice);

@@ -6,15 +6,15 @@
 
 namespace xm {
 
-// What a form keeps where.  One row of quads: the coefficients in registers.  Two:
-// in shared memory.  Four (the lean form): P and PCG live in shared memory too --
+// What a form keeps where.  One quad side by side: the coefficients in registers.
+// Two by two: in shared memory.  Four (the lean form): P and PCG live in shared memory too --
 // PCG where the rows above and below read it anyway --, CCCI as well, and the
 // other coefficients are read and scaled anew (24 of the 112 B per cell-iteration
 // of the multi-kernel CG, from L2).
 __host__ __device__ constexpr bool res_lean(int Q) { return Q == 4; }
 constexpr int RES_NC = 5;  // CCC, CCS, CCW, CCN and CCCI (symmetric) or CCE (MA)
 template <int W, int Q>
-using Coef64 = ResCoef<double, W, Q, res_lean(Q) ? 2 : RES_NC, Q == 1>;  // lean: CCCI, P
+using Coef64 = ResCoef<double, W, Q, res_lean(Q) ? 2 : RES_NC, Q == 1 || W == 1>;  // lean: CCCI, P
 template <int W, int Q, bool CLUSTER>
 constexpr size_t res_smem64() {
   return size_t(W) * Q * TILES_PER_CTA * TILE * sizeof(double) + Coef64<W, Q>::bytes +
@@ -29,10 +29,10 @@ constexpr size_t res_smem64() {
 // 0.57 -> 0.33, 256 lakes of 1,100 cells in one batch 0.50 -> 0.38; lean: 900x860
 // 0.65 -> 0.49, 1,000x1,000 0.80 -> 0.56 (an iteration 31 -> 20 us, of which the row
 // work is 13, the exchanges' waits for the slowest CTA 3 and the exchanges 4).
-// 128 registers a thread: one row of quads keeps the coefficients in registers
-// too, two keep them in shared memory, four read them (see res_lean).
+// Registers: one quad side by side keeps the coefficients there too (255 a thread with
+// two rows), two by two (128 a thread) in shared memory; the lean form reads them.
 template <bool MA, int W, int Q, bool CLUSTER>
-__global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
+__global__ void __launch_bounds__(NT *W, W == 1 && Q == 1 && CLUSTER ? 2 : 1)
     k_cg_res(DevStatic S, SysView V, DevSystem Y, double *P, Ctl *ctl, Glob *glob, ResPlan R,
              ResEnds ends) {
   extern __shared__ __align__(16) double dyn[];

@@ -470,8 +470,8 @@ void launch_resident(void (*kernel)(P...), int ncta, int threads, size_t smem, i
 }
 
 // Calls go with a form as compile-time constants; false for one that is not
-// compiled (LEAN: four rows of quads are, for grid groups).
-template <bool LEAN, class F>
+// compiled (F64: for FP64).
+template <bool F64, class F>
 bool res_form(const ResForm &f, F &&go) {
   auto call = [&](auto w, auto q) {
     if (f.cluster > 0)
@@ -483,11 +483,14 @@ bool res_form(const ResForm &f, F &&go) {
   using I1 = std::integral_constant<int, 1>;
   using I2 = std::integral_constant<int, 2>;
   if (f.w == 1 && f.q == 1) return call(I1{}, I1{});
-  if (f.w == 2 && f.q == 1) return call(I2{}, I1{});
   if (f.w == 2 && f.q == 2) return call(I2{}, I2{});
-  if constexpr (LEAN)
+  if constexpr (F64) {
+    if (f.w == 1 && f.q == 2) return call(I1{}, I2{});
     if (f.w == 2 && f.q == 4 && f.cluster == 0)
       return go(I2{}, std::integral_constant<int, 4>{}, std::false_type{}), true;
+  } else {
+    if (f.w == 2 && f.q == 1) return call(I2{}, I1{});
+  }
   return false;
 }
 
