@@ -66,7 +66,7 @@ constexpr int NSTAGE = 8;     // staging buffers (each holds one array of every 
 constexpr int NCHUNK = 32;    // most member chunks of a pipelined efdc_xm_step_batch
 constexpr int NCOPY = 4;      // streams for host<->device copies
 constexpr size_t STAGE_BYTES = size_t(64) << 20;  // staging of a transfer in one round, at most
-constexpr int NPIECE = 16;    // slots of the page-locked buffer for pageable arrays
+constexpr int NPIECE = 8;     // slots of the page-locked buffer for pageable arrays
 // Contexts of at most this many members fold the member reductions into the
 // CG kernels by default.  In a larger batch the CTA that stores last often
 // completes many members at once and sums them one after another at the end
@@ -273,9 +273,7 @@ struct efdc_xm_ctx {
   double *mom_hp = nullptr;
   void *mom_lists = nullptr;  // the serial lists on the device (rebuilt after a set-up call)
   char *pack_h = nullptr, *pack_d = nullptr;  // packed small transfers (page-locked, device)
-  // pageable transfers: the page-locked ring and its slots' events
-  char *ring_h = nullptr;
-  cudaEvent_t piece_event[NPIECE] = {};
+  cudaEvent_t piece_event[NPIECE] = {};       // of pack_h as the ring of pageable arrays
   bool mom_inputs = false;    // a call has left U, V, UHDY, VHDX on the device
   std::vector<char> has_mom;
   std::vector<int> mom_ld;
@@ -506,14 +504,15 @@ int download_packed(efdc_xm_ctx *c, const std::vector<Xfer> &xs) {
   return EFDC_XM_OK;
 }
 
-// Larger transfers of pageable host arrays: pieces through a page-locked ring, the
-// host copies by up to NCOPY threads (of this call only: joined before it returns),
-// each with its own slots of the ring and its own copy stream, so that host copies and
+// Larger transfers of pageable host arrays: pieces through the same page-locked buffer
+// as a ring, the host copies by up to NCOPY threads (of this call only: joined before
+// it returns), each with its own slots and its own copy stream, so that host copies and
 // link run side by side.  The driver's own staging of pageable copies moved 450 KB
 // arrays at 18 GB/s in and 7.5 out.  Measured (16 cores): the calls of a coupled step of
-// 56,000 cells and four layers 3.6 -> 2.65 ms, one thread 2.9; slots of 256 KB 3.1, a
-// ring of 4 MB 2.66, slabs of 1 MB across arrays in a ring of 16 MB 3.0 (it no longer
-// stays in the caches).
+// 56,000 cells and four layers 3.6 -> 2.65 ms, with one thread 2.9, with slots of 256 KB
+// 3.1; a ring of 8 MB was even there and 5 % faster at 160,000 cells, but doubles what a
+// context locks; slabs of 1 MB across arrays in a ring of 16 MB 3.0 (it no longer stays
+// in the caches).
 struct Piece {
   char *host, *dev;
   size_t n;
@@ -521,6 +520,7 @@ struct Piece {
 constexpr size_t PIECE_MAX = size_t(512) << 10;     // bytes of a slot
 constexpr size_t PIECE_THREAD = size_t(1) << 20;    // bytes that are worth another thread
 constexpr int PIECE_SLOTS = NPIECE / NCOPY;  // of a thread
+static_assert(NPIECE * PIECE_MAX <= PACK_MAX, "the slots fit the buffer");
 
 void add_pieces(std::vector<Piece> &v, char *host, char *dev, size_t n) {
   for (size_t o = 0; o < n; o += PIECE_MAX)
@@ -533,7 +533,7 @@ cudaError_t move_pieces(efdc_xm_ctx *c, const std::vector<Piece> &v, std::atomic
                         int w, bool up) {
   cudaError_t e = cudaSetDevice(c->device);
   const cudaStream_t st = c->copy_stream[w];
-  char *buf = c->ring_h + size_t(w) * PIECE_SLOTS * PIECE_MAX;
+  char *buf = c->pack_h + size_t(w) * PIECE_SLOTS * PIECE_MAX;
   cudaEvent_t *ev = c->piece_event + w * PIECE_SLOTS;
   size_t held[PIECE_SLOTS] = {}, k0 = 0, k1 = 0;  // copies k0..k1-1 are in flight, k in slot k % SLOTS
   auto retire = [&] {
@@ -605,11 +605,7 @@ bool pageable(efdc_xm_ctx *c, const Xfer &x) {
 }
 // The ring of pageable transfers.
 bool pieces_ready(efdc_xm_ctx *c) {
-  if (!c->ring_h && cudaHostAlloc(&c->ring_h, NPIECE * PIECE_MAX, cudaHostAllocDefault) != cudaSuccess) {
-    cudaGetLastError();
-    c->ring_h = nullptr;
-    return false;
-  }
+  if (!pack_buffer(c)) return false;
   for (cudaEvent_t &e : c->piece_event)
     if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
       cudaGetLastError();
@@ -621,14 +617,15 @@ bool pieces_ready(efdc_xm_ctx *c) {
 
 // More staging buffers, for transfers in which every array takes its own.
 int ensure_stages(efdc_xm_ctx *c, size_t n) {
-  while (c->stage.size() < n) {
-    double *p = c->alloc<double>(size_t(c->stage_len), false);
-    if (!p) {
-      set_error("cudaMalloc failed (staging)");
-      return EFDC_XM_CUDA_ERROR;
-    }
-    c->stage.push_back(p);
+  if (c->stage.size() >= n) return EFDC_XM_OK;
+  // one allocation for all of them, each at a 256-byte boundary
+  const size_t more = n - c->stage.size(), each = (size_t(c->stage_len) + 31) / 32 * 32;
+  double *p = c->alloc<double>(more * each, false);
+  if (!p) {
+    set_error("cudaMalloc failed (staging)");
+    return EFDC_XM_CUDA_ERROR;
   }
+  for (size_t k = 0; k < more; ++k) c->stage.push_back(p + k * each);
   return EFDC_XM_OK;
 }
 
@@ -1230,7 +1227,6 @@ void efdc_xm_destroy(efdc_xm_ctx *c) {
   for (auto &b : c->bufs) cudaFree(b.p);
   if (c->mom_lists) cudaFree(c->mom_lists);
   if (c->pack_h) cudaFreeHost(c->pack_h);
-  if (c->ring_h) cudaFreeHost(c->ring_h);
   for (cudaEvent_t e : c->piece_event)
     if (e) cudaEventDestroy(e);
   void *pinned[] = {c->ctl_h, c->glob_h, c->act_h, c->mpoly_h, c->sc_h, c->jobs_h, c->pser_h};
@@ -1935,7 +1931,7 @@ int upload_batch(efdc_xm_ctx *c, const efdc_xm_fields *f, bool skip_wetdry, bool
   int rc = plan_upload(c, f, skip_wetdry, skip_sbxy, levels, xs, &sent);
   // (upload_small waits); an upload by itself may be the only one: it sets up no ring,
   // whose page-locking takes several milliseconds
-  if (!rc) rc = upload_arrays(c, xs, false, !wait || c->ring_h);
+  if (!rc) rc = upload_arrays(c, xs, false, !wait || c->pack_h);
   if (!rc && !levels) rc = copy_levels(c, f, 0, size_t(c->nslot), c->stream);
   if (!rc) rc = upload_small(c, f, wait);
   if (rc) {

@@ -25,9 +25,9 @@ constexpr size_t res_smem64() {
 // exchange (see xm_resident.cuh) and the latency of the row work around it.
 // Measured against the multi-kernel CG with folded reductions (one CTA per
 // member before, for members of up to 4,000 slots), ms per step, device-resident:
-// 60x60 cells 0.35 -> 0.13, 260x250 0.36 -> 0.17, 500x500 0.45 -> 0.24, 700x700
+// 60x60 cells 0.33 -> 0.083, 260x250 0.36 -> 0.13, 500x500 0.45 -> 0.177, 700x700
 // 0.57 -> 0.33, 256 lakes of 1,100 cells in one batch 0.50 -> 0.38; lean: 900x860
-// 0.65 -> 0.49, 1,000x1,000 0.80 -> 0.56 (an iteration 31 -> 20 us, of which the row
+// 0.65 -> 0.49, 1,000x1,000 0.80 -> 0.55 (an iteration 31 -> 20 us, of which the row
 // work is 13, the exchanges' waits for the slowest CTA 3 and the exchanges 4).
 // Registers: one quad side by side keeps the coefficients there too (255 a thread with
 // two rows), two by two (128 a thread) in shared memory; the lean form reads them.
