@@ -2793,12 +2793,9 @@ int step_range(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_stats *stats, 
   // there from the mapped mirrors
   auto controls = [&]() -> int {
     int r = to_device(c, c->sc, c->sc_h, c->sc_hd, sizeof(xm::StepScalars) * M);
-    if (r) return r;
-    if (c->in_chunks)  // counters of this step (no copy engine: see to_device)
-      xm::launch_words(c->stream, c->ctl, nullptr, sizeof(Ctl) * M);
-    else
-      CK(cudaMemsetAsync(c->ctl, 0, sizeof(Ctl) * M, c->stream));
-    return write_act(c);
+    if (r || (r = write_act(c))) return r;
+    xm::launch_ctl_enter(c->stream, c->ctl, c->act, M);
+    return EFDC_XM_OK;
   };
   int rc = 0;
   bool sent = false;

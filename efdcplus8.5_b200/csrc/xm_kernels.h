@@ -201,6 +201,7 @@ void launch_loop_next(cudaStream_t st, Glob *g, int which, cudaGraphConditionalH
                       int inner, int nmember);
 void launch_step_enter(cudaStream_t st, const StepIn &in, StepScalars *sc, int *act, int *mpoly,
                        Ctl *ctl, Glob *g, int nmember);
+void launch_ctl_enter(cudaStream_t st, Ctl *ctl, const int *act, int nmember);
 void launch_inner_done(cudaStream_t st, Ctl *ctl, const int *act, int nmember);
 void launch_after_solve(cudaStream_t st, Ctl *ctl, int *act, int nmember, int mixed);
 void launch_sweep_next(cudaStream_t st, const DevStatic &S, Ctl *ctl, int *act, Glob *g,

@@ -38,6 +38,26 @@ __global__ void k_loop_next(Glob *g, int which, cudaGraphConditionalHandle h, in
   cudaGraphSetConditional(h, (more && c < cap) ? 1u : 0u);
 }
 
+// A member's control block at the start of a step.  One that takes no part keeps
+// what describes its assembled system -- the minimum diagonal and the symmetry --:
+// the chunks of an efdc_xm_step_batch are steps of a few members each, and the
+// scaled system of every member may be asked for after the last.
+__device__ __forceinline__ void member_enter(Ctl &c, bool active) {
+  Ctl k{};
+  if (!active) {
+    k.ccmnm_int = c.ccmnm_int;
+    k.ccmnm_bc = c.ccmnm_bc;
+    k.asym = c.asym;
+  }
+  k.stepping = active ? 1 : 0;
+  member_sweep_reset(k, active);
+  c = k;
+}
+// The control blocks of a step driven by the host.
+__global__ void k_ctl_enter(Ctl *ctl, const int *act, int nmember) {
+  for (int m = threadIdx.x; m < nmember; m += blockDim.x) member_enter(ctl[m], act[m] != 0);
+}
+
 // Start of a step, and of its first sweep: the members' scalars, activity and
 // inner preconditioner from the host's mirrors, their control blocks, the
 // step's counters.  One kernel of the graph in place of four small copies
@@ -53,10 +73,7 @@ __global__ void k_step_enter(StepIn in, StepScalars *sc, int *act, int *mpoly, C
     const int a = in.act[m];
     act[m] = a;
     mpoly[m] = in.mpoly[m];
-    Ctl k{};
-    k.stepping = a ? 1 : 0;
-    member_sweep_reset(k, a != 0);
-    ctl[m] = k;
+    member_enter(ctl[m], a != 0);
   }
   if (blockIdx.x == 0) {
     __shared__ int out;
@@ -141,6 +158,10 @@ void launch_step_enter(cudaStream_t st, const StepIn &in, StepScalars *sc, int *
   const int words = nmember * int(sizeof(StepScalars) / 4);
   k_step_enter<<<std::min(64, (words + 255) / 256), 256, 0, st>>>(in, sc, act, mpoly, ctl, g,
                                                                  nmember);
+  count_launches(1);
+}
+void launch_ctl_enter(cudaStream_t st, Ctl *ctl, const int *act, int nmember) {
+  k_ctl_enter<<<1, 256, 0, st>>>(ctl, act, nmember);
   count_launches(1);
 }
 void launch_inner_done(cudaStream_t st, Ctl *ctl, const int *act, int nmember) {

@@ -1671,7 +1671,7 @@ void launch_tbxy(const Launch &l, const DevStatic &S, const DevState &X, const D
 // they do not queue behind bulk copies in flight on other streams.
 __global__ void k_words(const unsigned *src, unsigned *dst, int n) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    dst[i] = src ? src[i] : 0u;
+    dst[i] = src[i];
 }
 void launch_words(cudaStream_t st, void *dst, const void *src, size_t bytes) {
   const int n = int(bytes / sizeof(unsigned));
