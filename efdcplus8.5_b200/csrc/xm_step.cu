@@ -868,7 +868,7 @@ __global__ void __launch_bounds__(NT, 4) k_backsub(DevStatic S, DevState X, int 
       hp = hb + c.deltd2 * dxyip * (2. * qsume - (ue + u1e - u - u1 + vn + v1n - v - v1));
     else
       hp = hb + c.delt * dxyip * (qsume - 0.5 * (ue + u1e - u - u1 + vn + v1n - v - v1));
-    if (kd == OPENBC && c.isdry == 0) hp = c.gi * P - S.belv[d];
+    if (kd == OPENBC && c.isdry <= 0) hp = c.gi * P - S.belv[d];
     X.uhdye[d] = u;
     X.vhdxe[d] = v;
     X.uhe[d] = u * dyiu;
@@ -884,7 +884,7 @@ __global__ void k_obc_hp(DevStatic S, DevState X, DevObc B, const int *act) {
     const int m = B.member[k];
     if (!act[m]) continue;
     const StepScalars &c = S.sc[m];
-    if (c.isdry == 0) continue;  // k_backsub's
+    if (c.isdry <= 0) continue;  // k_backsub's
     const int d = B.slot[k];
     double hp = c.gi * X.p[d] - S.belv[d];
     {
