@@ -221,6 +221,7 @@ struct efdc_xm_ctx {
   xm::SysView mxview{};  // the system the MIXED solve refines (the step's assembly, or CONGRAD's)
   bool last_mixed = false;  // the last step ran MIXED
   bool scaled_ready = true;  // Y holds the last step's scaled FP64 system (else formed on request)
+  bool inner_ready = false;  // and mxview's FP32 operator (else formed on request)
   bool sys_external = false;  // the system being solved is a caller's (efdc_xm_congrad)
   // calibration (efdc_xm_calib_*): adjoint state, step-start snapshots,
   // the CG solution of the last step, gauge gathers
@@ -828,6 +829,17 @@ int scaled_system(efdc_xm_ctx *c) {
   CK(cudaGetLastError());
   c->last_mixed = false;
   c->scaled_ready = true;
+  return EFDC_XM_OK;
+}
+
+// The FP32 operator of the multi-kernel MIXED iteration, which resident and FP64
+// solves do not form; for kernel timing and tuning.
+int inner_operator(efdc_xm_ctx *c) {
+  if (c->inner_ready) return EFDC_XM_OK;
+  const xm::Launch l = c->L();
+  xm::launch_scale32(l, c->S, c->mxview, c->Y, l.may_asym);
+  CK(cudaGetLastError());
+  c->inner_ready = true;
   return EFDC_XM_OK;
 }
 
@@ -2651,6 +2663,7 @@ int tune_time(efdc_xm_ctx *c, bool mixed, double fac, int reps, double *ms) {
   pl.mixed = mixed;
   pl.resident = resident_solve(c, mixed);
   if (!mixed && !pl.resident && !c->scaled_ready && (rc = scaled_system(c))) return rc;
+  if (mixed && !pl.resident && (rc = inner_operator(c))) return rc;
   pl.iters = c->graph_iters;
   pl.max_iterm = 1;
   for (int m = 0; m < c->M; ++m) pl.max_iterm = std::max(pl.max_iterm, c->sc_h[m].iterm);
@@ -2764,6 +2777,7 @@ int step_range(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_stats *stats, 
   c->last_mixed = mixed;
   const bool resident = resident_solve(c, mixed);
   c->scaled_ready = !mixed && !resident;
+  c->inner_ready = mixed && !resident;
   c->sys_external = false;
   c->step_baro = false;
   for (int m = m0; m < m1; ++m) c->step_baro |= prm[m].bsc > 1.E-6;
@@ -4164,6 +4178,7 @@ int32_t efdc_xm_congrad(efdc_xm_ctx *c, const double *ccc, const double *ccs, co
   c->mxview = xm::SysView{c->Y.fptmp, c->Y.ccc, c->Y.ccs, c->Y.ccw, c->Y.cce, c->Y.ccn, 0};
   c->last_mixed = false;
   c->scaled_ready = true;
+  c->inner_ready = mixed;
   c->sys_external = true;
   xm::launch_sys_prepare(c->L(), c->S, c->Y, c->ctl, mixed ? 1 : 0);
   CK(cudaGetLastError());
@@ -4384,18 +4399,16 @@ int32_t efdc_xm_time_kernels(efdc_xm_ctx *c, int32_t precision, int32_t reps, ef
   CK(cudaSetDevice(c->device));
   const xm::Launch l = c->L();
   const bool mixed = precision == EFDC_XM_PREC_MIXED;
-  if (!mixed && !c->scaled_ready) {
-    const int rc0 = scaled_system(c);
-    if (rc0) return rc0;
-  }
+  int rc = EFDC_XM_OK;
+  if (!mixed && !c->scaled_ready && (rc = scaled_system(c))) return rc;
+  if (mixed && (rc = inner_operator(c))) return rc;
   // the iterations run on a scratch copy of P with the stop tests disabled;
   // all launches are queued back to back (one untimed warm-up pair first),
   // so the events bracket device execution only, not host launch latency
   CK(cudaMemcpyAsync(c->ptmp, c->X.p, size_t(c->nslot) * sizeof(double), cudaMemcpyDeviceToDevice,
                      c->stream));
   for (int m = 0; m < c->M; ++m) c->act_h[m] = 1;
-  int rc = write_act(c);
-  if (rc) return rc;
+  if ((rc = write_act(c))) return rc;
   xm::launch_solve_reset(l, c->ctl, c->glob, c->act, c->M);
   if (mixed)
     xm::launch_mx_resid(l, c->S, c->mxview, c->Y, c->ptmp, c->ctl, c->glob, c->part, 1.0, 0.0,

@@ -120,6 +120,9 @@ void launch_obc_reset(const Launch &l, const DevStatic &S, const DevObc &B, cons
                       const int *act);
 void launch_scale(const Launch &l, const DevStatic &S, const DevState &X, const DevSystem &Y,
                   Ctl *ctl, const int *act, int mixed, int write_cross);
+// the FP32 operator of the system V, every member's
+void launch_scale32(const Launch &l, const DevStatic &S, const SysView &V, const DevSystem &Y,
+                    int write_cross);
 void launch_solve_reset(const Launch &l, Ctl *ctl, Glob *glob, const int *act, int nmember);
 void launch_outer_reset(const Launch &l, Glob *glob);
 void launch_cg_init(const Launch &l, const DevStatic &S, const DevSystem &Y, double *P, Ctl *ctl,

@@ -1350,6 +1350,11 @@ void launch_scale(const Launch &l, const DevStatic &S, const DevState &X, const 
   }
   count_launches(1);
 }
+void launch_scale32(const Launch &l, const DevStatic &S, const SysView &V, const DevSystem &Y,
+                    int write_cross) {
+  k_scale32<<<l.grid, NT, 0, l.stream>>>(S, V, Y, l.ntile, nullptr, write_cross);
+  count_launches(1);
+}
 void launch_solve_reset(const Launch &l, Ctl *ctl, Glob *glob, const int *act, int nmember) {
   k_solve_reset<<<1, 256, 0, l.stream>>>(ctl, glob, act, nmember);
   count_launches(1);
@@ -1716,9 +1721,7 @@ void launch_sys_prepare(const Launch &l, const DevStatic &S, const DevSystem &Y,
   k_sys_prepare<<<l.grid, NT, 0, l.stream>>>(S, Y, l.ntile, ctl);
   count_launches(1);
   if (mixed) {  // the standalone system may be unsymmetric: always the 4-array form
-    const SysView V{Y.fptmp, Y.ccc, Y.ccs, Y.ccw, Y.cce, Y.ccn, 0};
-    k_scale32<<<l.grid, NT, 0, l.stream>>>(S, V, Y, l.ntile, nullptr, 1);
-    count_launches(1);
+    launch_scale32(l, S, SysView{Y.fptmp, Y.ccc, Y.ccs, Y.ccw, Y.cce, Y.ccn, 0}, Y, 1);
   }
 }
 
