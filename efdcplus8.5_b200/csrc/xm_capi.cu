@@ -81,6 +81,8 @@ constexpr int KERNELS_PER_ITER = 4;  // matvec, its reduce, update, its reduce
 
 namespace xm {
 void count_launches(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
+thread_local int g_wait_polls = WAIT_POLLS;
+int wait_polls() { return g_wait_polls; }
 void set_last_error_str(const char *msg) { g_last_error = msg ? msg : ""; }
 }  // namespace xm
 
@@ -914,7 +916,8 @@ bool build_resident(efdc_xm_ctx *c, int (*capacity)(const xm::ResForm &, bool, i
 }
 
 xm::ResPlan res_plan(const efdc_xm_ctx *c, const ResSet &r, const ResSet::Wave &w) {
-  return xm::ResPlan{r.cta ? r.cta + w.cta0 : nullptr, c->res_part, c->res_count};
+  return xm::ResPlan{r.cta ? r.cta + w.cta0 : nullptr, c->res_part, c->res_count,
+                     xm::wait_polls()};
 }
 
 void launch_resident64(efdc_xm_ctx *c, const xm::Launch &l, const xm::SysView &V, double *P,
@@ -2138,7 +2141,7 @@ struct StepPlan {
   int mixed, istl, all, any_isdry, any_legacy, any99, any_waste, iters;
   int max_iterm, max_sweeps, grid, grid_cg, grid_cg32, grid_up32;
   int mx_jac, mx_poly, may_asym, chan, baro, obc_serial, any_may_asym, nmember;
-  int variant, ctas_mv, ctas_up, any_drag, resident;
+  int variant, ctas_mv, ctas_up, any_drag, resident, polls;
   double fac, inner_margin;
   const void *psol;
 };
@@ -2890,6 +2893,7 @@ int step_range(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_stats *stats, 
     pl.nmember = M;
     pl.fac = mixed ? (prm[0].mixed_rsq_factor > 0 ? prm[0].mixed_rsq_factor : 0.1) : 0.0;
     pl.psol = c->psol;
+    pl.polls = xm::wait_polls();  // (a captured launch keeps it)
     rc = run_step_graph(c, pl, x_pre, prm, stats, m0, m1);
     if (rc >= 0) {
       if (istl == 0) c->tl3_ready = false;  // CALPUV2C does not keep the three levels
@@ -4202,6 +4206,12 @@ void *efdc_xm_stream(efdc_xm_ctx *c) { return c ? static_cast<void *>(c->stream)
 int64_t efdc_xm_kernel_launches(void) { return g_launches.load(); }
 
 int64_t efdc_xm_host_waits(void) { return g_waits.load(); }
+
+int32_t efdc_xm_set_wait_limit(int32_t polls) {
+  const int32_t old = xm::g_wait_polls;
+  xm::g_wait_polls = polls >= 0 ? polls : xm::WAIT_POLLS;
+  return old;
+}
 
 int32_t efdc_xm_tune_key(const efdc_xm_ctx *c, int32_t precision, char *buf, int32_t len) {
   if (!c || !buf || len < 1) {

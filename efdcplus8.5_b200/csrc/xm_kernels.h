@@ -75,6 +75,7 @@ struct ResPlan {
   double2 *part;    // grid groups: [2][nquad] the quads' partial sums, by turns
   unsigned *count;  // grid groups: [M*RES_COUNT_STRIDE] the member's arrivals, and next to it
                     // the arrivals at the end of its last launch
+  int polls;        // of that counter, before a wait is given up
 };
 constexpr int RES_COUNT_STRIDE = 32;  // a 128-byte line per member
 // What a resident solve does at its ends besides solving.
@@ -209,6 +210,11 @@ void launch_inner_done(cudaStream_t st, Ctl *ctl, const int *act, int nmember);
 void launch_after_solve(cudaStream_t st, Ctl *ctl, int *act, int nmember, int mixed);
 void launch_sweep_next(cudaStream_t st, const DevStatic &S, Ctl *ctl, int *act, Glob *g,
                        cudaGraphConditionalHandle h, int cap, int nmember);
+
+// Polls of a counter before a device-side wait is given up, for the launches of this
+// host thread (efdc_xm_set_wait_limit).
+constexpr int WAIT_POLLS = 1 << 20;  // about a second
+int wait_polls();
 
 // sets the message returned by efdc_xm_last_error() for this thread
 void set_last_error_str(const char *msg);

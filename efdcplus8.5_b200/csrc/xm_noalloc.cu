@@ -43,8 +43,8 @@ static __device__ __align__(256) double g_na_scratch[NA_DOUBLES];
 
 struct NaCtl {  // lives in the last NA_CTL doubles of the scratch
   double rpcg, alpha, beta, rsq;
-  int iter, done, status, pad;
-  unsigned int counter, pad2;
+  int iter, status;
+  unsigned int counter, pad;
 };
 static_assert(sizeof(NaCtl) <= NA_CTL * sizeof(double), "control block too large");
 
@@ -55,6 +55,7 @@ struct NaArgs {
   double *P;
   double *z, *pa, *pb, *part;
   NaCtl *ctl;
+  int polls;  // of a wait, before it is given up
 };
 
 using xm::NT;
@@ -95,7 +96,7 @@ __device__ __forceinline__ bool na_sum(const NaArgs &a, unsigned &count, int &tu
     if (t == 0) {
       xm::red_release(&a.ctl->counter, 1u);
       for (int k = 0; int(xm::ld_acquire(&a.ctl->counter) - count) < 0; ++k)
-        if (k >= xm::RES_TRIES) {
+        if (k >= a.polls) {
           dead = 1;
           break;
         }
@@ -138,11 +139,10 @@ __global__ void __launch_bounds__(NA_NT) k_na_solve(NaArgs a, double rsqm, int i
       q[0] = 0.0;
       q[a.lc - 1] = 0.0;
     }
+  // a CTA whose last wait ran out has left its cells of P unsolved although the others
+  // may have come to the end: its status stays
   auto fail = [&] {
-    if (threadIdx.x == 0) {
-      a.ctl->status = EFDC_XM_DEVICE_TIMEOUT;
-      a.ctl->done = 1;
-    }
+    if (threadIdx.x == 0) atomicExch(&a.ctl->status, EFDC_XM_DEVICE_TIMEOUT);
   };
   double rpcg, alpha = 0.0, beta = 0.0, rsq = 0.0;
   int iter = 0, status = 0;
@@ -233,8 +233,7 @@ __global__ void __launch_bounds__(NA_NT) k_na_solve(NaArgs a, double rsqm, int i
     a.ctl->beta = beta;
     a.ctl->rsq = rsq;
     a.ctl->iter = iter;
-    a.ctl->status = status;
-    a.ctl->done = 1;
+    atomicCAS(&a.ctl->status, EFDC_XM_OK, status);
   }
 }
 
@@ -318,6 +317,7 @@ int32_t efdc_xm_congrad_noalloc(int32_t la, const int32_t *lnc, const int32_t *l
   a.cce = cce;
   a.fptmp = fptmp;
   a.P = p;
+  a.polls = xm::wait_polls();
   a.z = base;
   a.pa = base + NA_LEN;
   a.pb = base + 2 * size_t(NA_LEN);

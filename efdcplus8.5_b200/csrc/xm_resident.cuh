@@ -38,8 +38,6 @@
 
 namespace xm {
 
-constexpr int RES_TRIES = 1 << 20;  // polls of the counter before the wait is given up (about 1 s)
-
 __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -280,7 +278,7 @@ __device__ __forceinline__ bool res_exchange(const ResPlan &R, const DevStatic &
         unsigned *n = R.count + size_t(c.m) * RES_COUNT_STRIDE;
         red_release(n, 1u);
         for (int k = 0; int(ld_acquire(n) - bar.count) < 0; ++k)
-          if (k >= RES_TRIES) {
+          if (k >= R.polls) {
             dead = 1;
             break;
           }

@@ -475,6 +475,11 @@ def host_waits() -> int:
     return int(load().efdc_xm_host_waits())
 
 
+def set_wait_limit(polls: int = -1) -> int:
+    """efdc_xm_set_wait_limit (-1: the default); returns the old limit."""
+    return int(load().efdc_xm_set_wait_limit(int(polls)))
+
+
 class CudaLibraryMissing(RuntimeError):
     pass
 
@@ -522,6 +527,8 @@ def load(path: str | os.PathLike | None = None):
     lib.efdc_xm_stream.argtypes = [C.c_void_p]
     lib.efdc_xm_kernel_launches.restype = C.c_int64
     lib.efdc_xm_host_waits.restype = C.c_int64
+    lib.efdc_xm_set_wait_limit.restype = C.c_int32
+    lib.efdc_xm_set_wait_limit.argtypes = [C.c_int32]
     lib.efdc_xm_autotune.restype = C.c_int32
     lib.efdc_xm_autotune.argtypes = [C.c_void_p, C.c_int32, C.c_char_p, C.c_int32,
                                      C.POINTER(Schedule), C.POINTER(C.c_double)]

@@ -1,0 +1,72 @@
+"""Waits between the CTAs of a solve that run out (efdc_xm_set_wait_limit): a call
+returns EFDC_XM_DEVICE_TIMEOUT unless its results are those of a call that waits as
+long as it takes, and the next call with the default limit gives these results."""
+import numpy as np
+import pytest
+
+import efdc_xm as X
+import scenario as S
+
+pytestmark = pytest.mark.gpu
+
+LIMITS = [0] * 6 + [1, 2, 4, 8] * 4
+
+
+@pytest.fixture(autouse=True)
+def default_limit():
+    yield
+    X.set_wait_limit()
+
+
+def system(nx, ny):
+    scn = S.make_scenario(nx, ny, seed=41, obc_sides=("W",), amp=0.5, dt=10.0)
+    st, g = scn.copy_state(), scn.grid
+    sol = X.Solver(g)
+    sol.step(X.make_params(scn.params, n=1, tn=scn.tn(1)), st, diag=True)
+    i0 = np.arange(1, scn.la)
+    for k, src, nb in (("cce", "ccw", "lec"), ("ccn", "ccs", "lnc")):
+        st[k][i0] = np.where(g[nb][i0] <= scn.la, st[src][g[nb][i0] - 1], 0.0)
+    return scn, st, sol
+
+
+def check(call, limits=LIMITS):
+    """call() -> (status, results)."""
+    rc0, want = call()
+    assert rc0 in (X.OK, X.CG_MAXITER)
+    seen = []
+    for limit in limits:
+        old = X.set_wait_limit(limit)
+        rc, got = call()
+        assert X.set_wait_limit(old) == limit
+        seen.append(rc)
+        if rc != X.DEVICE_TIMEOUT:
+            assert rc == rc0
+            for a, b in zip(got, want):
+                np.testing.assert_array_equal(a, b)
+        rc, got = call()
+        assert rc == rc0
+        for a, b in zip(got, want):
+            np.testing.assert_array_equal(a, b)
+    assert X.DEVICE_TIMEOUT in seen  # CTAs that look once cannot all find the others
+
+
+@pytest.mark.parametrize("iterm", [1, 500])
+def test_noalloc(iterm):
+    import torch
+    scn, st, sol = system(300, 250)
+    sol.close()
+    t = {k: torch.from_numpy(np.ascontiguousarray(scn.grid[k], dtype=np.int32)).cuda()
+         for k in ("lnc", "lsc", "lec", "lwc")}
+    for k in ("ccc", "ccs", "ccn", "ccw", "cce", "fptmp"):
+        t[k] = torch.from_numpy(st[k]).cuda()
+
+    def call():
+        p = torch.from_numpy(scn.state["p"]).cuda()
+        torch.cuda.synchronize()
+        rc = X.load().efdc_xm_congrad_noalloc(
+            scn.la, *(t[k].data_ptr() for k in ("lnc", "lsc", "lec", "lwc", "ccc", "ccs", "ccn",
+                                                "ccw", "cce", "fptmp")),
+            p.data_ptr(), 1e-10, iterm, None, None, None)
+        return rc, (p.cpu().numpy(),)
+
+    check(call)
