@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(NT *W, W == 1 && Q == 1 && CLUSTER ? 2 : 1)
       o.alpha = k.alpha;
     }
     o.iter = k.iter;
-    o.status = k.status;
+    res_status(o, k.status);
     o.parity = k.parity;
     member_done(o, glob);
     if (ends.act) member_after_solve(o, ends.act[m], atomicOr(&o.asym, 0), false);

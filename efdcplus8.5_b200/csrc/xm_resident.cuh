@@ -331,12 +331,17 @@ __device__ __forceinline__ void res_check_faces(const DevStatic &S, const SysVie
     if (kinds[c] == OPENBC && unsymmetric_faces(S, V, r.d0 + c)) atomicOr(&k.asym, 2);
 }
 
-// A wait ran out: the step fails with a timeout status.
+// A wait ran out: the call fails with a timeout status.  The CTA has not stored its part
+// of the solution, and the others may have come through the same exchange: the status
+// of the one that ends the solve (res_status) does not replace this one.
 __device__ __forceinline__ void res_fail(Ctl &k, int *err) {
   if (threadIdx.x == 0) {
-    k.status = EFDC_XM_DEVICE_TIMEOUT;
+    atomicExch(&k.status, EFDC_XM_DEVICE_TIMEOUT);
     atomicExch(err, 1);
   }
+}
+__device__ __forceinline__ void res_status(Ctl &k, int status) {  // OK at the entry
+  atomicCAS(&k.status, EFDC_XM_OK, status);
 }
 
 // Row vectors of NC coefficients of the thread's quads: in registers (REG), or

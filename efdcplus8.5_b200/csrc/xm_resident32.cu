@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
       t.alpha = k.alpha;
     }
     t.iter = k.iter;
-    t.status = k.status;
+    res_status(t, k.status);
     t.parity = k.parity;
     t.inner_iter = k.inner_iter;
     t.outer = k.outer;

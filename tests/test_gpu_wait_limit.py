@@ -70,3 +70,43 @@ def test_noalloc(iterm):
         return rc, (p.cpu().numpy(),)
 
     check(call)
+
+
+def large():
+    """A context whose member takes more CTAs than a cluster holds.  MIXED: one
+    preconditioner (else each solve's choice follows from the iterations of the last)."""
+    scn, st, sol = system(520, 515)
+    sol.set_option(X.OPT_POLY_THRESHOLD, 0)
+    return scn, st, sol
+
+
+@pytest.mark.parametrize("iterm", [1, 500])
+@pytest.mark.parametrize("precision", [X.PREC_FP64, X.PREC_MIXED])
+def test_congrad(precision, iterm):
+    scn, st, sol = large()
+
+    def call():
+        p = scn.state["p"].copy()
+        args = (st["ccc"], st["ccs"], st["ccn"], st["ccw"], st["cce"], st["ccc"], st["fptmp"], p)
+        rc, it, rsq = sol.congrad(*args, 1e-10, iterm, precision)
+        return rc, (p, it, rsq)
+
+    check(call, LIMITS[:12])
+    sol.close()
+
+
+@pytest.mark.parametrize("precision", [X.PREC_FP64, X.PREC_MIXED])
+def test_step(precision):
+    scn, _, sol = large()
+
+    def call():
+        st = scn.copy_state()
+        try:
+            r = sol.step(X.make_params(scn.params, n=1, tn=scn.tn(1), precision=precision), st)
+        except RuntimeError as e:
+            assert "DEVICE_TIMEOUT" in str(e)
+            return X.DEVICE_TIMEOUT, ()
+        return r.status, (st["p"], st["hp"], st["uhdye"])
+
+    check(call, LIMITS[:12])
+    sol.close()
