@@ -110,7 +110,8 @@ __global__ void k_after_solve(Ctl *ctl, int *act, int nmember, int mixed) {
 // End of a sweep (calpuv2c.f90:597-601, 726-749): a member whose faces
 // changed sweeps again unless it has reached its cap (then its status is
 // WETDRY_MAXSWEEP); the sweep loop runs again while some member does, and
-// the members are reset for it.
+// the members are reset for it.  After a wait that ran out (Glob::err) the step
+// has failed and no solve's arrivals match any more: no further sweep.
 __global__ void k_sweep_next(DevStatic S, Ctl *ctl, int *act, Glob *g,
                              cudaGraphConditionalHandle h, int cap, int nmember) {
   __shared__ int any;
@@ -139,7 +140,7 @@ __global__ void k_sweep_next(DevStatic S, Ctl *ctl, int *act, Glob *g,
     g->nidone = 0;
     g->tot[LOOP_SWEEP] += 1;
     const int c = ++g->loop[LOOP_SWEEP];
-    cudaGraphSetConditional(h, (any && c < cap) ? 1u : 0u);
+    cudaGraphSetConditional(h, (any && c < cap && !g->err) ? 1u : 0u);
   }
 }
 

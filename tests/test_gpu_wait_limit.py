@@ -110,3 +110,25 @@ def test_step(precision):
 
     check(call, LIMITS[:12])
     sol.close()
+
+
+def test_no_further_sweeps():
+    """A wetting and drying step (three or four solves) whose first solve runs out of
+    time ends with its sweep, and the next one is as if it had not been."""
+    scn = S.tidal_flat(n=280, seed=13, dt=5.0)
+    sol = X.Solver(scn.grid)
+    sweeps, states = [], []
+    for limit in (-1, 0, 0, 0, -1):
+        X.set_wait_limit(limit)
+        st, n0 = scn.copy_state(), X.load().efdc_xm_kernel_launches()
+        try:
+            r = sol.step(X.make_params(scn.params, n=1, tn=1200.0), st)
+            assert r.status == X.OK and r.solves >= 2
+            states.append(st)
+        except RuntimeError as e:
+            assert "DEVICE_TIMEOUT" in str(e)
+        sweeps.append(X.load().efdc_xm_kernel_launches() - n0)
+    sol.close()
+    assert len(states) == 2 and sweeps[0] == sweeps[4] > max(sweeps[1:4])
+    for k in ("p", "hp", "uhdye", "lmaskdry"):
+        np.testing.assert_array_equal(states[0][k], states[1][k], err_msg=k)
