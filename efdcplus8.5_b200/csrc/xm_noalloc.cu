@@ -20,8 +20,10 @@
 // two reductions of an iteration are also its barriers.
 
 #include <cstdarg>
+#include <algorithm>
 #include <cstdio>
 #include <mutex>
+#include <type_traits>
 
 #include "../../include/efdc_xm.h"
 #include "xm_kernels.h"
@@ -63,46 +65,55 @@ using xm::NWARP;
 
 constexpr int NA_NT = NA_HALVES * NT;
 
-// The sums of NS values over all blocks, in every thread, and the barrier of the
-// grid: each block of 256 threads (half a CTA) sums its values and stores them,
-// the CTA adds its arrival with release semantics and waits for the others'
-// (bounded), then sums the blocks' values as one block of 256 threads does.
-// False (in every thread) when the wait ran out.
+__device__ __forceinline__ double na_tree(const double *w) {  // block_sum's last stage (its
+  return ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));  // further lanes add 0)
+}
+
+// The barrier of the grid: the CTA adds its arrival with release semantics and waits for
+// the others' (bounded).  False (in every thread) when the wait ran out.
+__device__ __forceinline__ bool na_meet(const NaArgs &a, unsigned &count) {
+  count += gridDim.x;
+  int dead = 0;
+  if (threadIdx.x == 0) {
+    xm::red_release(&a.ctl->counter, 1u);
+    for (int k = 0; int(xm::ld_acquire(&a.ctl->counter) - count) < 0; ++k)
+      if (k >= a.polls) {
+        dead = 1;
+        break;
+      }
+  }
+  return !__syncthreads_or(dead);
+}
+
+// The sums of NS values of the 512 threads `vb` of the launch (a CTA of k_na_solve): each
+// block of 256 threads (half of them) sums its values and stores them.
 template <int NS>
-__device__ __forceinline__ bool na_sum(const NaArgs &a, unsigned &count, int &turn,
-                                       const double (&v)[NS], double (&out)[NS]) {
+__device__ __forceinline__ void na_part(const NaArgs &a, int turn, int vb, const double (&v)[NS]) {
   __shared__ double sh[NS][NA_HALVES][NWARP];
-  __shared__ double red[NS][NWARP];
   const int t = threadIdx.x, lane = t & 31, half = t / NT, warp = (t % NT) >> 5;
-  const int nblk = gridDim.x * NA_HALVES;
   double2 *part = reinterpret_cast<double2 *>(a.part) + turn * NA_GRID;
-  turn ^= 1;
-  auto tree = [](const double *w) {  // block_sum's last stage (its further lanes add zeros)
-    return ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
-  };
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
     const double x = xm::warp_sum(v[s]);
     if (lane == 0) sh[s][half][warp] = x + 0.0;
   }
-  __syncthreads();  // also: every thread's z or p is before the release below
-  count += gridDim.x;
-  int dead = 0;
-  if (t < 32) {
-    if (t < NA_HALVES)
-      part[blockIdx.x * NA_HALVES + t] =
-          make_double2(tree(sh[0][t]), NS > 1 ? tree(sh[NS - 1][t]) : 0.0);
-    __syncwarp();
-    if (t == 0) {
-      xm::red_release(&a.ctl->counter, 1u);
-      for (int k = 0; int(xm::ld_acquire(&a.ctl->counter) - count) < 0; ++k)
-        if (k >= a.polls) {
-          dead = 1;
-          break;
-        }
-    }
-  }
-  if (__syncthreads_or(dead)) return false;
+  __syncthreads();  // also: every thread's stores are before the release in na_meet
+  if (t < NA_HALVES)
+    part[vb * NA_HALVES + t] =
+        make_double2(na_tree(sh[0][t]), NS > 1 ? na_tree(sh[NS - 1][t]) : 0.0);
+  if (t < 32) __syncwarp();  // (the arrival is the first warp's)
+}
+
+// na_meet, and the sums over all nvb*NA_HALVES blocks' values, in every thread: as one
+// block of 256 threads sums them.
+template <int NS>
+__device__ __forceinline__ bool na_total(const NaArgs &a, unsigned &count, int &turn, int nvb,
+                                         double (&out)[NS]) {
+  __shared__ double red[NS][NWARP];
+  const int t = threadIdx.x, nblk = nvb * NA_HALVES;
+  const double2 *part = reinterpret_cast<const double2 *>(a.part) + turn * NA_GRID;
+  turn ^= 1;
+  if (!na_meet(a, count)) return false;
   if (t < NT) {  // reduce_partials
     double z[NS];
 #pragma unroll
@@ -115,37 +126,89 @@ __device__ __forceinline__ bool na_sum(const NaArgs &a, unsigned &count, int &tu
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
       const double x = xm::warp_sum(z[s]);
-      if (lane == 0) red[s][warp] = x + 0.0;
+      if ((t & 31) == 0) red[s][t >> 5] = x + 0.0;
     }
   }
   __syncthreads();
 #pragma unroll
-  for (int s = 0; s < NS; ++s) out[s] = tree(red[s]);
+  for (int s = 0; s < NS; ++s) out[s] = na_tree(red[s]);
   return true;
+}
+
+// The sums of a launch whose CTAs are the blocks' pairs.
+template <int NS>
+__device__ __forceinline__ bool na_sum(const NaArgs &a, unsigned &count, int &turn,
+                                       const double (&v)[NS], double (&out)[NS]) {
+  na_part(a, turn, blockIdx.x, v);
+  return na_total(a, count, turn, gridDim.x, out);
+}
+
+// What a solve leaves for the host.  A CTA whose last wait ran out has left its cells
+// of P unsolved although the others may have come to the end: its status stays.
+__device__ __forceinline__ void na_fail(const NaArgs &a) {
+  if (threadIdx.x == 0) atomicExch(&a.ctl->status, EFDC_XM_DEVICE_TIMEOUT);
+}
+struct NaScalars {
+  double rpcg, alpha = 0.0, beta = 0.0, rsq = 0.0;
+  int iter = 0, status = EFDC_XM_OK;
+  // :88, and :143-169; true when the solve has ended
+  __device__ __forceinline__ bool start(double sum) {
+    rpcg = sum;
+    if (!isfinite(rpcg)) status = EFDC_XM_NONFINITE;
+    return rpcg == 0.0 || !isfinite(rpcg);
+  }
+  __device__ __forceinline__ bool next(const double (&sum)[2], double rsqm, int iterm) {
+    beta = sum[0] / rpcg;
+    rpcg = sum[0];
+    rsq = sum[1];
+    ++iter;
+    if (!isfinite(rsq) || !isfinite(alpha)) {
+      status = EFDC_XM_NONFINITE;
+      return true;
+    }
+    if (rsq <= rsqm) return true;
+    if (iter >= iterm) {
+      status = EFDC_XM_CG_MAXITER;
+      return true;
+    }
+    return false;
+  }
+  __device__ __forceinline__ void leave(const NaArgs &a) const {
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    a.ctl->rpcg = rpcg;
+    a.ctl->alpha = alpha;
+    a.ctl->beta = beta;
+    a.ctl->rsq = rsq;
+    a.ctl->iter = iter;
+    atomicCAS(&a.ctl->status, EFDC_XM_OK, status);
+  }
+};
+// congrad.f90:42: PCG(1)=PCG(LC)=0
+__device__ __forceinline__ void na_ghosts(const NaArgs &a) {
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    for (double *q : {a.z, a.pa, a.pb}) {
+      q[0] = 0.0;
+      q[a.lc - 1] = 0.0;
+    }
+}
+// RCG of cell L = i + 1 (:72)
+__device__ __forceinline__ double na_resid(const NaArgs &a, int i, double c, double x) {
+  return a.fptmp[i] - c * x - a.ccn[i] * a.P[a.lnc[i] - 1] - a.ccs[i] * a.P[a.lsc[i] - 1] -
+         a.ccw[i] * a.P[a.lwc[i] - 1] - a.cce[i] * a.P[a.lec[i] - 1];
 }
 
 // congrad.f90:54-187 with NC cells per thread.  What bounds it is the exchange,
 // as for the resident solves (xm_resident.cuh): three kernels per iteration and a
 // copy to the host every 8 took 410 us for 16 iterations on 112,000 cells; one
-// launch takes 181 us (a call of efdc_xm_congrad_noalloc, its copy of P included).
+// launch takes 168 us (a call of efdc_xm_congrad_noalloc, its copy of P included).
 template <int NC>
 __global__ void __launch_bounds__(NA_NT) k_na_solve(NaArgs a, double rsqm, int iterm) {
   const int first = 2 + int(blockIdx.x) * NA_NT + int(threadIdx.x), stride = gridDim.x * NA_NT;
   unsigned count = 0u;
   int turn = 0;
   double x[NC], r[NC], p[NC], ap[NC], ci[NC];
-  if (blockIdx.x == 0 && threadIdx.x == 0)  // congrad.f90:42: PCG(1)=PCG(LC)=0
-    for (double *q : {a.z, a.pa, a.pb}) {
-      q[0] = 0.0;
-      q[a.lc - 1] = 0.0;
-    }
-  // a CTA whose last wait ran out has left its cells of P unsolved although the others
-  // may have come to the end: its status stays
-  auto fail = [&] {
-    if (threadIdx.x == 0) atomicExch(&a.ctl->status, EFDC_XM_DEVICE_TIMEOUT);
-  };
-  double rpcg, alpha = 0.0, beta = 0.0, rsq = 0.0;
-  int iter = 0, status = 0;
+  na_ghosts(a);
+  NaScalars q;
   bool done;
   {  // :54-88
     double v[1] = {0.0}, sum[1];
@@ -156,23 +219,19 @@ __global__ void __launch_bounds__(NA_NT) k_na_solve(NaArgs a, double rsqm, int i
       const int i = L - 1;
       x[k] = a.P[i];
       const double c = a.ccc[i];
-      r[k] = a.fptmp[i] - c * x[k] - a.ccn[i] * a.P[a.lnc[i] - 1] -
-             a.ccs[i] * a.P[a.lsc[i] - 1] - a.ccw[i] * a.P[a.lwc[i] - 1] -
-             a.cce[i] * a.P[a.lec[i] - 1];
+      r[k] = na_resid(a, i, c, x[k]);
       ci[k] = 1. / c;
       p[k] = r[k] * ci[k];
       a.z[i] = p[k];
       a.pa[i] = p[k];
       v[0] += r[k] * p[k];
     }
-    if (!na_sum(a, count, turn, v, sum)) return fail();
-    rpcg = sum[0];
-    if (!isfinite(rpcg)) status = EFDC_XM_NONFINITE;
-    done = rpcg == 0.0 || !isfinite(rpcg);
+    if (!na_sum(a, count, turn, v, sum)) return na_fail(a);
+    done = q.start(sum[0]);
   }
   while (!done) {  // ITERM bounds the loop
-    const double *pold = iter & 1 ? a.pb : a.pa;
-    double *pnew = iter & 1 ? a.pa : a.pb;
+    const double *pold = q.iter & 1 ? a.pb : a.pa;
+    double *pnew = q.iter & 1 ? a.pa : a.pb;
     {  // :151-162 of the iteration before, :107-125
       double v[1] = {0.0}, sum[1];
 #pragma unroll
@@ -180,17 +239,17 @@ __global__ void __launch_bounds__(NA_NT) k_na_solve(NaArgs a, double rsqm, int i
         const int L = first + k * stride;
         if (L > a.la) continue;
         const int i = L - 1;
-        auto at = [&](int n) { return __ldcg(a.z + n) + beta * __ldcg(pold + n); };
+        auto at = [&](int n) { return __ldcg(a.z + n) + q.beta * __ldcg(pold + n); };
         const double ps = at(__ldg(a.lsc + i) - 1), pn = at(__ldg(a.lnc + i) - 1),
                      pw = at(__ldg(a.lwc + i) - 1), pe = at(__ldg(a.lec + i) - 1);
-        p[k] = ci[k] * r[k] + beta * p[k];
+        p[k] = ci[k] * r[k] + q.beta * p[k];
         pnew[i] = p[k];
         ap[k] = __ldg(a.ccc + i) * p[k] + __ldg(a.ccs + i) * ps + __ldg(a.ccn + i) * pn +
                 __ldg(a.ccw + i) * pw + __ldg(a.cce + i) * pe;
         v[0] += ap[k] * p[k];
       }
-      if (!na_sum(a, count, turn, v, sum)) return fail();
-      alpha = rpcg / sum[0];
+      if (!na_sum(a, count, turn, v, sum)) return na_fail(a);
+      q.alpha = q.rpcg / sum[0];
     }
     {  // :127-149
       double v[2] = {0.0, 0.0}, sum[2];
@@ -198,43 +257,87 @@ __global__ void __launch_bounds__(NA_NT) k_na_solve(NaArgs a, double rsqm, int i
       for (int k = 0; k < NC; ++k) {
         const int L = first + k * stride;
         if (L > a.la) continue;
-        x[k] = x[k] + alpha * p[k];
-        r[k] = r[k] - alpha * ap[k];
+        x[k] = x[k] + q.alpha * p[k];
+        r[k] = r[k] - q.alpha * ap[k];
         const double z = ci[k] * r[k];
         a.z[L - 1] = z;
         v[0] += r[k] * z;
         v[1] += r[k] * r[k];
       }
-      if (!na_sum(a, count, turn, v, sum)) return fail();
-      beta = sum[0] / rpcg;
-      rpcg = sum[0];
-      rsq = sum[1];
-    }
-    ++iter;
-    if (!isfinite(rsq) || !isfinite(alpha)) {
-      status = EFDC_XM_NONFINITE;
-      done = true;
-    } else if (rsq <= rsqm) {
-      done = true;
-    } else if (iter >= iterm) {
-      status = EFDC_XM_CG_MAXITER;
-      done = true;
+      if (!na_sum(a, count, turn, v, sum)) return na_fail(a);
+      done = q.next(sum, rsqm, iterm);
     }
   }
-  if (iter > 0)
+  if (q.iter > 0)
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
       const int L = first + k * stride;
       if (L <= a.la) a.P[L - 1] = x[k];
     }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    a.ctl->rpcg = rpcg;
-    a.ctl->alpha = alpha;
-    a.ctl->beta = beta;
-    a.ctl->rsq = rsq;
-    a.ctl->iter = iter;
-    atomicCAS(&a.ctl->status, EFDC_XM_OK, status);
+  q.leave(a);
+}
+
+// The same solve where fewer CTAs than that can be resident together (a partition of the
+// GPU): each CTA does the work of some of the nvb CTAs of k_na_solve, one after another,
+// with RCG, PCG and APCG in the scratch and PCG's update in a pass of its own.  The same
+// operations and sums, so the same bits; on the whole GPU 112,000 cells take 168 us in
+// the launch above.
+__global__ void __launch_bounds__(NA_NT) k_na_passes(NaArgs a, double rsqm, int iterm, int nvb) {
+  double *const r = a.z, *const p = a.pa, *const ap = a.pb;
+  unsigned count = 0u;
+  int turn = 0;
+  na_ghosts(a);
+  NaScalars q;
+  // body(i, v) on the CTA's cells, with the sums of each of its nvb CTAs
+  auto sweep = [&](auto ns, auto body) {
+    constexpr int NS = decltype(ns)::value;
+    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
+      double v[NS] = {};
+      for (int L = 2 + vb * NA_NT + int(threadIdx.x); L <= a.la; L += nvb * NA_NT) body(L - 1, v);
+      na_part(a, turn, vb, v);
+      __syncthreads();  // the warps' sums have been read
+    }
+  };
+  using One = std::integral_constant<int, 1>;
+  using Two = std::integral_constant<int, 2>;
+  double sum[1], sums[2];
+  sweep(One{}, [&](int i, double *v) {  // :54-88
+    const double c = a.ccc[i];
+    const double ri = na_resid(a, i, c, a.P[i]), pi = ri * (1. / c);
+    r[i] = ri;
+    p[i] = pi;
+    v[0] += ri * pi;
+  });
+  if (!na_total(a, count, turn, nvb, sum)) return na_fail(a);
+  bool done = q.start(sum[0]);
+  while (!done) {  // ITERM bounds the loop
+    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x)  // :151-162 of the iteration before
+      for (int L = 2 + vb * NA_NT + int(threadIdx.x); L <= a.la; L += nvb * NA_NT)
+        p[L - 1] = (1. / a.ccc[L - 1]) * r[L - 1] + q.beta * p[L - 1];
+    __syncthreads();  // every thread's p is before the release
+    if (!na_meet(a, count)) return na_fail(a);
+    sweep(One{}, [&](int i, double *v) {  // :107-125
+      auto at = [&](int n) { return __ldcg(p + n - 1); };
+      const double pi = p[i], ps = at(a.lsc[i]), pn = at(a.lnc[i]), pw = at(a.lwc[i]),
+                   pe = at(a.lec[i]);
+      const double api = a.ccc[i] * pi + a.ccs[i] * ps + a.ccn[i] * pn + a.ccw[i] * pw +
+                         a.cce[i] * pe;
+      ap[i] = api;
+      v[0] += api * pi;
+    });
+    if (!na_total(a, count, turn, nvb, sum)) return na_fail(a);
+    q.alpha = q.rpcg / sum[0];
+    sweep(Two{}, [&](int i, double *v) {  // :127-149
+      a.P[i] = a.P[i] + q.alpha * p[i];
+      const double ri = r[i] - q.alpha * ap[i], z = (1. / a.ccc[i]) * ri;
+      r[i] = ri;
+      v[0] += ri * z;
+      v[1] += ri * ri;
+    });
+    if (!na_total(a, count, turn, nvb, sums)) return na_fail(a);
+    done = q.next(sums, rsqm, iterm);
   }
+  q.leave(a);
 }
 
 thread_local char g_na_msg[512];
@@ -337,10 +440,15 @@ int32_t efdc_xm_congrad_noalloc(int32_t la, const int32_t *lnc, const int32_t *l
                        : nc <= 2 ? reinterpret_cast<const void *>(k_na_solve<2>)
                        : nc <= 4 ? reinterpret_cast<const void *>(k_na_solve<4>)
                                  : reinterpret_cast<const void *>(k_na_solve<8>);
-  void *args[] = {&a, &rsqm, &iterm};
-  if ((e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(NA_NT), args, 0, st)) !=
-      cudaSuccess)
-    return fail(e, "launch");
+  void *args[] = {&a, &rsqm, &iterm, const_cast<int *>(&grid)};  // (grid: k_na_passes alone)
+  e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(NA_NT), args, 0, st);
+  // the stream's part of the GPU holds fewer CTAs at once
+  for (int g = grid / 2; e == cudaErrorCooperativeLaunchTooLarge && g > 0; g /= 2) {
+    cudaGetLastError();
+    e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_na_passes), dim3(g),
+                                    dim3(NA_NT), args, 0, st);
+  }
+  if (e != cudaSuccess) return fail(e, "launch");
   NaCtl h{};
   if ((e = cudaMemcpyAsync(&h, a.ctl, sizeof(NaCtl), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
     return fail(e, "copy of the control block");

@@ -642,8 +642,9 @@ int32_t efdc_xm_time_kernels(efdc_xm_ctx *ctx, int32_t precision, int32_t reps,
  *   - all calls share the array: calls that overlap on the GPU (other
  *     streams, other host threads) race; the call returns after its work on
  *     `stream` (a cudaStream_t, NULL = legacy default stream) finished;
- *   - a call is one cooperative launch of up to 148 CTAs that wait on one
- *     another (bounded: EFDC_XM_DEVICE_TIMEOUT); it copies its control block to
+ *   - a call is one cooperative launch of up to 148 CTAs (fewer where `stream`
+ *     has part of the GPU) that wait on one another (bounded:
+ *     EFDC_XM_DEVICE_TIMEOUT); it copies its control block to
  *     host memory and synchronizes `stream`, so it must not be called while a
  *     stream capture is active (on `stream` or, in global capture mode, anywhere
  *     in the process). */
