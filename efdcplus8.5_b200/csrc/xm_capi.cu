@@ -456,29 +456,42 @@ bool pack_buffer(efdc_xm_ctx *c) {
   return true;
 }
 bool packed(efdc_xm_ctx *c, size_t njobs) {
-  return njobs <= size_t(xm::JobTable::CAP) &&
-         njobs * size_t(c->stage_len) * sizeof(double) <= PACK_MAX && pack_buffer(c);
+  return njobs * size_t(c->stage_len) * sizeof(double) <= PACK_MAX && pack_buffer(c);
 }
 
-// The job table goes with the kernel's arguments.  wait: until the transfer is done
-// (else the caller waits for the solver stream before the host buffer is used again).
+// The kernels of a packed transfer (go: one launch), JobTable::CAP arrays each: the job
+// table goes with the kernel's arguments.
+template <class Go>
+void packed_launches(efdc_xm_ctx *c, const std::vector<Xfer> &xs, Go go) {
+  const size_t L = size_t(c->stage_len), n = xs.size();
+  for (size_t j0 = 0; j0 < n; j0 += size_t(xm::JobTable::CAP)) {
+    const size_t m = std::min(n - j0, size_t(xm::JobTable::CAP));
+    xm::JobTable jobs;
+    for (size_t j = 0; j < m; ++j)
+      jobs.j[j] = CopyJob{reinterpret_cast<double *>(c->pack_d + (j0 + j) * L * sizeof(double)),
+                          xs[j0 + j].dev, xs[j0 + j].kind};
+    go(jobs, int(m));
+  }
+}
+
+// wait: until the transfer is done (else the caller waits for the solver stream before
+// the host buffer is used again).
 int upload_packed(efdc_xm_ctx *c, const std::vector<Xfer> &xs, bool wait) {
   const size_t L = size_t(c->stage_len), n = xs.size();
-  xm::JobTable jobs;
   for (size_t j = 0; j < n; ++j) {
     const size_t es = esize(xs[j].kind);
     char *dst = c->pack_h + j * L * sizeof(double);
     for (int m = 0; m < c->M; ++m)
       if (xs[j].host[m])
         std::memcpy(dst + size_t(c->mem[m].off) * es, xs[j].host[m], size_t(c->mem[m].lc) * es);
-    jobs.j[j] = CopyJob{reinterpret_cast<double *>(c->pack_d + j * L * sizeof(double)),
-                        xs[j].dev, xs[j].kind};
   }
   const size_t bytes = n * L * sizeof(double);
   CK(cudaMemcpyAsync(c->pack_d, c->pack_h, bytes, cudaMemcpyHostToDevice, c->stream));
   g_h2d.fetch_add(static_cast<long long>(bytes), std::memory_order_relaxed);
-  xm::launch_scatter_table(c->stream, jobs, int(n), c->lidx, c->tile_member, c->moff, c->mlc, 0,
-                           c->nslot);
+  packed_launches(c, xs, [&](const xm::JobTable &jobs, int m) {
+    xm::launch_scatter_table(c->stream, jobs, m, c->lidx, c->tile_member, c->moff, c->mlc, 0,
+                             c->nslot);
+  });
   CK(cudaGetLastError());
   if (wait) CK(cudaStreamSynchronize(c->stream));
   return EFDC_XM_OK;
@@ -486,12 +499,10 @@ int upload_packed(efdc_xm_ctx *c, const std::vector<Xfer> &xs, bool wait) {
 
 int download_packed(efdc_xm_ctx *c, const std::vector<Xfer> &xs) {
   const size_t L = size_t(c->stage_len), n = xs.size();
-  xm::JobTable jobs;
-  for (size_t j = 0; j < n; ++j)
-    jobs.j[j] = CopyJob{reinterpret_cast<double *>(c->pack_d + j * L * sizeof(double)),
-                        xs[j].dev, xs[j].kind};
   const size_t bytes = n * L * sizeof(double);
-  xm::launch_gather_table(c->stream, jobs, int(n), c->lidx, c->tile_member, c->moff, 0, c->nslot);
+  packed_launches(c, xs, [&](const xm::JobTable &jobs, int m) {
+    xm::launch_gather_table(c->stream, jobs, m, c->lidx, c->tile_member, c->moff, 0, c->nslot);
+  });
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(c->pack_h, c->pack_d, bytes, cudaMemcpyDeviceToHost, c->stream));
   g_d2h.fetch_add(static_cast<long long>(bytes), std::memory_order_relaxed);

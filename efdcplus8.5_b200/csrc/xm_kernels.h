@@ -42,7 +42,7 @@ struct CopyJob {
   void *dev;               // tile-order device array
   int is_int;              // 0 double, 1 LOGICAL (0/1), 2 raw int, 3 double water-only
 };
-// The jobs of a small transfer, as a kernel argument.
+// The jobs of a small transfer, as a kernel argument (up to CAP of them a launch).
 struct JobTable {
   static constexpr int CAP = 64;
   CopyJob j[CAP];
