@@ -62,7 +62,8 @@ uint64_t morton2(uint32_t x, uint32_t y) {
   return spread(x) | (spread(y) << 1);
 }
 
-constexpr int NSTAGE = 8;     // staging buffers (each holds one array of every member)
+constexpr int NSTAGE = 8;     // staging buffers (each holds one array of every member), at least
+constexpr int NARRAYS = 32;   // arrays of a step's upload
 constexpr int NCHUNK = 32;    // most member chunks of a pipelined efdc_xm_step_batch
 constexpr int NCOPY = 4;      // streams for host<->device copies
 constexpr size_t STAGE_BYTES = size_t(64) << 20;  // staging of a transfer in one round, at most
@@ -275,6 +276,7 @@ struct efdc_xm_ctx {
   xm::MomDev md{};
   double *mom_hp = nullptr;
   void *mom_lists = nullptr;  // the serial lists on the device (rebuilt after a set-up call)
+  char *pinned = nullptr;  // page-locked: the control mirrors, the job table, the series
   char *pack_h = nullptr, *pack_d = nullptr;  // packed small transfers (page-locked, device)
   cudaEvent_t piece_event[NPIECE] = {};       // of pack_h as the ring of pageable arrays
   bool mom_inputs = false;    // a call has left U, V, UHDY, VHDX on the device
@@ -440,20 +442,10 @@ int d2h_range(efdc_xm_ctx *c, const Xfer &x, const char *stage, int m0, int m1, 
 // array: those, not bytes, bound a small basin's step on host arrays.
 constexpr size_t PACK_MAX = size_t(4) << 20;  // bytes of one packed transfer
 
+// Its device side is allocated by the first packed transfer (a small context's creation).
 bool pack_buffer(efdc_xm_ctx *c) {
-  if (!c->pack_h) {
-    if (cudaHostAlloc(&c->pack_h, PACK_MAX, cudaHostAllocDefault) != cudaSuccess) {
-      cudaGetLastError();
-      c->pack_h = nullptr;
-      return false;
-    }
-    if (!(c->pack_d = c->alloc<char>(PACK_MAX, false))) {
-      cudaFreeHost(c->pack_h);
-      c->pack_h = nullptr;
-      return false;
-    }
-  }
-  return true;
+  if (c->pack_h && !c->pack_d && !(c->pack_d = c->alloc<char>(PACK_MAX, false))) cudaGetLastError();
+  return c->pack_d != nullptr;
 }
 bool packed(efdc_xm_ctx *c, size_t njobs) {
   return njobs * size_t(c->stage_len) * sizeof(double) <= PACK_MAX && pack_buffer(c);
@@ -654,7 +646,7 @@ bool pageable(efdc_xm_ctx *c, const Xfer &x) {
 }
 // The ring of pageable transfers.
 bool pieces_ready(efdc_xm_ctx *c) {
-  if (!pack_buffer(c)) return false;
+  if (!c->pack_h) return false;
   for (cudaEvent_t &e : c->piece_event)
     if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
       cudaGetLastError();
@@ -685,14 +677,13 @@ size_t group_size(efdc_xm_ctx *c, size_t n) {
   size_t g = std::min(n, std::max<size_t>(NSTAGE, STAGE_BYTES / std::max<size_t>(each, 1)));
   if (g > c->stage.size() && ensure_stages(c, g) != EFDC_XM_OK) {
     cudaGetLastError();
-    g = NSTAGE;
+    if (c->stage.empty() && ensure_stages(c, NSTAGE) != EFDC_XM_OK) cudaGetLastError();
+    g = c->stage.size();
   }
   return g;
 }
 
-// ring = false: without the ring of pageable arrays.
-int upload_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs, bool wait = true,
-                  bool ring = true) {
+int upload_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs, bool wait = true) {
   if (xs.empty()) return EFDC_XM_OK;
   if (xs.size() > size_t(MAX_JOBS)) {
     set_error("internal: too many arrays in one transfer");
@@ -712,7 +703,7 @@ int upload_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs, bool wait = true,
     Pieces v;
     for (size_t j = g0; j < g1; ++j) {
       char *stage = reinterpret_cast<char *>(c->stage[j % G]);
-      if (ring && pageable(c, xs[j]) && pieces_ready(c)) {
+      if (pageable(c, xs[j]) && pieces_ready(c)) {
         const size_t es = esize(xs[j].kind);
         PieceMaker mk{v};
         for (int m = 0; m < c->M; ++m)
@@ -1289,12 +1280,10 @@ void efdc_xm_destroy(efdc_xm_ctx *c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   for (auto &b : c->bufs) cudaFree(b.p);
   if (c->mom_lists) cudaFree(c->mom_lists);
-  if (c->pack_h) cudaFreeHost(c->pack_h);
   for (cudaEvent_t e : c->piece_event)
     if (e) cudaEventDestroy(e);
-  void *pinned[] = {c->ctl_h, c->glob_h, c->act_h, c->mpoly_h, c->sc_h, c->jobs_h, c->pser_h};
-  for (void *p : pinned)
-    if (p) cudaFreeHost(p);
+  if (c->pinned) cudaFreeHost(c->pinned);
+  if (c->pack_h) cudaFreeHost(c->pack_h);
   if (c->gslot) cudaFree(c->gslot);
   if (c->gbuf) cudaFree(c->gbuf);
   for (cudaGraphExec_t g : c->graph_cg)
@@ -1605,15 +1594,35 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
   c->mxview = xm::SysView{X.fp, X.cc, X.cs, X.cw, X.ce, X.cn, 1};
   if (!c->ptmp || !Y.x32 || !Y.z32 || !Y.r32b || !X.rcy)
     return bail("cudaMalloc failed (device memory)");
-  auto pin = [](void *pp, size_t bytes) {
-    return cudaHostAlloc(static_cast<void **>(pp), std::max<size_t>(bytes, 1),
-                         cudaHostAllocMapped) == cudaSuccess;
-  };
-  if (!pin(&c->ctl_h, sizeof(Ctl) * M) || !pin(&c->glob_h, sizeof(Glob)) ||
-      !pin(&c->act_h, sizeof(int) * M) || !pin(&c->mpoly_h, sizeof(int) * M) ||
-      !pin(&c->sc_h, sizeof(xm::StepScalars) * M) ||
-      !pin(&c->jobs_h, sizeof(CopyJob) * MAX_JOBS))
-    return bail("cudaHostAlloc failed");
+  {  // the control mirrors and the job table, one page-locked block
+    size_t need = 0;
+    auto part = [&need](size_t bytes) {
+      const size_t at = need;
+      need += (bytes + 255) / 256 * 256;
+      return at;
+    };
+    const size_t ctl = part(sizeof(Ctl) * M), glob = part(sizeof(Glob)),
+                 act = part(sizeof(int) * M), mpoly = part(sizeof(int) * M),
+                 sc = part(sizeof(xm::StepScalars) * M), jobs = part(sizeof(CopyJob) * MAX_JOBS),
+                 pser = part(sizeof(double) * c->nobc);
+    if (cudaHostAlloc(&c->pinned, need, cudaHostAllocMapped) != cudaSuccess) {
+      c->pinned = nullptr;
+      return bail("cudaHostAlloc failed");
+    }
+    // and the transfers' buffer, here rather than in the first call that wants it, which
+    // it would cost several milliseconds; without it they go through the driver
+    if (cudaHostAlloc(&c->pack_h, PACK_MAX, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      c->pack_h = nullptr;
+    }
+    c->ctl_h = reinterpret_cast<Ctl *>(c->pinned + ctl);
+    c->glob_h = reinterpret_cast<Glob *>(c->pinned + glob);
+    c->act_h = reinterpret_cast<int *>(c->pinned + act);
+    c->mpoly_h = reinterpret_cast<int *>(c->pinned + mpoly);
+    c->sc_h = reinterpret_cast<xm::StepScalars *>(c->pinned + sc);
+    c->jobs_h = reinterpret_cast<CopyJob *>(c->pinned + jobs);
+    if (c->nobc > 0) c->pser_h = reinterpret_cast<double *>(c->pinned + pser);
+  }
   std::memset(c->ctl_h, 0, sizeof(Ctl) * M);
   std::memset(c->sc_h, 0, sizeof(xm::StepScalars) * M);
   {  // the control mirrors' device addresses (pinned memory is mapped under UVA)
@@ -1646,11 +1655,9 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
     cudaMemcpy(st[16], fu.data(), ns * sizeof(double), cudaMemcpyHostToDevice);
     cudaMemcpy(st[17], fv.data(), ns * sizeof(double), cudaMemcpyHostToDevice);
   }
-  for (int k = 0; k < NSTAGE; ++k) {
-    double *p = c->alloc<double>(size_t(c->stage_len), false);
-    if (!p) return bail("cudaMalloc failed (staging)");
-    c->stage.push_back(p);
-  }
+  // the staging buffers of a step's arrays in one allocation
+  group_size(c, NARRAYS);
+  if (c->stage.empty()) return bail("cudaMalloc failed (staging)");
   xm::DevObc &Bo = c->B;
   Bo.n = c->nobc;
   Bo.mtmax = mtmax;
@@ -1685,7 +1692,6 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
     Bo.pcb = pc;
     Bo.psb = ps;
     Bo.pser = c->pser_d;
-    if (!pin(&c->pser_h, n * sizeof(double))) return bail("cudaHostAlloc failed");
   }
   // the zero-fills above ran on the legacy stream; finish them before any
   // work on the non-blocking solver stream
@@ -1704,7 +1710,7 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
       {&efdc_xm_grid::sbxo, st[12]},  {&efdc_xm_grid::sbyo, st[13]}, {&efdc_xm_grid::belv, st[14]}};
   std::vector<Xfer> xs;
   for (const auto &mt : metrics) xs.push_back(Xfer{per(mt.first), mt.second, 0});
-  if (upload_arrays(c, xs, true, false) != EFDC_XM_OK)
+  if (upload_arrays(c, xs) != EFDC_XM_OK)
     return bail("upload of the static arrays failed");
   if (cudaDeviceSynchronize() != cudaSuccess) return bail("device error during set-up");
   for (int m = 0; m < M; ++m) c->mem[m].slot_of = std::move(slot_of[m]);
@@ -1992,9 +1998,7 @@ int upload_batch(efdc_xm_ctx *c, const efdc_xm_fields *f, bool skip_wetdry, bool
   std::vector<Xfer> xs;
   uint32_t sent = 0;
   int rc = plan_upload(c, f, skip_wetdry, skip_sbxy, levels, xs, &sent);
-  // (upload_small waits); an upload by itself may be the only one: it sets up no ring,
-  // whose page-locking takes several milliseconds
-  if (!rc) rc = upload_arrays(c, xs, false, !wait || c->pack_h);
+  if (!rc) rc = upload_arrays(c, xs, false);  // (upload_small waits)
   if (!rc && !levels) rc = copy_levels(c, f, 0, size_t(c->nslot), c->stream);
   if (!rc) rc = upload_small(c, f, wait);
   if (rc) {
