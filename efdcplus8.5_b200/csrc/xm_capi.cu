@@ -900,7 +900,15 @@ bool resident_solve(const efdc_xm_ctx *c, bool mixed) {
 
 // The form of a resident solve.  One cluster per member where the largest
 // member fits 16 CTAs, with as few quads per CTA as that takes (the members
-// are independent: a launch holds any number of clusters).  Else grid groups,
+// are independent: a launch holds any number of clusters).  In MIXED the multi-kernel
+// CG moves half the bytes of the FP64 one, and passes the clusters when too many of
+// them run one after another.  ms per step, clusters against the multi-kernel CG, by
+// rounds (members over the clusters that fit at once): one quad a CTA, 64 members of
+// 12,000 cells (4.6 rounds) 0.58 / 0.59, 512 of 1,100 (5.5) 0.66 / 0.69, 96 of 12,000
+// (6.9) 0.81 / 0.73, 256 of 12,000 (18) 2.10 / 1.49; more quads a CTA, 48 of 30,000 (3.2)
+// 0.72 / 0.75, 24 of 58,000 (3.4) 0.77 / 0.73, 32 of 20,000 (4.6) 0.51 / 0.48, 48 of
+// 58,000 (6.9) 1.35 / 1.19.  FP64 gains by any number of rounds (256 of 12,000: 2.05 /
+// 2.59).  Else grid groups,
 // the first form that holds every member at once, or, up to max_waves, the
 // last in as few launches as that takes.  Several launches, one after another,
 // are still faster than the multi-kernel CG in FP64 (24 basins of 2.5 M cells:
@@ -912,8 +920,10 @@ bool resident_solve(const efdc_xm_ctx *c, bool mixed) {
 // side by side in MIXED (0.159 against 0.173 and 0.110 against 0.119).
 const std::vector<xm::ResForm> FORMS64 = {{1, 1, 0}, {1, 2, 0}, {2, 2, 0}, {2, 4, 0}};
 const std::vector<xm::ResForm> FORMS32 = {{1, 1, 0}, {2, 1, 0}, {2, 2, 0}};
+constexpr int MX_ROUNDS1 = 6, MX_ROUNDS = 4;  // of one and of more quads a CTA
 bool build_resident(efdc_xm_ctx *c, int (*capacity)(const xm::ResForm &, bool, int),
-                    const std::vector<xm::ResForm> &forms, size_t max_waves, ResSet &out) {
+                    const std::vector<xm::ResForm> &forms, bool mixed, ResSet &out) {
+  const size_t max_waves = mixed ? 1 : SIZE_MAX;
   const int M = c->M, mq = c->max_units;
   auto cap_of = [&](const xm::ResForm &f) {
     return std::min(capacity(f, false, c->nsm), capacity(f, true, c->nsm));
@@ -922,7 +932,9 @@ bool build_resident(efdc_xm_ctx *c, int (*capacity)(const xm::ResForm &, bool, i
     const int per = f.w * f.q, n = (mq + per - 1) / per;
     if (n > 16) continue;
     f.cluster = n;
-    if (cap_of(f) < 1) continue;
+    const int cap = cap_of(f);
+    if (cap < 1) continue;
+    if (mixed && M > (per == 1 ? MX_ROUNDS1 : MX_ROUNDS) * cap) return true;
     out.form = f;
     out.waves = {{0, n * M}};
     return true;
@@ -1542,8 +1554,8 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
   c->qstart_h = qstart;
   for (int m = 0; m < M; ++m) c->max_units = std::max(c->max_units, qstart[m + 1] - qstart[m]);
   c->has_layers.assign(M, 0);
-  if (reset_resident(c) || !build_resident(c, xm::cg_res_capacity, FORMS64, SIZE_MAX, c->res64) ||
-      !build_resident(c, xm::mx_res_capacity, FORMS32, 1, c->res32))
+  if (reset_resident(c) || !build_resident(c, xm::cg_res_capacity, FORMS64, false, c->res64) ||
+      !build_resident(c, xm::mx_res_capacity, FORMS32, true, c->res32))
     return bail("cudaMalloc failed (resident solves)");
   cudaMemcpy(quads_d, quads.data(), quads.size() * sizeof(int4), cudaMemcpyHostToDevice);
   cudaMemcpy(qstart_d, qstart.data(), (M + 1) * sizeof(int), cudaMemcpyHostToDevice);
