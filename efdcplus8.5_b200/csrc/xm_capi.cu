@@ -900,48 +900,66 @@ bool resident_solve(const efdc_xm_ctx *c, bool mixed) {
 
 // The form of a resident solve.  One cluster per member where the largest
 // member fits 16 CTAs, with as few quads per CTA as that takes (the members
-// are independent: a launch holds any number of clusters).  In MIXED the multi-kernel
-// CG moves half the bytes of the FP64 one, and passes the clusters when too many of
-// them run one after another.  ms per step, clusters against the multi-kernel CG, by
-// rounds (members over the clusters that fit at once): one quad a CTA, 64 members of
-// 12,000 cells (4.6 rounds) 0.58 / 0.59, 512 of 1,100 (5.5) 0.66 / 0.69, 96 of 12,000
-// (6.9) 0.81 / 0.73, 256 of 12,000 (18) 2.10 / 1.49; more quads a CTA, 48 of 30,000 (3.2)
-// 0.72 / 0.75, 24 of 58,000 (3.4) 0.77 / 0.73, 32 of 20,000 (4.6) 0.51 / 0.48, 48 of
-// 58,000 (6.9) 1.35 / 1.19.  FP64 gains by any number of rounds (256 of 12,000: 2.05 /
-// 2.59).  Else grid groups,
-// the first form that holds every member at once, or, up to max_waves, the
-// last in as few launches as that takes.  Several launches, one after another,
-// are still faster than the multi-kernel CG in FP64 (24 basins of 2.5 M cells:
-// 1.46 against 1.72 ms per step) and slower in MIXED (1.29 against 1.16 ms).  Four
-// rows of quads exist in FP64 only: of the same form in MIXED, a basin of 770,000
+// are independent: a launch holds any number of clusters).  Else, or where the clusters
+// cost too much, grid groups, each member with the CTAs that it needs: the first form
+// that holds every member at once, or, in FP64, the last in as few launches as that
+// takes.  Else none: the multi-kernel CG.
+//
+// What it costs decides, counted in quads of the multi-kernel CG's row work: a form's
+// `round` for each time the chip fills with clusters (members over the clusters that fit
+// at once; every cluster has the size of the largest member's), or for each launch of
+// grid groups, against the quads of all members and `launches`, what the multi-kernel CG
+// spends between its kernels.  The constants are from steps, ms, resident against
+// multi-kernel.  FP64 clusters: 256 members of 12,000 cells 2.05 / 2.59, 96 of 20,000 1.23
+// / 1.45, 48 of 58,000 1.61 / 2.09; of uneven members, 15 of 1,100 and one of 58,000 0.71 /
+// 0.40, 255 and one 8.4 / 0.71.  Launches of grid groups, FP64: 24 of 2.5 M together 1.46 /
+// 1.72 (3 launches), 4 of 610,000 1.94 / 1.96 (4), 255 of 1,100 and one of 100,000 0.79 /
+// 0.72 (2).  MIXED, where the multi-kernel CG moves half the bytes: 512 of 1,100 0.66 /
+// 0.69, 1,024 of them 1.26 / 1.12, 48 of 12,000 0.47 / 0.52, 256 of them 2.10 / 1.49, 32 of
+// 20,000 0.51 / 0.48, 48 of 30,000 0.72 / 0.75, 24 of 58,000 0.77 / 0.73; several launches
+// of grid groups are slower (24 of 2.5 M together 1.29 / 1.16).
+//
+// Four rows of quads exist in FP64 only: of the same form in MIXED, a basin of 770,000
 // cells took 0.50 ms against the multi-kernel CG's 0.49, one of a million 0.53
 // against 0.56.  Two quads a CTA: one after another in FP64, each thread with the
 // registers of two (500x500 cells 0.186 -> 0.177 ms per step, 160x150 0.102 -> 0.099),
 // side by side in MIXED (0.159 against 0.173 and 0.110 against 0.119).
-const std::vector<xm::ResForm> FORMS64 = {{1, 1, 0}, {1, 2, 0}, {2, 2, 0}, {2, 4, 0}};
-const std::vector<xm::ResForm> FORMS32 = {{1, 1, 0}, {2, 1, 0}, {2, 2, 0}};
-constexpr int MX_ROUNDS1 = 6, MX_ROUNDS = 4;  // of one and of more quads a CTA
-bool build_resident(efdc_xm_ctx *c, int (*capacity)(const xm::ResForm &, bool, int),
-                    const std::vector<xm::ResForm> &forms, bool mixed, ResSet &out) {
-  const size_t max_waves = mixed ? 1 : SIZE_MAX;
+struct FormCost {
+  xm::ResForm form;
+  int round;
+};
+struct SolveForms {
+  int (*capacity)(const xm::ResForm &, bool, int);
+  int launches;
+  bool several;  // several launches of grid groups
+  std::vector<FormCost> forms;
+};
+const SolveForms FORMS64 = {xm::cg_res_capacity, 330, true,
+                            {{{1, 1, 0}, 170}, {{1, 2, 0}, 170}, {{2, 2, 0}, 340}, {{2, 4, 0}, 640}}};
+const SolveForms FORMS32 = {xm::mx_res_capacity, 667, false,
+                            {{{1, 1, 0}, 370}, {{2, 1, 0}, 370}, {{2, 2, 0}, 667}}};
+bool build_resident(efdc_xm_ctx *c, const SolveForms &sf, ResSet &out) {
   const int M = c->M, mq = c->max_units;
+  const double multi = double(sf.launches) + c->nquad;
   auto cap_of = [&](const xm::ResForm &f) {
-    return std::min(capacity(f, false, c->nsm), capacity(f, true, c->nsm));
+    return std::min(sf.capacity(f, false, c->nsm), sf.capacity(f, true, c->nsm));
   };
-  for (xm::ResForm f : forms) {
+  for (const FormCost &fc : sf.forms) {
+    xm::ResForm f = fc.form;
     const int per = f.w * f.q, n = (mq + per - 1) / per;
     if (n > 16) continue;
     f.cluster = n;
     const int cap = cap_of(f);
     if (cap < 1) continue;
-    if (mixed && M > (per == 1 ? MX_ROUNDS1 : MX_ROUNDS) * cap) return true;
+    if (fc.round * std::max(1.0, double(M) / cap) > multi) break;
     out.form = f;
     out.waves = {{0, n * M}};
     return true;
   }
-  for (const xm::ResForm &f : forms) {
+  for (const FormCost &fc : sf.forms) {
+    const xm::ResForm &f = fc.form;
     const int per = f.w * f.q, cap = cap_of(f);
-    const bool last = &f == &forms.back();
+    const bool several = sf.several && &fc == &sf.forms.back();
     // one CTA per SM exchanges faster than two: the narrow form only up to there
     const int lim = f.w == 1 ? std::min(cap, c->nsm) : cap;
     std::vector<int4> cta;
@@ -954,7 +972,8 @@ bool build_resident(efdc_xm_ctx *c, int (*capacity)(const xm::ResForm &, bool, i
       waves.back().ncta += n;
       for (int q = q0; q < q1; q += per) cta.push_back(int4{m, q, std::min(per, q1 - q), 0});
     }
-    if (!fits || (waves.size() > 1 && !last) || waves.size() > max_waves) continue;
+    if (!fits) continue;
+    if (waves.size() > 1 && !(several && fc.round * double(waves.size()) <= multi)) continue;
     out.cta = c->alloc<int4>(cta.size(), false);
     if (!out.cta || cudaMemcpy(out.cta, cta.data(), cta.size() * sizeof(int4),
                                cudaMemcpyHostToDevice) != cudaSuccess)
@@ -1554,8 +1573,8 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
   c->qstart_h = qstart;
   for (int m = 0; m < M; ++m) c->max_units = std::max(c->max_units, qstart[m + 1] - qstart[m]);
   c->has_layers.assign(M, 0);
-  if (reset_resident(c) || !build_resident(c, xm::cg_res_capacity, FORMS64, false, c->res64) ||
-      !build_resident(c, xm::mx_res_capacity, FORMS32, true, c->res32))
+  if (reset_resident(c) || !build_resident(c, FORMS64, c->res64) ||
+      !build_resident(c, FORMS32, c->res32))
     return bail("cudaMalloc failed (resident solves)");
   cudaMemcpy(quads_d, quads.data(), quads.size() * sizeof(int4), cudaMemcpyHostToDevice);
   cudaMemcpy(qstart_d, qstart.data(), (M + 1) * sizeof(int), cudaMemcpyHostToDevice);
