@@ -2643,8 +2643,10 @@ bool schedule_valid(const efdc_xm_schedule &s) {
 }
 
 // The workload key of a table line: the precision, the buckets (floor log2)
-// of the member count and of the water cells, and the operator's form.
-std::string tune_key(const efdc_xm_ctx *c, int precision) {
+// of the member count and of the water cells, the operator's form, and whether the
+// solves are resident: those do not use the multi-kernel iteration's knobs, so their
+// lines say nothing about a workload that does.
+std::string workload_key(const efdc_xm_ctx *c, int precision) {
   long long cells = 0;
   for (const Member &mb : c->mem) cells += mb.la - 1;
   auto lg = [](long long v) {
@@ -2660,6 +2662,11 @@ std::string tune_key(const efdc_xm_ctx *c, int precision) {
            precision == EFDC_XM_PREC_MIXED ? "mixed" : "fp64", lg(c->M), lg(cells),
            c->any_may_asym ? 1 : 0, c->S.ch.n > 0 ? 1 : 0);
   return buf;
+}
+
+std::string tune_key(const efdc_xm_ctx *c, int precision) {
+  const bool resident = resident_solve(c, precision == EFDC_XM_PREC_MIXED);
+  return workload_key(c, precision) + (resident ? " solve=resident" : "");
 }
 
 // "key | variant=.. ctas_mv=.. ctas_up=.. iters=.. poly=.. margin=.. tol=.. | ms=.."
@@ -4327,7 +4334,10 @@ int32_t efdc_xm_autotune(efdc_xm_ctx *c, int32_t precision, const char *table, i
   const std::string key = tune_key(c, precision);
   efdc_xm_schedule best{};
   if (solve_ms) *solve_ms = 0.0;
-  if (!(flags & EFDC_XM_TUNE_MEASURE) && table && table_lookup(table, key, &best)) {
+  // (a resident workload without a line of its own: one from before its key said so)
+  if (!(flags & EFDC_XM_TUNE_MEASURE) && table &&
+      (table_lookup(table, key, &best) ||
+       table_lookup(table, workload_key(c, precision), &best))) {
     apply_schedule(c, best);  // replayed: no measurement
     if (chosen) *chosen = best;
     return EFDC_XM_OK;
@@ -4378,9 +4388,11 @@ int32_t efdc_xm_autotune(efdc_xm_ctx *c, int32_t precision, const char *table, i
     apply_schedule(c, best);
     return EFDC_XM_OK;
   };
+  // a resident solve runs none of the kernels and loops of these; variant 3 is variant 1
+  const bool multi = !resident_solve(c, mixed);
   if (mixed) {
-    if ((rc = knob(&efdc_xm_schedule::kernel_variant, {0, 1, 2, 3}))) return rc;
-    if (best.kernel_variant > 0) {
+    if (multi && (rc = knob(&efdc_xm_schedule::kernel_variant, {0, 1, 2}))) return rc;
+    if (multi && best.kernel_variant > 0) {
       if ((rc = knob(&efdc_xm_schedule::ctas_matvec, {0, 2, 3, 4}))) return rc;
       if ((rc = knob(&efdc_xm_schedule::ctas_update, {0, 2, 3, 4}))) return rc;
     }
@@ -4388,7 +4400,7 @@ int32_t efdc_xm_autotune(efdc_xm_ctx *c, int32_t precision, const char *table, i
     if ((rc = knob(&efdc_xm_schedule::inner_margin, {0, 1, 2}))) return rc;
     if ((rc = knob(&efdc_xm_schedule::inner_tol, {40, 50, 60, 70}))) return rc;
   }
-  if ((rc = knob(&efdc_xm_schedule::graph_iters, {2, 4, 8}))) return rc;
+  if (multi && (rc = knob(&efdc_xm_schedule::graph_iters, {2, 4, 8}))) return rc;
   // P as the last step left it
   CK(cudaMemcpyAsync(c->X.p, c->ptune, size_t(c->nslot) * sizeof(double),
                      cudaMemcpyDeviceToDevice, c->stream));

@@ -504,8 +504,12 @@ int64_t efdc_xm_kernel_launches(void);
  * each the median of 5 timed solves, a candidate replacing the incumbent only
  * when 2 % faster -- applies the result and appends it to the table.  *solve_ms: the measured
  * solve time of the chosen schedule (0 when replayed).  The key holds the
- * precision, the floor log2 of the member count and of the water cells, and
- * whether the operator may be unsymmetric or has sub-grid channels. */
+ * precision, the floor log2 of the member count and of the water cells,
+ * whether the operator may be unsymmetric or has sub-grid channels, and whether
+ * the solves are resident (EFDC_XM_OPT_SMALL_SOLVE): of those only the options
+ * they use are tuned, the preconditioner's threshold and the inner target and
+ * tolerance of MIXED.  Without a line of its own a resident workload replays
+ * the line of its key without that word. */
 typedef struct efdc_xm_schedule {
   int32_t kernel_variant;  /* EFDC_XM_OPT_KERNEL_VARIANT */
   int32_t ctas_matvec;     /* EFDC_XM_OPT_CTAS_MATVEC */
