@@ -11,6 +11,9 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <unordered_set>
@@ -67,7 +70,7 @@ constexpr int NARRAYS = 32;   // arrays of a step's upload
 constexpr int NCHUNK = 32;    // most member chunks of a pipelined efdc_xm_step_batch
 constexpr int NCOPY = 4;      // streams for host<->device copies
 constexpr size_t STAGE_BYTES = size_t(64) << 20;  // staging of a transfer in one round, at most
-constexpr int NPIECE = 8;     // slots of the page-locked buffer for pageable arrays
+constexpr int NPIECE = 8;     // slots of a ring for pageable arrays
 // Contexts of at most this many members fold the member reductions into the
 // CG kernels by default.  In a larger batch the CTA that stores last often
 // completes many members at once and sums them one after another at the end
@@ -278,7 +281,7 @@ struct efdc_xm_ctx {
   void *mom_lists = nullptr;  // the serial lists on the device (rebuilt after a set-up call)
   char *pinned = nullptr;  // page-locked: the control mirrors, the job table, the series
   char *pack_h = nullptr, *pack_d = nullptr;  // packed small transfers (page-locked, device)
-  cudaEvent_t piece_event[NPIECE] = {};       // of pack_h as the ring of pageable arrays
+  bool in_ring_pool = false;  // counted among the contexts that the pool of rings serves
   bool mom_inputs = false;    // a call has left U, V, UHDY, VHDX on the device
   std::vector<char> has_mom;
   std::vector<int> mom_ld;
@@ -442,13 +445,22 @@ int d2h_range(efdc_xm_ctx *c, const Xfer &x, const char *stage, int m0, int m1, 
 // array: those, not bytes, bound a small basin's step on host arrays.
 constexpr size_t PACK_MAX = size_t(4) << 20;  // bytes of one packed transfer
 
-// Its device side is allocated by the first packed transfer (a small context's creation).
-bool pack_buffer(efdc_xm_ctx *c) {
-  if (c->pack_h && !c->pack_d && !(c->pack_d = c->alloc<char>(PACK_MAX, false))) cudaGetLastError();
-  return c->pack_d != nullptr;
-}
 bool packed(efdc_xm_ctx *c, size_t njobs) {
-  return njobs * size_t(c->stage_len) * sizeof(double) <= PACK_MAX && pack_buffer(c);
+  const size_t bytes = njobs * size_t(c->stage_len) * sizeof(double);
+  if (bytes > PACK_MAX) return false;
+  if (!c->pack_h) {
+    if (cudaHostAlloc(&c->pack_h, PACK_MAX, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      c->pack_h = nullptr;
+      return false;
+    }
+    if (!(c->pack_d = c->alloc<char>(PACK_MAX, false))) {
+      cudaFreeHost(c->pack_h);
+      c->pack_h = nullptr;
+      return false;
+    }
+  }
+  return true;
 }
 
 // The kernels of a packed transfer (go: one launch), JobTable::CAP arrays each: the job
@@ -510,15 +522,14 @@ int download_packed(efdc_xm_ctx *c, const std::vector<Xfer> &xs) {
   return EFDC_XM_OK;
 }
 
-// Larger transfers of pageable host arrays: pieces through the same page-locked buffer
-// as a ring, the host copies by up to NCOPY threads (of this call only: joined before
-// it returns), each with its own slots and its own copy stream, so that host copies and
-// link run side by side.  The driver's own staging of pageable copies moved 450 KB
-// arrays at 18 GB/s in and 7.5 out.  Measured (16 cores): the calls of a coupled step of
-// 56,000 cells and four layers 3.6 -> 2.65 ms, with one thread 2.9, with slots of 256 KB
-// 3.1; a ring of 8 MB was even there and 5 % faster at 160,000 cells, but doubles what a
-// context locks; slabs of 1 MB across arrays in a ring of 16 MB 3.0 (it no longer stays
-// in the caches).
+// Larger transfers of pageable host arrays: pieces through a page-locked ring, the host
+// copies by up to NCOPY threads (of this call only: joined before it returns), each with
+// its own slots and its own copy stream, so that host copies and link run side by side.
+// The driver's own staging of pageable copies moved 450 KB arrays at 18 GB/s in and 7.5
+// out.  Measured: the calls of a coupled step of 56,000 cells and four layers 3.9 -> 2.95
+// ms; when the ring was written 3.6 -> 2.65, with one thread 2.9, with slots of 256 KB 3.1,
+// with a ring of 8 MB the same (5 % faster at 160,000 cells), with slabs of 1 MB across
+// arrays in a ring of 16 MB 3.0 (it no longer stays in the caches).
 // A piece is a range of one array's staging buffer: part of a long member's, or several
 // short members' (each a segment of it): all arrays of 256 lakes of 1,100 cells, 9 KB an
 // array and member, go up in 2.8 ms and down in 2.4 (with a copy and an event per array
@@ -539,7 +550,91 @@ struct Pieces {
 constexpr size_t PIECE_MAX = size_t(512) << 10;     // bytes of a slot
 constexpr size_t PIECE_THREAD = size_t(1) << 20;    // bytes that are worth another thread
 constexpr int PIECE_SLOTS = NPIECE / NCOPY;  // of a thread
-static_assert(NPIECE * PIECE_MAX <= PACK_MAX, "the slots fit the buffer");
+
+// A ring is lent to a transfer for its duration by its device's pool, so that the contexts
+// of a process share a few.  Page-locking one takes 2 to 5 ms, what it saves on about 128
+// MB: until the pool's contexts have moved that much, transfers go through the driver, as
+// they do when RING_MAX others are on their way.  The rings are freed, and the count starts
+// anew, when the device's last context is destroyed.
+constexpr size_t RING_AFTER = size_t(128) << 20;
+constexpr int RING_MAX = 4;
+struct Ring {
+  char *h = nullptr;
+  cudaEvent_t ev[NPIECE] = {};
+  ~Ring() {
+    for (cudaEvent_t e : ev)
+      if (e) cudaEventDestroy(e);
+    if (h) cudaFreeHost(h);
+  }
+};
+struct RingPool {
+  std::mutex mu;
+  int contexts = 0, made = 0;
+  size_t moved = 0;
+  std::vector<std::unique_ptr<Ring>> idle;
+};
+RingPool &ring_pool(int device) {
+  static std::mutex mu;
+  static auto *pools = new std::map<int, RingPool>;  // not destroyed: CUDA may be gone by then
+  std::lock_guard<std::mutex> lock(mu);
+  return (*pools)[device];
+}
+void ring_pool_enter(efdc_xm_ctx *c) {
+  RingPool &p = ring_pool(c->device);
+  std::lock_guard<std::mutex> lock(p.mu);
+  ++p.contexts;
+  c->in_ring_pool = true;
+}
+void ring_pool_leave(efdc_xm_ctx *c) {  // (on the context's device)
+  if (!c->in_ring_pool) return;
+  RingPool &p = ring_pool(c->device);
+  std::lock_guard<std::mutex> lock(p.mu);
+  if (--p.contexts > 0) return;
+  p.idle.clear();
+  p.made = 0;
+  p.moved = 0;
+}
+// The ring of one transfer of `bytes` pageable bytes (ring null: none to be had).
+struct RingLoan {
+  efdc_xm_ctx *c;
+  std::unique_ptr<Ring> ring;
+  RingLoan(efdc_xm_ctx *ctx, size_t bytes) : c(ctx) {
+    if (bytes == 0) return;
+    RingPool &p = ring_pool(c->device);
+    {
+      std::lock_guard<std::mutex> lock(p.mu);
+      p.moved += bytes;
+      if (!p.idle.empty()) {
+        ring = std::move(p.idle.back());
+        p.idle.pop_back();
+        return;
+      }
+      if (p.moved <= RING_AFTER || p.made >= RING_MAX) return;
+      ++p.made;
+    }
+    ring = std::make_unique<Ring>();
+    bool ok = cudaHostAlloc(&ring->h, NPIECE * PIECE_MAX, cudaHostAllocDefault) == cudaSuccess;
+    if (!ok) ring->h = nullptr;
+    for (cudaEvent_t &e : ring->ev)
+      if (ok && !(ok = cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess))
+        e = nullptr;
+    if (ok) return;
+    cudaGetLastError();
+    ring.reset();
+    std::lock_guard<std::mutex> lock(p.mu);
+    --p.made;
+  }
+  ~RingLoan() {
+    if (!ring) return;
+    // (after an error: copies may still be on their way)
+    for (cudaStream_t s : c->copy_stream) cudaStreamSynchronize(s);
+    RingPool &p = ring_pool(c->device);
+    std::lock_guard<std::mutex> lock(p.mu);
+    p.idle.push_back(std::move(ring));
+  }
+  RingLoan(const RingLoan &) = delete;
+  RingLoan &operator=(const RingLoan &) = delete;
+};
 
 // The pieces of one array: add_range for its members in order.
 struct PieceMaker {
@@ -565,13 +660,13 @@ struct PieceMaker {
 
 // One thread's share: the pieces it takes from the counter.  Up: a slot is filled
 // again when its copy has left it.  Down: as many copies ahead as slots.
-cudaError_t move_pieces(efdc_xm_ctx *c, const Pieces &ps, std::atomic<size_t> &next, int w,
-                        bool up) {
+cudaError_t move_pieces(efdc_xm_ctx *c, Ring &ring, const Pieces &ps, std::atomic<size_t> &next,
+                        int w, bool up) {
   const std::vector<Piece> &v = ps.v;
   cudaError_t e = cudaSetDevice(c->device);
   const cudaStream_t st = c->copy_stream[w];
-  char *buf = c->pack_h + size_t(w) * PIECE_SLOTS * PIECE_MAX;
-  cudaEvent_t *ev = c->piece_event + w * PIECE_SLOTS;
+  char *buf = ring.h + size_t(w) * PIECE_SLOTS * PIECE_MAX;
+  cudaEvent_t *ev = ring.ev + w * PIECE_SLOTS;
   size_t held[PIECE_SLOTS] = {}, k0 = 0, k1 = 0;  // copies k0..k1-1 are in flight, k in slot k % SLOTS
   auto retire = [&] {
     const int q = int(k0 % PIECE_SLOTS);
@@ -603,8 +698,9 @@ cudaError_t move_pieces(efdc_xm_ctx *c, const Pieces &ps, std::atomic<size_t> &n
   return e;
 }
 
-int move_all_pieces(efdc_xm_ctx *c, const Pieces &ps, bool up) {
+int move_all_pieces(efdc_xm_ctx *c, const RingLoan &loan, const Pieces &ps, bool up) {
   if (ps.v.empty()) return EFDC_XM_OK;
+  Ring &ring = *loan.ring;
   size_t bytes = 0;
   for (const Piece &p : ps.v) bytes += p.n;
   (up ? g_h2d : g_d2h).fetch_add(static_cast<long long>(bytes), std::memory_order_relaxed);
@@ -614,12 +710,12 @@ int move_all_pieces(efdc_xm_ctx *c, const Pieces &ps, bool up) {
   std::thread th[NCOPY];
   for (int w = 1; w < nw; ++w) {
     try {
-      th[w] = std::thread([&, w] { err[w] = move_pieces(c, ps, next, w, up); });
+      th[w] = std::thread([&, w] { err[w] = move_pieces(c, ring, ps, next, w, up); });
     } catch (...) {
       break;  // no thread to be had: the ones there are take the pieces
     }
   }
-  err[0] = move_pieces(c, ps, next, 0, up);
+  err[0] = move_pieces(c, ring, ps, next, 0, up);
   for (std::thread &t : th)
     if (t.joinable()) t.join();
   for (cudaError_t e : err) CK(e);
@@ -644,16 +740,15 @@ bool pageable(efdc_xm_ctx *c, const Xfer &x) {
   }
   return true;
 }
-// The ring of pageable transfers.
-bool pieces_ready(efdc_xm_ctx *c) {
-  if (!c->pack_h) return false;
-  for (cudaEvent_t &e : c->piece_event)
-    if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
-      cudaGetLastError();
-      e = nullptr;
-      return false;
-    }
-  return true;
+// Which arrays of a transfer are pageable, and their bytes.
+size_t pageable_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs, std::vector<char> &pg) {
+  size_t n = 0;
+  pg.resize(xs.size());
+  for (size_t j = 0; j < xs.size(); ++j) {
+    pg[j] = pageable(c, xs[j]);
+    if (pg[j]) n += esize(xs[j].kind) * size_t(c->stage_len);
+  }
+  return n;
 }
 
 // More staging buffers, for transfers in which every array takes its own.
@@ -695,6 +790,8 @@ int upload_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs, bool wait = true)
     c->jobs_h[j] = CopyJob{c->stage[j % G], xs[j].dev, xs[j].kind};
   CK(cudaMemcpyAsync(c->jobs_d, c->jobs_h, xs.size() * sizeof(CopyJob), cudaMemcpyHostToDevice,
                      c->stream));
+  std::vector<char> pg;
+  const RingLoan loan(c, pageable_arrays(c, xs, pg));
   int rc = 0, k = 0;
   for (size_t g0 = 0; g0 < xs.size(); g0 += G) {
     const size_t g1 = std::min(xs.size(), g0 + G);
@@ -703,7 +800,7 @@ int upload_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs, bool wait = true)
     Pieces v;
     for (size_t j = g0; j < g1; ++j) {
       char *stage = reinterpret_cast<char *>(c->stage[j % G]);
-      if (pageable(c, xs[j]) && pieces_ready(c)) {
+      if (pg[j] && loan.ring) {
         const size_t es = esize(xs[j].kind);
         PieceMaker mk{v};
         for (int m = 0; m < c->M; ++m)
@@ -713,7 +810,7 @@ int upload_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs, bool wait = true)
         return rc;
       }
     }
-    if ((rc = move_all_pieces(c, v, true))) return rc;
+    if ((rc = move_all_pieces(c, loan, v, true))) return rc;
     if ((rc = compute_after_copies(c))) return rc;
     xm::launch_scatter(c->stream, c->jobs_d + g0, int(g1 - g0), c->lidx, c->tile_member, c->moff,
                        c->mlc, 0, c->nslot);
@@ -736,6 +833,8 @@ int download_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs) {
   CK(cudaMemcpyAsync(c->jobs_d, c->jobs_h, xs.size() * sizeof(CopyJob), cudaMemcpyHostToDevice,
                      c->stream));
   std::vector<Keep> keep;  // put back once the copies are done (the caller waits here)
+  std::vector<char> pg;
+  const RingLoan loan(c, pageable_arrays(c, xs, pg));
   int rc = 0, k = 0;
   for (size_t g0 = 0; g0 < xs.size(); g0 += G) {
     const size_t g1 = std::min(xs.size(), g0 + G);
@@ -747,7 +846,7 @@ int download_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs) {
     Pieces v;
     for (size_t j = g0; j < g1; ++j) {
       char *stage = reinterpret_cast<char *>(c->stage[j % G]);
-      if (pageable(c, xs[j]) && pieces_ready(c)) {
+      if (pg[j] && loan.ring) {
         const size_t es = esize(xs[j].kind);
         PieceMaker mk{v};
         for (int m = 0; m < c->M; ++m)  // the water elements L = 2..LA
@@ -757,7 +856,7 @@ int download_arrays(efdc_xm_ctx *c, const std::vector<Xfer> &xs) {
         return rc;
       }
     }
-    if ((rc = move_all_pieces(c, v, false))) return rc;
+    if ((rc = move_all_pieces(c, loan, v, false))) return rc;
   }
   for (cudaStream_t s : c->copy_stream) CK(cudaStreamSynchronize(s));
   CK(cudaStreamSynchronize(c->stream));
@@ -1311,8 +1410,7 @@ void efdc_xm_destroy(efdc_xm_ctx *c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   for (auto &b : c->bufs) cudaFree(b.p);
   if (c->mom_lists) cudaFree(c->mom_lists);
-  for (cudaEvent_t e : c->piece_event)
-    if (e) cudaEventDestroy(e);
+  ring_pool_leave(c);
   if (c->pinned) cudaFreeHost(c->pinned);
   if (c->pack_h) cudaFreeHost(c->pack_h);
   if (c->gslot) cudaFree(c->gslot);
@@ -1399,6 +1497,7 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
     delete c;
     return nullptr;
   }
+  ring_pool_enter(c);
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
     return bail("stream creation failed");
   for (cudaStream_t &s : c->copy_stream)
@@ -1639,12 +1738,6 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
     if (cudaHostAlloc(&c->pinned, need, cudaHostAllocMapped) != cudaSuccess) {
       c->pinned = nullptr;
       return bail("cudaHostAlloc failed");
-    }
-    // and the transfers' buffer, here rather than in the first call that wants it, which
-    // it would cost several milliseconds; without it they go through the driver
-    if (cudaHostAlloc(&c->pack_h, PACK_MAX, cudaHostAllocDefault) != cudaSuccess) {
-      cudaGetLastError();
-      c->pack_h = nullptr;
     }
     c->ctl_h = reinterpret_cast<Ctl *>(c->pinned + ctl);
     c->glob_h = reinterpret_cast<Glob *>(c->pinned + glob);
