@@ -1085,8 +1085,7 @@ bool build_resident(efdc_xm_ctx *c, const SolveForms &sf, ResSet &out) {
 }
 
 xm::ResPlan res_plan(const efdc_xm_ctx *c, const ResSet &r, const ResSet::Wave &w) {
-  return xm::ResPlan{r.cta ? r.cta + w.cta0 : nullptr, c->res_part, c->res_count,
-                     xm::wait_polls()};
+  return xm::ResPlan{r.cta ? r.cta + w.cta0 : nullptr, c->res_part, c->res_count};
 }
 
 void launch_resident64(efdc_xm_ctx *c, const xm::Launch &l, const xm::SysView &V, double *P,
@@ -1109,12 +1108,22 @@ int reset_resident(efdc_xm_ctx *c) {
   return EFDC_XM_OK;
 }
 
+// With a short limit of the waits (efdc_xm_set_wait_limit): the groups of CTAs of the
+// next solves wait for arrivals that never come.
+int spoil_resident(efdc_xm_ctx *c) {
+  if (xm::wait_polls() < xm::WAIT_POLLS)
+    CK(cudaMemset2DAsync(c->res_count + 1, xm::RES_COUNT_STRIDE * sizeof(unsigned), 1,
+                         sizeof(unsigned), c->M, c->stream));
+  return EFDC_XM_OK;
+}
+
 // Of the system V: a resident solve's, the step's unscaled assembly or Y's
 // scaled system; the multi-kernel CG takes Y's whatever V is.
 int solve_fp64(efdc_xm_ctx *c, const xm::SysView &V, double *P) {
   const xm::Launch l = c->L();
   xm::launch_solve_reset(l, c->ctl, c->glob, c->act, c->M);
   if (resident_solve(c, false)) {  // the whole CG of each member in one launch
+    if (const int rs = spoil_resident(c)) return rs;
     launch_resident64(c, l, V, P, xm::ResEnds{});
     CK(cudaGetLastError());
     int rc = read_ctl(c);
@@ -1199,6 +1208,7 @@ int solve_mixed(efdc_xm_ctx *c, double *P, double factor) {
   xm::launch_chan_p0(lk, c->S, c->mxview, P, c->act);
   int rc = 0;
   if (resident_solve(c, true)) {
+    if ((rc = spoil_resident(c))) return rc;
     launch_resident32(c, lk, P, fac, xm::ResEnds{});
     CK(cudaGetLastError());
     if ((rc = read_ctl(c))) return rc;
@@ -2317,7 +2327,7 @@ struct StepPlan {
   int mixed, istl, all, any_isdry, any_legacy, any99, any_waste, iters;
   int max_iterm, max_sweeps, grid, grid_cg, grid_cg32, grid_up32;
   int mx_jac, mx_poly, may_asym, chan, baro, obc_serial, any_may_asym, nmember;
-  int variant, ctas_mv, ctas_up, any_drag, resident, polls;
+  int variant, ctas_mv, ctas_up, any_drag, resident;
   double fac, inner_margin;
   const void *psol;
 };
@@ -2629,6 +2639,7 @@ int run_step_graph(efdc_xm_ctx *c, const StepPlan &pl, const xm::DevState &x_pre
                    const efdc_xm_params *prm, efdc_xm_stats *stats, int m0, int m1) {
   StepGraph *sg = step_graph(c, pl, x_pre);
   if (!sg) return -1;
+  if (const int rs = pl.resident ? spoil_resident(c) : EFDC_XM_OK) return rs;
   CK(cudaGraphLaunch(sg->exec, c->stream));
   if (!mirrors_mapped(c)) {
     CK(cudaMemcpyAsync(c->ctl_h, c->ctl, sizeof(Ctl) * c->M, cudaMemcpyDeviceToHost, c->stream));
@@ -3076,7 +3087,6 @@ int step_range(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_stats *stats, 
     pl.nmember = M;
     pl.fac = mixed ? (prm[0].mixed_rsq_factor > 0 ? prm[0].mixed_rsq_factor : 0.1) : 0.0;
     pl.psol = c->psol;
-    pl.polls = xm::wait_polls();  // (a captured launch keeps it)
     rc = run_step_graph(c, pl, x_pre, prm, stats, m0, m1);
     if (rc >= 0) {
       if (istl == 0) c->tl3_ready = false;  // CALPUV2C does not keep the three levels

@@ -75,7 +75,6 @@ struct ResPlan {
   double2 *part;    // grid groups: [2][nquad] the quads' partial sums, by turns
   unsigned *count;  // grid groups: [M*RES_COUNT_STRIDE] the member's arrivals, and next to it
                     // the arrivals at the end of its last launch
-  int polls;        // of that counter, before a wait is given up
 };
 constexpr int RES_COUNT_STRIDE = 32;  // a 128-byte line per member
 // What a resident solve does at its ends besides solving.
@@ -211,8 +210,8 @@ void launch_after_solve(cudaStream_t st, Ctl *ctl, int *act, int nmember, int mi
 void launch_sweep_next(cudaStream_t st, const DevStatic &S, Ctl *ctl, int *act, Glob *g,
                        cudaGraphConditionalHandle h, int cap, int nmember);
 
-// Polls of a counter before a device-side wait is given up, for the launches of this
-// host thread (efdc_xm_set_wait_limit).
+// Polls of a counter before a device-side wait is given up, and the limit in force for
+// the calls of this host thread (efdc_xm_set_wait_limit).
 constexpr int WAIT_POLLS = 1 << 20;  // about a second
 int wait_polls();
 

@@ -278,7 +278,7 @@ __device__ __forceinline__ bool res_exchange(const ResPlan &R, const DevStatic &
         unsigned *n = R.count + size_t(c.m) * RES_COUNT_STRIDE;
         red_release(n, 1u);
         for (int k = 0; int(ld_acquire(n) - bar.count) < 0; ++k)
-          if (k >= R.polls) {
+          if (k >= WAIT_POLLS) {
             dead = 1;
             break;
           }
@@ -333,15 +333,19 @@ __device__ __forceinline__ void res_check_faces(const DevStatic &S, const SysVie
 
 // A wait ran out: the call fails with a timeout status.  The CTA has not stored its part
 // of the solution, and the others may have come through the same exchange: the status
-// of the one that ends the solve (res_status) does not replace this one.
+// of the one that ends the solve (res_status) does not replace this one, the largest.
+// (A limit of the waits as a kernel argument, or a compare-and-swap here, cost the
+// registers of the MIXED 2x1 form: 512x512 cells 0.163 -> 0.166 ms per step.)
 __device__ __forceinline__ void res_fail(Ctl &k, int *err) {
   if (threadIdx.x == 0) {
-    atomicExch(&k.status, EFDC_XM_DEVICE_TIMEOUT);
+    atomicMax(&k.status, EFDC_XM_DEVICE_TIMEOUT);
     atomicExch(err, 1);
   }
 }
 __device__ __forceinline__ void res_status(Ctl &k, int status) {  // OK at the entry
-  atomicCAS(&k.status, EFDC_XM_OK, status);
+  static_assert(EFDC_XM_DEVICE_TIMEOUT > EFDC_XM_NONFINITE &&
+                EFDC_XM_DEVICE_TIMEOUT > EFDC_XM_CG_MAXITER, "the largest of a solve");
+  atomicMax(&k.status, status);
 }
 
 // Row vectors of NC coefficients of the thread's quads: in registers (REG), or

@@ -533,10 +533,11 @@ int32_t efdc_xm_tune_lookup(const char *table, const char *key, efdc_xm_schedule
  * device (EFDC_XM_OPT_DEVICE_LOOPS) waits once, when it has finished. */
 int64_t efdc_xm_host_waits(void);
 
-/* How often a CTA of a solve that runs in one launch looks for the others before it gives
- * up and the call returns EFDC_XM_DEVICE_TIMEOUT, in the calls that this host thread makes
- * from now on.  The default (restored by a negative value) takes about a second; a short
- * limit is for testing what a host program does on that status.  Returns the old limit. */
+/* For testing what a host program does on EFDC_XM_DEVICE_TIMEOUT: how often a CTA of
+ * efdc_xm_congrad_noalloc looks for the others before it gives up, in the calls that this
+ * host thread makes from now on.  The default (restored by a negative value) takes about
+ * a second.  With a smaller limit the solves of contexts that run in groups of CTAs wait
+ * for one that never comes, about a second.  Returns the old limit. */
 int32_t efdc_xm_set_wait_limit(int32_t polls);
 
 /* Options of a context (no counterpart in the reference).
