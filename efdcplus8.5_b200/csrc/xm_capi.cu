@@ -192,7 +192,7 @@ struct efdc_xm_ctx {
        *sc_hd = nullptr;
   bool in_chunks = false;  // inside a chunked efdc_xm_step_batch (see to_device)
   double *part = nullptr;
-  ResSet res64, res32;          // resident solves, FP64 and MIXED
+  ResSet res64[2], res32[2];    // resident solves, FP64 and MIXED: of all members, of a chunk's
   double2 *res_part = nullptr;   // their grid groups' partial sums
   unsigned *res_count = nullptr; // and arrival counters
   int *lidx = nullptr;
@@ -993,8 +993,10 @@ double inner_rel_tol(const efdc_xm_ctx *c) { return std::pow(10.0, -0.1 * c->inn
 // How a solve runs: iteration kernels of every member in lockstep, or resident
 // groups of CTAs (contexts without sub-grid channels, whose terms are separate
 // kernels of the multi-kernel CG).
-bool resident_solve(const efdc_xm_ctx *c, bool mixed) {
-  return c->resident && c->S.ch.n == 0 && !(mixed ? c->res32 : c->res64).waves.empty();
+// part: of some of the members (a chunk of an efdc_xm_step_batch), else of all.
+bool resident_solve(const efdc_xm_ctx *c, bool mixed, bool part = false) {
+  return c->resident && c->S.ch.n == 0 &&
+         !(mixed ? c->res32[part] : c->res64[part]).waves.empty();
 }
 
 // The form of a resident solve.  One cluster per member where the largest
@@ -1037,9 +1039,11 @@ const SolveForms FORMS64 = {xm::cg_res_capacity, 330, true,
                             {{{1, 1, 0}, 170}, {{1, 2, 0}, 170}, {{2, 2, 0}, 340}, {{2, 4, 0}, 640}}};
 const SolveForms FORMS32 = {xm::mx_res_capacity, 667, false,
                             {{{1, 1, 0}, 370}, {{2, 1, 0}, 370}, {{2, 2, 0}, 667}}};
-bool build_resident(efdc_xm_ctx *c, const SolveForms &sf, ResSet &out) {
+// active: the members that step together, all or (a chunk of an efdc_xm_step_batch) some;
+// the others' clusters and launches end at once.
+bool build_resident(efdc_xm_ctx *c, const SolveForms &sf, int active, ResSet &out) {
   const int M = c->M, mq = c->max_units;
-  const double multi = double(sf.launches) + c->nquad;
+  const double share = double(active) / M, multi = sf.launches + c->nquad * share;
   auto cap_of = [&](const xm::ResForm &f) {
     return std::min(sf.capacity(f, false, c->nsm), sf.capacity(f, true, c->nsm));
   };
@@ -1050,7 +1054,7 @@ bool build_resident(efdc_xm_ctx *c, const SolveForms &sf, ResSet &out) {
     f.cluster = n;
     const int cap = cap_of(f);
     if (cap < 1) continue;
-    if (fc.round * std::max(1.0, double(M) / cap) > multi) break;
+    if (fc.round * std::max(1.0, double(active) / cap) > multi) break;
     out.form = f;
     out.waves = {{0, n * M}};
     return true;
@@ -1072,7 +1076,9 @@ bool build_resident(efdc_xm_ctx *c, const SolveForms &sf, ResSet &out) {
       for (int q = q0; q < q1; q += per) cta.push_back(int4{m, q, std::min(per, q1 - q), 0});
     }
     if (!fits) continue;
-    if (waves.size() > 1 && !(several && fc.round * double(waves.size()) <= multi)) continue;
+    // (a launch of members that take no part: 5 us)
+    const double n = double(waves.size()), cost = fc.round * std::max(1.0, n * share) + 10 * n;
+    if (n > 1 && !(several && cost <= multi)) continue;
     out.cta = c->alloc<int4>(cta.size(), false);
     if (!out.cta || cudaMemcpy(out.cta, cta.data(), cta.size() * sizeof(int4),
                                cudaMemcpyHostToDevice) != cudaSuccess)
@@ -1088,17 +1094,19 @@ xm::ResPlan res_plan(const efdc_xm_ctx *c, const ResSet &r, const ResSet::Wave &
   return xm::ResPlan{r.cta ? r.cta + w.cta0 : nullptr, c->res_part, c->res_count};
 }
 
-void launch_resident64(efdc_xm_ctx *c, const xm::Launch &l, const xm::SysView &V, double *P,
-                       const xm::ResEnds &ends) {
-  for (const ResSet::Wave &w : c->res64.waves)
-    xm::launch_cg_res(l, c->S, V, c->Y, P, c->ctl, c->glob, res_plan(c, c->res64, w),
-                      c->res64.form, w.ncta, ends);
+void launch_resident64(efdc_xm_ctx *c, bool part, const xm::Launch &l, const xm::SysView &V,
+                       double *P, const xm::ResEnds &ends) {
+  const ResSet &r = c->res64[part];
+  for (const ResSet::Wave &w : r.waves)
+    xm::launch_cg_res(l, c->S, V, c->Y, P, c->ctl, c->glob, res_plan(c, r, w), r.form, w.ncta,
+                      ends);
 }
-void launch_resident32(efdc_xm_ctx *c, const xm::Launch &l, double *P, double fac,
+void launch_resident32(efdc_xm_ctx *c, bool part, const xm::Launch &l, double *P, double fac,
                        const xm::ResEnds &ends) {
-  for (const ResSet::Wave &w : c->res32.waves)
-    xm::launch_mx_res(l, c->S, c->mxview, c->Y, P, c->ctl, c->glob, res_plan(c, c->res32, w),
-                      c->res32.form, w.ncta, fac, inner_rel_tol(c), MAX_OUTER, ends);
+  const ResSet &r = c->res32[part];
+  for (const ResSet::Wave &w : r.waves)
+    xm::launch_mx_res(l, c->S, c->mxview, c->Y, P, c->ctl, c->glob, res_plan(c, r, w), r.form,
+                      w.ncta, fac, inner_rel_tol(c), MAX_OUTER, ends);
 }
 
 // No arrivals counted: at the start, and after a wait that ran out.
@@ -1119,12 +1127,12 @@ int spoil_resident(efdc_xm_ctx *c) {
 
 // Of the system V: a resident solve's, the step's unscaled assembly or Y's
 // scaled system; the multi-kernel CG takes Y's whatever V is.
-int solve_fp64(efdc_xm_ctx *c, const xm::SysView &V, double *P) {
+int solve_fp64(efdc_xm_ctx *c, const xm::SysView &V, double *P, bool part = false) {
   const xm::Launch l = c->L();
   xm::launch_solve_reset(l, c->ctl, c->glob, c->act, c->M);
-  if (resident_solve(c, false)) {  // the whole CG of each member in one launch
+  if (resident_solve(c, false, part)) {  // the whole CG of each member in one launch
     if (const int rs = spoil_resident(c)) return rs;
-    launch_resident64(c, l, V, P, xm::ResEnds{});
+    launch_resident64(c, part, l, V, P, xm::ResEnds{});
     CK(cudaGetLastError());
     int rc = read_ctl(c);
     if (rc) return rc;
@@ -1199,7 +1207,7 @@ int send_inner(efdc_xm_ctx *c) {
 
 // MIXED: FP64 refinement around the FP32 inner PCG, all active members in
 // lockstep outer passes.
-int solve_mixed(efdc_xm_ctx *c, double *P, double factor) {
+int solve_mixed(efdc_xm_ctx *c, double *P, double factor, bool part = false) {
   const double fac = factor > 0 ? factor : 0.1;  // stop at fac*RSQM in FP64
   xm::launch_solve_reset(c->L(), c->ctl, c->glob, c->act, c->M);
   choose_inner(c);
@@ -1207,9 +1215,9 @@ int solve_mixed(efdc_xm_ctx *c, double *P, double factor) {
   const xm::Launch lk = c->L();  // with the kinds in use
   xm::launch_chan_p0(lk, c->S, c->mxview, P, c->act);
   int rc = 0;
-  if (resident_solve(c, true)) {
+  if (resident_solve(c, true, part)) {
     if ((rc = spoil_resident(c))) return rc;
-    launch_resident32(c, lk, P, fac, xm::ResEnds{});
+    launch_resident32(c, part, lk, P, fac, xm::ResEnds{});
     CK(cudaGetLastError());
     if ((rc = read_ctl(c))) return rc;
     for (int m = 0; m < c->M; ++m) {
@@ -1682,8 +1690,10 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
   c->qstart_h = qstart;
   for (int m = 0; m < M; ++m) c->max_units = std::max(c->max_units, qstart[m + 1] - qstart[m]);
   c->has_layers.assign(M, 0);
-  if (reset_resident(c) || !build_resident(c, FORMS64, c->res64) ||
-      !build_resident(c, FORMS32, c->res32))
+  if (reset_resident(c) || !build_resident(c, FORMS64, M, c->res64[0]) ||
+      !build_resident(c, FORMS32, M, c->res32[0]) ||
+      (M > 1 && (!build_resident(c, FORMS64, (M + 7) / 8, c->res64[1]) ||
+                 !build_resident(c, FORMS32, (M + 7) / 8, c->res32[1]))))
     return bail("cudaMalloc failed (resident solves)");
   cudaMemcpy(quads_d, quads.data(), quads.size() * sizeof(int4), cudaMemcpyHostToDevice);
   cudaMemcpy(qstart_d, qstart.data(), (M + 1) * sizeof(int), cudaMemcpyHostToDevice);
@@ -2327,7 +2337,7 @@ struct StepPlan {
   int mixed, istl, all, any_isdry, any_legacy, any99, any_waste, iters;
   int max_iterm, max_sweeps, grid, grid_cg, grid_cg32, grid_up32;
   int mx_jac, mx_poly, may_asym, chan, baro, obc_serial, any_may_asym, nmember;
-  int variant, ctas_mv, ctas_up, any_drag, resident;
+  int variant, ctas_mv, ctas_up, any_drag, resident, part;
   double fac, inner_margin;
   const void *psol;
 };
@@ -2420,9 +2430,9 @@ cudaError_t capture_solve(efdc_xm_ctx *c, const StepPlan &pl, int d, StepGraph &
   if (pl.resident) {  // the loops inside the kernel
     const xm::ResEnds ends{step ? c->act : nullptr, step && !c->any_may_asym ? 1 : 0};
     if (pl.mixed)
-      launch_resident32(c, l, P, pl.fac, ends);
+      launch_resident32(c, pl.part, l, P, pl.fac, ends);
     else
-      launch_resident64(c, l, c->mxview, P, ends);
+      launch_resident64(c, pl.part, l, c->mxview, P, ends);
     take_count(mark, mine);
     return cudaGetLastError();
   }
@@ -2972,7 +2982,8 @@ int step_range(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_stats *stats, 
   const bool mixed = prm[0].precision == EFDC_XM_PREC_MIXED;
   c->mxview = xm::SysView{c->X.fp, c->X.cc, c->X.cs, c->X.cw, c->X.ce, c->X.cn, 1};
   c->last_mixed = mixed;
-  const bool resident = resident_solve(c, mixed);
+  const bool part = m0 != 0 || m1 != M;
+  const bool resident = resident_solve(c, mixed, part);
   c->scaled_ready = !mixed && !resident;
   c->inner_ready = mixed && !resident;
   c->sys_external = false;
@@ -3055,6 +3066,7 @@ int step_range(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_stats *stats, 
     const xm::Launch lk = c->L();
     pl.mixed = mixed;
     pl.resident = resident;
+    pl.part = part;
     pl.istl = istl;
     pl.all = all;
     pl.any_isdry = any_isdry;
@@ -3118,8 +3130,8 @@ int step_range(efdc_xm_ctx *c, const efdc_xm_params *prm, efdc_xm_stats *stats, 
       xm::launch_scale(l, c->S, c->X, c->Y, c->ctl, c->act, mixed ? 1 : 0,
                        c->any_may_asym ? 1 : 0);
     CK(cudaGetLastError());
-    rc = mixed ? solve_mixed(c, c->X.p, prm[0].mixed_rsq_factor)
-               : solve_fp64(c, c->mxview, c->X.p);
+    rc = mixed ? solve_mixed(c, c->X.p, prm[0].mixed_rsq_factor, part)
+               : solve_fp64(c, c->mxview, c->X.p, part);
     if (rc) return rc;
     if ((rc = read_glob(c))) return rc;
     if (c->glob_h->err) return device_timeout(c, stats, m0, m1);
