@@ -90,6 +90,11 @@ int wait_polls() { return g_wait_polls; }
 void set_last_error_str(const char *msg) { g_last_error = msg ? msg : ""; }
 }  // namespace xm
 
+// The set-up work of a context, which runs on the legacy stream, is done.  (Not the whole
+// device: that is refused while another host thread captures its first step, whose capture
+// it invalidates.)
+static cudaError_t legacy_done() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 // A device buffer owned by the context.
 struct DevBuf {
   void *p = nullptr;
@@ -1839,7 +1844,7 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
   }
   // the zero-fills above ran on the legacy stream; finish them before any
   // work on the non-blocking solver stream
-  if (cudaDeviceSynchronize() != cudaSuccess) return bail("device error during allocation");
+  if (legacy_done() != cudaSuccess) return bail("device error during allocation");
   // static metrics into tile order (land slots take element LC of their member)
   auto per = [&](const double *efdc_xm_grid::*f) {
     std::vector<const void *> v(M);
@@ -1856,7 +1861,7 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
   for (const auto &mt : metrics) xs.push_back(Xfer{per(mt.first), mt.second, 0});
   if (upload_arrays(c, xs) != EFDC_XM_OK)
     return bail("upload of the static arrays failed");
-  if (cudaDeviceSynchronize() != cudaSuccess) return bail("device error during set-up");
+  if (legacy_done() != cudaSuccess) return bail("device error during set-up");
   for (int m = 0; m < M; ++m) c->mem[m].slot_of = std::move(slot_of[m]);
   return c;
 }
@@ -1895,7 +1900,7 @@ int ensure_levels(efdc_xm_ctx *c) {
   X.p1 = b[0]; X.h2p = b[1]; X.uhdy2e = b[2]; X.vhdx2e = b[3]; X.h1u = b[4]; X.h1v = b[5];
   X.hutmp = b[6]; X.hvtmp = b[7]; X.fpgxe = b[8]; X.fpgye = b[9];
   X.tsx1 = b[10]; X.tsy1 = b[11]; X.tbx1 = b[12]; X.tby1 = b[13];
-  CK(cudaDeviceSynchronize());  // the zeroing ran on the legacy stream
+  CK(legacy_done());  // the zeroing ran on the legacy stream
   c->tl3_alloc = true;
   return EFDC_XM_OK;
 }
@@ -3619,7 +3624,7 @@ int rebuild_channels(efdc_xm_ctx *c) {
   CK(cudaMemcpy(const_cast<uint8_t *>(c->S.kind), kind.data(), kind.size(), cudaMemcpyHostToDevice));
   drop_graphs(c);
   if (n == 0) {
-    CK(cudaDeviceSynchronize());  // the kinds are in place before the next launch
+    CK(legacy_done());  // the kinds are in place before the next launch
     return EFDC_XM_OK;
   }
   auto dev = [&](const void *src, size_t bytes) -> void * {
@@ -3664,7 +3669,7 @@ int rebuild_channels(efdc_xm_ctx *c) {
   }
   // copies and zeroing ran on the legacy stream, which the context's stream
   // does not wait for
-  CK(cudaDeviceSynchronize());
+  CK(legacy_done());
   C.n = n;
   return EFDC_XM_OK;
 }
@@ -3726,7 +3731,7 @@ int32_t efdc_xm_set_layers(efdc_xm_ctx *c, int32_t member, const efdc_xm_layers 
   }
   // the context's stream does not wait for the legacy stream: the zeroing of
   // new planes and these copies must be complete before the scatter runs
-  if (cudaDeviceSynchronize() != cudaSuccess ||
+  if (legacy_done() != cudaSuccess ||
       cudaMemcpyAsync(idx_d, idx.data(), sizeof(int) * n, cudaMemcpyHostToDevice, c->stream) !=
           cudaSuccess ||
       cudaMemcpyAsync(val_d, val.data(), sizeof(double) * val.size(), cudaMemcpyHostToDevice,
@@ -3780,7 +3785,7 @@ int32_t efdc_xm_set_bed(efdc_xm_ctx *c, int32_t member, const efdc_xm_bed *bed) 
     Bd.ub = b[9]; Bd.vb = b[10]; Bd.vu = b[11]; Bd.uv = b[12]; Bd.h1u = b[13]; Bd.h1v = b[14];
     c->has_bed.assign(c->M, 0);
     c->bed_sc.assign(c->M, xm::DragScalars{});
-    CK(cudaDeviceSynchronize());  // the zeroing ran on the legacy stream
+    CK(legacy_done());  // the zeroing ran on the legacy stream
     c->bed_alloc = true;
   }
   // the member's arrays into tile order (its slots; tile 0, the ghost tile,
@@ -4006,7 +4011,7 @@ int32_t efdc_xm_set_momentum(efdc_xm_ctx *c, int32_t member, const efdc_xm_momen
     c->mom_t2.assign(M, {});
     c->mom_bc.assign(M, {});
     c->mom_sc_h.assign(M, xm::MomScalars{});
-    CK(cudaDeviceSynchronize());  // the zeroing ran on the legacy stream
+    CK(legacy_done());  // the zeroing ran on the legacy stream
     c->mom_alloc = true;
   }
   const int kc = mo->kc;
@@ -4783,7 +4788,7 @@ int32_t efdc_xm_calib_enable(efdc_xm_ctx *c, int32_t nsnap) {
   }
   A.tbx = const_cast<double *>(c->X.tbx);
   A.tby = const_cast<double *>(c->X.tby);
-  CK(cudaDeviceSynchronize());  // the zero-fills of the legacy stream
+  CK(legacy_done());  // the zero-fills of the legacy stream
   c->calib = true;
   return EFDC_XM_OK;
 }
