@@ -805,14 +805,17 @@ __global__ void __launch_bounds__(NT) k_sys_prepare(DevStatic S, DevSystem Y, in
 // ---------------------------------------------------------------------------
 // calpuv2c.f90:416-437 face discharges and unit-width discharges.
 //
-// Back-substitution and continuity in one kernel: the continuity takes the new
-// discharges of the cell's east and north faces from the next lane (a warp is a
-// tile row) and, through shared memory, from the warp of the next row; only the
-// tile's last column and row form the neighbour tile's again from its inputs.
-// Two kernels read the discharges back from memory: 184 instead of 168 B per
-// cell and one more launch (2.5 M cells: 4 CTAs per SM 1.12 ms per MIXED step, 3 or
-// fewer 1.15; two kernels 1.16).  Open-boundary cells of members without wetting and
-// drying get their depth here (:489-490); the others' is k_obc_hp's.
+// Back-substitution and continuity, in one kernel (k_backsub) or two (k_flows,
+// k_continuity).  In one, the continuity takes the new discharges of the cell's east
+// and north faces from the next lane (a warp is a tile row) and, through shared memory,
+// from the warp of the next row; only the tile's last column and row form the neighbour
+// tile's again from its inputs: 168 instead of 184 B per cell and one launch less.  But
+// a tile's loads, its barrier and its stores follow one another, with few other tiles
+// on the SM to hide them (64 registers, 4 CTAs): where a CTA has several tiles two
+// kernels are faster.  ms per MIXED step, one / two: 80,000 cells 0.121 / 0.122, 243,000
+// 0.162 / 0.161, 974,000 0.534 / 0.529, 3.9 million 1.386 / 1.362, 21.8 million (256
+// members) 7.15 / 6.86.  Open-boundary cells of members without wetting and drying get
+// their depth here (:489-490); the others' is k_obc_hp's.
 __device__ __forceinline__ double face_flow(const StepScalars &c, double sw, double f, double hr,
                                             double rc, double h, double P, double PB) {
   return sw * (f - c.deltd2 * hr * rc * h * (P - PB));
@@ -828,6 +831,17 @@ __device__ __forceinline__ double flow_v(const DevStatic &S, const DevState &X,
                                          const StepScalars &c, int x, double PB) {
   if (S.kind[x] == LAND) return X.vhdxe[x];
   return face_flow(c, X.svb[x], X.fvhdxe[x], S.hrvo[x], rc_y(X, c, x), X.hvc[x], X.p[x], PB);
+}
+// :466-486 from H1P, UHDY1E, VHDX1E (hb, u1, v1, at the east and north face u1e, v1n);
+// CALPUV9C's (calpuv9c.f90:500-525) is written DELT*(Q - S/2), from H2P, UHDY2E, VHDX2E
+// for ISTL_ = 3 (the views hb, ub, vb)
+__device__ __forceinline__ double continuity(const StepScalars &c, double hb, double dxyip,
+                                             double qsume, double ue, double u1e, double u,
+                                             double u1, double vn, double v1n, double v,
+                                             double v1) {
+  if (c.istl == 0)
+    return hb + c.deltd2 * dxyip * (2. * qsume - (ue + u1e - u - u1 + vn + v1n - v - v1));
+  return hb + c.delt * dxyip * (qsume - 0.5 * (ue + u1e - u - u1 + vn + v1n - v - v1));
 }
 __global__ void __launch_bounds__(NT, 4) k_backsub(DevStatic S, DevState X, int ntile,
                                                const int *act) {
@@ -860,19 +874,49 @@ __global__ void __launch_bounds__(NT, 4) k_backsub(DevStatic S, DevState X, int 
     if (!north) vn = sv[turn][threadIdx.x + TX];
     turn ^= 1;
     if (kd == LAND) continue;
-    // :466-486 from H1P, UHDY1E, VHDX1E; CALPUV9C's (calpuv9c.f90:500-525) is
-    // written DELT*(Q - S/2), from H2P, UHDY2E, VHDX2E for ISTL_ = 3 (the views
-    // hb, ub, vb)
-    double hp;
-    if (c.istl == 0)
-      hp = hb + c.deltd2 * dxyip * (2. * qsume - (ue + u1e - u - u1 + vn + v1n - v - v1));
-    else
-      hp = hb + c.delt * dxyip * (qsume - 0.5 * (ue + u1e - u - u1 + vn + v1n - v - v1));
+    double hp = continuity(c, hb, dxyip, qsume, ue, u1e, u, u1, vn, v1n, v, v1);
     if (kd == OPENBC && c.isdry <= 0) hp = c.gi * P - S.belv[d];
     X.uhdye[d] = u;
     X.vhdxe[d] = v;
     X.uhe[d] = u * dyiu;
     X.vhe[d] = v * dxiv;
+    X.hp[d] = hp;
+  }
+}
+
+__global__ void __launch_bounds__(NT) k_flows(DevStatic S, DevState X, int ntile,
+                                             const int *act) {
+  TILE_LOOP(ntile) {
+    TILE_MEMBER(S);
+    if (!act[m]) continue;
+    const Nb q = neighbours(S.tnbr, tile, threadIdx.x);
+    const int d = q.d;
+    if (S.kind[d] == LAND) continue;
+    // the loads first (the stores below could alias them for the compiler)
+    const double P = X.p[d], PW = X.p[q.w], PS = X.p[q.s];
+    const double sub = X.sub[d], svb = X.svb[d], fuh = X.fuhdye[d], fvh = X.fvhdxe[d];
+    const double hruo = S.hruo[d], hrvo = S.hrvo[d], huc = X.huc[d], hvc = X.hvc[d];
+    const double rx = rc_x(X, c, d), ry = rc_y(X, c, d), dyiu = S.dyiu[d], dxiv = S.dxiv[d];
+    const double u = face_flow(c, sub, fuh, hruo, rx, huc, P, PW);
+    const double v = face_flow(c, svb, fvh, hrvo, ry, hvc, P, PS);
+    X.uhdye[d] = u;
+    X.vhdxe[d] = v;
+    X.uhe[d] = u * dyiu;
+    X.vhe[d] = v * dxiv;
+  }
+}
+__global__ void __launch_bounds__(NT) k_continuity(DevStatic S, DevState X, int ntile,
+                                                  const int *act) {
+  TILE_LOOP(ntile) {
+    TILE_MEMBER(S);
+    if (!act[m]) continue;
+    const Nb q = neighbours(S.tnbr, tile, threadIdx.x);
+    const int d = q.d;
+    const uint8_t kd = S.kind[d];
+    if (kd == LAND) continue;
+    double hp = continuity(c, X.hb[d], S.dxyip[d], X.qsume[d], X.uhdye[q.e], X.ub[q.e],
+                           X.uhdye[d], X.ub[d], X.vhdxe[q.n], X.vb[q.n], X.vhdxe[d], X.vb[d]);
+    if (kd == OPENBC && c.isdry <= 0) hp = c.gi * X.p[d] - S.belv[d];
     X.hp[d] = hp;
   }
 }
@@ -1498,8 +1542,15 @@ void launch_mx_apply(const Launch &l, const DevStatic &S, const SysView &V, cons
   count_launches(1);
 }
 void launch_backsub(const Launch &l, const DevStatic &S, const DevState &X, const int *act) {
-  k_backsub<<<cell_grid(l, k_backsub), NT, 0, l.stream>>>(S, X, l.ntile, act);
-  count_launches(1);
+  const int grid = cell_grid(l, k_backsub);
+  if (l.ntile - 1 <= grid) {  // a tile per CTA
+    k_backsub<<<grid, NT, 0, l.stream>>>(S, X, l.ntile, act);
+    count_launches(1);
+    return;
+  }
+  k_flows<<<cell_grid(l, k_flows), NT, 0, l.stream>>>(S, X, l.ntile, act);
+  k_continuity<<<cell_grid(l, k_continuity), NT, 0, l.stream>>>(S, X, l.ntile, act);
+  count_launches(2);
 }
 void launch_obc_hp(const Launch &l, const DevStatic &S, const DevState &X, const DevObc &B,
                    const int *act) {
