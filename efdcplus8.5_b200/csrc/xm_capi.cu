@@ -1804,8 +1804,10 @@ efdc_xm_ctx *efdc_xm_create_batch(const efdc_xm_grid *grids, int32_t nmembers, i
     cudaMemcpy(st[16], fu.data(), ns * sizeof(double), cudaMemcpyHostToDevice);
     cudaMemcpy(st[17], fv.data(), ns * sizeof(double), cudaMemcpyHostToDevice);
   }
-  // the staging buffers of a step's arrays in one allocation
-  group_size(c, NARRAYS);
+  // the staging buffers of a step's arrays (or, where those go packed, the fewest) in one
+  // allocation
+  const bool small = NARRAYS * size_t(c->stage_len) * sizeof(double) <= PACK_MAX;
+  group_size(c, small ? NSTAGE : NARRAYS);
   if (c->stage.empty()) return bail("cudaMalloc failed (staging)");
   xm::DevObc &Bo = c->B;
   Bo.n = c->nobc;
