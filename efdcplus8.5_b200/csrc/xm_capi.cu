@@ -531,7 +531,7 @@ int download_packed(efdc_xm_ctx *c, const std::vector<Xfer> &xs) {
 // copies by up to NCOPY threads (of this call only: joined before it returns), each with
 // its own slots and its own copy stream, so that host copies and link run side by side.
 // The driver's own staging of pageable copies moved 450 KB arrays at 18 GB/s in and 7.5
-// out.  Measured: the calls of a coupled step of 56,000 cells and four layers 3.9 -> 2.95
+// out.  Measured: the calls of a coupled step of 56,000 cells and four layers 4.1 -> 2.85
 // ms; when the ring was written 3.6 -> 2.65, with one thread 2.9, with slots of 256 KB 3.1,
 // with a ring of 8 MB the same (5 % faster at 160,000 cells), with slabs of 1 MB across
 // arrays in a ring of 16 MB 3.0 (it no longer stays in the caches).

@@ -766,7 +766,7 @@ __device__ __forceinline__ V4<float> x_plus_alpha_p(const V4<float> &x, float al
 // stored: 20 of a pass's 56 n + 113 B per cell).
 // Here and in the other MIXED rows every global load is issued before the first
 // shuffle or dependent operation, so that one round trip to memory serves the row:
-// more values live, fewer CTAs per SM (see mx_ctas).
+// more values live, fewer CTAs per SM (MX_CTAS).
 __device__ __forceinline__ double matvec_row_scaled(const RowGeo &g, bool valid,
                                                     const float *__restrict__ r,
                                                     const float *__restrict__ pold,

@@ -30,7 +30,10 @@ constexpr size_t res_smem64() {
 // 0.65 -> 0.49, 1,000x1,000 0.80 -> 0.55 (an iteration 31 -> 20 us, of which the row
 // work is 13, the exchanges' waits for the slowest CTA 3 and the exchanges 4).
 // Registers: one quad side by side keeps the coefficients there too (255 a thread with
-// two rows), two by two (128 a thread) in shared memory; the lean form reads them.
+// two rows), two by two (128 a thread) in shared memory; the lean form reads them.  These
+// two spill, 312 to 400 bytes stored and 424 to 560 loaded a thread (the forms with one
+// quad side by side at most 64); one quad side by side and four or eight rows, which
+// would have 255 registers, were not tried.
 template <bool MA, int W, int Q, bool CLUSTER>
 __global__ void __launch_bounds__(NT *W, W == 1 && Q == 1 && CLUSTER ? 2 : 1)
     k_cg_res(DevStatic S, SysView V, DevSystem Y, double *P, Ctl *ctl, Glob *glob, ResPlan R,

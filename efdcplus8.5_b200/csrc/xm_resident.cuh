@@ -6,9 +6,9 @@
 // another, a thread holding its row vectors of each quad in registers from the
 // first residual to the stop test.  What leaves a CTA is the border of its
 // tiles (the rows and columns a neighbour tile reads) and one partial sum per
-// quad, through L2 (FP64 clusters: through shared memory).  The multi-kernel CG pays two kernel boundaries per
-// iteration (launch, ramp, tail and a folded reduction: 7 us each on a
-// 60,000-cell basin whose row work is below 1 us); here a boundary is one
+// quad, through L2 (FP64 clusters: through shared memory).  The multi-kernel CG pays
+// two kernel boundaries per iteration (launch, ramp, tail and a folded reduction: 7 us
+// each on a 60,000-cell basin whose row work is below 1 us); here a boundary is one
 // exchange between the CTAs of the member, which is also their barrier:
 //  * a group of up to 16 CTAs is a thread-block cluster: each CTA stores its
 //    quads' partial sums into the shared memory of every CTA, and the cluster

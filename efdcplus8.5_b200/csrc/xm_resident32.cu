@@ -35,8 +35,8 @@ constexpr size_t res_smem32() {
 
 // What bounds it: the exchanges (two per inner iteration, three per pass) and
 // the latency of the row work around them; see k_cg_res.  Measured against the
-// multi-kernel form, ms per MIXED step: 60x60 cells 0.33 -> 0.13, 260x250 0.35 ->
-// 0.17, 500x500 0.38 -> 0.21, 700x700 0.45 -> 0.29.
+// multi-kernel form, ms per MIXED step: 317x203 cells 0.124, 400x390 0.147, 512x512
+// 0.38 -> 0.163, 700x700 0.45 -> 0.257.
 template <bool MA, int W, int Q, bool CLUSTER>
 __global__ void __launch_bounds__(NT *W, W == 1 && CLUSTER ? 2 : 1)
     k_mx_res(DevStatic S, SysView V, DevSystem Y, double *P, Ctl *ctl, Glob *glob, ResPlan R,

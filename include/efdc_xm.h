@@ -568,11 +568,13 @@ int32_t efdc_xm_set_wait_limit(int32_t polls);
  *     its residual by at least 10^(-value/10) in norm before the next FP64
  *     refinement pass, where the FP64 stop needs more than that.
  *   EFDC_XM_OPT_SMALL_SOLVE (default 1): 1 runs the solves of contexts whose
- *     members fit the chip (FP64: up to about 600,000 cells each; MIXED: all
- *     members together up to about that) and have no sub-grid channels as one
- *     launch per solve, or per run of members that fit, with the vectors in
- *     registers; 0 runs them as the kernels of every other context.  Both give
- *     the same results bit for bit.
+ *     members fit the chip and have no sub-grid channels in one launch, with the
+ *     vectors in registers and shared memory, where that is faster: FP64 members
+ *     of up to about 1.2 million cells, a batch that does not fit at once in
+ *     several launches; MIXED members of up to about 600,000 cells together, or
+ *     a few hundred small ones (up to about 60,000 cells each).  0, and every
+ *     other context, runs the multi-kernel CG.  Both give the same results bit
+ *     for bit.
  *   EFDC_XM_OPT_FOLD_REDUCE (default 1, 0..2): 2 finishes each member's CG
  *     sums (its dot products, ALPHA, BETA and stop tests) inside the kernel
  *     that forms them, in the CTA that stores the member's last partial sum;
